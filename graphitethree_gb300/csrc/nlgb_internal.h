@@ -102,10 +102,51 @@ struct SolveResult {
   int precision = 0;             // precision that ran (0 FP64, 1 mixed, 3 double-float)
 };
 
+// The persistent PCG kernel's view of one matrix (nlgb_persist.cu): how its
+// tiles are dealt to CTAs, and per CTA the columns outside its own rows
+// ("halo"), the matrix's columns renumbered to its own rows and that halo, and
+// its rows sorted by length.  Laid out once per matrix and layout.
+struct PersistLayout {
+  int ctas = 0;                        // CTAs that own tiles
+  int slots = 0;                       // tiles per CTA at most
+  int halo_stride = 0;                 // entries of `halo` per CTA
+  int halo_cap = 0;                    // halo entries per CTA the shared memory is laid out for (even)
+  const unsigned short* lci = nullptr; // per nonzero: own row, or slots * tile_rows + halo entry
+  const unsigned short* perm = nullptr;// per CTA (at its first row): own rows by length
+  const int* halo = nullptr;           // per CTA: columns (grid form) or rank << 16 | row (cluster form)
+  const int* halo_n = nullptr;         // per CTA
+};
+struct PersistPlan {
+  bool usable = false;
+  bool cluster = false;                // one thread-block cluster; else a cooperative grid
+  int grid = 0, block = 0, smem = 0;
+  const void* kernel = nullptr;
+};
+struct DeviceCRS;
+class PersistTables {
+ public:
+  PersistTables() = default;
+  ~PersistTables() { release(); }
+  PersistTables(const PersistTables&) = delete;
+  PersistTables& operator=(const PersistTables&) = delete;
+  // Lays a matrix out for the persistent kernel; usable() tells whether it
+  // fits (sizes and halos).
+  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s);
+  bool usable() const { return lay_.ctas > 0; }
+  const PersistLayout& layout() const { return lay_; }
+  PersistPlan plan(int tile_rows, int tpr, int mode) const;
+  void release();
+
+ private:
+  PersistLayout lay_;
+  bool cluster_ = false;
+  void* mem_ = nullptr;
+};
+
 // Plain FP64, double-float, or mixed FP32/FP64-refined Jacobi-PCG on one
 // resident matrix.
-// The whole iteration loop is a single CUDA-graph launch (while-conditional
-// node); the host waits once per solve.
+// The iteration runs in the persistent kernel when the system fits it, else
+// as a single CUDA-graph launch (while-conditional node).
 class PcgSolver {
  public:
   PcgSolver() = default;
@@ -124,6 +165,7 @@ class PcgSolver {
   cudaError_t run_graph(bool mixed, bool df, const SolveParams& prm, long long max_iter,
                         long long done, int outer, float* ms);
   cudaError_t run_eager(bool mixed, bool df, SysState* h, bool cont = false);
+  cudaError_t run_persist(int mode, const SolveParams& prm);
   // continuation after a failed true-residual check (state: running, stage 4)
   cudaError_t run_cont(bool df, float* ms);
   cudaError_t add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysView* v, bool df,
@@ -143,10 +185,11 @@ class PcgSolver {
   const volatile int* abort_flag_ = nullptr;
   cudaGraphExec_t plain_exec_ = nullptr, mixed_exec_ = nullptr, df_exec_ = nullptr;
   cudaGraphExec_t cont_exec_ = nullptr, cont_df_exec_ = nullptr;
-  // single-kernel cooperative iterations (small and mid-size systems)
-  bool use_coop_ = false;
-  int coop_grid_ = 0;
-  unsigned long long* coop_bar_ = nullptr;
+  // persistent kernel (small and mid-size systems): the matrix's tables,
+  // launch shapes per mode (FP64, double-float, mixed) and the exchange area
+  PersistTables tables_;
+  PersistPlan plan_[3];
+  void* exch_ = nullptr;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   bool mixed_alloc_ = false;
   long long graph_launches_ = 0;

@@ -1,0 +1,45 @@
+// nlgb_persist.h -- the persistent single-system PCG kernel (nlgb_persist.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "nlgb_core.cuh"
+#include "nlgb_internal.h"
+
+namespace nlgb {
+
+enum { kPersistDouble = 0, kPersistDf = 1, kPersistMixed = 2 };
+
+constexpr int kPersistBlock = 512;        // threads per CTA at most (128 registers each)
+constexpr int kPersistSlots = 9;          // tiles per CTA at most (1,216 tiles on 151 CTAs)
+constexpr int kPersistCluster = 16;       // CTAs of the cluster form at most
+constexpr int kPersistClusterTiles = 64;  // tiles of the cluster form at most
+constexpr int kPersistRed = 8 * 36;       // 8-byte words of one staged value of a tile
+
+struct PersistArgs {
+  SysView s;
+  ulonglong2* slot;            // grid form: 3 x n_tiles, p.q, r.z, r.r of every tile as (value, epoch)
+  ulonglong2* ctl;             // grid form: [0] alpha, [8] beta as (value, 256 epoch + code)
+  ulonglong2* zslot;           // grid form: z of every row as (value, epoch)
+  int* err;                    // nonzero: a wait ran out
+  PersistLayout lay;
+  long long iters;             // iterations of this launch at most
+};
+
+// Exchange area (zeroed before a solve): partial slots, control slots, z
+// slots, the error word.
+inline size_t persist_bytes(int n, int n_tiles) {
+  return ((size_t)3 * n_tiles + 16 + (size_t)n + 1) * sizeof(ulonglong2);
+}
+inline void persist_bind(PersistArgs& a, void* exch) {
+  a.slot = reinterpret_cast<ulonglong2*>(exch);
+  a.ctl = a.slot + (size_t)3 * a.s.n_tiles;
+  a.zslot = a.ctl + 16;
+  a.err = reinterpret_cast<int*>(a.zslot + a.s.n);
+}
+cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& a, cudaStream_t s);
+// The kernel for a layout (nlgb_persist_*.cu): nc rows per lane group in registers.
+const void* persist_kernel_f64(int tpr, bool cluster, int nc);
+const void* persist_kernel_df(int tpr, bool cluster, int nc);
+const void* persist_kernel_mx(int tpr, bool cluster, int nc);
+
+}  // namespace nlgb

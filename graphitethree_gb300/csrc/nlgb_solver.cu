@@ -4,7 +4,9 @@
 // (call sites: src/lib/OGF/scene_graph/NL/matrix.cpp:364,390-393; nlSolve at
 // plugins/OGF/WarpDrive/commands/voxel_grob_transport_commands.cpp:281).
 //
-// One PCG iteration = three kernels (SpMV + p.q; x/r update + r.z, r.r;
+// Small and mid-size systems run in the persistent kernel of
+// nlgb_persist.cu; here is the rest.  One PCG iteration = three kernels (SpMV
+// + p.q; x/r update + r.z, r.r;
 // p update).  Each kernel's last CTA reduces the tile partials in a fixed
 // order and advances the scalar state in HBM, so the host never reads a
 // scalar during the solve: the loop is a CUDA-graph while-node whose
@@ -13,6 +15,7 @@
 #include "nlgb_batch.h"
 #include "nlgb_core.cuh"
 #include "nlgb_internal.h"
+#include "nlgb_persist.h"
 
 #include <algorithm>
 #include <chrono>
@@ -220,103 +223,6 @@ __global__ void __launch_bounds__(kCTA, 8) k_update_p(SysView s) {
   if (ld_status(s.st) != ST_RUNNING) return;
   const double beta = __ldcg(&s.st->beta);
   for (int t = vec_t0(s), t1 = vec_t1(s); t < t1; ++t) phase_update_p<D>(s, t, beta);
-}
-
-// ---------------------------------------------------------------------------
-// One whole FP64 PCG iteration in one cooperative kernel (small and mid-size
-// systems, all tiles in one resident wave): SpMV + p.q, grid barrier, x / r
-// update, grid barrier, p update; the kernel boundary orders the next
-// iteration's SpMV after this p update.  Every CTA reduces the tile partials
-// in the canonical order and applies the same scalar steps to its own copy
-// of the state (identical results), so the phases need no extra barrier for
-// the scalars; CTA 0 writes the state back.  The tile procedures, reductions
-// and scalar steps are those of the three-kernel iteration: the iterates are
-// bit-identical.  Replaces three kernel boundaries and three last-CTA
-// reduction tails per iteration by two barriers.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long coop_atom_add(unsigned long long* p) {
-  unsigned long long old;
-  asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], 1;" : "=l"(old) : "l"(p) : "memory");
-  return old;
-}
-__device__ __forceinline__ unsigned long long coop_ld_acquire(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned long long coop_clock_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Grid barrier on a monotonic counter (one arrival per CTA per barrier):
-// returns false in every thread if the wait exceeded 4 s.
-__device__ bool coop_grid_sync(unsigned long long* bar, unsigned long long target) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = 1;
-    coop_atom_add(bar);
-    const unsigned long long t0 = coop_clock_ns();
-    unsigned int spins = 0;
-    while (coop_ld_acquire(bar) < target) {
-      if ((++spins & 63u) == 0u && coop_clock_ns() - t0 > 4000000000ULL) { ok = 0; break; }
-    }
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
-template <int T, bool D>
-__global__ void __launch_bounds__(kCTA) k_iter(SysView s, unsigned long long* bar) {
-  __shared__ SysState sst;
-  if (threadIdx.x == 0) sst = *s.st;      // written by the previous kernel
-  __syncthreads();
-  if (sst.status != ST_RUNNING) return;
-  const int G = gridDim.x;
-  const unsigned long long base = (unsigned long long)sst.coop_epoch * 2ULL * (unsigned long long)G;
-  for (int t = blockIdx.x; t < s.n_tiles; t += G) {
-    const double v = phase_spmv_pq<D, T>(s, t);
-    if (threadIdx.x == 0) __stcg(s.part + (size_t)t * kParts + kSlotPQ, v);
-  }
-  bool ok = coop_grid_sync(bar, base + G);
-  if (ok) {
-    const int comp[1] = {kSlotPQ};
-    double o[1];
-    canon_reduce<1>(s.part, s.n_tiles, comp, o);
-    if (threadIdx.x == 0) scalar_after_pq(&sst, o[0]);
-    __syncthreads();
-    if (sst.status == ST_RUNNING) {
-      const double alpha = sst.alpha;
-      for (int t = blockIdx.x; t < s.n_tiles; t += G) {
-        double v[2];
-        phase_update_xr<D>(s, t, alpha, v);
-        if (threadIdx.x == 0) {
-          __stcg(s.part + (size_t)t * kParts + kSlotXR, v[0]);
-          __stcg(s.part + (size_t)t * kParts + kSlotXR + 1, v[1]);
-        }
-      }
-    }
-    // every CTA takes the second barrier (the epoch arithmetic counts both)
-    ok = coop_grid_sync(bar, base + 2ULL * G);
-    if (ok && sst.status == ST_RUNNING) {
-      const int comp2[2] = {kSlotXR, kSlotXR + 1};
-      double o2[2];
-      canon_reduce<2>(s.part, s.n_tiles, comp2, o2);
-      if (threadIdx.x == 0) scalar_after_xr(&sst, o2[0], o2[1]);
-      __syncthreads();
-      if (sst.status == ST_RUNNING) {
-        const double beta = sst.beta;
-        for (int t = blockIdx.x; t < s.n_tiles; t += G) phase_update_p<D>(s, t, beta);
-      }
-    }
-  }
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    if (!ok) sst.status = ST_DEVICE_ERR;
-    sst.coop_epoch += 1;
-    *s.st = sst;
-  }
 }
 
 // Termination guard of a while-node body (single thread).  use_handle == 0:
@@ -674,48 +580,16 @@ static long long resident_slots() {
 }
 long long phase_resident_slots() { return resident_slots(); }
 
-// CTAs of the single-kernel iteration k_iter<T> resident at once (0 if the
-// occupancy cannot be queried).
-// Above ~640 CTAs the single-counter barrier and the per-CTA canonical
-// reductions (CTAs x tiles partial reads) cost more than the two kernel
-// boundaries they replace (measured on GB300: 512 CTAs 30 vs 38 us per
-// iteration, 834-1,024 CTAs 47-64 vs 39-50 us).
-constexpr long long kCoopMaxCtas = 640;
-
-template <bool D>
-static const void* iter_kernel(int tpr) {
-  switch (tpr) {
-    case 1: return (const void*)k_iter<1, D>;
-    case 2: return (const void*)k_iter<2, D>;
-    case 4: return (const void*)k_iter<4, D>;
-    case 8: return (const void*)k_iter<8, D>;
-    case 16: return (const void*)k_iter<16, D>;
-    default: return (const void*)k_iter<32, D>;
-  }
-}
-
-// Resident CTAs per SM of the single-kernel iteration: the smaller of its
-// FP64 and double-float forms, so that a matrix's layout and executor do not
-// depend on the precision it is solved in (0 if it cannot be queried).
-static int coop_per_sm(int tpr) {
-  int a = 0, b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, iter_kernel<false>(tpr), kCTA, 0) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, iter_kernel<true>(tpr), kCTA, 0) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return std::min(a, b);
-}
-
-static long long coop_wave(int tpr) {
+// Tiles of the smallest systems' layouts (128 and 256 rows): at most this
+// many, so that a system above 128 x this takes 256-row tiles.
+static long long small_tiles() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  const int per_sm = coop_per_sm(tpr);
-  return std::min<long long>((long long)per_sm * sms, kCoopMaxCtas);
+  return std::min(6LL * sms, 640LL);
 }
 
 TuneChoice autotune(int n, long long nnz, int max_row, const int* hist33) {
@@ -747,11 +621,11 @@ TuneChoice autotune(int n, long long nnz, int max_row, const int* hist33) {
   // rows with at most 4,096 tiles; among equal costs the fewest tiles (each
   // scalar is a reduction over the tiles, so three waves of 384-row tiles
   // are slower than one wave of 1,152).  Small systems keep 128-row tiles:
-  // one wave of CTAs as small as they go; systems just above one resident
-  // wave of the single-kernel iteration (k_iter) at 128 rows take 256-row
-  // tiles, so that they still fit that wave (one tile per CTA).
+  // one wave of CTAs as small as they go; systems just above 640 of them take
+  // 256-row tiles (few tiles per CTA of the persistent iteration, few
+  // partials per scalar).
   const long long slots = resident_slots();
-  const long long cw = coop_wave(tpr);
+  const long long cw = small_tiles();
   int tile = 128;
   if (cw > 0 && (long long)n > 128 * cw && (long long)n <= 256 * cw) {
     tile = 256;
@@ -991,15 +865,14 @@ static cudaError_t add_while(cudaGraph_t g, cudaGraphNode_t* node, cudaGraphNode
 // The kernels of one threads-per-row variant; df selects the double-float
 // form of the plain iteration (init, SpMV, vector updates, final residual).
 struct KernelSet {
-  const void *init, *spmv, *fin, *mx_outer, *mx_spmv, *iter, *update_xr, *update_p, *resume_p,
-      *init_chunk, *fin_if;
+  const void *init, *spmv, *fin, *mx_outer, *mx_spmv, *update_xr, *update_p, *resume_p, *init_chunk,
+      *fin_if;
 };
 template <int T, bool D>
 static KernelSet kernel_set() {
   return {(const void*)k_init<T, D>, (const void*)k_spmv_pq<T, D>, (const void*)k_final<T, D>,
-          (const void*)k_mx_outer<T>, (const void*)k_mx_spmv_pq<T>, (const void*)k_iter<T, D>,
-          (const void*)k_update_xr<D>, (const void*)k_update_p<D>, (const void*)k_resume_p<D>,
-          (const void*)k_init_chunk<T, D>, (const void*)k_final_if<T, D>};
+          (const void*)k_mx_outer<T>, (const void*)k_mx_spmv_pq<T>, (const void*)k_update_xr<D>, (const void*)k_update_p<D>,
+          (const void*)k_resume_p<D>, (const void*)k_init_chunk<T, D>, (const void*)k_final_if<T, D>};
 }
 template <bool D>
 static KernelSet kernels_for_t(int tpr) {
@@ -1017,7 +890,6 @@ static KernelSet kernels_for(int tpr, bool df) {
 }
 
 constexpr int kUnrollPlain = 4;   // CG iterations per while-body pass
-constexpr int kCoopTilesPerCta = 1;   // measured: two tiles per CTA lose to three kernels
 constexpr int kUnrollInner = 4;
 constexpr long long kMaxItersBetweenUpdates = 1000;   // mixed: forced reliable update
 
@@ -1031,8 +903,9 @@ void PcgSolver::release() {
   if (cont_df_exec_) cudaGraphExecDestroy(cont_df_exec_);
   plain_exec_ = mixed_exec_ = df_exec_ = cont_exec_ = cont_df_exec_ = nullptr;
   cudaFree(b_); cudaFree(x_); cudaFree(r_); cudaFree(p_); cudaFree(q_); cudaFree(part_);
-  cudaFree(coop_bar_);
-  coop_bar_ = nullptr;
+  cudaFree(exch_);
+  exch_ = nullptr;
+  tables_.release();
   cudaFree(r32_); cudaFree(p32_); cudaFree(q32_); cudaFree(c32_); cudaFree(st_);
   if (st_host_) cudaFreeHost(st_host_);
   if (ev0_) cudaEventDestroy(ev0_);
@@ -1052,19 +925,8 @@ cudaError_t PcgSolver::bind(DeviceCRS* A, cudaStream_t stream) {
   tpr_ = A->tpr;
   tile_rows_ = A->tile_rows;
   n_tiles_ = std::max(1, (n_ + tile_rows_ - 1) / tile_rows_);
-  // One cooperative kernel per iteration when the tiles fit in one resident
-  // wave of it at no more than kCoopTilesPerCta tiles per CTA (latency-bound
-  // sizes); larger systems keep one kernel per phase at full occupancy.
-  int dev = 0, sms = 0, per_sm = 0;
-  use_coop_ = false;
-  if (cudaGetDevice(&dev) == cudaSuccess &&
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-      (per_sm = coop_per_sm(tpr_)) > 0) {
-    const long long wave = std::min<long long>((long long)per_sm * sms, kCoopMaxCtas);
-    use_coop_ = n_tiles_ <= kCoopTilesPerCta * wave;
-    coop_grid_ = (int)std::min<long long>(n_tiles_, wave);
-  }
-  cudaGetLastError();
+  NLGB_CUDA_TRY(tables_.build(*A, tile_rows_, n_tiles_, stream));
+  for (int m = 0; m < 3; ++m) plan_[m] = tables_.plan(tile_rows_, tpr_, m);
   return alloc(false);
 }
 
@@ -1078,10 +940,10 @@ cudaError_t PcgSolver::alloc(bool mixed) {
     NLGB_CUDA_TRY(cudaMalloc(&q_, n8));
     NLGB_CUDA_TRY(cudaMalloc(&part_, (size_t)n_tiles_ * kParts * sizeof(double)));
     NLGB_CUDA_TRY(cudaMalloc(&st_, sizeof(SysState)));
-    NLGB_CUDA_TRY(cudaMallocHost(&st_host_, sizeof(SysState)));
+    NLGB_CUDA_TRY(cudaMallocHost(&st_host_, sizeof(SysState) + 16));
     NLGB_CUDA_TRY(cudaEventCreate(&ev0_));
     NLGB_CUDA_TRY(cudaEventCreate(&ev1_));
-    NLGB_CUDA_TRY(cudaMalloc(&coop_bar_, 256));
+    if (tables_.usable()) NLGB_CUDA_TRY(cudaMalloc(&exch_, persist_bytes(n_, n_tiles_)));
   }
   if (mixed && !mixed_alloc_) {
     const size_t n4 = (size_t)std::max(4, n_ + 4) * sizeof(float);
@@ -1110,8 +972,8 @@ static SysView make_view(DeviceCRS* A, int tile_rows, int n_tiles, double* b, do
 }
 
 // The while loop of the plain (FP64 or double-float) iteration, after
-// `dep`: kUnrollPlain iterations per pass (one cooperative kernel each, or
-// three phase kernels), then the guard.
+// `dep`: kUnrollPlain iterations per pass (three phase kernels each), then
+// the guard.
 cudaError_t PcgSolver::add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysView* v, bool df,
                                       cudaGraphNode_t* loop_out) {
   const KernelSet ks = kernels_for(tpr_, df);
@@ -1121,19 +983,7 @@ cudaError_t PcgSolver::add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysVie
   cudaGraph_t body;
   NLGB_CUDA_TRY(add_while(g, loop_out, dep, h, &body));
   cudaGraphNode_t prev = nullptr;
-  unsigned long long* bar = coop_bar_;
-  void* a_it[] = {v, &bar};
   for (int u = 0; u < kUnrollPlain; ++u) {
-    if (use_coop_) {
-      cudaGraphNode_t n1;
-      NLGB_CUDA_TRY(add_kernel(body, &n1, prev, ks.iter, coop_grid_, kCTA, a_it));
-      cudaKernelNodeAttrValue coop;
-      std::memset(&coop, 0, sizeof(coop));
-      coop.cooperative = 1;
-      NLGB_CUDA_TRY(cudaGraphKernelNodeSetAttribute(n1, cudaKernelNodeAttributeCooperative, &coop));
-      prev = n1;
-      continue;
-    }
     cudaGraphNode_t n1, n2, n3;
     NLGB_CUDA_TRY(add_kernel(body, &n1, prev, ks.spmv, n_tiles_, kCTA, a1));
     const int vg = (n_tiles_ + vec_tiles_for(tile_rows_) - 1) / vec_tiles_for(tile_rows_);
@@ -1549,8 +1399,68 @@ cudaError_t PcgSolver::run_cont(bool df, float* ms) {
   if (eager_mode()) return cudaSuccess;   // run_eager counted its launches
   ++graph_launches_;
   // resume p update, mark, final residual, check + every while-body pass
-  const long long per_iter = use_coop_ ? 1 : 3;
-  count_launches(4 + (h->guard - guard0) * (per_iter * kUnrollPlain + 1));
+  count_launches(4 + (h->guard - guard0) * (3 * kUnrollPlain + 1));
+  return cudaSuccess;
+}
+
+// The solve of a system that fits the persistent kernel (nlgb_persist.cu),
+// from the state in st_: initial residual, then the iteration in launches of
+// at most kPersistIters iterations (so that a long solve leaves the GPU to
+// other streams' kernels now and then), the reliable updates of a mixed
+// system between them, the final residual and the true-residual check.  The
+// kernels return at once when it is not their turn, so several launches are
+// queued before the state is read.  Leaves the state in st_.
+constexpr long long kPersistIters = 1024;
+
+cudaError_t PcgSolver::run_persist(int mode, const SolveParams& prm) {
+  const bool mixed = mode == kPersistMixed, df = mode == kPersistDf;
+  PersistArgs pa;
+  std::memset(&pa, 0, sizeof(pa));
+  pa.s = make_view(A_, tile_rows_, n_tiles_, b_, x_, r_, p_, q_, r32_, p32_, q32_, c32_, part_, st_,
+                   abort_flag_, df);
+  persist_bind(pa, exch_);
+  pa.lay = tables_.layout();
+  pa.iters = kPersistIters;
+  const KernelSet ks = kernels_for(tpr_, df);
+  const int vg = (n_tiles_ + vec_tiles_for(tile_rows_) - 1) / vec_tiles_for(tile_rows_);
+  SysState* h = (SysState*)st_host_;
+  SysState* st = (SysState*)st_;
+  long long launched = 0;
+  auto go = [&](const void* fn, int grid, int block, void** args) {
+    ++launched;
+    return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, stream_);
+  };
+  void* a1[] = {&pa.s};
+  void* ast[] = {&st};
+  NLGB_CUDA_TRY(cudaMemsetAsync(exch_, 0, persist_bytes(n_, n_tiles_), stream_));   // coop_epoch = 0 too
+  NLGB_CUDA_TRY(go(mixed ? ks.mx_outer : ks.init, n_tiles_, kCTA, a1));
+  // Mixed: a round per reliable update that is expected (one per inner_eps).
+  int rounds = 1;
+  if (mixed && prm.eps > 0.0 && prm.eps < 1.0)
+    rounds = (int)std::max(1.0, std::min(16.0, std::ceil(std::log(prm.eps) / std::log(prm.inner_eps))));
+  for (;;) {
+    for (int k = 0; k < rounds; ++k) {
+      NLGB_CUDA_TRY(persist_launch(plan_[mode], pa, stream_));
+      if (mixed) {
+        NLGB_CUDA_TRY(go((const void*)k_mx_apply, vg, kCTA, a1));
+        NLGB_CUDA_TRY(go(ks.mx_outer, n_tiles_, kCTA, a1));
+      }
+    }
+    NLGB_CUDA_TRY(go(ks.fin_if, n_tiles_, kCTA, a1));
+    if (!mixed) NLGB_CUDA_TRY(go((const void*)k_check, 1, 1, ast));
+    int* err = reinterpret_cast<int*>(h + 1);
+    NLGB_CUDA_TRY(cudaMemcpyAsync(h, st_, sizeof(SysState), cudaMemcpyDeviceToHost, stream_));
+    NLGB_CUDA_TRY(cudaMemcpyAsync(err, pa.err, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    NLGB_CUDA_TRY(cudaStreamSynchronize(stream_));
+    if (*err) h->status = ST_DEVICE_ERR;
+    if (h->status != ST_RUNNING) break;
+    rounds = mixed ? 2 : 1;
+    if (h->stage == 4) {   // the true residual missed eps: the pending p update, then more iterations
+      NLGB_CUDA_TRY(go(ks.resume_p, vg, kCTA, a1));
+      NLGB_CUDA_TRY(go((const void*)k_resume_mark, 1, 1, ast));
+    }
+  }
+  count_launches(launched);
   return cudaSuccess;
 }
 
@@ -1562,23 +1472,10 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
                                  long long done, int outer, float* ms) {
   if (mixed) df = false;
   cudaGraphExec_t* plain = df ? &df_exec_ : &plain_exec_;
-  if (mixed && !mixed_exec_) NLGB_CUDA_TRY(build_mixed_graph());
-  if (!mixed && !*plain) {
-    cudaError_t e = build_plain_graph(df);
-    if (e != cudaSuccess && use_coop_) {
-      // cooperative kernel nodes refused here: one kernel per phase instead
-      // (both plain graphs are rebuilt so that they keep one executor)
-      cudaGetLastError();
-      use_coop_ = false;
-      if (plain_exec_) cudaGraphExecDestroy(plain_exec_);
-      if (df_exec_) cudaGraphExecDestroy(df_exec_);
-      if (cont_exec_) cudaGraphExecDestroy(cont_exec_);
-      if (cont_df_exec_) cudaGraphExecDestroy(cont_df_exec_);
-      plain_exec_ = df_exec_ = cont_exec_ = cont_df_exec_ = nullptr;
-      e = build_plain_graph(df);
-    }
-    NLGB_CUDA_TRY(e);
-  }
+  const int mode = mixed ? kPersistMixed : df ? kPersistDf : kPersistDouble;
+  const bool persist = plan_[mode].usable && !eager_mode();
+  if (mixed && !persist && !eager_mode() && !mixed_exec_) NLGB_CUDA_TRY(build_mixed_graph());
+  if (!mixed && !persist && !eager_mode() && !*plain) NLGB_CUDA_TRY(build_plain_graph(df));
   SysState* h = (SysState*)st_host_;
   std::memset(h, 0, sizeof(SysState));
   h->thresh2 = prm.eps * prm.eps;
@@ -1599,13 +1496,14 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
   const int unroll = mixed ? kUnrollInner : kUnrollPlain;
   h->guard_cap = std::max(0LL, max_iter - done) / unroll + 2LL * (h->max_outer + 2) + 4;
   NLGB_CUDA_TRY(cudaMemcpyAsync(st_, h, sizeof(SysState), cudaMemcpyHostToDevice, stream_));
-  NLGB_CUDA_TRY(cudaMemsetAsync(coop_bar_, 0, sizeof(unsigned long long), stream_));   // coop_epoch = 0 too
   if (mixed) {
     NLGB_CUDA_TRY(cudaMemsetAsync(c32_, 0, (size_t)n_ * sizeof(float), stream_));
     NLGB_CUDA_TRY(cudaMemsetAsync(p32_, 0, (size_t)n_ * sizeof(float), stream_));
   }
   NLGB_CUDA_TRY(cudaEventRecord(ev0_, stream_));
-  if (eager_mode()) {
+  if (persist) {
+    NLGB_CUDA_TRY(run_persist(mode, prm));
+  } else if (eager_mode()) {
     NLGB_CUDA_TRY(run_eager(mixed, df, h));
   } else {
     NLGB_CUDA_TRY(cudaGraphLaunch(mixed ? mixed_exec_ : *plain, stream_));
@@ -1614,15 +1512,14 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
   NLGB_CUDA_TRY(cudaMemcpyAsync(h, st_, sizeof(SysState), cudaMemcpyDeviceToHost, stream_));
   NLGB_CUDA_TRY(cudaStreamSynchronize(stream_));
   NLGB_CUDA_TRY(cudaEventElapsedTime(ms, ev0_, ev1_));
-  if (eager_mode()) return cudaSuccess;   // run_eager counted its launches
+  if (persist || eager_mode()) return cudaSuccess;   // counted their launches
   ++graph_launches_;
   // Kernel nodes executed: every while-body pass runs all of its kernels
   // (3 per unrolled iteration + the guard); the mixed graph adds 2 kernels
   // per reliable update after the first; plus the first and final kernels
   // (and the true-residual check of the plain graph).
   const long long passes = h->guard;
-  const long long per_iter = (!mixed && use_coop_) ? 1 : 3;
-  long long k = (mixed ? 2 : 3) + passes * (per_iter * unroll + 1);
+  long long k = (mixed ? 2 : 3) + passes * (3LL * unroll + 1);
   if (mixed) k += 2LL * std::max(0, h->outer - outer - 1);
   count_launches(k);
   return cudaSuccess;
