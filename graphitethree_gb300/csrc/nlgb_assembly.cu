@@ -9,12 +9,14 @@
 //
 // GPU row-merge: (1) per LS row, s_r = b_r - sum_locked a x (coefficient
 // order); (2) transpose the free coefficients into per-variable column lists;
-// (3) for each output row i, merge the rows that contain i: candidates
-// (j, r) -> (w a_ri) a_rj are sorted by (j, r) in shared memory and each run
-// of equal j is summed sequentially in ascending r.  The sum order is exactly
-// that of a sequential row-by-row CPU build, and products and sums use
-// explicitly rounded intrinsics (no FMA contraction), so the assembled
-// matrix and right-hand side are bit-identical to the CPU oracle's.
+// (3) for each output row i, merge the rows that contain i: the candidates
+// (j, r) -> (w a_ri) a_rj of equal j are summed in ascending r.  One thread
+// per output row keeps its columns and sums in a small table (k_merge_rows);
+// rows with more LS rows or columns than that table holds sort their
+// candidates in shared memory, a warp or a CTA per row (k_merge).  The sum
+// order is exactly that of a sequential row-by-row CPU build, and products
+// and sums use explicitly rounded intrinsics (no FMA contraction), so the
+// assembled matrix and right-hand side are bit-identical to the CPU oracle's.
 #include "nlgb_internal.h"
 
 #include <algorithm>
@@ -76,18 +78,7 @@ __global__ void k_col_scatter(LSRowsDevice R, const long long* __restrict__ colp
   }
 }
 
-// ---- (3a) candidate count per output row ----
-__global__ void k_cand_count(int n_free, const long long* __restrict__ colptr,
-                             const int* __restrict__ colrow, const int* __restrict__ nfree,
-                             int* __restrict__ cand) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_free) return;
-  long long c = 0;
-  for (long long e = colptr[i]; e < colptr[i + 1]; ++e) c += nfree[colrow[e]];
-  cand[i] = (int)(c < (1LL << 30) ? c : (1LL << 30));
-}
-
-// ---- (3b) merge: shared-memory sort of (j, r) candidates ----
+// ---- (3) merge ----
 struct MergeArgs {
   LSRowsDevice R;
   int n_free;
@@ -96,8 +87,7 @@ struct MergeArgs {
   const double* colwa;
   const int* nfree;
   const double* s;       // n_systems * n_rows
-  const int* cand;
-  const int* rows;       // output rows handled by this launch (null: all)
+  const int* rows;       // output rows handled by this launch of k_merge
   int n_rows_list;
   int* row_nnz;          // symbolic output
   const int* rp;         // numeric: CRS row pointers
@@ -107,6 +97,102 @@ struct MergeArgs {
   int numeric;
   int* err;              // set to 1 when a row exceeds the CTA cap
 };
+
+// One thread per output row.  The row's LS rows are put in ascending order
+// (at most kRowLists of them), then walked coefficient by coefficient; the
+// thread's table in shared memory (at most kRowCols columns) holds one column
+// index and running sum per distinct column, found by a linear search, and
+// the row is written sorted by ranks.  A warp thus adds 32 rows' terms per
+// FP64 instruction, where one warp per row (k_merge) adds in a single lane: on
+// GB300, whose FP64 instructions occupy the SM for 16 cycles whatever the
+// number of active lanes, the merge of a 640 x 481 LSCM mesh (615,676 rows,
+// 8.6 M nonzeros, 44 M candidates) took 10.3 ms with k_merge alone.
+// Bound by L2 latency and the FP64 pipe.  The limits fit mesh operators (LSCM
+// rows merge 12 LS rows into 14 columns, the cotangent Laplacian 13 into 7,
+// the 7-point voxel rows 7 into 25) at 64 KB per 128 threads.
+// NUMERIC false: row_nnz, and the rows that do not fit into the lists mid (at
+// most kWarpCap candidates) and big.  NUMERIC true: values and right-hand side.
+constexpr int kRowLists = 24, kRowCols = 32, kRowCTA = 128;
+constexpr size_t kRowSmem = (size_t)kRowCTA * (kRowLists * (sizeof(int) + 2) + kRowCols * (sizeof(int) + sizeof(double)));
+
+template <bool NUMERIC>
+__global__ void __launch_bounds__(kRowCTA) k_merge_rows(MergeArgs A, int* mid, int* mid_n, int* big, int* big_n) {
+  extern __shared__ __align__(16) unsigned char row_smem[];
+  double* sum = reinterpret_cast<double*>(row_smem) + threadIdx.x;             // [kRowCols][kRowCTA]
+  int* col = reinterpret_cast<int*>(row_smem + sizeof(double) * kRowCols * kRowCTA) + threadIdx.x;
+  int* lst = col + kRowCols * kRowCTA;                                         // [kRowLists][kRowCTA]
+  unsigned char* ent = reinterpret_cast<unsigned char*>(lst - threadIdx.x + kRowLists * kRowCTA) + threadIdx.x;
+  unsigned char* hits = ent + kRowLists * kRowCTA;
+  const int i = blockIdx.x * kRowCTA + threadIdx.x;
+  if (i >= A.n_free) return;
+  const long long e0 = A.colptr[i];
+  const int L = (int)min(A.colptr[i + 1] - e0, (long long)kRowLists + 1);
+  bool fits = L <= kRowLists;
+  int nc = 0;
+  if (NUMERIC && fits) fits = A.rp[i + 1] - A.rp[i] <= kRowCols;
+  if (fits) {
+    for (int u = 0; u < L; ++u) {
+      const int r = A.colrow[e0 + u];
+      int t = u;
+      if (NUMERIC)   // insertion by r
+        for (; t > 0 && lst[(t - 1) * kRowCTA] > r; --t) {
+          lst[t * kRowCTA] = lst[(t - 1) * kRowCTA];
+          ent[t * kRowCTA] = ent[(t - 1) * kRowCTA];
+        }
+      lst[t * kRowCTA] = r;
+      ent[t * kRowCTA] = (unsigned char)u;
+    }
+    for (int u = 0; u < L && fits; ++u) {
+      const int r = lst[u * kRowCTA];
+      const double wa = NUMERIC ? A.colwa[e0 + ent[u * kRowCTA]] : 0.0;
+      const long long k1 = A.R.row_ptr[r + 1];
+      int own = 0;
+      for (long long k = A.R.row_ptr[r]; k < k1; ++k) {
+        const int j = A.R.col[k];
+        if (j < 0) continue;
+        int t = 0;
+        while (t < nc && col[t * kRowCTA] != j) ++t;
+        if (t == nc) {
+          if (nc == kRowCols) { fits = false; break; }
+          col[t * kRowCTA] = j;
+          if (NUMERIC) sum[t * kRowCTA] = 0.0;
+          ++nc;
+        }
+        if (NUMERIC) {
+          sum[t * kRowCTA] = __dadd_rn(sum[t * kRowCTA], __dmul_rn(wa, A.R.val[k]));
+          own += j == i;
+        }
+      }
+      if (NUMERIC) hits[u * kRowCTA] = (unsigned char)min(own, 255);
+    }
+  }
+  if (!NUMERIC) {
+    if (fits) { A.row_nnz[i] = nc; return; }
+    long long c = 0;
+    const long long e1 = A.colptr[i + 1];
+    for (long long e = e0; e < e1; ++e) c += A.nfree[A.colrow[e]];
+    if (c <= kWarpCap) mid[atomicAdd(mid_n, 1)] = i;
+    else big[atomicAdd(big_n, 1)] = i;
+    return;
+  }
+  if (!fits || nc == 0) return;
+  const int o = A.rp[i];
+  for (int t = 0; t < nc; ++t) {
+    const int j = col[t * kRowCTA];
+    int rank = 0;
+    for (int u = 0; u < nc; ++u) rank += col[u * kRowCTA] < j;
+    A.ci[o + rank] = j;
+    A.va[o + rank] = sum[t * kRowCTA];
+  }
+  for (int sys = 0; sys < A.R.n_systems; ++sys) {
+    double acc = 0.0;
+    for (int u = 0; u < L; ++u) {
+      const double v = __dmul_rn(A.colwa[e0 + ent[u * kRowCTA]], A.s[(size_t)sys * A.R.n_rows + lst[u * kRowCTA]]);
+      for (int h = hits[u * kRowCTA]; h > 0; --h) acc = __dadd_rn(acc, v);
+    }
+    A.rhs[(size_t)sys * A.n_free + i] = acc;
+  }
+}
 
 // Exclusive scan of v over a group of G threads (G == 32: one warp,
 // G == kAsmCTA: the whole CTA, which then must call it uniformly).
@@ -208,10 +294,8 @@ __global__ void __launch_bounds__(kAsmCTA) k_merge(MergeArgs A) {
                 (size_t)grp * CAP;
   __shared__ int heads_cnt[kGroups];
   const long long idx = (long long)blockIdx.x * kGroups + grp;
-  const long long total = A.rows ? A.n_rows_list : A.n_free;
-  const bool active = idx < total;
-  const int i = active ? (A.rows ? A.rows[idx] : (int)idx) : 0;
-  const bool mine = active && (A.rows != nullptr || A.cand[i] <= CAP);
+  const bool mine = idx < A.n_rows_list;
+  const int i = mine ? A.rows[idx] : 0;
   // All threads take part in fills/sorts (they contain __syncthreads); an
   // inactive group fills nothing.
   int cnt = fill_candidates<G>(A, i, mine, key, val, aux, g, CAP);
@@ -271,12 +355,6 @@ __global__ void __launch_bounds__(kAsmCTA) k_merge(MergeArgs A) {
       t = t2;
     }
   }
-}
-
-// Rows whose candidates exceed the warp cap (compacted list).
-__global__ void k_collect_big(int n_free, const int* cand, int cap, int* list, int* count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n_free && cand[i] > cap) list[atomicAdd(count, 1)] = i;
 }
 
 // Rows with no candidates still need an RHS of 0 (and no entries).
@@ -385,7 +463,7 @@ cudaError_t assemble_normal_equations(const LSRowsDevice& R, DeviceCRS& out, dou
     set_error("least-squares assembly: more than 2^31-1 rows");
     return cudaErrorInvalidValue;
   }
-  DevBuf<double> sbuf; DevBuf<int> nfree, colcnt, cursor, colrow, cand, row_nnz, big, big_n, err;
+  DevBuf<double> sbuf; DevBuf<int> nfree, colcnt, cursor, colrow, row_nnz, mid, big, ctl;
   DevBuf<long long> colptr, rp64;
   DevBuf<double> colwa;
   NLGB_CUDA_TRY(sbuf.alloc((size_t)R.n_systems * R.n_rows, s));
@@ -410,45 +488,47 @@ cudaError_t assemble_normal_equations(const LSRowsDevice& R, DeviceCRS& out, dou
     k_col_scatter<<<blocks_for(R.n_rows), 256, 0, s>>>(R, colptr.p, cursor.p, colrow.p, colwa.p);
     count_launches(1);
   }
-  NLGB_CUDA_TRY(cand.alloc(nf + 1, s));
   NLGB_CUDA_TRY(row_nnz.alloc(nf + 1, s));
+  NLGB_CUDA_TRY(mid.alloc(nf + 1, s));
   NLGB_CUDA_TRY(big.alloc(nf + 1, s));
-  NLGB_CUDA_TRY(big_n.alloc(1, s));
-  NLGB_CUDA_TRY(err.alloc(1, s));
-  NLGB_CUDA_TRY(cudaMemsetAsync(big_n.p, 0, sizeof(int), s));
-  NLGB_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(int), s));
+  NLGB_CUDA_TRY(ctl.alloc(3, s));   // rows in mid, rows in big, error
+  NLGB_CUDA_TRY(cudaMemsetAsync(ctl.p, 0, 3 * sizeof(int), s));
   NLGB_CUDA_TRY(cudaMemsetAsync(row_nnz.p, 0, sizeof(int) * (nf + 1), s));
-  if (nf > 0) {
-    k_cand_count<<<blocks_for(nf), 256, 0, s>>>(nf, colptr.p, colrow.p, nfree.p, cand.p);
-    count_launches(1);
-    k_collect_big<<<blocks_for(nf), 256, 0, s>>>(nf, cand.p, kWarpCap, big.p, big_n.p);
-    count_launches(1);
-  }
-  NLGB_CUDA_TRY(cudaGetLastError());
-  int n_big = 0;
-  NLGB_CUDA_TRY(cudaMemcpyAsync(&n_big, big_n.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  NLGB_CUDA_TRY(cudaStreamSynchronize(s));
 
   MergeArgs M;
   M.R = R; M.n_free = nf; M.colptr = colptr.p; M.colrow = colrow.p; M.colwa = colwa.p;
-  M.nfree = nfree.p; M.s = sbuf.p; M.cand = cand.p; M.row_nnz = row_nnz.p; M.err = err.p;
+  M.nfree = nfree.p; M.s = sbuf.p; M.row_nnz = row_nnz.p; M.err = ctl.p + 2;
   M.rp = nullptr; M.ci = nullptr; M.va = nullptr; M.rhs = rhs_out; M.numeric = 0;
   constexpr int kWarpGroups = kAsmCTA / 32;
   const size_t smem_warp = (size_t)kWarpCap * kWarpGroups * 24;
   const size_t smem_block = (size_t)kBlockCap * 24;
   NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge<32, kWarpCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_warp));
   NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge<kAsmCTA, kBlockCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_block));
+  NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem));
+  NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem));
+  int listed[2] = {0, 0};   // rows in mid, big
   auto run_merge = [&](int numeric) -> cudaError_t {
     M.numeric = numeric;
-    M.rows = nullptr; M.n_rows_list = 0;
     if (nf > 0) {
-      k_merge<32, kWarpCap><<<blocks_for(nf, kWarpGroups), kAsmCTA, smem_warp, s>>>(M);
+      const unsigned g = blocks_for(nf, kRowCTA);
+      if (numeric) k_merge_rows<true><<<g, kRowCTA, kRowSmem, s>>>(M, nullptr, nullptr, nullptr, nullptr);
+      else k_merge_rows<false><<<g, kRowCTA, kRowSmem, s>>>(M, mid.p, ctl.p, big.p, ctl.p + 1);
       count_launches(1);
     }
     NLGB_CUDA_TRY(cudaGetLastError());
-    if (n_big > 0) {
-      M.rows = big.p; M.n_rows_list = n_big;
-      k_merge<kAsmCTA, kBlockCap><<<(unsigned)n_big, kAsmCTA, smem_block, s>>>(M);
+    if (!numeric) {
+      NLGB_CUDA_TRY(cudaMemcpyAsync(listed, ctl.p, sizeof(listed), cudaMemcpyDeviceToHost, s));
+      NLGB_CUDA_TRY(cudaStreamSynchronize(s));
+    }
+    if (listed[0] > 0) {
+      M.rows = mid.p; M.n_rows_list = listed[0];
+      k_merge<32, kWarpCap><<<blocks_for(listed[0], kWarpGroups), kAsmCTA, smem_warp, s>>>(M);
+      count_launches(1);
+      NLGB_CUDA_TRY(cudaGetLastError());
+    }
+    if (listed[1] > 0) {
+      M.rows = big.p; M.n_rows_list = listed[1];
+      k_merge<kAsmCTA, kBlockCap><<<(unsigned)listed[1], kAsmCTA, smem_block, s>>>(M);
       count_launches(1);
       NLGB_CUDA_TRY(cudaGetLastError());
     }
@@ -456,7 +536,7 @@ cudaError_t assemble_normal_equations(const LSRowsDevice& R, DeviceCRS& out, dou
   };
   NLGB_CUDA_TRY(run_merge(0));
   int herr = 0;
-  NLGB_CUDA_TRY(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  NLGB_CUDA_TRY(cudaMemcpyAsync(&herr, ctl.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
   NLGB_CUDA_TRY(rp64.alloc(nf + 1, s));
   long long nnz = 0;
   NLGB_CUDA_TRY(exclusive_scan<int>(row_nnz.p, nf + 1, rp64.p, &nnz, s));
