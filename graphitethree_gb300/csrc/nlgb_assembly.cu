@@ -100,27 +100,31 @@ struct MergeArgs {
 
 // One thread per output row.  The row's LS rows are put in ascending order
 // (at most kRowLists of them), then walked coefficient by coefficient; the
-// thread's table in shared memory (at most kRowCols columns) holds one column
-// index and running sum per distinct column, found by a linear search, and
-// the row is written sorted by ranks.  A warp thus adds 32 rows' terms per
-// FP64 instruction, where one warp per row (k_merge) adds in a single lane: on
-// GB300, whose FP64 instructions occupy the SM for 16 cycles whatever the
-// number of active lanes, the merge of a 640 x 481 LSCM mesh (615,676 rows,
-// 8.6 M nonzeros, 44 M candidates) took 10.3 ms with k_merge alone.
-// Bound by L2 latency and the FP64 pipe.  The limits fit mesh operators (LSCM
-// rows merge 12 LS rows into 14 columns, the cotangent Laplacian 13 into 7,
-// the 7-point voxel rows 7 into 25) at 64 KB per 128 threads.
+// thread's hash table in shared memory (at most kRowCols columns) holds one
+// column index and running sum per distinct column, and the row is written
+// sorted by ranks.  A warp thus adds 32 rows' terms per FP64 instruction,
+// where one warp per row (k_merge) adds in a single lane: on GB300, whose FP64
+// instructions occupy the SM for 16 cycles whatever the number of active
+// lanes, the merge of a 640 x 481 LSCM mesh (615,676 rows, 8.6 M nonzeros,
+// 44 M candidates) took 10.3 ms with k_merge alone and takes 0.64 ms here.
+// Bound by L2 latency (the rows a thread reads are scattered), so the row
+// pointers of the next LS row and eight coefficients are loaded at once; a
+// linear search of the columns instead of the hash took 0.67 + 1.16 ms.  The
+// limits fit mesh operators (LSCM rows merge 12 LS rows into 14 columns, the
+// cotangent Laplacian 13 into 7, the 7-point voxel rows 7 into 25) at 66 KB
+// per 128 threads.
 // NUMERIC false: row_nnz, and the rows that do not fit into the lists mid (at
 // most kWarpCap candidates) and big.  NUMERIC true: values and right-hand side.
 constexpr int kRowLists = 24, kRowCols = 32, kRowCTA = 128;
-constexpr size_t kRowSmem = (size_t)kRowCTA * (kRowLists * (sizeof(int) + 2) + kRowCols * (sizeof(int) + sizeof(double)));
+constexpr size_t kRowSmemCols = (size_t)kRowCTA * kRowCols * sizeof(int);
+constexpr size_t kRowSmem = kRowSmemCols + (size_t)kRowCTA * (kRowCols * sizeof(double) + kRowLists * (sizeof(int) + 2));
 
 template <bool NUMERIC>
 __global__ void __launch_bounds__(kRowCTA) k_merge_rows(MergeArgs A, int* mid, int* mid_n, int* big, int* big_n) {
   extern __shared__ __align__(16) unsigned char row_smem[];
-  double* sum = reinterpret_cast<double*>(row_smem) + threadIdx.x;             // [kRowCols][kRowCTA]
-  int* col = reinterpret_cast<int*>(row_smem + sizeof(double) * kRowCols * kRowCTA) + threadIdx.x;
-  int* lst = col + kRowCols * kRowCTA;                                         // [kRowLists][kRowCTA]
+  int* col = reinterpret_cast<int*>(row_smem) + threadIdx.x;                   // [kRowCols][kRowCTA], -1: free
+  double* sum = reinterpret_cast<double*>(row_smem + kRowSmemCols) + threadIdx.x;
+  int* lst = reinterpret_cast<int*>(sum - threadIdx.x + kRowCols * kRowCTA) + threadIdx.x;   // [kRowLists][kRowCTA]
   unsigned char* ent = reinterpret_cast<unsigned char*>(lst - threadIdx.x + kRowLists * kRowCTA) + threadIdx.x;
   unsigned char* hits = ent + kRowLists * kRowCTA;
   const int i = blockIdx.x * kRowCTA + threadIdx.x;
@@ -131,36 +135,68 @@ __global__ void __launch_bounds__(kRowCTA) k_merge_rows(MergeArgs A, int* mid, i
   int nc = 0;
   if (NUMERIC && fits) fits = A.rp[i + 1] - A.rp[i] <= kRowCols;
   if (fits) {
-    for (int u = 0; u < L; ++u) {
-      const int r = A.colrow[e0 + u];
-      int t = u;
-      if (NUMERIC)   // insertion by r
+#pragma unroll 8
+    for (int t = 0; t < kRowCols; ++t) col[t * kRowCTA] = -1;
+    if (NUMERIC) {   // insertion by r
+      for (int u = 0; u < L; ++u) {
+        const int r = A.colrow[e0 + u];
+        int t = u;
         for (; t > 0 && lst[(t - 1) * kRowCTA] > r; --t) {
           lst[t * kRowCTA] = lst[(t - 1) * kRowCTA];
           ent[t * kRowCTA] = ent[(t - 1) * kRowCTA];
         }
-      lst[t * kRowCTA] = r;
-      ent[t * kRowCTA] = (unsigned char)u;
+        lst[t * kRowCTA] = r;
+        ent[t * kRowCTA] = (unsigned char)u;
+      }
     }
+    auto row_at = [&](int u) { return NUMERIC ? lst[u * kRowCTA] : A.colrow[e0 + u]; };
+    long long kn = 0, kn1 = 0;      // the next row's coefficients
+    double wn = 0.0;
+    auto fetch = [&](int u) {
+      if (u < L) {
+        const int r = row_at(u);
+        kn = A.R.row_ptr[r];
+        kn1 = A.R.row_ptr[r + 1];
+        if (NUMERIC) wn = A.colwa[e0 + ent[u * kRowCTA]];
+      }
+    };
+    fetch(0);
     for (int u = 0; u < L && fits; ++u) {
-      const int r = lst[u * kRowCTA];
-      const double wa = NUMERIC ? A.colwa[e0 + ent[u * kRowCTA]] : 0.0;
-      const long long k1 = A.R.row_ptr[r + 1];
+      const long long k0 = kn, k1 = kn1;
+      const double wa = wn;
+      fetch(u + 1);
       int own = 0;
-      for (long long k = A.R.row_ptr[r]; k < k1; ++k) {
-        const int j = A.R.col[k];
-        if (j < 0) continue;
-        int t = 0;
-        while (t < nc && col[t * kRowCTA] != j) ++t;
-        if (t == nc) {
-          if (nc == kRowCols) { fits = false; break; }
-          col[t * kRowCTA] = j;
-          if (NUMERIC) sum[t * kRowCTA] = 0.0;
-          ++nc;
+      for (long long k = k0; k < k1 && fits; k += 8) {
+        int c[8];
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          c[q] = -1;
+          if (k + q < k1) {
+            c[q] = A.R.col[k + q];
+            if (NUMERIC) v[q] = A.R.val[k + q];
+          }
         }
-        if (NUMERIC) {
-          sum[t * kRowCTA] = __dadd_rn(sum[t * kRowCTA], __dmul_rn(wa, A.R.val[k]));
-          own += j == i;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int j = c[q];
+          if (j < 0 || !fits) continue;
+          unsigned h = ((unsigned)j * 2654435761u) >> 27;
+          int x = col[h * kRowCTA];
+          for (int t = 1; x != j && x != -1 && t < kRowCols; ++t) {
+            h = (h + 1) % kRowCols;
+            x = col[h * kRowCTA];
+          }
+          if (x != j) {
+            if (x != -1) { fits = false; continue; }   // more than kRowCols columns
+            col[h * kRowCTA] = j;
+            if (NUMERIC) sum[h * kRowCTA] = 0.0;
+            ++nc;
+          }
+          if (NUMERIC) {
+            sum[h * kRowCTA] = __dadd_rn(sum[h * kRowCTA], __dmul_rn(wa, v[q]));
+            own += j == i;
+          }
         }
       }
       if (NUMERIC) hits[u * kRowCTA] = (unsigned char)min(own, 255);
@@ -176,6 +212,16 @@ __global__ void __launch_bounds__(kRowCTA) k_merge_rows(MergeArgs A, int* mid, i
     return;
   }
   if (!fits || nc == 0) return;
+  // the used slots moved to the front, then every column to its rank
+  for (int t = 0, to = 0; t < kRowCols; ++t) {
+    const int j = col[t * kRowCTA];
+    if (j < 0) continue;
+    if (to != t) {
+      col[to * kRowCTA] = j;
+      sum[to * kRowCTA] = sum[t * kRowCTA];
+    }
+    ++to;
+  }
   const int o = A.rp[i];
   for (int t = 0; t < nc; ++t) {
     const int j = col[t * kRowCTA];
@@ -504,7 +550,7 @@ cudaError_t assemble_normal_equations(const LSRowsDevice& R, DeviceCRS& out, dou
   const size_t smem_block = (size_t)kBlockCap * 24;
   NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge<32, kWarpCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_warp));
   NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge<kAsmCTA, kBlockCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_block));
-  NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem));
+  NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmemCols));
   NLGB_CUDA_TRY(cudaFuncSetAttribute(k_merge_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem));
   int listed[2] = {0, 0};   // rows in mid, big
   auto run_merge = [&](int numeric) -> cudaError_t {
@@ -512,7 +558,7 @@ cudaError_t assemble_normal_equations(const LSRowsDevice& R, DeviceCRS& out, dou
     if (nf > 0) {
       const unsigned g = blocks_for(nf, kRowCTA);
       if (numeric) k_merge_rows<true><<<g, kRowCTA, kRowSmem, s>>>(M, nullptr, nullptr, nullptr, nullptr);
-      else k_merge_rows<false><<<g, kRowCTA, kRowSmem, s>>>(M, mid.p, ctl.p, big.p, ctl.p + 1);
+      else k_merge_rows<false><<<g, kRowCTA, kRowSmemCols, s>>>(M, mid.p, ctl.p, big.p, ctl.p + 1);
       count_launches(1);
     }
     NLGB_CUDA_TRY(cudaGetLastError());
