@@ -46,7 +46,7 @@ struct KrState {
   int pad_;
   double H[(kMaxRestart + 1) * kMaxRestart];   // column-major, (m + 1) x m
   double cs[kMaxRestart], sn[kMaxRestart], g[kMaxRestart + 1], y[kMaxRestart];
-  double hr[kMaxRestart + 1];       // GMRES: coefficients of the current Gram-Schmidt round
+  int act[kMaxRestart + 1];         // GMRES: step j of this cycle is to be run
 };
 
 struct KrView {
@@ -57,8 +57,9 @@ struct KrView {
   const double* dinv;
   double* part;      // n_tiles * kParts
   KrState* st;
-  double* mpart;     // GMRES: n_tiles * (m + 1) multi-dot partials
+  double* mpart;     // GMRES: per CTA of a step kernel m + 1 multi-dot partials, then its w.w
   int mstride;
+  int step_ctas, step_rows;   // GMRES: CTAs of the step kernels and rows of each
 };
 
 __device__ __forceinline__ bool running(const KrView& v) {
@@ -259,9 +260,10 @@ __global__ void __launch_bounds__(kCTA) k_gm_residual(KrView v, GmVecs w) {
 }
 
 __global__ void k_gm_start(KrView v, int first) {
+  if ((int)threadIdx.x <= kMaxRestart) v.st->act[threadIdx.x] = 0;   // no step of this cycle yet
   if (*((volatile int*)&v.st->status) != ST_RUNNING) return;
   double o[2];
-  sums<2>(v, 0, o);
+  sums<2>(v, 0, o);                // (synchronises the CTA)
   if (threadIdx.x != 0) return;
   KrState* st = v.st;
   if (first) {
@@ -279,131 +281,242 @@ __global__ void k_gm_start(KrView v, int first) {
   st->j = 0;
   st->cyc_done = 0;
   st->beta = beta;
+  st->act[0] = 1;
 }
 
-__global__ void k_gm_scale0(KrView v, GmVecs w) {
-  if (*((volatile int*)&v.st->status) != ST_RUNNING || v.st->cyc_done) return;
+// A step of a cycle is four kernels of one 1,024-thread CTA per SM (ten
+// launches over the matrix's tiles before):
+//   k_gm_spmv    w = A u, and the partials of h = V^T w;
+//   k_gm_orth    h summed by every CTA, w -= V h, partials of h2 = V^T w;
+//   k_gm_orth    h2 summed, w -= V h2, partials of w.w;
+//   k_gm_next    the norm, V_{j+1} = w / ||w||, u = M^-1 V_{j+1}; one thread
+//                turns column j of H into the QR factors and decides whether
+//                the cycle goes on.
+// V fits L2 up to about 16 M entries; the FP64 pipe bounds the rest: 4 n (j + 1)
+// products per step, 32 of the 104 us a step takes at 314,323 rows (j = 15 on
+// average).  What was slow before: a block sum per coefficient and tile of 384
+// rows cost three times its products (67 us per round), and the reductions and
+// the norm were kernels of one CTA.  Measured on GB300, convection-diffusion
+// 601 x 523, GMRES(30): 231 -> 104 us per step.
+constexpr int kGmThreads = 1024;
+constexpr int kGmWarps = kGmThreads / 32;
+
+// Sums of eight per-lane values over the warp: lane l returns value
+// (l / 4) mod 8 (the lanes that carry a value halve at each level, so eight
+// sums take nine additions).
+__device__ __forceinline__ double warp_sum8(const double (&a)[8]) {
+  const int l = threadIdx.x & 31;
+  double u[4], t[2];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    u[q] = ((l & 16) ? a[q + 4] : a[q]) + __shfl_xor_sync(0xffffffffu, (l & 16) ? a[q] : a[q + 4], 16);
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    t[q] = ((l & 8) ? u[q + 2] : u[q]) + __shfl_xor_sync(0xffffffffu, (l & 8) ? u[q] : u[q + 2], 8);
+  double s = ((l & 4) ? t[1] : t[0]) + __shfl_xor_sync(0xffffffffu, (l & 4) ? t[0] : t[1], 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+__device__ __forceinline__ int step_lo(const KrView& v) { return (int)blockIdx.x * v.step_rows; }
+__device__ __forceinline__ int step_hi(const KrView& v) { return min(v.n, ((int)blockIdx.x + 1) * v.step_rows); }
+__device__ __forceinline__ bool step_active(const KrView& v, int j) { return *((volatile int*)&v.st->act[j]) != 0; }
+
+// This CTA's partials of V_i . w, i <= j (every thread calls it).
+__device__ __forceinline__ void step_dots(const KrView& v, const GmVecs& w, const double* wn, int j) {
+  __shared__ double red[kGmWarps][kMaxRestart + 1];
+  const int lo = step_lo(v), hi = step_hi(v), warp = threadIdx.x >> 5, l = threadIdx.x & 31;
+  for (int i0 = 0; i0 <= j; i0 += 8) {
+    double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const int c = min(8, j + 1 - i0);
+    const double* Vi = w.V + (size_t)i0 * w.ld;
+    for (int r = lo + (int)threadIdx.x; r < hi; r += kGmThreads) {
+      const double x = wn[r];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < c) a[q] = fma(x, Vi[(size_t)q * w.ld + r], a[q]);
+    }
+    const double s = warp_sum8(a);
+    if ((l & 3) == 0 && (l >> 2) < c) red[warp][i0 + (l >> 2)] = s;
+  }
+  __syncthreads();
+  // eight lanes per coefficient
+  const int i = threadIdx.x >> 3, p = threadIdx.x & 7;
+  double s = 0.0;
+  if (i <= j) {
+    s = red[p][i];
+#pragma unroll
+    for (int k = 1; k < kGmWarps / 8; ++k) s += red[p + 8 * k][i];
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  if (i <= j && p == 0) v.mpart[(size_t)blockIdx.x * v.mstride + i] = s;
+}
+
+// The coefficients i <= j summed over the CTAs into h (shared memory).
+__device__ __forceinline__ void step_sums(const KrView& v, int j, double* h) {
+  const int l = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i <= j; i += kGmWarps) {
+    double s = 0.0;
+    for (int g = l; g < v.step_ctas; g += 32) s += v.mpart[(size_t)g * v.mstride + i];
+    s = warp_sum(s);
+    if (l == 0) h[i] = s;
+  }
+  __syncthreads();
+}
+
+// V_0 = r / ||r||, u = M^-1 V_0 (prec 0: a general preconditioner follows).
+__global__ void k_gm_scale0(KrView v, GmVecs w, int prec) {
+  if (!step_active(v, 0)) return;
   const double inv = 1.0 / v.st->beta;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < v.n; i += (long long)gridDim.x * blockDim.x)
-    w.V[i] *= inv;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < v.n; i += (long long)gridDim.x * blockDim.x) {
+    const double x = w.V[i] * inv;
+    w.V[i] = x;
+    if (prec) w.u[i] = v.dinv[i] * x;
+  }
 }
 
-__device__ __forceinline__ bool gm_active(const KrView& v, int j) {
-  return *((volatile int*)&v.st->status) == ST_RUNNING && !v.st->cyc_done && v.st->j == j;
-}
-
-// u = M^-1 V_j
-__global__ void k_gm_precond(KrView v, GmVecs w, int j) {
-  if (!gm_active(v, j)) return;
-  const double* Vj = w.V + (size_t)j * w.ld;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < v.n; i += (long long)gridDim.x * blockDim.x)
-    w.u[i] = v.dinv[i] * Vj[i];
-}
-
-// V_{j+1} = A u
 template <int T>
-__global__ void __launch_bounds__(kCTA) k_gm_spmv(KrView v, GmVecs w, int j) {
-  if (!gm_active(v, j)) return;
+__global__ void __launch_bounds__(kGmThreads, 1) k_gm_spmv(KrView v, GmVecs w, int j) {
+  if (!step_active(v, j)) return;
   double* Wn = w.V + (size_t)(j + 1) * w.ld;
-  tile_spmv<T>(v, w.u, [&](int i, double q) { Wn[i] = q; });
-}
-
-// Gram-Schmidt round, 1/3: per-tile partials of V_i . w for every i <= j
-// (one sweep over the tile per i; w stays in L1 between them).  Measured on
-// GB300: grouping eight coefficients per sweep was not faster.
-__global__ void __launch_bounds__(kCTA) k_gm_multidot(KrView v, GmVecs w, int j) {
-  if (!gm_active(v, j)) return;
-  const double* Wn = w.V + (size_t)(j + 1) * w.ld;
-  for (int i = 0; i <= j; ++i) {
-    const double* Vi = w.V + (size_t)i * w.ld;
-    double a[1] = {0.0};
-    for (int r = lo_of(v) + threadIdx.x; r < hi_of(v); r += kCTA) a[0] = fma(Wn[r], Vi[r], a[0]);
-    block_sum<1>(a);
-    if (threadIdx.x == 0) v.mpart[(size_t)blockIdx.x * v.mstride + i] = a[0];
+  const int lo = step_lo(v), hi = step_hi(v);
+  constexpr int RPP = kGmThreads / T;
+  for (int base = lo; base < hi; base += RPP) {
+    const int row = base + (int)threadIdx.x / T, lane = threadIdx.x % T;
+    // (row_dot with up to eight nonzeros per lane in flight: one CTA per SM
+    // hides less latency than the tiles' eight)
+    double q = 0.0;
+    if (row < hi) {
+      const int k1 = __ldg(v.rp + row + 1);
+      for (int k = __ldg(v.rp + row) + lane; k < k1; k += 8 * T) {
+        double x[8], a[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (k + u * T < k1) {
+            x[u] = __ldg(w.u + __ldg(v.ci + k + u * T));
+            a[u] = __ldg(v.va + k + u * T);
+          }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (k + u * T < k1) q = fma(a[u], x[u], q);
+      }
+    }
+    q = subwarp_sum<T, double>(q);
+    if (row < hi && lane == 0) Wn[row] = q;
   }
+  __syncthreads();
+  step_dots(v, w, Wn, j);
 }
 
-// 2/3: CTA i reduces coefficient i over the tiles in the canonical order
-// (thread t sums tiles t, t + 256, ..., then the fixed block tree).
-__global__ void __launch_bounds__(kCTA) k_gm_hreduce(KrView v, int j, int round) {
-  if (!gm_active(v, j)) return;
-  const int i = blockIdx.x;
-  double a[1] = {0.0};
-  for (int t = threadIdx.x; t < v.n_tiles; t += kCTA) a[0] += v.mpart[(size_t)t * v.mstride + i];
-  block_sum<1>(a);
-  if (threadIdx.x == 0) {
+// One Gram-Schmidt round: the sums of the partials, w -= V h (i in order);
+// then the second round's partials, or after it (round 1) those of w.w.
+__global__ void __launch_bounds__(kGmThreads, 1) k_gm_orth(KrView v, GmVecs w, int j, int round, const double* pin) {
+  if (!step_active(v, j)) return;
+  __shared__ double h[kMaxRestart + 1];
+  __shared__ double rr[kGmWarps];
+  {
+    KrView in = v;
+    in.mpart = const_cast<double*>(pin);
+    step_sums(in, j, h);
+  }
+  if (blockIdx.x == 0 && (int)threadIdx.x <= j) {
     double* Hj = v.st->H + j * (kMaxRestart + 1);
-    v.st->hr[i] = a[0];
-    Hj[i] = round == 0 ? a[0] : Hj[i] + a[0];
+    Hj[threadIdx.x] = round == 0 ? h[threadIdx.x] : Hj[threadIdx.x] + h[threadIdx.x];
   }
-}
-
-// 3/3: w -= sum_i hr_i V_i (i in order); after the second round also the
-// partial of w.w for the norm.
-__global__ void __launch_bounds__(kCTA) k_gm_update(KrView v, GmVecs w, int j, int with_norm) {
-  if (!gm_active(v, j)) return;
   double* Wn = w.V + (size_t)(j + 1) * w.ld;
-  const double* hr = v.st->hr;
-  double a[1] = {0.0};
-  for (int r = lo_of(v) + threadIdx.x; r < hi_of(v); r += kCTA) {
+  const int lo = step_lo(v), hi = step_hi(v);
+  double a = 0.0;
+  for (int r = lo + (int)threadIdx.x; r < hi; r += kGmThreads) {
     double x = Wn[r];
-    for (int i = 0; i <= j; ++i) x -= hr[i] * w.V[(size_t)i * w.ld + r];
+#pragma unroll 8
+    for (int i = 0; i <= j; ++i) x -= h[i] * w.V[(size_t)i * w.ld + r];
     Wn[r] = x;
-    a[0] = fma(x, x, a[0]);
+    a = fma(x, x, a);
   }
-  if (with_norm) put_tile<1>(v, 0, a);
+  if (round == 0) {
+    step_dots(v, w, Wn, j);      // (each thread reads back its own rows)
+    return;
+  }
+  a = warp_sum(a);
+  if ((threadIdx.x & 31) == 0) rr[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    a = warp_sum(rr[threadIdx.x]);
+    if (threadIdx.x == 0) v.mpart[(size_t)blockIdx.x * v.mstride] = a;
+  }
 }
 
-// H_{j+1,j} = ||w||, V_{j+1} /= it; Givens rotations; cycle control.
-__global__ void k_gm_norm(KrView v, int j) {
-  if (!gm_active(v, j)) return;
-  double o[1];
-  sums<1>(v, 0, o);
-  if (threadIdx.x != 0) return;
+// H_{j+1,j} = ||w||, V_{j+1} = w / it, u = M^-1 V_{j+1}; Givens rotations and
+// cycle control by one thread.
+__global__ void __launch_bounds__(kGmThreads, 1) k_gm_next(KrView v, GmVecs w, int j, int prec) {
+  if (!step_active(v, j)) return;
+  __shared__ double nrm[1];
+  __shared__ double hc[kMaxRestart + 1], cs[kMaxRestart], sn[kMaxRestart];
   KrState* st = v.st;
   double* Hj = st->H + j * (kMaxRestart + 1);
-  const double hn = sqrt(o[0]);
-  Hj[j + 1] = hn;
-  for (int k = 0; k < j; ++k) {              // previous rotations on column j
-    const double a = Hj[k], b = Hj[k + 1];
-    Hj[k] = st->cs[k] * a + st->sn[k] * b;
-    Hj[k + 1] = -st->sn[k] * a + st->cs[k] * b;
+  const bool last = blockIdx.x == gridDim.x - 1;
+  if (last && (int)threadIdx.x <= j) {       // column j and the previous rotations
+    hc[threadIdx.x] = Hj[threadIdx.x];
+    if ((int)threadIdx.x < j) { cs[threadIdx.x] = st->cs[threadIdx.x]; sn[threadIdx.x] = st->sn[threadIdx.x]; }
   }
-  const double a = Hj[j], b = Hj[j + 1];
+  step_sums(v, 0, nrm);
+  const double hn = sqrt(nrm[0]);
+  if (hn > 0.0) {                // (a lucky breakdown, H_{j+1,j} = 0, leaves w)
+    double* Wn = w.V + (size_t)(j + 1) * w.ld;
+    const double inv = 1.0 / hn;
+    const int hi = step_hi(v);
+    for (int r = step_lo(v) + (int)threadIdx.x; r < hi; r += kGmThreads) {
+      const double x = Wn[r] * inv;
+      Wn[r] = x;
+      if (prec) w.u[r] = v.dinv[r] * x;
+    }
+  }
+  if (!last || threadIdx.x != 0) return;
+  // previous rotations on column j, then the new one
+  double a = hc[0];
+  for (int k = 0; k < j; ++k) {
+    const double b = hc[k + 1], c = cs[k], s = sn[k];
+    const double up = c * a + s * b;
+    Hj[k] = up;
+    a = -s * a + c * b;
+  }
+  const double b = hn;
   const double den = hypot(a, b);
   const double c = den > 0.0 ? a / den : 1.0, s = den > 0.0 ? b / den : 0.0;
+  const double gj = st->g[j];
   st->cs[j] = c; st->sn[j] = s;
   Hj[j] = den; Hj[j + 1] = 0.0;
-  st->g[j + 1] = -s * st->g[j];
-  st->g[j] = c * st->g[j];
-  st->gnorm = fabs(st->g[j + 1]);
+  const double gn = -s * gj;
+  st->g[j + 1] = gn;
+  st->g[j] = c * gj;
+  st->gnorm = fabs(gn);
   st->iter += 1;
   st->j = j + 1;
   if (!(den > 0.0) || !(hn == hn)) { st->cyc_done = 1; if (!(den > 0.0)) st->status = ST_BREAKDOWN; return; }
-  if (st->gnorm * st->gnorm <= st->thresh2 * st->bnorm2 || j + 1 >= st->m ||
-      st->iter >= st->max_iter || !(hn > 0.0))
+  if (gn * gn <= st->thresh2 * st->bnorm2 || j + 1 >= st->m || st->iter >= st->max_iter || !(hn > 0.0)) {
     st->cyc_done = 1;
-  st->beta = hn;        // for the scaling of V_{j+1}
-}
-
-__global__ void k_gm_scale(KrView v, GmVecs w, int j) {
-  // V_{j+1} /= H_{j+1,j} (skipped after a lucky breakdown, H_{j+1,j} = 0)
-  if (*((volatile int*)&v.st->status) != ST_RUNNING || v.st->j != j + 1 || !(v.st->beta > 0.0)) return;
-  double* Wn = w.V + (size_t)(j + 1) * w.ld;
-  const double inv = 1.0 / v.st->beta;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < v.n; i += (long long)gridDim.x * blockDim.x)
-    Wn[i] *= inv;
+    return;
+  }
+  st->act[j + 1] = 1;
 }
 
 // End of a cycle: y = H^-1 g (back substitution over the k = j steps done)
+// (one warp: lane c holds the right-hand sides c and c + 32, and the columns are
+// eliminated from the last; one thread doing the rows took 59 us at k = 30)
 __global__ void k_gm_solve_y(KrView v) {
   KrState* st = v.st;
-  if (*((volatile int*)&st->status) != ST_RUNNING || threadIdx.x != 0) return;
-  const int k = st->j;
+  if (*((volatile int*)&st->status) != ST_RUNNING) return;
+  const int k = st->j, l = threadIdx.x;
+  double g0 = l < k ? st->g[l] : 0.0, g1 = l + 32 < k ? st->g[l + 32] : 0.0;
   for (int i = k - 1; i >= 0; --i) {
-    double s = st->g[i];
-    for (int c = i + 1; c < k; ++c) s -= st->H[c * (kMaxRestart + 1) + i] * st->y[c];
-    st->y[i] = s / st->H[i * (kMaxRestart + 1) + i];
+    const double* Hi = st->H + i * (kMaxRestart + 1);
+    const double y = __shfl_sync(0xffffffffu, i < 32 ? g0 : g1, i & 31) / Hi[i];
+    if (l == (i & 31)) st->y[i] = y;
+    if (l < i) g0 = fma(-Hi[l], y, g0);
+    if (l + 32 < i) g1 = fma(-Hi[l + 32], y, g1);
   }
 }
 
@@ -468,8 +581,18 @@ cudaError_t krylov_solve(const DeviceCRS& A, const double* dinv, const double* b
   cudaError_t e = cudaMallocAsync(&part, sizeof(double) * (size_t)n_tiles * kParts, s);
   if (e == cudaSuccess) e = cudaMallocAsync(&st, sizeof(KrState), s);
   double* mpart = nullptr;
-  if (e == cudaSuccess && method == KRYLOV_GMRES)
-    e = cudaMallocAsync(&mpart, sizeof(double) * (size_t)n_tiles * (m + 1), s);
+  // GMRES step kernels: one CTA per SM (at least 256 rows each), two areas of
+  // partials (a kernel reads one and writes the other)
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    sms = 152;
+  }
+  const int step_rows = std::max(256, (n + sms - 1) / sms);
+  const int step_ctas = std::max(1, (n + step_rows - 1) / step_rows);
+  const size_t part_area = (size_t)step_ctas * (m + 1);
+  if (e == cudaSuccess && method == KRYLOV_GMRES) e = cudaMallocAsync(&mpart, sizeof(double) * 2 * part_area, s);
   KrState h;
   std::memset(&h, 0, sizeof(h));
   h.thresh2 = eps * eps;
@@ -477,7 +600,7 @@ cudaError_t krylov_solve(const DeviceCRS& A, const double* dinv, const double* b
   h.status = ST_RUNNING;
   h.m = m;
   if (e == cudaSuccess) e = cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-  KrView v{n, tile_rows, n_tiles, A.rp, A.ci, A.va, dinv, part, st, mpart, m + 1};
+  KrView v{n, tile_rows, n_tiles, A.rp, A.ci, A.va, dinv, part, st, mpart, m + 1, step_ctas, step_rows};
   long long launches = 0;
   auto poll = [&](int* status) {
     cudaError_t pe = cudaMemcpyAsync(status, &st->status, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -518,24 +641,18 @@ cudaError_t krylov_solve(const DeviceCRS& A, const double* dinv, const double* b
     while (e == cudaSuccess && status == ST_RUNNING) {
       NLGB_KR_T((k_gm_residual<T><<<n_tiles, kCTA, 0, s>>>(v, w)));
       k_gm_start<<<1, kCTA, 0, s>>>(v, first ? 1 : 0);
-      k_gm_scale0<<<grid1(n), 256, 0, s>>>(v, w);
+      k_gm_scale0<<<grid1(n), 256, 0, s>>>(v, w, P ? 0 : 1);
       launches += 3;
       first = false;
+      KrView v1 = v;               // the other area of partials
+      v1.mpart = mpart + part_area;
       for (int j = 0; j < m; ++j) {
-        if (P) {
-          if (e == cudaSuccess) e = P->apply(w.V + (size_t)j * ld, w.u, s);   // u = M^-1 V_j
-        } else {
-          k_gm_precond<<<grid1(n), 256, 0, s>>>(v, w, j);
-        }
-        NLGB_KR_T((k_gm_spmv<T><<<n_tiles, kCTA, 0, s>>>(v, w, j)));
-        for (int round = 0; round < 2; ++round) {     // CGS2
-          k_gm_multidot<<<n_tiles, kCTA, 0, s>>>(v, w, j);
-          k_gm_hreduce<<<j + 1, kCTA, 0, s>>>(v, j, round);
-          k_gm_update<<<n_tiles, kCTA, 0, s>>>(v, w, j, round);
-        }
-        k_gm_norm<<<1, kCTA, 0, s>>>(v, j);
-        k_gm_scale<<<grid1(n), 256, 0, s>>>(v, w, j);
-        launches += 10;
+        if (P && e == cudaSuccess) e = P->apply(w.V + (size_t)j * ld, w.u, s);   // u = M^-1 V_j
+        NLGB_KR_T((k_gm_spmv<T><<<step_ctas, kGmThreads, 0, s>>>(v, w, j)));
+        k_gm_orth<<<step_ctas, kGmThreads, 0, s>>>(v1, w, j, 0, v.mpart);        // CGS2
+        k_gm_orth<<<step_ctas, kGmThreads, 0, s>>>(v, w, j, 1, v1.mpart);
+        k_gm_next<<<step_ctas, kGmThreads, 0, s>>>(v, w, j, P ? 0 : 1);
+        launches += 4;
       }
       k_gm_solve_y<<<1, 32, 0, s>>>(v);
       if (P) {
