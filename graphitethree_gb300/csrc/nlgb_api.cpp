@@ -3,11 +3,13 @@
 #include "../../include/nl_gb300.h"
 #include "nlgb_batch.h"
 #include "nlgb_internal.h"
+#include "nlgb_sell.h"
 
 #include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 using namespace nlgb;
@@ -18,6 +20,8 @@ struct nlgb_matrix_s {
   bool bound = false;
   cudaStream_t stream = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
+  std::mutex spmv_mu;
+  long long spmvs = 0;       // products asked for so far
   ~nlgb_matrix_s() {
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -67,6 +71,20 @@ struct Stage {
     return cudaSuccess;
   }
 };
+
+// y = A x, `count` products at a time.  From the fifth product on a large
+// matrix is multiplied in its sliced layout (nlgb_sell.cu): laying it out
+// costs about as much as four products, a user of one or two never pays it.
+cudaError_t spmv_many(nlgb_matrix M, const double* x, double* y, int count) {
+  bool sell = false;
+  {
+    std::lock_guard<std::mutex> lk(M->spmv_mu);
+    M->spmvs += count;
+    if (M->spmvs > 4) NLGB_CUDA_TRY(sell_prepare(M->A, &sell, M->stream));
+  }
+  for (int r = 0; r < count; ++r) NLGB_CUDA_TRY(sell ? sell_spmv64(M->A, x, y, M->stream) : spmv64(M->A, x, y, M->stream));
+  return cudaSuccess;
+}
 
 cudaError_t matrix_stream(nlgb_matrix M) {
   if (!M->stream) {
@@ -190,7 +208,7 @@ int nlgb_spmv(nlgb_matrix A, const double* x, double* y) {
   Stage sx, sy;
   if (sx.in(x, A->A.m, s, true) != cudaSuccess || sy.in(y, A->A.n, s, false) != cudaSuccess)
     return NLGB_E_DEVICE;
-  if (spmv64(A->A, sx.d, sy.d, s) != cudaSuccess) return NLGB_E_DEVICE;
+  if (spmv_many(A, sx.d, sy.d, 1) != cudaSuccess) return NLGB_E_DEVICE;
   if (sy.out(y, A->A.n, s) != cudaSuccess) return NLGB_E_DEVICE;
   if (cudaStreamSynchronize(s) != cudaSuccess) return fail(NLGB_E_DEVICE, cudaGetErrorString(cudaGetLastError()));
   return NLGB_OK;
@@ -207,9 +225,9 @@ int nlgb_spmv32(nlgb_matrix A, const float* x, float* y) {
 int nlgb_spmv_timed(nlgb_matrix A, const double* x, double* y, int reps, double* ms) {
   if (!A || reps <= 0) return fail(NLGB_E_INVALID, "nlgb_spmv_timed: bad arguments");
   cudaStream_t s = A->stream;
+  if (reps > 4 && spmv_many(A, x, y, 5) != cudaSuccess) return NLGB_E_DEVICE;   // (the layout outside the timing)
   if (cudaEventRecord(A->e0, s) != cudaSuccess) return NLGB_E_DEVICE;
-  for (int r = 0; r < reps; ++r)
-    if (spmv64(A->A, x, y, s) != cudaSuccess) return NLGB_E_DEVICE;
+  if (spmv_many(A, x, y, reps) != cudaSuccess) return NLGB_E_DEVICE;
   cudaEventRecord(A->e1, s);
   if (cudaEventSynchronize(A->e1) != cudaSuccess) return fail(NLGB_E_DEVICE, cudaGetErrorString(cudaGetLastError()));
   float t = 0.f;

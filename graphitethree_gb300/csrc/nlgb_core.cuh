@@ -117,6 +117,20 @@ inline __host__ __device__ int vec_tiles_for(int tile_rows) {
   return tile_rows >= 512 ? 1 : 512 / tile_rows;
 }
 
+// Row-sorted sliced layout of a matrix with two threads per row (nlgb_sell.cu);
+// va null: none.  A CTA processes its tile in passes of 128 rows; the rows of a
+// pass are sorted by length and dealt to the eight warps in slices of 16.
+// Element k of lane l of a slice (the k-th nonzero row_dot gives that lane) is
+// at (off + k) * 32 + l.
+struct SellView {
+  const uint2* shape;          // per slice: offset / 32, width
+  const unsigned char* len;    // per lane: its nonzeros
+  const unsigned char* perm;   // per row position: the row within the pass
+  const int* ci;
+  const double* va;
+  int passes;                  // per tile
+};
+
 // Everything a tile procedure needs about one system.
 struct SysView {
   int n;                 // rows (== columns)
@@ -145,6 +159,7 @@ struct SysView {
   SysState* st;
   const volatile int* abort_flag;   // host-mapped; nonzero -> stop
   long long budget;      // persistent kernel: iterations in this launch (> 0; else the launch's own)
+  SellView sell;
 };
 
 // ---------------------------------------------------------------------------

@@ -29,6 +29,19 @@ long long launch_count();
     }                                                                           \
   } while (0)
 
+// Row-sorted sliced copy of a matrix for the FP64 phase kernels of large
+// systems with two threads per row (nlgb_sell.cu), built on demand.
+struct SellLayout {
+  int state = 0;                    // 0 not built, 1 usable, -1 not worth it or no room
+  int tpr = 0, tile_rows = 0, passes = 0;
+  unsigned units = 0;               // slices' widths, summed (32 elements each)
+  uint2* shape = nullptr;
+  unsigned char* len = nullptr;
+  unsigned char* perm = nullptr;
+  int* ci = nullptr;
+  double* va = nullptr;
+};
+
 // A CRS matrix resident in GPU memory (int32 indices, FP64 values).
 struct DeviceCRS {
   int n = 0;               // rows
@@ -47,7 +60,15 @@ struct DeviceCRS {
   int tile_rows = 0;
   int max_row = 0;         // longest row (nnz)
   bool owns = true;        // false: a view sharing another matrix's arrays
+  SellLayout sell;
 };
+// Matrices below this have SpMVs of a few microseconds, bound by latency.
+constexpr long long kSellMinNnz = 1LL << 21;
+// Builds the sliced layout; *usable false: the CRS kernels run (other threads
+// per row, small or uneven matrix, no memory for the copy).
+cudaError_t sell_prepare(DeviceCRS& A, bool* usable, cudaStream_t s);
+void sell_free(SellLayout& L, cudaStream_t s, bool async);
+long long sell_bytes(const DeviceCRS& A);
 
 cudaError_t crs_upload(DeviceCRS& A, int n, int m, const int* rp, const int* ci,
                        const double* va, cudaStream_t s);

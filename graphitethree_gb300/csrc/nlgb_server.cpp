@@ -337,6 +337,8 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
   r->t_prepared = S->now();
   bool dfl = false;   // false also when the matrix is outside double-float's range: FP64 runs
   if (e == cudaSuccess && prec == NL_GB300_PRECISION_DOUBLE_FLOAT) e = crs_prepare_df(r->A, &dfl, s);
+  bool sell = false;  // the chunks' SpMV layout (false: CRS)
+  if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && !mixed && !dfl) e = sell_prepare(r->A, &sell, s);
   if (e == cudaSuccess) {
     // true footprint now known
     const size_t actual = (size_t)device_bytes(r->A) + (size_t)r->n_rhs * SystemSlot::bytes_for(r->n, r->A.tile_rows, mixed);

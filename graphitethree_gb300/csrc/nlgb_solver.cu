@@ -16,6 +16,7 @@
 #include "nlgb_core.cuh"
 #include "nlgb_internal.h"
 #include "nlgb_persist.h"
+#include "nlgb_sell.h"
 
 #include <algorithm>
 #include <chrono>
@@ -688,6 +689,7 @@ void crs_free(DeviceCRS& A) {
   cudaFree(A.rp); cudaFree(A.ci); cudaFree(A.va); cudaFree(A.va32);
   cudaFree(A.dinv); cudaFree(A.dinv32);
   cudaFree(A.vadf); cudaFree(A.dinvdf);
+  sell_free(A.sell, nullptr, false);
   A = DeviceCRS();
 }
 
@@ -696,6 +698,7 @@ void crs_free_async(DeviceCRS& A, cudaStream_t s) {
   for (void* p : {(void*)A.rp, (void*)A.ci, (void*)A.va, (void*)A.va32, (void*)A.dinv, (void*)A.dinv32,
                   (void*)A.vadf, (void*)A.dinvdf})
     if (p) cudaFreeAsync(p, s);
+  sell_free(A.sell, s, true);
   A = DeviceCRS();
 }
 
@@ -706,6 +709,7 @@ long long device_bytes(const DeviceCRS& A) {
   if (A.dinv32) b += (long long)A.n * 4;
   if (A.vadf) b += A.nnz * 8;
   if (A.dinvdf) b += (long long)A.n * 8;
+  b += sell_bytes(A);
   return b;
 }
 
@@ -968,6 +972,7 @@ static SysView make_view(DeviceCRS* A, int tile_rows, int n_tiles, double* b, do
   v.b = b; v.x = x; v.r = r; v.p = p; v.q = q;
   v.r32 = r32; v.p32 = p32; v.q32 = q32; v.c32 = c32;
   v.part = part; v.st = (SysState*)st; v.abort_flag = abort_flag;
+  v.sell = sell_view(*A);
   return v;
 }
 
@@ -977,6 +982,8 @@ static SysView make_view(DeviceCRS* A, int tile_rows, int n_tiles, double* b, do
 cudaError_t PcgSolver::add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysView* v, bool df,
                                       cudaGraphNode_t* loop_out) {
   const KernelSet ks = kernels_for(tpr_, df);
+  const void* spmv = df ? nullptr : sell_pq_kernel(*v);
+  if (!spmv) spmv = ks.spmv;
   cudaGraphConditionalHandle h;
   NLGB_CUDA_TRY(cudaGraphConditionalHandleCreate(&h, g, 1u, cudaGraphCondAssignDefault));
   void* a1[] = {v};
@@ -985,7 +992,7 @@ cudaError_t PcgSolver::add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysVie
   cudaGraphNode_t prev = nullptr;
   for (int u = 0; u < kUnrollPlain; ++u) {
     cudaGraphNode_t n1, n2, n3;
-    NLGB_CUDA_TRY(add_kernel(body, &n1, prev, ks.spmv, n_tiles_, kCTA, a1));
+    NLGB_CUDA_TRY(add_kernel(body, &n1, prev, spmv, n_tiles_, kCTA, a1));
     const int vg = (n_tiles_ + vec_tiles_for(tile_rows_) - 1) / vec_tiles_for(tile_rows_);
     NLGB_CUDA_TRY(add_kernel(body, &n2, n1, ks.update_xr, vg, kCTA, a1));
     NLGB_CUDA_TRY(add_kernel(body, &n3, n2, ks.update_p, vg, kCTA, a1));
@@ -1104,7 +1111,8 @@ cudaError_t ViewGraph::build(const SysView& v, bool mixed) {
   if (!e1_) NLGB_CUDA_TRY(cudaEventCreate(&e1_));
   view_ = v;
   mixed_ = mixed;
-  const KernelSet ks = kernels_for(v.tpr, !mixed && v.df != 0);
+  KernelSet ks = kernels_for(v.tpr, !mixed && v.df != 0);
+  if (!mixed && v.df == 0 && sell_pq_kernel(v)) ks.spmv = sell_pq_kernel(v);
   cudaGraph_t g;
   NLGB_CUDA_TRY(cudaGraphCreate(&g, 0));
   cudaGraphConditionalHandle h;
@@ -1184,7 +1192,8 @@ static bool same_view(const SysView& a, const SysView& b) {
          a.rp == b.rp && a.ci == b.ci && a.va == b.va && a.dinv == b.dinv && a.b == b.b &&
          a.x == b.x && a.r == b.r && a.p == b.p && a.q == b.q && a.part == b.part && a.st == b.st &&
          a.va32 == b.va32 && a.dinv32 == b.dinv32 && a.r32 == b.r32 && a.p32 == b.p32 &&
-         a.q32 == b.q32 && a.c32 == b.c32 && a.abort_flag == b.abort_flag;
+         a.q32 == b.q32 && a.c32 == b.c32 && a.abort_flag == b.abort_flag &&
+         a.sell.shape == b.sell.shape && a.sell.ci == b.sell.ci && a.sell.va == b.sell.va;
 }
 
 cudaError_t ViewGraph::prepare(const SysView& v, bool mixed) { return prepare(v, mixed, nullptr); }
@@ -1474,6 +1483,10 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
   cudaGraphExec_t* plain = df ? &df_exec_ : &plain_exec_;
   const int mode = mixed ? kPersistMixed : df ? kPersistDf : kPersistDouble;
   const bool persist = plan_[mode].usable && !eager_mode();
+  if (mode == kPersistDouble && !persist && !eager_mode()) {
+    bool sell = false;   // (false: the CRS kernels)
+    NLGB_CUDA_TRY(sell_prepare(*A_, &sell, stream_));
+  }
   if (mixed && !persist && !eager_mode() && !mixed_exec_) NLGB_CUDA_TRY(build_mixed_graph());
   if (!mixed && !persist && !eager_mode() && !*plain) NLGB_CUDA_TRY(build_plain_graph(df));
   SysState* h = (SysState*)st_host_;

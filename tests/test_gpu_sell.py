@@ -1,0 +1,60 @@
+"""Sliced layout of large matrices with two threads per row (csrc/nlgb_sell.cu):
+the products and the phase-kernel iterates are those of the CRS kernels bit for
+bit -- short last tiles and passes, tiles that are not a multiple of a pass,
+rows without entries -- and matrices it does not suit keep the CRS kernels."""
+import os
+
+import numpy as np
+import pytest
+
+from graphitethree_gb300 import meshes, solver, systems
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(M, rng):
+    x = rng.standard_normal(M.n)
+    x[:3] = [np.inf, -np.inf, np.nan]          # reach only their own rows
+    y = [M.spmv(x) for _ in range(7)]          # the layout is built by the fifth
+    assert all(np.array_equal(y[0], v, equal_nan=True) for v in y)
+
+
+@pytest.mark.parametrize("tile", [1024, 1088, 576, 4096])
+def test_lscm_products_and_iterates(gpu_ok, tile):
+    V, F = meshes.height_field(331, 307, 5)
+    M, b, _ = solver.build_lscm(V, F)
+    M.set_layout(2, tile)                       # (above 512 rows: phase kernels)
+    _check(M, np.random.default_rng(1))
+    os.environ["NLGB_EAGER_SOLVE"] = "1"
+    try:
+        want = M.solve(b, max_iter=60)
+    finally:
+        del os.environ["NLGB_EAGER_SOLVE"]
+    x, i = M.solve(b, max_iter=60)
+    assert np.array_equal(x, want[0]) and i.iterations == want[1].iterations
+    assert i.true_rel_residual == want[1].true_rel_residual
+    M.set_layout(2, 832)                        # another layout: rebuilt
+    _check(M, np.random.default_rng(2))
+
+
+@pytest.mark.parametrize("kind", ["empty_rows", "one_dense_row", "uneven"])
+def test_rows_of_any_length(gpu_ok, kind):
+    n = 170_000
+    rng = np.random.default_rng(7)
+    lens = rng.integers(10, 19, n)
+    if kind == "empty_rows":
+        lens[rng.random(n) < 0.05] = 0
+    elif kind == "one_dense_row":
+        lens[n // 2] = 700                      # more than 255 per lane
+    else:
+        lens[::64] = 300
+    rp = np.zeros(n + 1, np.int64)
+    rp[1:] = np.cumsum(lens)
+    i = np.repeat(np.arange(n), lens)
+    ci = (i + rng.integers(-300, 300, rp[-1])) % n
+    va = rng.standard_normal(rp[-1])
+    M = solver.Matrix(rp, ci, va)
+    M.set_layout(2, 1024)
+    x = rng.standard_normal(n)
+    y = [M.spmv(x) for _ in range(7)]
+    assert all(np.array_equal(y[0], v) for v in y)
