@@ -273,11 +273,31 @@ __device__ __forceinline__ A row_dot(const int* __restrict__ rp, const int* __re
   A sum = A(0);
   if (valid) {
     const int k0 = __ldg(rp + row), k1 = __ldg(rp + row + 1);
+    if constexpr (sizeof(VT) == 4) {
+      // three nonzeros in flight: FP32 rows are bound by latency (FP64 ones by
+      // the FP64 pipe, where this costs: 176 -> 180 us per iteration at
+      // 4.2 M rows; FP32 122.5 -> 119.3)
+      for (int k = k0 + lane; k < k1; k += 3 * T) {
+        int c[3];
+        VT av[3];
+        XT xc[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (k + u * T < k1) { c[u] = __ldg(ci + k + u * T); av[u] = __ldg(va + k + u * T); }
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (k + u * T < k1) xc[u] = kCoh ? __ldcg(x + c[u]) : __ldg(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (k + u * T < k1) sum = fma(A(av[u]), A(xc[u]), sum);
+      }
+    } else {
 #pragma unroll 2
-    for (int k = k0 + lane; k < k1; k += T) {
-      const int c = __ldg(ci + k);
-      const XT xc = kCoh ? __ldcg(x + c) : __ldg(x + c);
-      sum = fma(A(__ldg(va + k)), A(xc), sum);
+      for (int k = k0 + lane; k < k1; k += T) {
+        const int c = __ldg(ci + k);
+        const XT xc = kCoh ? __ldcg(x + c) : __ldg(x + c);
+        sum = fma(A(__ldg(va + k)), A(xc), sum);
+      }
     }
   }
   return subwarp_sum<T, A>(sum);
@@ -696,6 +716,20 @@ __device__ __forceinline__ double phase_true_rr(const SysView& s, int tile) {
   else return tile_true_rr<T, kCoh>(s, tile);
 }
 
+// float -> double, exact, on the integer pipe: GB300 converts on the FP64 pipe
+// (16 cycles of the SM per warp instruction).  Subnormals, infinities and NaN
+// take the conversion (all 2^32 inputs compared with it).  4.2 M rows, mixed:
+// 126 -> 122.5 us per iteration.
+__device__ __forceinline__ double to_double_int(float f) {
+  const unsigned b = __float_as_uint(f), e = (b >> 23) & 255u;
+  if (e - 1u < 254u)
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+  if ((b << 1) == 0u) return __hiloint2double((int)b, 0);
+  double d;
+  asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d) : "f"(f));   // volatile: not computed ahead of the branch
+  return d;
+}
+
 // ---------------------------------------------------------------------------
 // Mixed-precision tile procedures: FP32 matrix values and Krylov vectors,
 // FP64 for the outer residual, the solution update and the accumulation of
@@ -752,7 +786,7 @@ __device__ double tile_mx_spmv_pq(const SysView& s, int tile) {
   tile_rows_dot<T, float, float, float, kCoh>(s.rp, s.ci, s.va32, s.p32, lo, hi,
     [&](int row, float qv) {
       s.q32[row] = qv;
-      acc[0] += double(__ldcg(s.p32 + row) * qv);   // FP32 product, FP64 accumulation
+      acc[0] += to_double_int(__ldcg(s.p32 + row) * qv);   // FP32 product, FP64 accumulation
     });
   block_sum<1>(acc);
   return acc[0];
@@ -786,8 +820,8 @@ __device__ __forceinline__ void tile_mx_update_cr(const SysView& s, int tile, do
       const float zx = dv.x * rv.x, zy = dv.y * rv.y;
       rz32 = fmaf(zy, rv.y, zx * rv.x);
       rr32 = fmaf(rv.y, rv.y, rv.x * rv.x);
-      rz += double(rz32);
-      rr += double(rr32);
+      rz += to_double_int(rz32);
+      rr += to_double_int(rr32);
     },
     [&](int i) {
       s.c32[i] = fmaf(a, __ldcg(s.p32 + i), __ldcg(s.c32 + i));

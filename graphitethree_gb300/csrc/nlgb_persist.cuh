@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
       if (one_pass) {
         if constexpr (MODE == kPersistDf)
           reinterpret_cast<float2*>(red)[pos] = df::mac(make_float2(0.f, 0.f), ps[row], q);
-        else if constexpr (MODE == kPersistMixed) red[pos] = double(ps[row] * q);
+        else if constexpr (MODE == kPersistMixed) red[pos] = to_double_int(ps[row] * q);
         else red[pos] = fma(ps[row], q, 0.0);
       }
     };
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
           double acc = 0.0;
 #pragma unroll 1
           for (int r = sl * R + j; r < hi; r += RPP) {
-            if constexpr (MODE == kPersistMixed) acc += double(ps[r] * qs[r]);
+            if constexpr (MODE == kPersistMixed) acc += to_double_int(ps[r] * qs[r]);
             else acc = fma(ps[r], qs[r], acc);
           }
           red[chain_at(sl, j)] = acc;
@@ -758,8 +758,8 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
             const float al = float(alpha);
             rv.x = fmaf(-al, qv.x, rv.x); rv.y = fmaf(-al, qv.y, rv.y);
             zv.x = dv.x * rv.x; zv.y = dv.y * rv.y;
-            rz = double(fmaf(zv.y, rv.y, zv.x * rv.x));
-            rr = double(fmaf(rv.y, rv.y, rv.x * rv.x));
+            rz = to_double_int(fmaf(zv.y, rv.y, zv.x * rv.x));
+            rr = to_double_int(fmaf(rv.y, rv.y, rv.x * rv.x));
           } else {
             rv.x = fma(-alpha, qv.x, rv.x); rv.y = fma(-alpha, qv.y, rv.y);
             zv.x = dv.x * rv.x; zv.y = dv.y * rv.y;
