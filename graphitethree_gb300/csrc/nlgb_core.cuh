@@ -181,32 +181,43 @@ __device__ __forceinline__ double warp_sum(double v) {
 // bounds the phase kernels.  us per iteration: mixed 119.0 -> 115.2 at 4.2 M
 // rows and 57.3 -> 52.6 at 1.05 M, FP64 72.2 -> 68.7 at 1.05 M; 40 charts in
 // one batch 65.3 -> 56.8 ms.
+constexpr int kStagePad = 36;                    // doubles per staged warp: the pad keeps the banks apart
+constexpr int kStage = kWarps * kStagePad;
+
+// The tree over 256 staged values (value t of the CTA at stage_at(t)): the
+// total, in every lane of the warp that calls it.
+__device__ __forceinline__ int stage_at(int t) { return (t >> 5) * kStagePad + (t & 31); }
+__device__ __forceinline__ double stage_sum(const double* red) {
+  const int l = threadIdx.x & 31;
+  const double* r = red + (l >> 2) * kStagePad + (l & 3);
+  double a[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) a[j] = r[4 * j];
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int j = 0; j < h; ++j) a[j] += a[j + h];
+  double s = a[0];
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  double t = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < kWarps; ++i) t += __shfl_sync(0xffffffffu, s, 4 * i);
+  return t;
+}
+
 template <int K>
 __device__ __forceinline__ void block_sum(double (&v)[K]) {
   static_assert(K >= 1 && K <= 4, "block_sum: 1 to 4 values");
-  constexpr int kStride = 36;          // doubles per warp: the pad keeps the banks apart
-  __shared__ double red[K][kWarps * kStride];
+  __shared__ double red[K][kStage];
   __shared__ double tot[K];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   __syncthreads();   // protect red[] from a previous use
 #pragma unroll
-  for (int k = 0; k < K; ++k) red[k][w * kStride + l] = v[k];
+  for (int k = 0; k < K; ++k) red[k][stage_at(threadIdx.x)] = v[k];
   __syncthreads();
   if (w < K) {
-    const double* r = red[w] + (l >> 2) * kStride + (l & 3);
-    double a[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = r[4 * j];
-#pragma unroll
-    for (int h = 4; h > 0; h >>= 1)
-#pragma unroll
-      for (int j = 0; j < h; ++j) a[j] += a[j + h];
-    double s = a[0];
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    double t = 0.0;
-#pragma unroll 1
-    for (int i = 0; i < kWarps; ++i) t += __shfl_sync(0xffffffffu, s, 4 * i);
+    const double t = stage_sum(red[w]);
     if (K == 1) v[0] = t;
     else if (l == 0) tot[w] = t;
   }

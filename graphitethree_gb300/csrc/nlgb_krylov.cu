@@ -18,7 +18,8 @@
 // every dot product is a set of per-tile partials reduced in a fixed order
 // by one CTA (canon_reduce), and every scalar step runs on the device, so the
 // host only enqueues kernels and polls the status once per chunk (BiCGSTAB)
-// or per restart cycle (GMRES).  Kernels return at once when the system is no
+// or per restart cycle (GMRES).  BiCGSTAB's scalar steps run in the prologue
+// of the vector kernel that uses them.  Kernels return at once when the system is no
 // longer running, which makes overshooting a chunk harmless.
 #include "nlgb_core.cuh"
 #include "nlgb_internal.h"
@@ -34,7 +35,8 @@ constexpr int kMaxRestart = 64;     // GMRES(m): m <= 64
 constexpr int kChunk = 16;          // BiCGSTAB iterations between status polls
 
 struct KrState {
-  double rho, alpha, omega, beta;   // BiCGSTAB scalars
+  double alpha, omega, beta;        // BiCGSTAB scalars (beta: GMRES too)
+  double rho[2];                    // by the parity of the iteration that uses it
   double bnorm2, thresh2, rr, rr_true;
   double gnorm;                     // GMRES: |g_{j+1}| (residual estimate)
   long long iter, max_iter;
@@ -59,12 +61,14 @@ struct KrView {
   KrState* st;
   double* mpart;     // GMRES: per CTA of a step kernel m + 1 multi-dot partials, then its w.w
   int mstride;
-  int step_ctas, step_rows;   // GMRES: CTAs of the step kernels and rows of each
+  int step_ctas, step_rows;   // CTAs of the step kernels and rows of each
 };
 
 __device__ __forceinline__ bool running(const KrView& v) {
   return *((volatile int*)&v.st->status) == ST_RUNNING;
 }
+__device__ __forceinline__ int step_lo(const KrView& v) { return (int)blockIdx.x * v.step_rows; }
+__device__ __forceinline__ int step_hi(const KrView& v) { return min(v.n, ((int)blockIdx.x + 1) * v.step_rows); }
 __device__ __forceinline__ int lo_of(const KrView& v) { return blockIdx.x * v.tile_rows; }
 __device__ __forceinline__ int hi_of(const KrView& v) { return min(v.n, (int)(blockIdx.x + 1) * v.tile_rows); }
 
@@ -120,7 +124,7 @@ __global__ void k_bi_init_scalar(KrView v) {
   KrState* st = v.st;
   st->bnorm2 = o[0];
   st->rr = o[1];
-  st->rho = o[1];               // rh = r
+  st->rho[0] = o[1];            // rh = r
   st->alpha = st->omega = 1.0;
   st->beta = o[1];              // (rho / 1) (1 / 1); p = r on the first step
   if (!(o[0] > 0.0)) { st->zero_rhs = o[0] == 0.0; st->status = o[0] == 0.0 ? ST_CONVERGED : ST_BREAKDOWN; return; }
@@ -129,45 +133,131 @@ __global__ void k_bi_init_scalar(KrView v) {
   st->status = ST_RUNNING;
 }
 
-__global__ void __launch_bounds__(kCTA) k_bi_p(KrView v, BiVecs w) {
-  if (!running(v)) return;
-  const double beta = v.st->beta, omega = v.st->omega;
-  for (int i = lo_of(v) + threadIdx.x; i < hi_of(v); i += kCTA) {
-    const double pi = w.r[i] + beta * (w.p[i] - omega * w.v[i]);
-    w.p[i] = pi;
-    w.y[i] = v.dinv[i] * pi;
+// The vector kernels of the iteration (p, s, x/r): CTAs of 1024 threads, at
+// most one per SM.  Each reduces the partials of the SpMV or update before it
+// in its prologue and takes the scalar step itself; CTA 0 also writes the
+// scalars to the state, where only later kernels read them (rho alternates
+// between two slots; a status that turns while a CTA starts tells it to return,
+// which its own step would).  As one-CTA kernels between the vector kernels
+// the three scalar steps took 28 of the 128.6 us of an iteration on 1024 x 1024
+// unknowns; 120.5 us now (601 x 523: 81.0 -> 76.5).  One CTA per SM, because
+// the reduction costs each CTA about 1,000 cycles of the SM's FP64 pipe: three
+// CTAs of 512 threads 133.9 us, six of 256 140.5.
+constexpr int kBiThreads = 1024;
+constexpr int kBiQuarters = kBiThreads / kCTA;
+
+// The sums of the tiles' partials (canon_reduce's order), in every thread.
+template <int K>
+__device__ __forceinline__ void wide_sums(const KrView& v, int slot, double (&o)[K]) {
+  __shared__ double red[K][kStage];
+  __shared__ double tot[K];
+  const int t = threadIdx.x;
+  if (t < kCTA) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) o[k] = 0.0;
+#pragma unroll 8
+    for (int i = t; i < v.n_tiles; i += kCTA)
+#pragma unroll
+      for (int k = 0; k < K; ++k) o[k] += __ldcg(v.part + (size_t)i * kParts + slot + k);
+#pragma unroll
+    for (int k = 0; k < K; ++k) red[k][stage_at(t)] = o[k];
+  }
+  __syncthreads();
+  if (t < 32 * K) {
+    const double s = stage_sum(red[t >> 5]);
+    if ((t & 31) == 0) tot[t >> 5] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) o[k] = tot[k];
+}
+
+// load and body over rows lo, lo + stride, ... < hi: U rows of a thread in flight.
+template <int U, int N, typename Load, typename Body>
+__device__ __forceinline__ void rows_in_flight(int lo, int hi, int stride, Load&& load, Body&& body) {
+  for (int i = lo; i < hi; i += U * stride) {
+    double a[U][N];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * stride < hi) load(i + u * stride, a[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * stride < hi) body(i + u * stride, a[u]);
   }
 }
 
+// The same answer in every thread, also while CTA 0 writes the status.
+__device__ __forceinline__ bool stopped(const KrView& v) { return __syncthreads_or(!running(v)) != 0; }
+
+// The end of iteration it (its r.r and rh.r): the stopping tests and beta.
+__device__ __forceinline__ int bi_end(const KrView& v, long long it, double rr, double rho, bool write, double* beta) {
+  KrState* st = v.st;
+  const double alpha = st->alpha, omega = st->omega, rho0 = st->rho[it & 1];
+  int status = ST_RUNNING;
+  if (!(rr <= 1e300)) status = ST_BREAKDOWN;
+  else if (rr <= st->thresh2 * st->bnorm2) status = ST_CONVERGED;
+  else if (it + 1 >= st->max_iter) status = ST_MAX_ITER;
+  else if (!finite_nz(rho) || !finite_nz(omega)) status = ST_BREAKDOWN;
+  else *beta = (rho / rho0) * (alpha / omega);
+  if (write) {
+    st->iter = it + 1;
+    st->rr = rr;
+    if (status == ST_RUNNING) st->rho[(it + 1) & 1] = rho;
+    else st->status = status;
+  }
+  return status;
+}
+
+// fold: the end of iteration it - 1 first.
+__global__ void __launch_bounds__(kBiThreads, 1) k_bi_p(KrView v, BiVecs w, long long it, int fold) {
+  if (stopped(v)) return;
+  double beta, omega = v.st->omega;
+  if (fold) {
+    double o[2];
+    wide_sums<2>(v, 3, o);
+    if (bi_end(v, it - 1, o[0], o[1], blockIdx.x == 0 && threadIdx.x == 0, &beta) != ST_RUNNING) return;
+  } else {
+    beta = v.st->beta;
+  }
+  rows_in_flight<4, 4>(step_lo(v) + (int)threadIdx.x, step_hi(v), kBiThreads,
+    [&](int i, double (&a)[4]) { a[0] = w.r[i]; a[1] = w.p[i]; a[2] = w.v[i]; a[3] = __ldg(v.dinv + i); },
+    [&](int i, double (&a)[4]) {
+      const double pi = a[0] + beta * (a[1] - omega * a[2]);
+      w.p[i] = pi;
+      w.y[i] = a[3] * pi;
+    });
+}
+
 template <int T>
-__global__ void __launch_bounds__(kCTA) k_bi_v(KrView v, BiVecs w) {
+__global__ void __launch_bounds__(kCTA, 8) k_bi_v(KrView v, BiVecs w) {
   if (!running(v)) return;
   double a[1] = {0.0};
   tile_spmv<T>(v, w.y, [&](int i, double q) { w.v[i] = q; a[0] = fma(w.rh[i], q, a[0]); });
   put_tile<1>(v, 0, a);
 }
 
-__global__ void k_bi_alpha(KrView v) {
-  if (!running(v)) return;
+__global__ void __launch_bounds__(kBiThreads, 1) k_bi_s(KrView v, BiVecs w, long long it) {
+  if (stopped(v)) return;
   double o[1];
-  sums<1>(v, 0, o);
-  if (threadIdx.x != 0) return;
-  if (!finite_nz(o[0])) { v.st->status = ST_BREAKDOWN; return; }
-  v.st->alpha = v.st->rho / o[0];
-}
-
-__global__ void __launch_bounds__(kCTA) k_bi_s(KrView v, BiVecs w) {
-  if (!running(v)) return;
-  const double alpha = v.st->alpha;
-  for (int i = lo_of(v) + threadIdx.x; i < hi_of(v); i += kCTA) {
-    const double si = w.r[i] - alpha * w.v[i];
-    w.r[i] = si;                      // r now holds s
-    w.z[i] = v.dinv[i] * si;
+  wide_sums<1>(v, 0, o);
+  const bool ok = finite_nz(o[0]);
+  const double alpha = v.st->rho[it & 1] / o[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (ok) v.st->alpha = alpha;
+    else v.st->status = ST_BREAKDOWN;
   }
+  if (!ok) return;
+  rows_in_flight<4, 3>(step_lo(v) + (int)threadIdx.x, step_hi(v), kBiThreads,
+    [&](int i, double (&a)[3]) { a[0] = w.r[i]; a[1] = w.v[i]; a[2] = __ldg(v.dinv + i); },
+    [&](int i, double (&a)[3]) {
+      const double si = a[0] - alpha * a[1];
+      w.r[i] = si;                      // r now holds s
+      w.z[i] = a[2] * si;
+    });
 }
 
 template <int T>
-__global__ void __launch_bounds__(kCTA) k_bi_t(KrView v, BiVecs w) {
+__global__ void __launch_bounds__(kCTA, 8) k_bi_t(KrView v, BiVecs w) {
   if (!running(v)) return;
   double a[2] = {0.0, 0.0};
   tile_spmv<T>(v, w.z, [&](int i, double q) {
@@ -178,42 +268,46 @@ __global__ void __launch_bounds__(kCTA) k_bi_t(KrView v, BiVecs w) {
   put_tile<2>(v, 1, a);
 }
 
-__global__ void k_bi_omega(KrView v) {
+// Each quarter of the CTA (256 threads, a barrier of its own) takes a tile.
+__global__ void __launch_bounds__(kBiThreads, 1) k_bi_xr(KrView v, BiVecs w) {
   if (!running(v)) return;
+  __shared__ double red[kBiQuarters][2][kStage];
   double o[2];
-  sums<2>(v, 1, o);
-  if (threadIdx.x != 0) return;
-  v.st->omega = o[1] > 0.0 ? o[0] / o[1] : 0.0;
-}
-
-__global__ void __launch_bounds__(kCTA) k_bi_xr(KrView v, BiVecs w) {
-  if (!running(v)) return;
-  const double alpha = v.st->alpha, omega = v.st->omega;
-  double a[2] = {0.0, 0.0};
-  for (int i = lo_of(v) + threadIdx.x; i < hi_of(v); i += kCTA) {
-    w.x[i] += alpha * w.y[i] + omega * w.z[i];
-    const double ri = w.r[i] - omega * w.t[i];
-    w.r[i] = ri;
-    a[0] = fma(ri, ri, a[0]);
-    a[1] = fma(w.rh[i], ri, a[1]);
+  wide_sums<2>(v, 1, o);
+  const double alpha = v.st->alpha, omega = o[1] > 0.0 ? o[0] / o[1] : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) v.st->omega = omega;
+  const int qd = threadIdx.x / kCTA, t = threadIdx.x % kCTA;
+  for (int tile = (int)blockIdx.x * kBiQuarters + qd; tile < v.n_tiles; tile += (int)gridDim.x * kBiQuarters) {
+    const int lo = tile * v.tile_rows, hi = min(v.n, lo + v.tile_rows);
+    double rr = 0.0, rhr = 0.0;
+    rows_in_flight<2, 6>(lo + t, hi, kCTA,
+      [&](int i, double (&a)[6]) {
+        a[0] = w.x[i]; a[1] = w.y[i]; a[2] = w.z[i]; a[3] = w.r[i]; a[4] = w.t[i]; a[5] = w.rh[i];
+      },
+      [&](int i, double (&a)[6]) {
+        w.x[i] = a[0] + (alpha * a[1] + omega * a[2]);
+        const double ri = a[3] - omega * a[4];
+        w.r[i] = ri;
+        rr = fma(ri, ri, rr);
+        rhr = fma(a[5], ri, rhr);
+      });
+    red[qd][0][stage_at(t)] = rr;
+    red[qd][1][stage_at(t)] = rhr;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(kCTA) : "memory");
+    if (t < 64) {
+      const double s = stage_sum(red[qd][t >> 5]);
+      if ((t & 31) == 0) v.part[(size_t)tile * kParts + 3 + (t >> 5)] = s;
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(kCTA) : "memory");   // red[qd] is free again
   }
-  put_tile<2>(v, 3, a);
 }
 
-__global__ void k_bi_end(KrView v) {
+// Before a poll: the end of iteration it, for the host and for a k_bi_p without it.
+__global__ void __launch_bounds__(kBiThreads, 1) k_bi_end(KrView v, long long it) {
   if (!running(v)) return;
-  double o[2];
-  sums<2>(v, 3, o);
-  if (threadIdx.x != 0) return;
-  KrState* st = v.st;
-  st->iter += 1;
-  st->rr = o[0];
-  if (!(o[0] <= 1e300)) { st->status = ST_BREAKDOWN; return; }
-  if (o[0] <= st->thresh2 * st->bnorm2) { st->status = ST_CONVERGED; return; }
-  if (st->iter >= st->max_iter) { st->status = ST_MAX_ITER; return; }
-  if (!finite_nz(o[1]) || !finite_nz(st->omega)) { st->status = ST_BREAKDOWN; return; }
-  st->beta = (o[1] / st->rho) * (st->alpha / st->omega);
-  st->rho = o[1];
+  double o[2], beta = 0.0;
+  wide_sums<2>(v, 3, o);
+  if (threadIdx.x == 0 && bi_end(v, it, o[0], o[1], true, &beta) == ST_RUNNING) v.st->beta = beta;
 }
 
 // True residual ||b - A x||^2 of the returned x (and x = 0 when b = 0).
@@ -319,8 +413,6 @@ __device__ __forceinline__ double warp_sum8(const double (&a)[8]) {
   return s;
 }
 
-__device__ __forceinline__ int step_lo(const KrView& v) { return (int)blockIdx.x * v.step_rows; }
-__device__ __forceinline__ int step_hi(const KrView& v) { return min(v.n, ((int)blockIdx.x + 1) * v.step_rows); }
 __device__ __forceinline__ bool step_active(const KrView& v, int j) { return *((volatile int*)&v.st->act[j]) != 0; }
 
 // This CTA's partials of V_i . w, i <= j (every thread calls it).
@@ -581,7 +673,7 @@ cudaError_t krylov_solve(const DeviceCRS& A, const double* dinv, const double* b
   cudaError_t e = cudaMallocAsync(&part, sizeof(double) * (size_t)n_tiles * kParts, s);
   if (e == cudaSuccess) e = cudaMallocAsync(&st, sizeof(KrState), s);
   double* mpart = nullptr;
-  // GMRES step kernels: one CTA per SM (at least 256 rows each), two areas of
+  // step kernels (and BiCGSTAB's p and s): one CTA per SM (at least 256 rows each), two areas of
   // partials (a kernel reads one and writes the other)
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -612,23 +704,24 @@ cudaError_t krylov_solve(const DeviceCRS& A, const double* dinv, const double* b
     NLGB_KR_T((k_bi_init<T><<<n_tiles, kCTA, 0, s>>>(v, w)));
     k_bi_init_scalar<<<1, kCTA, 0, s>>>(v);
     launches += 2;
+    const int xr_ctas = std::min(sms, (n_tiles + kBiQuarters - 1) / kBiQuarters);
     int status = ST_RUNNING;
+    long long it = 0;
     while (e == cudaSuccess && status == ST_RUNNING) {
-      for (int c = 0; c < kChunk; ++c) {
+      for (int c = 0; c < kChunk; ++c, ++it) {
         // (with a general preconditioner dinv is all ones: y = p, z = s,
         // then y = M^-1 p, z = M^-1 s)
-        k_bi_p<<<n_tiles, kCTA, 0, s>>>(v, w);
+        k_bi_p<<<step_ctas, kBiThreads, 0, s>>>(v, w, it, c > 0);
         if (P && e == cudaSuccess) e = P->apply(w.p, w.y, s);
         NLGB_KR_T((k_bi_v<T><<<n_tiles, kCTA, 0, s>>>(v, w)));
-        k_bi_alpha<<<1, kCTA, 0, s>>>(v);
-        k_bi_s<<<n_tiles, kCTA, 0, s>>>(v, w);
+        k_bi_s<<<step_ctas, kBiThreads, 0, s>>>(v, w, it);
         if (P && e == cudaSuccess) e = P->apply(w.r, w.z, s);
         NLGB_KR_T((k_bi_t<T><<<n_tiles, kCTA, 0, s>>>(v, w)));
-        k_bi_omega<<<1, kCTA, 0, s>>>(v);
-        k_bi_xr<<<n_tiles, kCTA, 0, s>>>(v, w);
-        k_bi_end<<<1, kCTA, 0, s>>>(v);
-        launches += 8;
+        k_bi_xr<<<xr_ctas, kBiThreads, 0, s>>>(v, w);
+        launches += 5;
       }
+      k_bi_end<<<1, kBiThreads, 0, s>>>(v, it - 1);
+      launches += 1;
       if (e == cudaSuccess) e = cudaGetLastError();
       if (e == cudaSuccess) e = poll(&status);
     }
