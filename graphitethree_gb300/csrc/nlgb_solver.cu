@@ -247,7 +247,8 @@ __global__ void k_guard(SysView s, cudaGraphConditionalHandle h, int need_mode, 
 }
 
 // Before a resumable chunk of at most `iters` iterations: pause point and a
-// matching cap on while-body passes.
+// matching cap on while-body passes.  unroll: iterations every pass makes
+// (a mixed pass ends early at a reliable update: at least one).
 __global__ void k_chunk_start(SysState* st, long long iters, int unroll) {
   st->iter_stop = st->iter + iters;
   st->guard_cap = st->guard + iters / unroll + 4;
@@ -1133,7 +1134,7 @@ cudaError_t ViewGraph::build(const SysView& v, bool mixed) {
   cudaGraphNode_t n_start, n_loop, n_fin, n_end, prev = nullptr, n_first = nullptr;
   cudaGraph_t body;
   ChunkMirror* mirror = mirror_;
-  int unroll = kUnrollPlain;
+  int unroll = mixed ? 1 : kUnrollPlain;
   void* am[] = {&st, &mirror, &unroll};
   if (mirror_) NLGB_CUDA_TRY(add_kernel(g, &n_first, nullptr, (const void*)k_chunk_start_m, 1, 1, am));
   if (!mixed) {
@@ -1221,7 +1222,7 @@ cudaError_t ViewGraph::prepare(const SysView& v, bool mixed, ChunkMirror* m, cud
 cudaError_t ViewGraph::launch(cudaStream_t s) {
   if (!mirror_) return cudaErrorInvalidValue;
   if (eager_mode()) {
-    k_chunk_start_m<<<1, 1, 0, s>>>(view_.st, mirror_, kUnrollPlain);
+    k_chunk_start_m<<<1, 1, 0, s>>>(view_.st, mirror_, mixed_ ? 1 : kUnrollPlain);
     NLGB_CUDA_TRY(cudaGetLastError());
     const long long budget = *reinterpret_cast<volatile long long*>(&mirror_->budget);
     return run_eager(s, budget > 0 ? budget : 1);
@@ -1246,7 +1247,7 @@ cudaError_t ViewGraph::run(const SysView& v, long long iters, cudaStream_t s, fl
   if (!e0_) NLGB_CUDA_TRY(cudaEventCreate(&e0_));
   if (!e1_) NLGB_CUDA_TRY(cudaEventCreate(&e1_));
   NLGB_CUDA_TRY(cudaEventRecord(e0_, s));
-  k_chunk_start<<<1, 1, 0, s>>>(v.st, std::max(1LL, iters), kUnrollPlain);
+  k_chunk_start<<<1, 1, 0, s>>>(v.st, std::max(1LL, iters), mixed ? 1 : kUnrollPlain);
   NLGB_CUDA_TRY(cudaGetLastError());
   if (eager_mode()) {
     NLGB_CUDA_TRY(run_eager(s, iters));

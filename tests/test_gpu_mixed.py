@@ -72,3 +72,15 @@ def test_products_out_of_the_normal_range(gpu_ok, scale):
     M = _band(1500, 2, 1.0)
     b = np.sin(np.arange(1500)) * scale
     _same(M.solve(b, precision="mixed", max_iter=40), _eager(M, b, max_iter=40))
+
+
+def test_chunk_with_many_updates(gpu_ok):
+    """A chunk in which many passes end early: an update every few iterations."""
+    sq = systems.fairing_system(1300, 1000, seed=3, n_rhs=1)
+    x, info = solver.Matrix(sq.rp, sq.ci, sq.va).solve(sq.rhs[0], precision="mixed", inner_eps=0.5)
+    srv = solver.Server(precision="mixed", inner_eps=0.5, epoch_ms=20.0)   # the second chunk: about 300 iterations
+    xs, infos, _ = srv.wait(srv.submit_square(sq))
+    srv.close()
+    assert infos[0].status == info.status == "converged"
+    assert infos[0].refinement_steps > 20
+    _same((xs[0], infos[0]), (x, info))
