@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "nlgb_core.cuh"
+#include "nlgb_internal.h"
 
 namespace nlgb {
 
@@ -145,8 +146,20 @@ class ViewGraph {
   cudaError_t prepare(const SysView& v, bool mixed, ChunkMirror* m, cudaStream_t upload = nullptr);
   cudaError_t launch(cudaStream_t s);
   void account(long long iters_before, long long iters_after);
+  // The persistent kernel (nlgb_persist.cuh) as an executor of the chunks:
+  // tables of the system's matrix, and an exchange area of persist_bytes(),
+  // zeroed when the system started.  Both outlive the chunks.  The chunks
+  // run there while persist(true) holds and the system fits.
+  void persist_bind(const PersistTables& t, void* exch, const SysView& v, bool mixed);
+  int persist_ctas(bool mixed) const { return plan_[mixed ? 1 : 0].usable ? plan_[mixed ? 1 : 0].grid : 0; }
+  void persist(bool on) { persist_ = on; }
 
  private:
+  bool persistent() const { return persist_ && plan_[mixed_ ? 1 : 0].usable; }
+  PersistPlan plan_[2];        // FP64 or double-float; mixed
+  PersistLayout lay_;
+  void* exch_ = nullptr;
+  bool persist_ = false;
   cudaError_t build(const SysView& v, bool mixed);
   cudaError_t run_eager(cudaStream_t s, long long iters);
   SysView view_{};
@@ -163,6 +176,12 @@ class ViewGraph {
 // switched to FP64 PCG from its current x (stage 0, iteration count kept);
 // stream-ordered, before the system's next chunk.
 cudaError_t chunk_fallback_fp64(SysState* st, cudaStream_t s);
+
+// Queues a chunk of a system on the persistent kernel: what a chunk graph
+// does (see nlgb_solver.cu), with `rounds` launches of at most `iters`
+// iterations each (a mixed system ends one at every reliable update).
+cudaError_t persist_chunk(const SysView& v, const PersistPlan& plan, const PersistLayout& lay, void* exch,
+                          bool mixed, long long iters, int rounds, cudaStream_t s);
 
 // Launches the persistent kernel over a set of resident systems.  Each
 // system's SysState (device) must be initialised by the caller (status

@@ -151,17 +151,21 @@ class PersistTables {
   PersistTables(const PersistTables&) = delete;
   PersistTables& operator=(const PersistTables&) = delete;
   // Lays a matrix out for the persistent kernel; usable() tells whether it
-  // fits (sizes and halos).
-  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s);
+  // fits (sizes and halos).  shared: for a system that shares the GPU with
+  // others (fewer CTAs, more tiles on each).
+  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared = false);
   bool usable() const { return lay_.ctas > 0; }
   const PersistLayout& layout() const { return lay_; }
   PersistPlan plan(int tile_rows, int tpr, int mode) const;
+  size_t bytes() const { return bytes_; }
   void release();
+  void release(cudaStream_t s);          // stream-ordered
 
  private:
   PersistLayout lay_;
   bool cluster_ = false;
   void* mem_ = nullptr;
+  size_t bytes_ = 0;
 };
 
 // Plain FP64, double-float, or mixed FP32/FP64-refined Jacobi-PCG on one

@@ -22,6 +22,7 @@
 #include "../../include/nl_gb300.h"
 #include "nlgb_batch.h"
 #include "nlgb_internal.h"
+#include "nlgb_persist.h"
 
 #include <algorithm>
 #include <atomic>
@@ -88,6 +89,8 @@ struct Req {
   // in flight, whether it runs the mixed iteration now, a pending switch to
   // FP64, and the measured time per iteration (ms; < 0 unknown)
   std::vector<std::unique_ptr<ViewGraph>> graphs;
+  PersistTables tables;              // of A, for chunks on the persistent kernel
+  void* exch = nullptr;              // their exchange areas, one per system
   std::vector<int> mirror_idx;       // per system, its ChunkMirror in the server's pool
   std::vector<int> running, mixed_now, need_fallback;
   std::vector<double> ms_per_iter;
@@ -269,6 +272,31 @@ SolveParams params_of(const nlgb_server_s* S, const Req& r, int precision) {
   return p;
 }
 
+size_t exchange_bytes(const Req& r) {
+  return (persist_bytes(r.n, r.slots.empty() ? 1 : r.slots[0].view.n_tiles) + 255) & ~(size_t)255;
+}
+
+// The tables and exchange areas for chunks on the persistent kernel, where
+// the request's systems fit it and the budget has room for them.
+cudaError_t persist_tables(nlgb_server_s* S, Req* r, cudaStream_t s) {
+  const SysView& v = r->slots[0].view;
+  cudaError_t e = r->tables.build(r->A, v.tile_rows, v.n_tiles, s, true);
+  if (e != cudaSuccess || !r->tables.usable()) return e;
+  const size_t exch = exchange_bytes(*r) * (size_t)r->n_rhs, extra = r->tables.bytes() + exch;
+  {
+    std::lock_guard<std::mutex> lk(S->mu);
+    if (S->used + extra > S->cfg.hbm_budget_bytes) {
+      r->tables.release(s);
+      return cudaSuccess;
+    }
+    add_used_locked(S, (long long)extra);
+  }
+  r->bytes += extra;
+  e = cudaMallocAsync(&r->exch, exch, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(r->exch, 0, exch, s);
+  return e;
+}
+
 // Upload / assemble a request on stream `s` and start its systems.
 // df_slots: the slots run the double-float iteration in the persistent
 // kernel (x packed as float pairs); the serial worker keeps FP64 slots and
@@ -356,6 +384,8 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
       e = r->slots[k].start(bk, xk, prm, s);
     }
   }
+  if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && S->cfg.schedule == NLGB_SCHEDULE_SRPT)
+    e = persist_tables(S, r, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   // host inputs are no longer needed
   std::vector<int>().swap(r->rp); std::vector<int>().swap(r->ci); std::vector<double>().swap(r->va);
@@ -403,6 +433,9 @@ void release(nlgb_server_s* S, Req* r, cudaStream_t s) {
     for (int i : r->mirror_idx) S->mirror_free.push_back(i);
     r->mirror_idx.clear();
   }
+  r->tables.release(s);
+  if (r->exch) cudaFreeAsync(r->exch, s);
+  r->exch = nullptr;
   crs_free_async(r->A, s);
   if (r->d_rhs) cudaFreeAsync(r->d_rhs, s);
   r->d_rhs = nullptr;
@@ -632,6 +665,11 @@ void admitter(nlgb_server_s* S) {
           ChunkMirror* m = &S->mirrors[pick->mirror_idx[k]];
           m->budget = 0;
           pick->graphs[k].reset(new ViewGraph());
+          if (pick->exch) {
+            pick->graphs[k]->persist_bind(pick->tables, static_cast<char*>(pick->exch) + (size_t)k * exchange_bytes(*pick),
+                                          pick->slots[k].view, pick->slots[k].mixed);
+            pick->graphs[k]->persist(true);
+          }
           ok = pick->graphs[k]->prepare(pick->slots[k].view, pick->slots[k].mixed, m, su) == cudaSuccess;
         }
         if (ok) ok = cudaStreamSynchronize(su) == cudaSuccess;
@@ -905,8 +943,8 @@ void worker_batched(nlgb_server_s* S) {
 }
 
 // SRPT executor of the BATCHED server: `streams` CUDA streams, each running
-// one system at a time as a chunk of CUDA-graph iterations (ViewGraph) of
-// about epoch_ms.  Whenever a stream is free it takes the system with the
+// one system at a time as a chunk of about epoch_ms (ViewGraph: on the
+// persistent single-system kernel or as CUDA-graph iterations).  Whenever a stream is free it takes the system with the
 // least estimated remaining work that is not running already (a new system
 // first, for a probe of kProbeIters iterations).  A system's chunks run one
 // after the other (the next one is queued only after the previous one was
@@ -973,12 +1011,23 @@ void worker_streams(nlgb_server_s* S) {
     long long iter_before = 0;
     double t_free = -1.0;       // server clock when the lane's last chunk was seen done (tracing)
     long long ctas = 0;         // CTAs per phase kernel of the running system
+    int sms = 0;                // SMs of a chunk on the persistent kernel (0: a graph)
   };
   std::vector<Lane> lanes((size_t)ns);
   // CTA budget of the chunks in flight (config.chunk_cta_budget; 0: none)
   const long long cta_cap = S->cfg.chunk_cta_budget < 0 ? phase_resident_slots()
                                                         : (long long)S->cfg.chunk_cta_budget;
   long long running_ctas = 0;
+  // Chunks run on the persistent kernel while every unfinished system fits it:
+  // 8 to 10 us per iteration of 2k to 33k rows, against 30 us on 16 lanes of
+  // graphs, and no graph to instantiate (which also held a burst's other
+  // requests back for up to 50 ms behind the first one's chunk).  24 requests
+  // of 1k to 20k vertices at once: 222 -> 73 ms, their median latency 72 ->
+  // 10 ms.  A chunk's CTAs each need a whole SM and wait for one another, so
+  // the chunks in flight share out the SMs, and they never run beside graph
+  // chunks, whose kernels would leave no SM empty.
+  int n_sm = 0, sms_busy = 0, graphs_busy = 0;
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, S->device);
   auto ctas_of = [](const Req* r) {
     return ((long long)r->A.n + r->A.tile_rows - 1) / std::max(1, r->A.tile_rows);
   };
@@ -1071,6 +1120,9 @@ void worker_streams(nlgb_server_s* S) {
     l.m = nullptr;
     running_ctas -= l.ctas;
     l.ctas = 0;
+    sms_busy -= l.sms;
+    graphs_busy -= l.sms == 0 ? 1 : 0;
+    l.sms = 0;
     busy_change(-1);
   };
   // requests whose systems are all done go to the completion threads
@@ -1141,8 +1193,13 @@ void worker_streams(nlgb_server_s* S) {
     }
     // give every free lane the least-work system that is not running
     cudaError_t e = cudaSuccess;
+    bool persist = n_busy < ns;
+    for (Req* r : S->active)
+      for (int k = 0; persist && k < r->n_rhs; ++k)
+        persist = r->sys_done[k] || r->graphs[k]->persist_ctas(r->mixed_now[k] != 0) > 0;
     for (Lane& l : lanes) {
       if (l.r) continue;
+      if (persist ? graphs_busy > 0 : sms_busy > 0) break;   // the other kind's chunks end first
       Req* best = nullptr;
       int bk = -1;
       double bkey = 0.0;
@@ -1152,6 +1209,8 @@ void worker_streams(nlgb_server_s* S) {
           // within the CTA budget (a system that does not fit waits; the
           // least-work one that fits runs meanwhile)
           if (cta_cap > 0 && running_ctas > 0 && running_ctas + ctas_of(r) > cta_cap) continue;
+          if (persist && sms_busy > 0 &&
+              sms_busy + r->graphs[k]->persist_ctas(r->mixed_now[k] != 0) > n_sm) continue;
           const double key = r->est_left[k] < 0.0 ? -1.0 : r->est_left[k] * r->iter_cost;
           if (!best || key < bkey || (key == bkey && r->id < best->id)) { best = r; bk = k; bkey = key; }
         }
@@ -1176,6 +1235,10 @@ void worker_streams(nlgb_server_s* S) {
       best->running[bk] = 1;
       l.ctas = ctas_of(best);
       running_ctas += l.ctas;
+      l.sms = persist ? best->graphs[bk]->persist_ctas(best->mixed_now[bk] != 0) : 0;
+      sms_busy += l.sms;
+      graphs_busy += l.sms == 0 ? 1 : 0;
+      best->graphs[bk]->persist(persist);
       // the budget is read by the chunk's first kernel
       __atomic_store_n(&m->budget, iters, __ATOMIC_RELEASE);
       const double tr = S->now();

@@ -261,6 +261,12 @@ __global__ void k_chunk_end(SysState* st) {
   if (st->status != ST_RUNNING) st->stage = 3;
 }
 
+// The same after a chunk on the persistent kernel, whose waits are bounded.
+__global__ void k_persist_end(SysState* st, const int* err) {
+  if (*err) st->status = ST_DEVICE_ERR;
+  if (st->status != ST_RUNNING) st->stage = 3;
+}
+
 __device__ __forceinline__ unsigned long long chunk_clock_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1108,6 +1114,10 @@ static bool eager_mode();
 // A chunk pauses on whole passes of 4 iterations (guard), the system stays
 // running; the server continues it with another chunk later.
 // ---------------------------------------------------------------------------
+// Reliable updates in a mixed system's chunk on the persistent kernel, which
+// ends a launch at each (a solve has about ten).
+constexpr int kPersistChunkRounds = 6;
+
 ViewGraph::~ViewGraph() {
   if (exec_) cudaGraphExecDestroy(exec_);
   if (e0_) cudaEventDestroy(e0_);
@@ -1211,6 +1221,16 @@ static bool same_view(const SysView& a, const SysView& b) {
 cudaError_t ViewGraph::prepare(const SysView& v, bool mixed) { return prepare(v, mixed, nullptr); }
 
 cudaError_t ViewGraph::prepare(const SysView& v, bool mixed, ChunkMirror* m, cudaStream_t upload) {
+  if (persist_ && plan_[mixed ? 1 : 0].usable) {
+    if (exec_ && (mixed != mixed_ || m != mirror_ || !same_view(v, view_))) {   // not this system's any more
+      cudaGraphExecDestroy(exec_);
+      exec_ = nullptr;
+    }
+    view_ = v;
+    mixed_ = mixed;
+    mirror_ = m;
+    return cudaSuccess;
+  }
   if (!exec_ || mixed != mixed_ || m != mirror_ || !same_view(v, view_)) {
     mirror_ = m;
     NLGB_CUDA_TRY(build(v, mixed));
@@ -1227,11 +1247,28 @@ cudaError_t ViewGraph::launch(cudaStream_t s) {
     const long long budget = *reinterpret_cast<volatile long long*>(&mirror_->budget);
     return run_eager(s, budget > 0 ? budget : 1);
   }
+  if (persistent()) {
+    const long long budget = *reinterpret_cast<volatile long long*>(&mirror_->budget);
+    k_chunk_start_m<<<1, 1, 0, s>>>(view_.st, mirror_, kUnrollPlain);
+    NLGB_CUDA_TRY(persist_chunk(view_, plan_[mixed_ ? 1 : 0], lay_, exch_, mixed_, std::max(1LL, budget),
+                                mixed_ ? kPersistChunkRounds : 1, s));
+    k_chunk_end_m<<<1, 32, 0, s>>>(view_.st, mirror_);
+    count_launches(2);
+    return cudaGetLastError();
+  }
   if (!exec_) return cudaErrorInvalidValue;
   return cudaGraphLaunch(exec_, s);
 }
 
+void ViewGraph::persist_bind(const PersistTables& t, void* exch, const SysView& v, bool mixed) {
+  lay_ = t.layout();
+  exch_ = exch;
+  plan_[0] = t.plan(v.tile_rows, v.tpr, v.df ? kPersistDf : kPersistDouble);   // (a mixed system may end in FP64)
+  if (mixed) plan_[1] = t.plan(v.tile_rows, v.tpr, kPersistMixed);
+}
+
 void ViewGraph::account(long long iters_before, long long iters_after) {
+  if (persistent()) return;   // launch() counted
   if (eager_counted_) {   // run_eager counted its launches (plus the chunk start)
     eager_counted_ = false;
     count_launches(1);
@@ -1257,6 +1294,47 @@ cudaError_t ViewGraph::run(const SysView& v, long long iters, cudaStream_t s, fl
   NLGB_CUDA_TRY(cudaEventRecord(e1_, s));
   pending_ = true;
   ms_ = ms;
+  return cudaSuccess;
+}
+
+cudaError_t persist_chunk(const SysView& v, const PersistPlan& plan, const PersistLayout& lay, void* exch,
+                          bool mixed, long long iters, int rounds, cudaStream_t s) {
+  PersistArgs pa;
+  std::memset(&pa, 0, sizeof(pa));
+  pa.s = v;
+  persist_bind(pa, exch);
+  pa.lay = lay;
+  pa.iters = iters;
+  const KernelSet ks = kernels_for(v.tpr, !mixed && v.df != 0);
+  const int vg = (v.n_tiles + vec_tiles_for(v.tile_rows) - 1) / vec_tiles_for(v.tile_rows);
+  SysState* st = v.st;
+  void* a1[] = {&pa.s};
+  void* ast[] = {&st};
+  long long launched = 0;
+  auto go = [&](const void* fn, int grid, int block, void** args) {
+    ++launched;
+    return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, s);
+  };
+  if (mixed) {
+    NLGB_CUDA_TRY(go(ks.mx_outer, v.n_tiles, kCTA, a1));
+    NLGB_CUDA_TRY(go((const void*)k_mark_started, 1, 1, ast));
+  } else {
+    NLGB_CUDA_TRY(go(ks.init_chunk, v.n_tiles, kCTA, a1));
+    NLGB_CUDA_TRY(go(ks.resume_p, vg, kCTA, a1));
+    NLGB_CUDA_TRY(go((const void*)k_resume_mark, 1, 1, ast));
+  }
+  for (int k = 0; k < rounds; ++k) {
+    NLGB_CUDA_TRY(persist_launch(plan, pa, s));
+    if (mixed) {
+      NLGB_CUDA_TRY(go((const void*)k_mx_apply, vg, kCTA, a1));
+      NLGB_CUDA_TRY(go(ks.mx_outer, v.n_tiles, kCTA, a1));
+    }
+  }
+  NLGB_CUDA_TRY(go(ks.fin_if, v.n_tiles, kCTA, a1));
+  if (!mixed) NLGB_CUDA_TRY(go((const void*)k_check, 1, 1, ast));
+  void* ae[] = {&st, &pa.err};
+  NLGB_CUDA_TRY(go((const void*)k_persist_end, 1, 1, ae));
+  count_launches(launched);
   return cudaSuccess;
 }
 

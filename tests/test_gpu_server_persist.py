@@ -1,0 +1,63 @@
+"""Chunks of the server on the persistent kernel (csrc/nlgb_persist.cuh): where
+their layout changes (four tiles per CTA; one CTA, one cluster, cluster to grid
+at 64 / 65 tiles, more than four tiles per CTA), every precision, a mixed system
+that continues in FP64, a budget without room for the tables, and a load that
+changes between systems that fit and systems that do not -- the same iterates
+bit for bit as the single-system solver."""
+import numpy as np
+import pytest
+
+from graphitethree_gb300 import meshes, solver, systems
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(srv, reqs, precision):
+    want = [solver.Matrix(s.rp, s.ci, s.va).solve(s.rhs[0], precision=precision) for s in reqs]
+    tickets = [srv.submit_square(s) for s in reqs]
+    for t, (y, j) in zip(tickets, want):
+        xs, infos, _ = srv.wait(t)
+        assert infos[0].status == j.status == "converged"
+        assert np.array_equal(xs[0], y)
+        assert (infos[0].iterations, infos[0].refinement_steps) == (j.iterations, j.refinement_steps)
+
+
+@pytest.mark.parametrize("precision", ["double", "mixed", "df"])
+@pytest.mark.parametrize("sizes", [[(3, 3)], [(32, 16)], [(37, 17)], [(128, 64)], [(131, 64)], [(363, 291)],
+                                   [(640, 600)], [(20, 20), (150, 131), (90, 80), (33, 31), (200, 180), (5, 4)]])
+def test_sizes(gpu_ok, sizes, precision):
+    srv = solver.Server(precision=precision, epoch_ms=0.5)
+    _check(srv, [systems.fairing_system(nx, ny, seed=nx, n_rhs=1) for nx, ny in sizes], precision)
+    srv.close()
+
+
+def test_mixed_continues_in_fp64(gpu_ok):
+    V, F = meshes.height_field(70, 60, 3)
+    M, rhs, _ = solver.build_lscm(V, F)
+    x, info = M.solve(rhs, precision="mixed", eps=1e-12)
+    srv = solver.Server(precision="mixed", eps=1e-12)
+    xs, infos, _ = srv.wait(srv.submit_mesh("lscm", V, F))
+    srv.close()
+    assert infos[0].status == info.status
+    assert np.array_equal(xs[0], x) and infos[0].iterations == info.iterations
+
+
+def test_no_room_for_tables(gpu_ok):
+    sq = systems.fairing_system(200, 180, seed=2, n_rhs=1)
+    srv = solver.Server(precision="double")
+    srv.wait(srv.submit_square(sq))
+    peak = srv.stats()["peak_bytes"]
+    srv.close()
+    srv = solver.Server(precision="double", budget_bytes=peak - 1024)
+    _check(srv, [sq], "double")
+    assert srv.stats()["peak_bytes"] <= peak - 1024
+    srv.close()
+
+
+def test_load_changes(gpu_ok):
+    small = [systems.fairing_system(60 + 10 * i, 50 + 7 * i, seed=i, n_rhs=1) for i in range(6)]
+    large = systems.fairing_system(1300, 1000, seed=3, n_rhs=1)
+    srv = solver.Server(precision="mixed", epoch_ms=1.0)
+    _check(srv, small + [large] + small, "mixed")
+    _check(srv, [large] + small, "mixed")
+    srv.close()
