@@ -504,8 +504,9 @@ def profile_case(which):
         print(json.dumps({"case": which, "iterations": its}))
         return
     if which == "batch_small":
-        # one small LSCM system (4,604 unknowns, 35 tiles) in the persistent
-        # kernel: a latency-bound team of 35 CTAs, 1000 FP64 iterations
+        # one small LSCM system (4,604 unknowns, 36 tiles) as a batch: the
+        # persistent single-system kernel on a cluster of nine CTAs, 1000 FP64
+        # iterations
         M, rhs, _ = solver.assemble(systems.lscm_system(48, 48, seed=1))
         xs, infos, ks = solver.batch_solve([M], [rhs[0]], max_iter=1000, eps=1e-30)
         print(json.dumps({"case": which, "kernel_ms": ks * 1e3, "iterations": infos[0].iterations,

@@ -2,6 +2,7 @@
 #include "../../include/nl.h"
 #include "../../include/nl_gb300.h"
 #include "nlgb_batch.h"
+#include "nlgb_persist.h"
 #include "nlgb_internal.h"
 #include "nlgb_sell.h"
 
@@ -22,6 +23,11 @@ struct nlgb_matrix_s {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   std::mutex spmv_mu;
   long long spmvs = 0;       // products asked for so far
+  // batches: the tables of the layout (tpr, tile_rows), built by the first
+  std::mutex batch_mu;
+  PersistTables tables;
+  PersistPlan plans[3];
+  int tables_tpr = -1, tables_rows = 0;
   ~nlgb_matrix_s() {
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -295,6 +301,60 @@ int nlgb_solve(nlgb_matrix A, const double* b, double* x, const nlgb_params* prm
   return NLGB_OK;
 }
 
+namespace {
+
+// The matrices' layouts and plans for the persistent kernel in a batch; false:
+// some system does not fit it in every precision, or an error (rc).
+bool batch_tables(int n_sys, const nlgb_matrix* A, const std::vector<SystemSlot>& slots, cudaStream_t s,
+                  std::vector<PersistSystem>& ps, int* rc) {
+  std::vector<nlgb_matrix> fresh(A, A + n_sys);
+  std::sort(fresh.begin(), fresh.end());   // (one order for every thread's locks)
+  fresh.erase(std::unique(fresh.begin(), fresh.end()), fresh.end());
+  std::vector<std::unique_lock<std::mutex>> held;
+  for (nlgb_matrix m : fresh) held.emplace_back(m->batch_mu);
+  fresh.erase(std::remove_if(fresh.begin(), fresh.end(), [](nlgb_matrix m) {
+    return m->tables_tpr == m->A.tpr && m->tables_rows == m->A.tile_rows;
+  }), fresh.end());
+  if (!fresh.empty()) {
+    std::vector<int> most(fresh.size(), 0);
+    int* d = nullptr;
+    cudaError_t e = cudaMallocAsync((void**)&d, sizeof(int) * most.size(), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, sizeof(int) * most.size(), s);
+    for (size_t i = 0; i < fresh.size() && e == cudaSuccess; ++i) {
+      const DeviceCRS& M = fresh[i]->A;
+      fresh[i]->tables_tpr = -1;
+      e = fresh[i]->tables.begin(M, M.tile_rows, std::max(1, (M.n + M.tile_rows - 1) / M.tile_rows), s, true, d + i);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(most.data(), d, sizeof(int) * most.size(), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (d) cudaFreeAsync(d, s);
+    if (e != cudaSuccess) {
+      *rc = NLGB_E_DEVICE;
+      return false;
+    }
+    for (size_t i = 0; i < fresh.size(); ++i) {
+      nlgb_matrix m = fresh[i];
+      m->tables.end(most[i], s);
+      for (int k = 0; k < 3; ++k) m->plans[k] = m->tables.plan(m->A.tile_rows, m->A.tpr, k);
+      m->tables_tpr = m->A.tpr;
+      m->tables_rows = m->A.tile_rows;
+    }
+  }
+  bool fit = true;
+  for (int i = 0; i < n_sys; ++i) {
+    const nlgb_matrix m = A[i];
+    ps[i].layout = m->tables.layout();
+    ps[i].plan[0] = m->plans[slots[i].df ? kPersistDf : kPersistDouble];
+    ps[i].plan[1] = m->plans[kPersistMixed];
+    ps[i].view = slots[i].view;
+    ps[i].mixed = slots[i].mixed;
+    fit = fit && m->plans[0].usable && m->plans[1].usable && m->plans[2].usable;
+  }
+  return fit;
+}
+
+}  // namespace
+
 int nlgb_batch_solve(int n_sys, const nlgb_matrix* A, const double* const* b, double* const* x,
                      const nlgb_params* prm, nlgb_result* res, double* kernel_seconds) {
   if (n_sys < 0 || (n_sys > 0 && (!A || !b || !x))) return fail(NLGB_E_INVALID, "nlgb_batch_solve: bad arguments");
@@ -340,7 +400,20 @@ int nlgb_batch_solve(int n_sys, const nlgb_matrix* A, const double* const* b, do
       work[i] = (long long)((double)(M.nnz + 8LL * M.n) * std::sqrt((double)std::max(1, M.n)));
     }
     BatchLaunchStats st;
-    if (rc == NLGB_OK && runner.run(views, work, 0, &st) != cudaSuccess) rc = NLGB_E_DEVICE;
+    std::vector<PersistSystem> ps((size_t)n_sys);
+    bool persist = rc == NLGB_OK && !runner.test_hooks() && persist_batch_pays(views) &&
+                   batch_tables(n_sys, A, slots, s, ps, &rc);
+    if (persist) {
+      float ms = 0.f;
+      const cudaError_t e = persist_batch(ps, s, &ms);
+      persist = e != cudaErrorMemoryAllocation;   // (nothing has run yet: the batched kernel needs less)
+      if (!persist) cudaGetLastError();
+      else if (e != cudaSuccess) rc = NLGB_E_DEVICE;
+      st.ms = ms;
+    }
+    if (!persist && rc == NLGB_OK && runner.run(views, work, 0, &st) != cudaSuccess) {
+      rc = NLGB_E_DEVICE;
+    }
     if (rc == NLGB_OK && kernel_seconds) *kernel_seconds = st.ms * 1e-3;
     std::vector<SysState> hs((size_t)n_sys);
     for (int i = 0; i < n_sys && rc == NLGB_OK; ++i) {

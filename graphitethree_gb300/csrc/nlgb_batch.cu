@@ -1,5 +1,7 @@
 // nlgb_batch.cu -- many independent Jacobi-PCG systems in one persistent
-// kernel launch (plain FP64 or mixed FP32/FP64 per system).
+// kernel launch (plain FP64 or mixed FP32/FP64 per system), or, where all of
+// them fit it and they are few enough, each on the persistent single-system
+// kernel (persist_batch).
 //
 // Reference context: geogram's mesh_make_atlas solves one LSCM system per
 // chart, one after another, each through nlSolve (called from
@@ -23,17 +25,28 @@
 #include "nlgb_batch.h"
 #include "nlgb_core.cuh"
 #include "nlgb_internal.h"
+#include "nlgb_persist.h"
 #include "nlgb_sell.h"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <numeric>
+#include <thread>
 
 namespace nlgb {
 
+static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
+
 namespace {
+
+// A batch on the persistent single-system kernel: systems at a time, iterations
+// of one launch, and the rule it is chosen by (persist_batch_pays).
+constexpr int kPersistLanes = 32;
+constexpr long long kPersistBatchIters = 1024;
+constexpr double kPersistBatchRatio = 0.5;
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
@@ -724,10 +737,168 @@ cudaError_t BatchRunner::gather_states(SysState* out, int n) {
 }
 
 // ---------------------------------------------------------------------------
+// A batch on the persistent single-system kernel.
+// ---------------------------------------------------------------------------
+namespace {
+
+int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();
+  return sms;
+}
+
+// Expected time of a system there, up to a factor: iterations of a Jacobi-CG on
+// a surface (sqrt(n)) times the time of one, us (kSharedTiles' figures).
+double persist_time(const SysView& v) {
+  return std::sqrt((double)v.n) * (5.0 + 1.2 * (double)(persist_shared_slots(v.n_tiles) - 1));
+}
+
+}  // namespace
+
+// The host starts one system there in about 35 us and builds a matrix's tables
+// in 15, while the batched kernel runs up to four systems per SM from one
+// launch.  So the line lies at the number of systems in the time of the
+// longest one.  LSCM charts, log-uniform long sides, whole call, ms, batched
+// kernel -> here with the tables built (first call), and that ratio:
+//   40 of 16..128      56.7 -> 27.6 (39.1)    0.03
+//   100 of 16..128    105.3 -> 59.7 (62.7)    0.07
+//   300 of 16..128    267.5 -> 225  (240)     0.22
+//   200 of 16..64      46.3 -> 25.5 (32.0)    0.29
+//   150 of 16..32      25.0 -> 11.1 (15.2)    0.44
+//   400 of 16..64      61.3 -> 50.7 (71.4)    0.53
+//   300 of 16..24      21.0 -> 20.6 (24.7)    1.09
+bool persist_batch_pays(const std::vector<SysView>& views) {
+  double longest = 0.0;
+  for (const SysView& v : views) longest = std::max(longest, persist_time(v));
+  return (double)views.size() <= kPersistBatchRatio * longest;
+}
+
+cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms) {
+  struct Lane {
+    cudaStream_t s = nullptr;
+    int sys = -1, sms = 0;
+    unsigned int seq0 = 0;
+  };
+  const int n = (int)systems.size(), n_sm = sm_count();
+  std::vector<Lane> lanes((size_t)std::min(n, kPersistLanes));
+  std::vector<std::unique_ptr<ViewGraph>> graphs;
+  std::vector<size_t> at((size_t)n + 1, 0);
+  ChunkMirror* mirrors = nullptr;
+  char* exch = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaError_t e = cudaSuccess;
+  auto ok = [&](cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+    return e == cudaSuccess;
+  };
+  for (int i = 0; i < n; ++i)
+    at[(size_t)i + 1] = at[(size_t)i] + align256(persist_bytes(systems[i].view.n, systems[i].view.n_tiles));
+  ok(cudaHostAlloc((void**)&mirrors, sizeof(ChunkMirror) * (size_t)n, cudaHostAllocMapped));
+  ok(cudaMallocAsync((void**)&exch, at[(size_t)n], s));
+  if (ok(e)) ok(cudaMemsetAsync(exch, 0, at[(size_t)n], s));
+  ok(cudaEventCreate(&e0));
+  ok(cudaEventCreate(&e1));
+  if (ok(e)) ok(cudaEventRecord(e0, s));
+  for (Lane& l : lanes) {
+    if (ok(e)) ok(cudaStreamCreateWithFlags(&l.s, cudaStreamNonBlocking));
+    if (ok(e)) ok(cudaStreamWaitEvent(l.s, e0, 0));
+  }
+  if (ok(e)) std::memset((void*)mirrors, 0, sizeof(ChunkMirror) * (size_t)n);
+  std::vector<int> order((size_t)n);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return persist_time(systems[a].view) > persist_time(systems[b].view);
+  });
+  for (int i = 0; i < n && ok(e); ++i) {
+    graphs.emplace_back(new ViewGraph());
+    graphs.back()->persist_bind(systems[i].layout, systems[i].plan, exch + at[(size_t)i]);
+    graphs.back()->persist(true);
+  }
+  std::vector<int> waiting(order);     // longest first
+  std::vector<char> fp64((size_t)n, 0);
+  int left = n, sms_busy = 0;
+  unsigned polls = 0;
+  auto seq_of = [&](int i) { return __atomic_load_n(&mirrors[i].seq, __ATOMIC_ACQUIRE); };
+  auto start = [&](Lane& l) {
+    const int i = l.sys;
+    const bool mixed = systems[i].mixed && !fp64[(size_t)i];
+    mirrors[i].budget = kPersistBatchIters;
+    l.seq0 = seq_of(i);
+    if (ok(graphs[(size_t)i]->prepare(systems[i].view, mixed, &mirrors[i], l.s))) ok(graphs[(size_t)i]->launch(l.s));
+  };
+  while (left > 0 && ok(e)) {
+    bool idle = true;
+    ++polls;
+    for (Lane& l : lanes) {
+      if (l.sys >= 0) {
+        if (seq_of(l.sys) == l.seq0) {
+          if (!ok(graphs[(size_t)l.sys]->advance(l.s))) break;
+          if ((polls & 4095u) == 0) {   // a failed kernel writes no mirror
+            const cudaError_t r = cudaStreamQuery(l.s);
+            if (r != cudaErrorNotReady && !ok(r)) break;
+          }
+          continue;
+        }
+        idle = false;
+        const int i = l.sys;
+        const SysState& h = mirrors[i].st;
+        if (h.status == ST_STAGNATION && !h.fell_back && h.precision == 1) {
+          // FP32 cannot track this system: it continues in FP64 from its x
+          fp64[(size_t)i] = 1;
+          mirrors[i].st.stage = 0;
+          if (ok(chunk_fallback_fp64(systems[i].view.st, l.s))) start(l);
+          continue;
+        }
+        if (h.stage != 3) {
+          start(l);
+          continue;
+        }
+        systems[i].state = h;
+        if (h.status == ST_DEVICE_ERR) {
+          set_error("batched solve: a wait of the persistent kernel timed out");
+          ok(cudaErrorLaunchTimeout);
+        }
+        sms_busy -= l.sms;
+        l.sys = -1;
+        --left;
+      }
+      for (size_t q = 0; q < waiting.size() && ok(e); ++q) {
+        const int c = graphs[(size_t)waiting[q]]->persist_ctas(systems[waiting[q]].mixed);
+        if (sms_busy > 0 && sms_busy + c > n_sm) continue;
+        l.sys = waiting[q];
+        l.sms = c;
+        sms_busy += c;
+        waiting.erase(waiting.begin() + (long)q);
+        start(l);
+        idle = false;
+        break;
+      }
+    }
+    if (idle) std::this_thread::yield();
+  }
+  for (Lane& l : lanes) {
+    if (!l.s) continue;
+    const cudaError_t r = cudaStreamSynchronize(l.s);
+    ok(r);
+    cudaStreamDestroy(l.s);
+  }
+  if (e1 && ok(e) && ok(cudaEventRecord(e1, s)) && ok(cudaEventSynchronize(e1))) {
+    float t = 0.f;
+    cudaEventElapsedTime(&t, e0, e1);
+    if (ms) *ms = t;
+  }
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  if (exch) cudaFreeAsync(exch, s);
+  if (mirrors) cudaFreeHost(mirrors);
+  return e;
+}
+
+// ---------------------------------------------------------------------------
 // Per-system device slot.
 // ---------------------------------------------------------------------------
-static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
-
 size_t SystemSlot::bytes_for(int n, int tile_rows, bool mixed) {
   const size_t n8 = align256((size_t)std::max(2, n + 2) * sizeof(double));
   const size_t n4 = align256((size_t)std::max(4, n + 4) * sizeof(float));

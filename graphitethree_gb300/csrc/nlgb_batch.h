@@ -113,12 +113,12 @@ struct SystemSlot {
 // here, stores the chunk's device duration and then bumps `seq`, so that a
 // host thread sees the end of a chunk by reading memory, without a CUDA call.
 struct ChunkMirror {
-  SysState st;                   // the system's state after the last chunk
+  SysState st;                   // the system's state after the last chunk (stage 0: none yet)
   long long budget;              // host: iterations of the next chunk
   unsigned long long t_start;    // device: %globaltimer at the chunk's start
   unsigned long long t_ns;       // device: the chunk's duration
   unsigned int seq;              // device: +1 after st and t_ns of a chunk are written
-  unsigned int pad_;
+  unsigned int persist;          // device: the last launch of the persistent kernel that ended
 };
 
 class ViewGraph {
@@ -147,19 +147,34 @@ class ViewGraph {
   cudaError_t launch(cudaStream_t s);
   void account(long long iters_before, long long iters_after);
   // The persistent kernel (nlgb_persist.cuh) as an executor of the chunks:
-  // tables of the system's matrix, and an exchange area of persist_bytes(),
-  // zeroed when the system started.  Both outlive the chunks.  The chunks
-  // run there while persist(true) holds and the system fits.
-  void persist_bind(const PersistTables& t, void* exch, const SysView& v, bool mixed);
+  // layout and plans (FP64 or double-float, mixed) of the system's matrix, and
+  // an exchange area of persist_bytes(), zeroed when the system started.  All
+  // outlive the chunks.  They run there while persist(true) holds and the
+  // system fits.
+  void persist_bind(const PersistLayout& layout, const PersistPlan (&plan)[2], void* exch);
   int persist_ctas(bool mixed) const { return plan_[mixed ? 1 : 0].usable ? plan_[mixed ? 1 : 0].grid : 0; }
   void persist(bool on) { persist_ = on; }
+  // A chunk there goes on in steps: the owner calls this while it polls m->seq.
+  // What follows a launch of the persistent kernel is queued only once that
+  // has ended: streams share hardware queues (eight, unless the process asked
+  // for more), and a kernel that waits for an earlier one of its stream would
+  // hold up every stream behind it for the whole chunk (40 LSCM charts 28 ->
+  // 38 ms).
+  cudaError_t advance(cudaStream_t s);
 
  private:
+  cudaError_t persist_head(long long iters, cudaStream_t s);
+  cudaError_t persist_next(cudaStream_t s);
   bool persistent() const { return persist_ && plan_[mixed_ ? 1 : 0].usable; }
   PersistPlan plan_[2];        // FP64 or double-float; mixed
   PersistLayout lay_;
   void* exch_ = nullptr;
   bool persist_ = false;
+  // the chunk in flight: its launch of the persistent kernel that has not been
+  // seen to end (0: none), iterations per launch, reliable updates left
+  unsigned int waiting_ = 0, launches_ = 0;
+  long long iters_ = 0;
+  int rounds_ = 0;
   cudaError_t build(const SysView& v, bool mixed);
   cudaError_t run_eager(cudaStream_t s, long long iters);
   SysView view_{};
@@ -177,11 +192,20 @@ class ViewGraph {
 // stream-ordered, before the system's next chunk.
 cudaError_t chunk_fallback_fp64(SysState* st, cudaStream_t s);
 
-// Queues a chunk of a system on the persistent kernel: what a chunk graph
-// does (see nlgb_solver.cu), with `rounds` launches of at most `iters`
-// iterations each (a mixed system ends one at every reliable update).
-cudaError_t persist_chunk(const SysView& v, const PersistPlan& plan, const PersistLayout& lay, void* exch,
-                          bool mixed, long long iters, int rounds, cudaStream_t s);
+// Many systems on the persistent single-system kernel (nlgb_persist.cuh), each
+// by itself on a few SMs, as many at a time as the SMs allow.
+struct PersistSystem {
+  PersistLayout layout;
+  PersistPlan plan[2];         // FP64 or double-float; mixed
+  SysView view{};              // started (SystemSlot::start)
+  bool mixed = false;
+  SysState state{};            // out
+};
+// Whether a batch is better off there than in one launch of the batched kernel.
+bool persist_batch_pays(const std::vector<SysView>& views);
+// Runs the systems (ready on stream s); on return they have ended.
+// cudaErrorMemoryAllocation: no room for the exchange areas, nothing was run.
+cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms);
 
 // Launches the persistent kernel over a set of resident systems.  Each
 // system's SysState (device) must be initialised by the caller (status
@@ -194,6 +218,7 @@ class BatchRunner {
   ~BatchRunner();
   BatchRunner(const BatchRunner&) = delete;
   BatchRunner& operator=(const BatchRunner&) = delete;
+  bool test_hooks() const { return test_shortfall_; }
 
   cudaError_t init(cudaStream_t s);
   // work[i]: relative cost estimate of system i (bytes per iteration x

@@ -154,6 +154,10 @@ class PersistTables {
   // fits (sizes and halos).  shared: for a system that shares the GPU with
   // others (fewer CTAs, more tiles on each).
   cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared = false);
+  // The same in two steps, for many matrices with one synchronisation: begin
+  // queues the work and raises *most (device, zero before), end takes its value.
+  cudaError_t begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared, int* most);
+  void end(int most, cudaStream_t s);
   bool usable() const { return lay_.ctas > 0; }
   const PersistLayout& layout() const { return lay_; }
   PersistPlan plan(int tile_rows, int tpr, int mode) const;
@@ -164,6 +168,7 @@ class PersistTables {
  private:
   PersistLayout lay_;
   bool cluster_ = false;
+  int ctas_ = 0;
   void* mem_ = nullptr;
   size_t bytes_ = 0;
 };

@@ -4,7 +4,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <vector>
 
 namespace nlgb {
 namespace {
@@ -24,7 +23,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_persist_prep(int n, int R, int
                                                                int cluster, int stride,
                                                                const int* __restrict__ rp, const int* __restrict__ ci,
                                                                unsigned short* lci, unsigned short* perm, int* halo,
-                                                               int* halo_n) {
+                                                               int* halo_n, int* most) {
   extern __shared__ unsigned words[];            // bitmap of the columns, then its exclusive counts
   __shared__ int sums[kPrepThreads];
   __shared__ int hist[65];
@@ -57,7 +56,10 @@ __global__ void __launch_bounds__(kPrepThreads) k_persist_prep(int n, int R, int
   }
   int at = sums[threadIdx.x] - mine;
   const int H = sums[kPrepThreads - 1];
-  if (threadIdx.x == 0) halo_n[cta] = H;
+  if (threadIdx.x == 0) {
+    halo_n[cta] = H;
+    atomicMax(most, H);
+  }
   for (int w = w0; w < w1; ++w) {
     off[w] = at;
     unsigned b = words[w];
@@ -122,6 +124,12 @@ size_t smem_bytes(int slots, int R, int halo, size_t word) {
 
 }  // namespace
 
+int persist_shared_slots(int n_tiles) {
+  const int most = n_tiles <= kPersistClusterTiles ? kPersistCluster : 151;
+  const int ctas = std::max(1, std::min((n_tiles + kSharedTiles - 1) / kSharedTiles, most));
+  return (n_tiles + ctas - 1) / ctas;
+}
+
 void PersistTables::release() {
   cudaFree(mem_);
   mem_ = nullptr;
@@ -136,6 +144,20 @@ void PersistTables::release(cudaStream_t s) {
 }
 
 cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared) {
+  int most = 0, *d = nullptr;
+  NLGB_CUDA_TRY(cudaMallocAsync((void**)&d, sizeof(int), s));
+  cudaError_t e = cudaMemsetAsync(d, 0, sizeof(int), s);
+  if (e == cudaSuccess) e = begin(A, tile_rows, n_tiles, s, shared, d);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&most, d, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFreeAsync(d, s);
+  NLGB_CUDA_TRY(e);
+  end(most, s);
+  return cudaSuccess;
+}
+
+cudaError_t PersistTables::begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared,
+                                 int* most) {
   release();
   int sms = 0, smem_max = 0;
   if (A.n <= 0 || A.nnz <= 0 || A.n != A.m || tile_rows > 512 || !device_limits(&sms, &smem_max)) return cudaSuccess;
@@ -157,7 +179,13 @@ cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles,
   const size_t perm_b = ((size_t)A.n * sizeof(unsigned short) + 255) & ~(size_t)255;
   const size_t halo_b = ((size_t)ctas * std::max(1, stride) * sizeof(int) + 255) & ~(size_t)255;
   const size_t bytes = lci_b + perm_b + halo_b + (size_t)ctas * sizeof(int);
-  NLGB_CUDA_TRY(shared ? cudaMallocAsync(&mem_, bytes, s) : cudaMalloc(&mem_, bytes));
+  const cudaError_t room = cudaMallocAsync(&mem_, bytes, s);
+  if (room == cudaErrorMemoryAllocation) {       // the other executors need no tables
+    cudaGetLastError();
+    mem_ = nullptr;
+    return cudaSuccess;
+  }
+  NLGB_CUDA_TRY(room);
   bytes_ = bytes;
   char* m = static_cast<char*>(mem_);
   unsigned short* lci = reinterpret_cast<unsigned short*>(m);
@@ -167,26 +195,27 @@ cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles,
   NLGB_CUDA_TRY(cudaFuncSetAttribute((const void*)k_persist_prep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      smem_max - 8192));
   k_persist_prep<<<ctas, kPrepThreads, prep_smem, s>>>(A.n, tile_rows, n_tiles, ctas, slots, A.tpr, cluster_ ? 1 : 0,
-                                                       stride, A.rp, A.ci, lci, perm, halo, halo_n);
+                                                       stride, A.rp, A.ci, lci, perm, halo, halo_n, most);
   count_launches(1);
   NLGB_CUDA_TRY(cudaGetLastError());
-  std::vector<int> hn((size_t)ctas);
-  NLGB_CUDA_TRY(cudaMemcpyAsync(hn.data(), halo_n, sizeof(int) * hn.size(), cudaMemcpyDeviceToHost, s));
-  NLGB_CUDA_TRY(cudaStreamSynchronize(s));
-  const int most = *std::max_element(hn.begin(), hn.end());
-  if (most > stride) {
-    shared ? release(s) : release();
-    return cudaSuccess;
-  }
-  lay_.ctas = ctas;
   lay_.slots = slots;
   lay_.halo_stride = stride;
-  lay_.halo_cap = (most + 1) & ~1;
+  ctas_ = ctas;
   lay_.lci = lci;
   lay_.perm = perm;
   lay_.halo = halo;
   lay_.halo_n = halo_n;
   return cudaSuccess;
+}
+
+void PersistTables::end(int most, cudaStream_t s) {
+  if (!mem_) return;
+  if (most > lay_.halo_stride) {
+    release(s);
+    return;
+  }
+  lay_.halo_cap = (most + 1) & ~1;
+  lay_.ctas = ctas_;
 }
 
 PersistPlan PersistTables::plan(int tile_rows, int tpr, int mode) const {

@@ -281,6 +281,17 @@ __device__ __forceinline__ double serial_sum(const double* v, int nw) {
   return s;
 }
 
+// Tells the host that this launch is over (one thread; the state itself is for
+// the kernels that the host queues then).
+template <int MODE>
+__device__ __forceinline__ void tell_done(const PersistArgs& a, const SysState& st) {
+  if (a.done == nullptr) return;
+  const unsigned end = st.status != ST_RUNNING                  ? kPersistStopped
+                       : MODE == kPersistMixed && st.mode == 0 ? kPersistUpdate
+                                                               : kPersistPaused;
+  *reinterpret_cast<volatile unsigned int*>(a.done) = a.done_value + end;
+}
+
 // ---------------------------------------------------------------------------
 // The reducing CTA of the grid form (256 threads): sums the tiles' partials
 // as they arrive, takes the scalar steps and publishes alpha and beta.
@@ -385,6 +396,7 @@ __device__ void reducer(const PersistArgs& a, SysState& sst) {
     sst.coop_epoch += it;
     sst.guard += (it + 3) / 4;
     *s.st = sst;
+    tell_done<MODE>(a, sst);
   }
 }
 
@@ -407,7 +419,10 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
 
   if (threadIdx.x == 0) { sst = *s.st; s_code[0] = s_code[1] = GO; s_failed = 0; s_abort = 0; }
   __syncthreads();
-  if (sst.status != ST_RUNNING || (MODE == kPersistMixed && sst.mode != 1)) return;
+  if (sst.status != ST_RUNNING || (MODE == kPersistMixed && sst.mode != 1)) {
+    if (cta == 0 && threadIdx.x == 0) tell_done<MODE>(a, sst);
+    return;
+  }
   if constexpr (!CLUSTER) {
     if (cta == C) { reducer<MODE>(a, sst); return; }
   }
@@ -915,6 +930,7 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
       sst.coop_epoch += it;
       sst.guard += (it + 3) / 4;
       *s.st = sst;
+      tell_done<MODE>(a, sst);
     }
     cluster_barrier();   // no CTA leaves while another may read its shared memory
   }

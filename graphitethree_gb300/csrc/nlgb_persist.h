@@ -15,6 +15,9 @@ constexpr int kPersistCluster = 16;       // CTAs of the cluster form at most
 constexpr int kPersistClusterTiles = 64;  // tiles of the cluster form at most
 constexpr int kPersistRed = 8 * 36;       // 8-byte words of one staged value of a tile
 
+// How a launch left its system: running, at a reliable update, or stopped.
+enum PersistEnd : unsigned { kPersistPaused = 0, kPersistUpdate = 1, kPersistStopped = 2 };
+
 struct PersistArgs {
   SysView s;
   ulonglong2* slot;            // grid form: 3 x n_tiles, p.q, r.z, r.r of every tile as (value, epoch)
@@ -23,6 +26,8 @@ struct PersistArgs {
   int* err;                    // nonzero: a wait ran out
   PersistLayout lay;
   long long iters;             // iterations of this launch at most
+  unsigned int* done;          // host-mapped, or null: done_value + a PersistEnd when the launch ends
+  unsigned int done_value;
 };
 
 // Exchange area (zeroed before a solve): partial slots, control slots, z
@@ -36,6 +41,8 @@ inline void persist_bind(PersistArgs& a, void* exch) {
   a.zslot = a.ctl + 16;
   a.err = reinterpret_cast<int*>(a.zslot + a.s.n);
 }
+// Tiles per CTA of a system that shares the GPU (PersistTables::build).
+int persist_shared_slots(int n_tiles);
 cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& a, cudaStream_t s);
 // The kernel for a layout (nlgb_persist_*.cu): nc rows per lane group in registers.
 const void* persist_kernel_f64(int tpr, bool cluster, int nc);

@@ -90,6 +90,7 @@ struct Req {
   // FP64, and the measured time per iteration (ms; < 0 unknown)
   std::vector<std::unique_ptr<ViewGraph>> graphs;
   PersistTables tables;              // of A, for chunks on the persistent kernel
+  PersistPlan plan[2];
   void* exch = nullptr;              // their exchange areas, one per system
   std::vector<int> mirror_idx;       // per system, its ChunkMirror in the server's pool
   std::vector<int> running, mixed_now, need_fallback;
@@ -292,7 +293,14 @@ cudaError_t persist_tables(nlgb_server_s* S, Req* r, cudaStream_t s) {
     add_used_locked(S, (long long)extra);
   }
   r->bytes += extra;
+  r->plan[0] = r->tables.plan(v.tile_rows, v.tpr, v.df ? kPersistDf : kPersistDouble);   // (a mixed one may end in FP64)
+  if (r->slots[0].mixed) r->plan[1] = r->tables.plan(v.tile_rows, v.tpr, kPersistMixed);
   e = cudaMallocAsync(&r->exch, exch, s);
+  if (e == cudaErrorMemoryAllocation) {   // no room: the chunks run as graphs
+    cudaGetLastError();
+    r->exch = nullptr;
+    return cudaSuccess;
+  }
   if (e == cudaSuccess) e = cudaMemsetAsync(r->exch, 0, exch, s);
   return e;
 }
@@ -664,10 +672,12 @@ void admitter(nlgb_server_s* S) {
         for (int k = 0; k < pick->n_rhs && ok; ++k) {
           ChunkMirror* m = &S->mirrors[pick->mirror_idx[k]];
           m->budget = 0;
+          m->st.stage = 0;
+          m->persist = 0;
           pick->graphs[k].reset(new ViewGraph());
           if (pick->exch) {
-            pick->graphs[k]->persist_bind(pick->tables, static_cast<char*>(pick->exch) + (size_t)k * exchange_bytes(*pick),
-                                          pick->slots[k].view, pick->slots[k].mixed);
+            pick->graphs[k]->persist_bind(pick->tables.layout(), pick->plan,
+                                          static_cast<char*>(pick->exch) + (size_t)k * exchange_bytes(*pick));
             pick->graphs[k]->persist(true);
           }
           ok = pick->graphs[k]->prepare(pick->slots[k].view, pick->slots[k].mixed, m, su) == cudaSuccess;
@@ -1022,8 +1032,8 @@ void worker_streams(nlgb_server_s* S) {
   // 8 to 10 us per iteration of 2k to 33k rows, against 30 us on 16 lanes of
   // graphs, and no graph to instantiate (which also held a burst's other
   // requests back for up to 50 ms behind the first one's chunk).  24 requests
-  // of 1k to 20k vertices at once: 222 -> 73 ms, their median latency 72 ->
-  // 10 ms.  A chunk's CTAs each need a whole SM and wait for one another, so
+  // of 1k to 20k vertices at once: 222 -> 65 ms, their median latency 72 ->
+  // 9 ms.  A chunk's CTAs each need a whole SM and wait for one another, so
   // the chunks in flight share out the SMs, and they never run beside graph
   // chunks, whose kernels would leave no SM empty.
   int n_sm = 0, sms_busy = 0, graphs_busy = 0;
@@ -1160,8 +1170,13 @@ void worker_streams(nlgb_server_s* S) {
     bool progress = have_admitted;
     double tw = S->now();
     ++w_loops;
+    cudaError_t e = cudaSuccess;
     for (Lane& l : lanes) {
-      if (!l.r || mirror_seq(l.m) == l.seq0) continue;
+      if (!l.r) continue;
+      if (mirror_seq(l.m) == l.seq0) {
+        if (l.sms > 0 && e == cudaSuccess) e = l.r->graphs[l.k]->advance(l.s);
+        continue;
+      }
       l.t_free = S->now();
       retire(l);
       progress = true;
@@ -1192,13 +1207,12 @@ void worker_streams(nlgb_server_s* S) {
       continue;
     }
     // give every free lane the least-work system that is not running
-    cudaError_t e = cudaSuccess;
     bool persist = n_busy < ns;
     for (Req* r : S->active)
       for (int k = 0; persist && k < r->n_rhs; ++k)
         persist = r->sys_done[k] || r->graphs[k]->persist_ctas(r->mixed_now[k] != 0) > 0;
     for (Lane& l : lanes) {
-      if (l.r) continue;
+      if (l.r || e != cudaSuccess) continue;
       if (persist ? graphs_busy > 0 : sms_busy > 0) break;   // the other kind's chunks end first
       Req* best = nullptr;
       int bk = -1;
@@ -1224,6 +1238,7 @@ void worker_streams(nlgb_server_s* S) {
       iters = (iters + kUnrollPlainIters - 1) / kUnrollPlainIters * kUnrollPlainIters;
       if (best->need_fallback[bk]) {
         e = chunk_fallback_fp64(best->slots[bk].view.st, l.s);
+        S->mirrors[best->mirror_idx[bk]].st.stage = 0;
         best->need_fallback[bk] = 0;
       }
       ChunkMirror* m = &S->mirrors[best->mirror_idx[bk]];
@@ -1269,7 +1284,9 @@ void worker_streams(nlgb_server_s* S) {
       // chunks in flight: poll their mirrors again shortly (the admission
       // threads' notifications are seen at the top of the loop); idle: sleep
       // until a request is admitted or the server stops
-      if (n_busy > 0) {
+      if (sms_busy > 0) {
+        std::this_thread::yield();   // (a sleep takes 70 us, and a chunk goes on in steps)
+      } else if (n_busy > 0) {
         std::this_thread::sleep_for(std::chrono::microseconds(20));
       } else {
         std::unique_lock<std::mutex> lk(S->mu);

@@ -261,12 +261,6 @@ __global__ void k_chunk_end(SysState* st) {
   if (st->status != ST_RUNNING) st->stage = 3;
 }
 
-// The same after a chunk on the persistent kernel, whose waits are bounded.
-__global__ void k_persist_end(SysState* st, const int* err) {
-  if (*err) st->status = ST_DEVICE_ERR;
-  if (st->status != ST_RUNNING) st->stage = 3;
-}
-
 __device__ __forceinline__ unsigned long long chunk_clock_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -285,9 +279,13 @@ __global__ void k_chunk_start_m(SysState* st, ChunkMirror* m, int unroll) {
 
 // End of a mirrored chunk (one warp): the k_chunk_end rule, then the state
 // copied to the mirror, the duration, a system-scope fence by every lane,
-// and last the sequence number the host polls.
-__global__ void k_chunk_end_m(SysState* st, ChunkMirror* m) {
-  if (threadIdx.x == 0 && st->status != ST_RUNNING) st->stage = 3;
+// and last the sequence number the host polls.  err: of a chunk on the
+// persistent kernel, set when one of its waits ran out (null: a graph).
+__global__ void k_chunk_end_m(SysState* st, ChunkMirror* m, const int* err) {
+  if (threadIdx.x == 0) {
+    if (err && *err) st->status = ST_DEVICE_ERR;
+    if (st->status != ST_RUNNING) st->stage = 3;
+  }
   __syncwarp();
   static_assert(sizeof(SysState) % 8 == 0, "SysState is copied in 8-byte words");
   const unsigned long long* src = reinterpret_cast<const unsigned long long*>(st);
@@ -954,7 +952,16 @@ cudaError_t PcgSolver::alloc(bool mixed) {
     NLGB_CUDA_TRY(cudaMallocHost(&st_host_, sizeof(SysState) + 16));
     NLGB_CUDA_TRY(cudaEventCreate(&ev0_));
     NLGB_CUDA_TRY(cudaEventCreate(&ev1_));
-    if (tables_.usable()) NLGB_CUDA_TRY(cudaMalloc(&exch_, persist_bytes(n_, n_tiles_)));
+    if (tables_.usable()) {
+      const cudaError_t e = cudaMalloc(&exch_, persist_bytes(n_, n_tiles_));
+      if (e == cudaErrorMemoryAllocation) {   // no room: the graph runs
+        cudaGetLastError();
+        exch_ = nullptr;
+        for (PersistPlan& p : plan_) p.usable = false;
+      } else {
+        NLGB_CUDA_TRY(e);
+      }
+    }
   }
   if (mixed && !mixed_alloc_) {
     const size_t n4 = (size_t)std::max(4, n_ + 4) * sizeof(float);
@@ -1194,7 +1201,8 @@ cudaError_t ViewGraph::build(const SysView& v, bool mixed) {
     n_fin = n_chk;
   }
   if (mirror_) {
-    void* aem[] = {&st, &mirror};
+    const int* err = nullptr;
+    void* aem[] = {&st, &mirror, &err};
     NLGB_CUDA_TRY(add_kernel(g, &n_end, n_fin, (const void*)k_chunk_end_m, 1, 32, aem));
   } else {
     NLGB_CUDA_TRY(add_kernel(g, &n_end, n_fin, (const void*)k_chunk_end, 1, 1, ae));
@@ -1250,21 +1258,17 @@ cudaError_t ViewGraph::launch(cudaStream_t s) {
   if (persistent()) {
     const long long budget = *reinterpret_cast<volatile long long*>(&mirror_->budget);
     k_chunk_start_m<<<1, 1, 0, s>>>(view_.st, mirror_, kUnrollPlain);
-    NLGB_CUDA_TRY(persist_chunk(view_, plan_[mixed_ ? 1 : 0], lay_, exch_, mixed_, std::max(1LL, budget),
-                                mixed_ ? kPersistChunkRounds : 1, s));
-    k_chunk_end_m<<<1, 32, 0, s>>>(view_.st, mirror_);
-    count_launches(2);
-    return cudaGetLastError();
+    return persist_head(std::max(1LL, budget), s);
   }
   if (!exec_) return cudaErrorInvalidValue;
   return cudaGraphLaunch(exec_, s);
 }
 
-void ViewGraph::persist_bind(const PersistTables& t, void* exch, const SysView& v, bool mixed) {
-  lay_ = t.layout();
+void ViewGraph::persist_bind(const PersistLayout& layout, const PersistPlan (&plan)[2], void* exch) {
+  lay_ = layout;
+  plan_[0] = plan[0];
+  plan_[1] = plan[1];
   exch_ = exch;
-  plan_[0] = t.plan(v.tile_rows, v.tpr, v.df ? kPersistDf : kPersistDouble);   // (a mixed system may end in FP64)
-  if (mixed) plan_[1] = t.plan(v.tile_rows, v.tpr, kPersistMixed);
 }
 
 void ViewGraph::account(long long iters_before, long long iters_after) {
@@ -1297,45 +1301,80 @@ cudaError_t ViewGraph::run(const SysView& v, long long iters, cudaStream_t s, fl
   return cudaSuccess;
 }
 
-cudaError_t persist_chunk(const SysView& v, const PersistPlan& plan, const PersistLayout& lay, void* exch,
-                          bool mixed, long long iters, int rounds, cudaStream_t s) {
-  PersistArgs pa;
-  std::memset(&pa, 0, sizeof(pa));
-  pa.s = v;
-  persist_bind(pa, exch);
-  pa.lay = lay;
-  pa.iters = iters;
-  const KernelSet ks = kernels_for(v.tpr, !mixed && v.df != 0);
-  const int vg = (v.n_tiles + vec_tiles_for(v.tile_rows) - 1) / vec_tiles_for(v.tile_rows);
+// What a chunk graph does, with launches of at most `iters` iterations of the
+// persistent kernel.  The stage after the system's last chunk (its mirror)
+// tells which kernels have nothing to do.
+cudaError_t ViewGraph::persist_head(long long iters, cudaStream_t s) {
+  const SysView& v = view_;
+  const KernelSet ks = kernels_for(v.tpr, !mixed_ && v.df != 0);
+  const int stage = mirror_->st.stage;
   SysState* st = v.st;
-  void* a1[] = {&pa.s};
+  void* a1[] = {&view_};
   void* ast[] = {&st};
-  long long launched = 0;
   auto go = [&](const void* fn, int grid, int block, void** args) {
-    ++launched;
+    count_launches(1);
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, s);
   };
-  if (mixed) {
+  count_launches(1);   // (the chunk's start)
+  if (mixed_ && stage == 0) {
     NLGB_CUDA_TRY(go(ks.mx_outer, v.n_tiles, kCTA, a1));
     NLGB_CUDA_TRY(go((const void*)k_mark_started, 1, 1, ast));
-  } else {
+  } else if (stage == 0) {
     NLGB_CUDA_TRY(go(ks.init_chunk, v.n_tiles, kCTA, a1));
+  } else if (stage == 4) {
+    const int vg = (v.n_tiles + vec_tiles_for(v.tile_rows) - 1) / vec_tiles_for(v.tile_rows);
     NLGB_CUDA_TRY(go(ks.resume_p, vg, kCTA, a1));
     NLGB_CUDA_TRY(go((const void*)k_resume_mark, 1, 1, ast));
   }
-  for (int k = 0; k < rounds; ++k) {
-    NLGB_CUDA_TRY(persist_launch(plan, pa, s));
-    if (mixed) {
-      NLGB_CUDA_TRY(go((const void*)k_mx_apply, vg, kCTA, a1));
-      NLGB_CUDA_TRY(go(ks.mx_outer, v.n_tiles, kCTA, a1));
-    }
+  iters_ = iters;
+  rounds_ = kPersistChunkRounds;
+  return persist_next(s);
+}
+
+cudaError_t ViewGraph::persist_next(cudaStream_t s) {
+  PersistArgs pa;
+  std::memset(&pa, 0, sizeof(pa));
+  pa.s = view_;
+  nlgb::persist_bind(pa, exch_);
+  pa.lay = lay_;
+  pa.iters = iters_;
+  launches_ = (launches_ + 1) & 0x3fffffffu;
+  if (launches_ == 0) launches_ = 1;
+  waiting_ = launches_;
+  pa.done = &mirror_->persist;
+  pa.done_value = launches_ << 2;
+  return persist_launch(plan_[mixed_ ? 1 : 0], pa, s);
+}
+
+cudaError_t ViewGraph::advance(cudaStream_t s) {
+  if (waiting_ == 0) return cudaSuccess;
+  const unsigned int done = __atomic_load_n(&mirror_->persist, __ATOMIC_ACQUIRE);
+  if ((done >> 2) != waiting_) return cudaSuccess;
+  waiting_ = 0;
+  const SysView& v = view_;
+  const KernelSet ks = kernels_for(v.tpr, !mixed_ && v.df != 0);
+  SysState* st = v.st;
+  void* a1[] = {&view_};
+  void* ast[] = {&st};
+  auto go = [&](const void* fn, int grid, int block, void** args) {
+    count_launches(1);
+    return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, s);
+  };
+  if ((done & 3u) == kPersistUpdate) {
+    const int vg = (v.n_tiles + vec_tiles_for(v.tile_rows) - 1) / vec_tiles_for(v.tile_rows);
+    NLGB_CUDA_TRY(go((const void*)k_mx_apply, vg, kCTA, a1));
+    NLGB_CUDA_TRY(go(ks.mx_outer, v.n_tiles, kCTA, a1));
+    if (--rounds_ > 0) return persist_next(s);
   }
   NLGB_CUDA_TRY(go(ks.fin_if, v.n_tiles, kCTA, a1));
-  if (!mixed) NLGB_CUDA_TRY(go((const void*)k_check, 1, 1, ast));
-  void* ae[] = {&st, &pa.err};
-  NLGB_CUDA_TRY(go((const void*)k_persist_end, 1, 1, ae));
-  count_launches(launched);
-  return cudaSuccess;
+  if (!mixed_) NLGB_CUDA_TRY(go((const void*)k_check, 1, 1, ast));
+  PersistArgs pa;
+  pa.s = view_;
+  nlgb::persist_bind(pa, exch_);
+  ChunkMirror* mirror = mirror_;
+  const int* err = pa.err;
+  void* ae[] = {&st, &mirror, &err};
+  return go((const void*)k_chunk_end_m, 1, 32, ae);
 }
 
 cudaError_t chunk_fallback_fp64(SysState* st, cudaStream_t s) {
@@ -1399,7 +1438,8 @@ cudaError_t ViewGraph::run_eager(cudaStream_t s, long long iters) {
   if (!mixed_) NLGB_CUDA_TRY(go((const void*)k_check, 1, 1, ae));
   if (mirror_) {
     ChunkMirror* mirror = mirror_;
-    void* aem[] = {&st, &mirror};
+    const int* err = nullptr;
+    void* aem[] = {&st, &mirror, &err};
     NLGB_CUDA_TRY(go((const void*)k_chunk_end_m, 1, 32, aem));
   } else {
     NLGB_CUDA_TRY(go((const void*)k_chunk_end, 1, 1, ae));

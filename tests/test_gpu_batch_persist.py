@@ -1,0 +1,80 @@
+"""Batches on the persistent single-system kernel (csrc/nlgb_batch.cu): its
+layouts (four tiles per CTA; one CTA, one cluster, cluster to grid at 64 / 65
+tiles, more than four tiles per CTA), more systems than run at a time, matrices
+used twice, mixed systems that continue in FP64, a layout changed between two
+batches, two threads with the same matrices, and both sides of the rule that
+chooses it -- the iterates of the single-system solver bit for bit."""
+import threading
+
+import numpy as np
+import pytest
+
+from graphitethree_gb300 import meshes, solver
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(kind, nx, ny, seed=3):
+    V, F = meshes.height_field(nx, ny, seed)
+    if kind == "lscm":
+        M, rhs, _ = solver.build_lscm(V, F)
+        return M, rhs
+    return solver.build_fairing(V, F, 1e-2)[0], 1e-2 * V[:, 0]
+
+
+def _check(systems, **kw):
+    want = [M.solve(b, **kw) for M, b in systems]
+    xs, infos, secs = solver.batch_solve([M for M, _ in systems], [b for _, b in systems], **kw)
+    assert secs > 0
+    for x, i, (y, j) in zip(xs, infos, want):
+        assert np.array_equal(x, y)
+        assert (i.status, i.iterations, i.refinement_steps) == (j.status, j.iterations, j.refinement_steps)
+
+
+@pytest.mark.parametrize("precision", ["double", "mixed", "df"])
+@pytest.mark.parametrize("sizes", [
+    [("fairing", 3, 3)], [("lscm", 4, 3), ("fairing", 32, 16)], [("fairing", 37, 17), ("fairing", 128, 64)],
+    [("fairing", 131, 64), ("lscm", 41, 29)], [("fairing", 363, 291)], [("fairing", 640, 600), ("fairing", 20, 20)]])
+def test_layouts(gpu_ok, sizes, precision):
+    _check([_system(*s) for s in sizes], precision=precision, max_iter=300)
+
+
+@pytest.mark.parametrize("n,side", [(40, 12), (400, 8)])   # here; in the batched kernel
+def test_more_systems_than_run_at_a_time(gpu_ok, n, side):
+    _check([_system("fairing", side + k % 7, side, k) for k in range(n)], precision="mixed")
+
+
+def test_a_matrix_twice_and_a_new_layout(gpu_ok):
+    M, b = _system("lscm", 60, 50)
+    F, c = _system("fairing", 150, 131)
+    _check([(M, b), (F, c), (M, 2.0 * b), (F, -c)])
+    M.set_layout(4, 256)
+    _check([(M, b), (F, c), (M, 2.0 * b)])
+
+
+def test_mixed_continues_in_fp64(gpu_ok):
+    _check([_system("lscm", 70, 60), _system("lscm", 30, 20)], precision="mixed", eps=1e-12)
+
+
+@pytest.mark.parametrize("max_iter", [0, 1, 1023, 1024, 1025])
+def test_iteration_limits(gpu_ok, max_iter):
+    _check([_system("lscm", 90, 80), _system("fairing", 40, 30)], max_iter=max_iter, eps=1e-13)
+
+
+def test_two_threads_share_matrices(gpu_ok):
+    systems = [_system("lscm", 50, 40), _system("fairing", 120, 100), _system("lscm", 33, 31)]
+    mats, bs = [M for M, _ in systems], [b for _, b in systems]
+    got = [None, None]
+
+    def run(k):
+        got[k] = [solver.batch_solve(mats[::1 - 2 * k], bs[::1 - 2 * k])[0][::1 - 2 * k] for _ in range(5)]
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    want = [M.solve(b)[0] for M, b in systems]
+    for k in range(2):
+        for xs in got[k]:
+            for x, y in zip(xs, want):
+                assert np.array_equal(x, y)
