@@ -133,18 +133,22 @@ __global__ void k_bi_init_scalar(KrView v) {
   st->status = ST_RUNNING;
 }
 
-// The vector kernels of the iteration (p, s, x/r): CTAs of 1024 threads, at
-// most one per SM.  Each reduces the partials of the SpMV or update before it
-// in its prologue and takes the scalar step itself; CTA 0 also writes the
-// scalars to the state, where only later kernels read them (rho alternates
-// between two slots; a status that turns while a CTA starts tells it to return,
-// which its own step would).  As one-CTA kernels between the vector kernels
-// the three scalar steps took 28 of the 128.6 us of an iteration on 1024 x 1024
-// unknowns; 120.5 us now (601 x 523: 81.0 -> 76.5).  One CTA per SM, because
-// the reduction costs each CTA about 1,000 cycles of the SM's FP64 pipe: three
-// CTAs of 512 threads 133.9 us, six of 256 140.5.
+// The vector kernels of the iteration (p, s, x/r): CTAs of 1024 threads, one
+// per SM, or of 256 up to kBiSmall rows per SM.  Each reduces the partials of
+// the SpMV or update before it in its prologue and takes the scalar step
+// itself; CTA 0 also writes the scalars to the state, where only later kernels
+// read them (rho alternates between two slots; a status that turns while a CTA
+// starts tells it to return, which its own step would).  As one-CTA kernels
+// between the vector kernels the three scalar steps took 28 of the 129 us of an
+// iteration on 1024 x 1024 unknowns; 120 us now.  One CTA per SM, because the
+// reduction costs each CTA about 1,000 cycles of the SM's FP64 pipe: three CTAs
+// of 512 threads 134 us, six of 256 140.  With few rows a CTA of 256 threads
+// starts and synchronises sooner (us per iteration, before, 256, 1024 threads):
+// 235 x 142 59.2, 51.2, 62.2; 400 x 380 65.0, 56.5, 65.4; 700 x 650 88.3, 75.0,
+// 81.8; 1024 x 1024 129.1, 122.2, 119.6.
 constexpr int kBiThreads = 1024;
 constexpr int kBiQuarters = kBiThreads / kCTA;
+constexpr int kBiSmall = 4096;
 
 // The sums of the tiles' partials (canon_reduce's order), in every thread.
 template <int K>
@@ -219,7 +223,7 @@ __global__ void __launch_bounds__(kBiThreads, 1) k_bi_p(KrView v, BiVecs w, long
   } else {
     beta = v.st->beta;
   }
-  rows_in_flight<4, 4>(step_lo(v) + (int)threadIdx.x, step_hi(v), kBiThreads,
+  rows_in_flight<4, 4>(step_lo(v) + (int)threadIdx.x, step_hi(v), (int)blockDim.x,
     [&](int i, double (&a)[4]) { a[0] = w.r[i]; a[1] = w.p[i]; a[2] = w.v[i]; a[3] = __ldg(v.dinv + i); },
     [&](int i, double (&a)[4]) {
       const double pi = a[0] + beta * (a[1] - omega * a[2]);
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(kBiThreads, 1) k_bi_s(KrView v, BiVecs w, long
     else v.st->status = ST_BREAKDOWN;
   }
   if (!ok) return;
-  rows_in_flight<4, 3>(step_lo(v) + (int)threadIdx.x, step_hi(v), kBiThreads,
+  rows_in_flight<4, 3>(step_lo(v) + (int)threadIdx.x, step_hi(v), (int)blockDim.x,
     [&](int i, double (&a)[3]) { a[0] = w.r[i]; a[1] = w.v[i]; a[2] = __ldg(v.dinv + i); },
     [&](int i, double (&a)[3]) {
       const double si = a[0] - alpha * a[1];
@@ -276,8 +280,8 @@ __global__ void __launch_bounds__(kBiThreads, 1) k_bi_xr(KrView v, BiVecs w) {
   wide_sums<2>(v, 1, o);
   const double alpha = v.st->alpha, omega = o[1] > 0.0 ? o[0] / o[1] : 0.0;
   if (blockIdx.x == 0 && threadIdx.x == 0) v.st->omega = omega;
-  const int qd = threadIdx.x / kCTA, t = threadIdx.x % kCTA;
-  for (int tile = (int)blockIdx.x * kBiQuarters + qd; tile < v.n_tiles; tile += (int)gridDim.x * kBiQuarters) {
+  const int quarters = (int)blockDim.x / kCTA, qd = threadIdx.x / kCTA, t = threadIdx.x % kCTA;
+  for (int tile = (int)blockIdx.x * quarters + qd; tile < v.n_tiles; tile += (int)gridDim.x * quarters) {
     const int lo = tile * v.tile_rows, hi = min(v.n, lo + v.tile_rows);
     double rr = 0.0, rhr = 0.0;
     rows_in_flight<2, 6>(lo + t, hi, kCTA,
@@ -704,23 +708,24 @@ cudaError_t krylov_solve(const DeviceCRS& A, const double* dinv, const double* b
     NLGB_KR_T((k_bi_init<T><<<n_tiles, kCTA, 0, s>>>(v, w)));
     k_bi_init_scalar<<<1, kCTA, 0, s>>>(v);
     launches += 2;
-    const int xr_ctas = std::min(sms, (n_tiles + kBiQuarters - 1) / kBiQuarters);
+    const int threads = n <= kBiSmall * sms ? kCTA : kBiThreads, quarters = threads / kCTA;
+    const int xr_ctas = std::min(threads == kCTA ? 2 * sms : sms, (n_tiles + quarters - 1) / quarters);
     int status = ST_RUNNING;
     long long it = 0;
     while (e == cudaSuccess && status == ST_RUNNING) {
       for (int c = 0; c < kChunk; ++c, ++it) {
         // (with a general preconditioner dinv is all ones: y = p, z = s,
         // then y = M^-1 p, z = M^-1 s)
-        k_bi_p<<<step_ctas, kBiThreads, 0, s>>>(v, w, it, c > 0);
+        k_bi_p<<<step_ctas, threads, 0, s>>>(v, w, it, c > 0);
         if (P && e == cudaSuccess) e = P->apply(w.p, w.y, s);
         NLGB_KR_T((k_bi_v<T><<<n_tiles, kCTA, 0, s>>>(v, w)));
-        k_bi_s<<<step_ctas, kBiThreads, 0, s>>>(v, w, it);
+        k_bi_s<<<step_ctas, threads, 0, s>>>(v, w, it);
         if (P && e == cudaSuccess) e = P->apply(w.r, w.z, s);
         NLGB_KR_T((k_bi_t<T><<<n_tiles, kCTA, 0, s>>>(v, w)));
-        k_bi_xr<<<xr_ctas, kBiThreads, 0, s>>>(v, w);
+        k_bi_xr<<<xr_ctas, threads, 0, s>>>(v, w);
         launches += 5;
       }
-      k_bi_end<<<1, kBiThreads, 0, s>>>(v, it - 1);
+      k_bi_end<<<1, kCTA, 0, s>>>(v, it - 1);
       launches += 1;
       if (e == cudaSuccess) e = cudaGetLastError();
       if (e == cudaSuccess) e = poll(&status);

@@ -1,6 +1,6 @@
 """BiCGSTAB's kernels (csrc/nlgb_krylov.cu) where their layout changes: one CTA
-to one per SM (256 rows each, 38,912 rows), tiles that do and do not fill the
-four quarters of a CTA, rows that do not divide, one or several threads per
+to one per SM (256 rows each, 38,912 rows), CTAs of 256 and of 1024 threads
+(622,592 rows), tiles that do and do not fill a CTA's quarters, rows that do not divide, one or several threads per
 row, and chunks of sixteen iterations cut anywhere -- against the definition
 (the true residual of the returned x) and the step count of the oracle's
 BiCGSTAB on the small systems."""
@@ -16,7 +16,8 @@ EPS = 1e-10
 
 @pytest.mark.parametrize("nx,ny,layout", [
     (1, 1, None), (16, 16, None), (257, 1, None), (40, 33, (1, 64)), (40, 33, (4, 256)), (40, 33, (32, 320)),
-    (73, 59, (2, 1024)), (256, 152, None), (1201, 33, (1, 192)), (311, 257, (1, 64)), (640, 611, None)])
+    (73, 59, (2, 1024)), (256, 152, None), (1201, 33, (1, 192)), (311, 257, (1, 64)), (640, 611, None),
+    (801, 777, None)])
 def test_kernels(gpu_ok, oracle_mod, nx, ny, layout):
     cd = systems.convection_diffusion(nx, ny, seed=nx + ny)
     b = cd.rhs[0]
