@@ -211,7 +211,8 @@ class PcgSolver {
   double *b_ = nullptr, *x_ = nullptr, *r_ = nullptr, *p_ = nullptr, *q_ = nullptr, *part_ = nullptr;
   float *r32_ = nullptr, *p32_ = nullptr, *q32_ = nullptr, *c32_ = nullptr;
   void* st_ = nullptr;          // SysState (device)
-  void* st_host_ = nullptr;     // pinned staging
+  void* st_host_ = nullptr;     // its copy on the host (pageable: pinning costs 300 us a solver)
+  void *mem_ = nullptr, *mem32_ = nullptr;   // one allocation for all of these, one for the floats
   const volatile int* abort_flag_ = nullptr;
   cudaGraphExec_t plain_exec_ = nullptr, mixed_exec_ = nullptr, df_exec_ = nullptr;
   cudaGraphExec_t cont_exec_ = nullptr, cont_df_exec_ = nullptr;

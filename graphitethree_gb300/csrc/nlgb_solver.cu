@@ -911,12 +911,11 @@ void PcgSolver::release() {
   if (cont_exec_) cudaGraphExecDestroy(cont_exec_);
   if (cont_df_exec_) cudaGraphExecDestroy(cont_df_exec_);
   plain_exec_ = mixed_exec_ = df_exec_ = cont_exec_ = cont_df_exec_ = nullptr;
-  cudaFree(b_); cudaFree(x_); cudaFree(r_); cudaFree(p_); cudaFree(q_); cudaFree(part_);
-  cudaFree(exch_);
-  exch_ = nullptr;
+  cudaFree(mem_);
+  cudaFree(mem32_);
+  mem_ = mem32_ = exch_ = nullptr;
   tables_.release();
-  cudaFree(r32_); cudaFree(p32_); cudaFree(q32_); cudaFree(c32_); cudaFree(st_);
-  if (st_host_) cudaFreeHost(st_host_);
+  ::operator delete(st_host_);
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
   b_ = x_ = r_ = p_ = q_ = part_ = nullptr;
@@ -939,36 +938,44 @@ cudaError_t PcgSolver::bind(DeviceCRS* A, cudaStream_t stream) {
   return alloc(false);
 }
 
+// One allocation each for the FP64 iteration and the mixed one's vectors: a
+// small solve through a fresh context spent 140 of 1,630 us on ten of them,
+// and as much on giving them back.
 cudaError_t PcgSolver::alloc(bool mixed) {
-  const size_t n8 = (size_t)std::max(2, n_ + 2) * sizeof(double);
+  auto up = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
   if (!x_) {
-    NLGB_CUDA_TRY(cudaMalloc(&b_, n8));
-    NLGB_CUDA_TRY(cudaMalloc(&x_, n8));
-    NLGB_CUDA_TRY(cudaMalloc(&r_, n8));
-    NLGB_CUDA_TRY(cudaMalloc(&p_, n8));
-    NLGB_CUDA_TRY(cudaMalloc(&q_, n8));
-    NLGB_CUDA_TRY(cudaMalloc(&part_, (size_t)n_tiles_ * kParts * sizeof(double)));
-    NLGB_CUDA_TRY(cudaMalloc(&st_, sizeof(SysState)));
-    NLGB_CUDA_TRY(cudaMallocHost(&st_host_, sizeof(SysState) + 16));
+    const size_t n8 = up((size_t)std::max(2, n_ + 2) * sizeof(double));
+    const size_t parts = up((size_t)n_tiles_ * kParts * sizeof(double)), st = up(sizeof(SysState));
+    const size_t exch = tables_.usable() ? persist_bytes(n_, n_tiles_) : 0;
+    char* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, 5 * n8 + parts + st + exch);
+    if (e == cudaErrorMemoryAllocation && exch > 0) {   // no room for the exchange area: the graph runs
+      cudaGetLastError();
+      for (PersistPlan& plan : plan_) plan.usable = false;
+      e = cudaMalloc(&p, 5 * n8 + parts + st);
+    }
+    NLGB_CUDA_TRY(e);
+    mem_ = p;
+    for (double** v : {&b_, &x_, &r_, &p_, &q_}) {
+      *v = reinterpret_cast<double*>(p);
+      p += n8;
+    }
+    part_ = reinterpret_cast<double*>(p);
+    st_ = p + parts;
+    exch_ = p + parts + st;      // (used where a plan is usable)
+    st_host_ = ::operator new(sizeof(SysState) + 16);
     NLGB_CUDA_TRY(cudaEventCreate(&ev0_));
     NLGB_CUDA_TRY(cudaEventCreate(&ev1_));
-    if (tables_.usable()) {
-      const cudaError_t e = cudaMalloc(&exch_, persist_bytes(n_, n_tiles_));
-      if (e == cudaErrorMemoryAllocation) {   // no room: the graph runs
-        cudaGetLastError();
-        exch_ = nullptr;
-        for (PersistPlan& p : plan_) p.usable = false;
-      } else {
-        NLGB_CUDA_TRY(e);
-      }
-    }
   }
   if (mixed && !mixed_alloc_) {
-    const size_t n4 = (size_t)std::max(4, n_ + 4) * sizeof(float);
-    NLGB_CUDA_TRY(cudaMalloc(&r32_, n4));
-    NLGB_CUDA_TRY(cudaMalloc(&p32_, n4));
-    NLGB_CUDA_TRY(cudaMalloc(&q32_, n4));
-    NLGB_CUDA_TRY(cudaMalloc(&c32_, n4));
+    const size_t n4 = up((size_t)std::max(4, n_ + 4) * sizeof(float));
+    char* p = nullptr;
+    NLGB_CUDA_TRY(cudaMalloc(&p, 4 * n4));
+    mem32_ = p;
+    for (float** v : {&r32_, &p32_, &q32_, &c32_}) {
+      *v = reinterpret_cast<float*>(p);
+      p += n4;
+    }
     mixed_alloc_ = true;
   }
   return cudaSuccess;
