@@ -382,21 +382,23 @@ __global__ void k_gm_start(KrView v, int first) {
   st->act[0] = 1;
 }
 
-// A step of a cycle is four kernels of one 1,024-thread CTA per SM (ten
+// A step of a cycle is four kernels of one 512-thread CTA per SM (ten
 // launches over the matrix's tiles before):
 //   k_gm_spmv    w = A u, and the partials of h = V^T w;
 //   k_gm_orth    h summed by every CTA, w -= V h, partials of h2 = V^T w;
 //   k_gm_orth    h2 summed, w -= V h2, partials of w.w;
-//   k_gm_next    the norm, V_{j+1} = w / ||w||, u = M^-1 V_{j+1}; one thread
+//   k_gm_next    the norm, V_{j+1} = w / ||w||, u = M^-1 V_{j+1}; one more CTA
 //                turns column j of H into the QR factors and decides whether
 //                the cycle goes on.
 // V fits L2 up to about 16 M entries; the FP64 pipe bounds the rest: 4 n (j + 1)
-// products per step, 32 of the 104 us a step takes at 314,323 rows (j = 15 on
+// products per step, 32 of the 98 us a step takes at 314,323 rows (j = 15 on
 // average).  What was slow before: a block sum per coefficient and tile of 384
 // rows cost three times its products (67 us per round), and the reductions and
 // the norm were kernels of one CTA.  Measured on GB300, convection-diffusion
-// 601 x 523, GMRES(30): 231 -> 104 us per step.
-constexpr int kGmThreads = 1024;
+// 601 x 523, GMRES(30): 231 -> 98 us per step (with 1,024 threads 108: a
+// group's eight sums cost every warp nine FP64 instructions, 2.4 us of the SM
+// with 32 warps).
+constexpr int kGmThreads = 512;
 constexpr int kGmWarps = kGmThreads / 32;
 
 // Sums of eight per-lane values over the warp: lane l returns value
@@ -540,45 +542,54 @@ __global__ void __launch_bounds__(kGmThreads, 1) k_gm_orth(KrView v, GmVecs w, i
   if ((threadIdx.x & 31) == 0) rr[threadIdx.x >> 5] = a;
   __syncthreads();
   if (threadIdx.x < 32) {
-    a = warp_sum(rr[threadIdx.x]);
+    a = warp_sum((int)threadIdx.x < kGmWarps ? rr[threadIdx.x] : 0.0);
     if (threadIdx.x == 0) v.mpart[(size_t)blockIdx.x * v.mstride] = a;
   }
 }
 
 // H_{j+1,j} = ||w||, V_{j+1} = w / it, u = M^-1 V_{j+1}; Givens rotations and
-// cycle control by one thread.
+// cycle control by the last CTA.
 __global__ void __launch_bounds__(kGmThreads, 1) k_gm_next(KrView v, GmVecs w, int j, int prec) {
   if (!step_active(v, j)) return;
-  __shared__ double nrm[1];
+  __shared__ double nrm[1], rotated;
   __shared__ double hc[kMaxRestart + 1], cs[kMaxRestart], sn[kMaxRestart];
   KrState* st = v.st;
   double* Hj = st->H + j * (kMaxRestart + 1);
-  const bool last = blockIdx.x == gridDim.x - 1;
-  if (last && (int)threadIdx.x <= j) {       // column j and the previous rotations
-    hc[threadIdx.x] = Hj[threadIdx.x];
-    if ((int)threadIdx.x < j) { cs[threadIdx.x] = st->cs[threadIdx.x]; sn[threadIdx.x] = st->sn[threadIdx.x]; }
+  const bool last = blockIdx.x == gridDim.x - 1;   // no rows: column j and the rotations
+  if (last) {
+    if ((int)threadIdx.x <= j) {
+      hc[threadIdx.x] = Hj[threadIdx.x];
+      if ((int)threadIdx.x < j) { cs[threadIdx.x] = st->cs[threadIdx.x]; sn[threadIdx.x] = st->sn[threadIdx.x]; }
+    }
+    __syncthreads();
+    if (threadIdx.x == 32) {                       // the previous rotations, while warp 0 sums
+      double a = hc[0];
+      for (int k = 0; k < j; ++k) {
+        const double b = hc[k + 1], c = cs[k], s = sn[k];
+        const double up = c * a + s * b;
+        Hj[k] = up;
+        a = -s * a + c * b;
+      }
+      rotated = a;
+    }
   }
   step_sums(v, 0, nrm);
   const double hn = sqrt(nrm[0]);
-  if (hn > 0.0) {                // (a lucky breakdown, H_{j+1,j} = 0, leaves w)
-    double* Wn = w.V + (size_t)(j + 1) * w.ld;
-    const double inv = 1.0 / hn;
-    const int hi = step_hi(v);
-    for (int r = step_lo(v) + (int)threadIdx.x; r < hi; r += kGmThreads) {
-      const double x = Wn[r] * inv;
-      Wn[r] = x;
-      if (prec) w.u[r] = v.dinv[r] * x;
+  if (!last) {
+    if (hn > 0.0) {              // (a lucky breakdown, H_{j+1,j} = 0, leaves w)
+      double* Wn = w.V + (size_t)(j + 1) * w.ld;
+      const double inv = 1.0 / hn;
+      const int hi = step_hi(v);
+      for (int r = step_lo(v) + (int)threadIdx.x; r < hi; r += kGmThreads) {
+        const double x = Wn[r] * inv;
+        Wn[r] = x;
+        if (prec) w.u[r] = v.dinv[r] * x;
+      }
     }
+    return;
   }
-  if (!last || threadIdx.x != 0) return;
-  // previous rotations on column j, then the new one
-  double a = hc[0];
-  for (int k = 0; k < j; ++k) {
-    const double b = hc[k + 1], c = cs[k], s = sn[k];
-    const double up = c * a + s * b;
-    Hj[k] = up;
-    a = -s * a + c * b;
-  }
+  if (threadIdx.x != 0) return;
+  const double a = rotated;      // (step_sums ends with a barrier)
   const double b = hn;
   const double den = hypot(a, b);
   const double c = den > 0.0 ? a / den : 1.0, s = den > 0.0 ? b / den : 0.0;
@@ -749,7 +760,7 @@ cudaError_t krylov_solve(const DeviceCRS& A, const double* dinv, const double* b
         NLGB_KR_T((k_gm_spmv<T><<<step_ctas, kGmThreads, 0, s>>>(v, w, j)));
         k_gm_orth<<<step_ctas, kGmThreads, 0, s>>>(v1, w, j, 0, v.mpart);        // CGS2
         k_gm_orth<<<step_ctas, kGmThreads, 0, s>>>(v, w, j, 1, v1.mpart);
-        k_gm_next<<<step_ctas, kGmThreads, 0, s>>>(v, w, j, P ? 0 : 1);
+        k_gm_next<<<step_ctas + 1, kGmThreads, 0, s>>>(v, w, j, P ? 0 : 1);
         launches += 4;
       }
       k_gm_solve_y<<<1, 32, 0, s>>>(v);
