@@ -750,10 +750,8 @@ int sm_count() {
 }
 
 // Expected time of a system there, up to a factor: iterations of a Jacobi-CG on
-// a surface (sqrt(n)) times the time of one, us (kSharedTiles' figures).
-double persist_time(const SysView& v) {
-  return std::sqrt((double)v.n) * (5.0 + 1.2 * (double)(persist_shared_slots(v.n_tiles) - 1));
-}
+// a surface (sqrt(n)) times the time of one.
+double persist_time(const SysView& v) { return std::sqrt((double)v.n) * persist_iteration_us(v.n_tiles); }
 
 }  // namespace
 

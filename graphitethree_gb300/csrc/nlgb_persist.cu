@@ -124,10 +124,10 @@ size_t smem_bytes(int slots, int R, int halo, size_t word) {
 
 }  // namespace
 
-int persist_shared_slots(int n_tiles) {
+double persist_iteration_us(int n_tiles) {
   const int most = n_tiles <= kPersistClusterTiles ? kPersistCluster : 151;
   const int ctas = std::max(1, std::min((n_tiles + kSharedTiles - 1) / kSharedTiles, most));
-  return (n_tiles + ctas - 1) / ctas;
+  return 5.0 + 1.2 * (double)((n_tiles + ctas - 1) / ctas - 1);   // (kSharedTiles' figures)
 }
 
 void PersistTables::release() {

@@ -41,8 +41,8 @@ inline void persist_bind(PersistArgs& a, void* exch) {
   a.zslot = a.ctl + 16;
   a.err = reinterpret_cast<int*>(a.zslot + a.s.n);
 }
-// Tiles per CTA of a system that shares the GPU (PersistTables::build).
-int persist_shared_slots(int n_tiles);
+// About the time of an iteration of a system that shares the GPU, us.
+double persist_iteration_us(int n_tiles);
 cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& a, cudaStream_t s);
 // The kernel for a layout (nlgb_persist_*.cu): nc rows per lane group in registers.
 const void* persist_kernel_f64(int tpr, bool cluster, int nc);

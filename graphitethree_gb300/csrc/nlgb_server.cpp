@@ -148,6 +148,7 @@ struct nlgb_server_s {
   nlgb_server_config cfg;
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
+  std::atomic<bool> graph_chunks{false};   // the chunks run as graphs now
   std::thread th;
   bool stop = false;
   bool aborting = false;
@@ -252,6 +253,7 @@ void add_used(nlgb_server_s* S, long long delta) {
 // ~608 slots: ~160 kB).
 constexpr double kServiceFloorBytes = 1.6e5;
 constexpr long long kProbeIters = 16;      // SRPT: first epoch of a new system
+constexpr double kGraphIterationUs = 30.0;    // of up to 16 systems on lanes of graph chunks
 constexpr int kReserveCtas = 16;           // persistent-kernel slots left to system builds
 constexpr long long kUnrollPlainIters = 4;  // a chunk pauses on whole passes of 4 iterations
 constexpr int kAdmitters = 4;               // admission threads of the batched server
@@ -678,7 +680,7 @@ void admitter(nlgb_server_s* S) {
           if (pick->exch) {
             pick->graphs[k]->persist_bind(pick->tables.layout(), pick->plan,
                                           static_cast<char*>(pick->exch) + (size_t)k * exchange_bytes(*pick));
-            pick->graphs[k]->persist(true);
+            pick->graphs[k]->persist(!S->graph_chunks.load());   // else its graph is wanted first
           }
           ok = pick->graphs[k]->prepare(pick->slots[k].view, pick->slots[k].mixed, m, su) == cudaSuccess;
         }
@@ -1028,15 +1030,23 @@ void worker_streams(nlgb_server_s* S) {
   const long long cta_cap = S->cfg.chunk_cta_budget < 0 ? phase_resident_slots()
                                                         : (long long)S->cfg.chunk_cta_budget;
   long long running_ctas = 0;
-  // Chunks run on the persistent kernel while every unfinished system fits it:
-  // 8 to 10 us per iteration of 2k to 33k rows, against 30 us on 16 lanes of
-  // graphs, and no graph to instantiate (which also held a burst's other
-  // requests back for up to 50 ms behind the first one's chunk).  24 requests
-  // of 1k to 20k vertices at once: 222 -> 65 ms, their median latency 72 ->
-  // 9 ms.  A chunk's CTAs each need a whole SM and wait for one another, so
-  // the chunks in flight share out the SMs, and they never run beside graph
-  // chunks, whose kernels would leave no SM empty.
+  // Chunks run on the persistent kernel or as graphs, all of them one way at a
+  // time: a persistent chunk's CTAs each need a whole SM and wait for one
+  // another, so these chunks share out the SMs, and kernels of graph chunks
+  // beside them would leave no SM empty.  Persistent chunks need an iteration
+  // time of 8 to 10 us (2k to 33k rows) on their SMs, graph chunks 30 us on 16
+  // lanes whatever the size, and a graph to instantiate (which also held a
+  // burst's other requests back for up to 50 ms behind the first one's chunk).
+  // So the persistent kernel it is when every unfinished system fits it and an
+  // iteration of all of them takes it no longer than the graphs (up to 1.5
+  // times before changing over, which waits for the chunks in flight).
+  // 24 requests of 1k to 20k vertices at once: 222 -> 65 ms, median latency
+  // 72 -> 9 ms.  Streams of requests, mean latency with graphs alone -> with
+  // the persistent kernel alone -> with the rule: 150 of 1k to 60k vertices at
+  // 100 a second 105 -> 109 -> 95 ms; 100 of 20k to 60k at 40 a second 390 ->
+  // 859 -> 275 ms.
   int n_sm = 0, sms_busy = 0, graphs_busy = 0;
+  bool persist = true;
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, S->device);
   auto ctas_of = [](const Req* r) {
     return ((long long)r->A.n + r->A.tile_rows - 1) / std::max(1, r->A.tile_rows);
@@ -1207,10 +1217,21 @@ void worker_streams(nlgb_server_s* S) {
       continue;
     }
     // give every free lane the least-work system that is not running
-    bool persist = n_busy < ns;
-    for (Req* r : S->active)
-      for (int k = 0; persist && k < r->n_rhs; ++k)
-        persist = r->sys_done[k] || r->graphs[k]->persist_ctas(r->mixed_now[k] != 0) > 0;
+    if (n_busy < ns) {
+      bool fit = true;
+      double us = 0.0, systems = 0.0;
+      for (Req* r : S->active)
+        for (int k = 0; fit && k < r->n_rhs; ++k) {
+          if (r->sys_done[k]) continue;
+          const int c = r->graphs[k]->persist_ctas(r->mixed_now[k] != 0);
+          fit = c > 0;
+          us += (double)c * persist_iteration_us(r->slots[k].view.n_tiles) / (double)std::max(1, n_sm);
+          systems += 1.0;
+        }
+      const double graph_us = kGraphIterationUs * std::max(1.0, systems / (double)std::min(ns, 16));
+      persist = fit && us <= (persist ? 1.5 : 1.0) * graph_us;
+      S->graph_chunks.store(!persist);
+    }
     for (Lane& l : lanes) {
       if (l.r || e != cudaSuccess) continue;
       if (persist ? graphs_busy > 0 : sms_busy > 0) break;   // the other kind's chunks end first

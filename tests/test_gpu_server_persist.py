@@ -61,3 +61,12 @@ def test_load_changes(gpu_ok):
     _check(srv, small + [large] + small, "mixed")
     _check(srv, [large] + small, "mixed")
     srv.close()
+
+
+def test_more_work_than_the_persistent_kernel_gains_on(gpu_ok):
+    """Enough mid-size systems that their chunks run as graphs, then the last
+    of them on the persistent kernel again."""
+    srv = solver.Server(precision="double", epoch_ms=1.0)
+    _check(srv, [systems.fairing_system(360 + 4 * i, 300, seed=i, n_rhs=1) for i in range(12)] +
+           [systems.fairing_system(60, 50 + i, seed=i, n_rhs=1) for i in range(8)], "double")
+    srv.close()
