@@ -124,15 +124,17 @@ int nlgb_spmv32_timed(nlgb_matrix A, const float* x, float* y, int reps, double*
 int nlgb_solve(nlgb_matrix A, const double* b, double* x, const nlgb_params* prm,
                nlgb_result* res);
 
-/* ---- many independent solves in one persistent-kernel launch ----
+/* ---- many independent solves in one call ----
  * The batched form of nlSolveSystemIterative for many uneven systems, e.g.
  * the per-chart LSCM solves of mesh_make_atlas (called at
  * src/lib/OGF/mesh/commands/mesh_grob_surface_commands.cpp:724).  A[i] may
  * repeat (several right-hand sides of one matrix).  b[i], x[i]: host or
  * device vectors of A[i]'s size; x[i] is the initial guess on entry.  Each
  * system converges (or stops) on its own; results are bit-identical to
- * nlgb_solve on the same system.  *kernel_seconds: device time of the
- * launch (CUDA events). */
+ * nlgb_solve on the same system.  The systems run side by side on the
+ * persistent single-system kernel, or in one launch of the batched kernel
+ * when one of them is too large for it or there are very many small ones.
+ * *kernel_seconds: device time of the solves (CUDA events). */
 int nlgb_batch_solve(int n_sys, const nlgb_matrix* A, const double* const* b, double* const* x,
                      const nlgb_params* prm, nlgb_result* res, double* kernel_seconds);
 
@@ -189,7 +191,8 @@ typedef struct nlgb_server_s* nlgb_server;
 
 /* Scheduling of the batched server.  SRPT (shortest remaining processing
  * time, the default): `streams` CUDA streams each run one system at a time
- * as a chunk of CUDA-graph PCG iterations lasting about epoch_ms; whenever a
+ * as a chunk of PCG iterations (on the persistent single-system kernel or as
+ * a CUDA graph) lasting about epoch_ms; whenever a
  * stream is free it takes the system with the least estimated remaining work
  * (iterations left, extrapolated from the system's residual history, times
  * its bytes per iteration); a new system first gets a short probe (16
@@ -260,12 +263,12 @@ typedef struct {
     double    algo_bytes;        /* algorithmic HBM bytes over all systems     */
     size_t    peak_bytes;        /* peak admitted device footprint             */
     size_t    budget_bytes;
-    double    graph_s;           /* part of kernel_s spent in graph chunks
+    double    graph_s;           /* part of kernel_s spent in single-system chunks
                                     (large FP64 systems continued on the
                                     single-system graph executor once only
                                     such systems are left)                   */
     double    graph_algo_bytes;  /* part of algo_bytes: iterations run there   */
-    long long graph_epochs;      /* part of epochs run as graph chunks         */
+    long long graph_epochs;      /* part of epochs run as such chunks          */
     size_t    used_bytes;        /* device footprint admitted now              */
     double    byte_seconds;      /* admitted footprint integrated over time
                                     since the clock (re)started: the mean HBM
