@@ -10,6 +10,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -23,11 +24,11 @@ struct nlgb_matrix_s {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   std::mutex spmv_mu;
   long long spmvs = 0;       // products asked for so far
-  // batches: the tables of the layout (tpr, tile_rows), built by the first
+  // batches: the tables of the layout (tpr, tile_rows, tiles per CTA), built by the first
   std::mutex batch_mu;
-  PersistTables tables;
+  std::shared_ptr<PersistTables> tables;
   PersistPlan plans[3];
-  int tables_tpr = -1, tables_rows = 0;
+  int tables_tpr = -1, tables_rows = 0, tables_per_cta = 0;
   ~nlgb_matrix_s() {
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -307,13 +308,29 @@ namespace {
 // some system does not fit it in every precision, or an error (rc).
 bool batch_tables(int n_sys, const nlgb_matrix* A, const std::vector<SystemSlot>& slots, cudaStream_t s,
                   std::vector<PersistSystem>& ps, int* rc) {
+  // Tiles per CTA: the fewest with which the SMs hold every system at once (a
+  // cluster of more than nine CTAs has one of the eight GPCs to itself).
+  int dev = 0, sms = 0, per_cta = 1;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    *rc = NLGB_E_DEVICE;
+    return false;
+  }
+  for (; per_cta < kSharedTiles; ++per_cta) {
+    int used = 0;
+    for (const SystemSlot& sl : slots) {
+      const int c = persist_ctas_for(sl.view.n_tiles, per_cta, sms);
+      used += sl.view.n_tiles > kPersistClusterTiles ? c + 1 : c > 9 ? sms / 8 : c;
+    }
+    if (used <= sms) break;
+  }
   std::vector<nlgb_matrix> fresh(A, A + n_sys);
   std::sort(fresh.begin(), fresh.end());   // (one order for every thread's locks)
   fresh.erase(std::unique(fresh.begin(), fresh.end()), fresh.end());
   std::vector<std::unique_lock<std::mutex>> held;
   for (nlgb_matrix m : fresh) held.emplace_back(m->batch_mu);
-  fresh.erase(std::remove_if(fresh.begin(), fresh.end(), [](nlgb_matrix m) {
-    return m->tables_tpr == m->A.tpr && m->tables_rows == m->A.tile_rows;
+  fresh.erase(std::remove_if(fresh.begin(), fresh.end(), [per_cta](nlgb_matrix m) {
+    return m->tables_tpr == m->A.tpr && m->tables_rows == m->A.tile_rows && m->tables_per_cta == per_cta;
   }), fresh.end());
   if (!fresh.empty()) {
     std::vector<int> most(fresh.size(), 0);
@@ -323,7 +340,8 @@ bool batch_tables(int n_sys, const nlgb_matrix* A, const std::vector<SystemSlot>
     for (size_t i = 0; i < fresh.size() && e == cudaSuccess; ++i) {
       const DeviceCRS& M = fresh[i]->A;
       fresh[i]->tables_tpr = -1;
-      e = fresh[i]->tables.begin(M, M.tile_rows, std::max(1, (M.n + M.tile_rows - 1) / M.tile_rows), s, true, d + i);
+      fresh[i]->tables = std::make_shared<PersistTables>();
+      e = fresh[i]->tables->begin(M, M.tile_rows, std::max(1, (M.n + M.tile_rows - 1) / M.tile_rows), s, per_cta, d + i);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(most.data(), d, sizeof(int) * most.size(), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -334,16 +352,18 @@ bool batch_tables(int n_sys, const nlgb_matrix* A, const std::vector<SystemSlot>
     }
     for (size_t i = 0; i < fresh.size(); ++i) {
       nlgb_matrix m = fresh[i];
-      m->tables.end(most[i], s);
-      for (int k = 0; k < 3; ++k) m->plans[k] = m->tables.plan(m->A.tile_rows, m->A.tpr, k);
+      m->tables->end(most[i], s);
+      for (int k = 0; k < 3; ++k) m->plans[k] = m->tables->plan(m->A.tile_rows, m->A.tpr, k);
       m->tables_tpr = m->A.tpr;
       m->tables_rows = m->A.tile_rows;
+      m->tables_per_cta = per_cta;
     }
   }
   bool fit = true;
   for (int i = 0; i < n_sys; ++i) {
     const nlgb_matrix m = A[i];
-    ps[i].layout = m->tables.layout();
+    ps[i].tables = m->tables;
+    ps[i].layout = m->tables->layout();
     ps[i].plan[0] = m->plans[slots[i].df ? kPersistDf : kPersistDouble];
     ps[i].plan[1] = m->plans[kPersistMixed];
     ps[i].view = slots[i].view;

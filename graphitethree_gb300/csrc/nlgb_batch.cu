@@ -809,6 +809,13 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     return persist_time(systems[a].view) > persist_time(systems[b].view);
   });
+  // with room for all at once the clusters go first: spread CTAs of the grids
+  // would leave no GPC with enough free SMs
+  int all = 0;
+  for (const PersistSystem& p : systems) all += p.plan[p.mixed ? 1 : 0].grid;
+  if (all <= n_sm)
+    std::stable_partition(order.begin(), order.end(),
+                          [&](int i) { return systems[i].plan[systems[i].mixed ? 1 : 0].cluster; });
   for (int i = 0; i < n && ok(e); ++i) {
     graphs.emplace_back(new ViewGraph());
     graphs.back()->persist_bind(systems[i].layout, systems[i].plan, exch + at[(size_t)i]);

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <vector>
 
 #include "nlgb_core.cuh"
@@ -195,6 +196,7 @@ cudaError_t chunk_fallback_fp64(SysState* st, cudaStream_t s);
 // Many systems on the persistent single-system kernel (nlgb_persist.cuh), each
 // by itself on a few SMs, as many at a time as the SMs allow.
 struct PersistSystem {
+  std::shared_ptr<const PersistTables> tables;   // (another thread may replace the matrix's own)
   PersistLayout layout;
   PersistPlan plan[2];         // FP64 or double-float; mixed
   SysView view{};              // started (SystemSlot::start)

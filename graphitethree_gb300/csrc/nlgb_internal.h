@@ -151,12 +151,12 @@ class PersistTables {
   PersistTables(const PersistTables&) = delete;
   PersistTables& operator=(const PersistTables&) = delete;
   // Lays a matrix out for the persistent kernel; usable() tells whether it
-  // fits (sizes and halos).  shared: for a system that shares the GPU with
-  // others (fewer CTAs, more tiles on each).
-  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared = false);
+  // fits (sizes and halos).  per_cta: tiles on a CTA (more where the GPU has
+  // fewer SMs than that takes).
+  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta = 1);
   // The same in two steps, for many matrices with one synchronisation: begin
   // queues the work and raises *most (device, zero before), end takes its value.
-  cudaError_t begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared, int* most);
+  cudaError_t begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta, int* most);
   void end(int most, cudaStream_t s);
   bool usable() const { return lay_.ctas > 0; }
   const PersistLayout& layout() const { return lay_; }

@@ -9,12 +9,6 @@ namespace nlgb {
 namespace {
 
 constexpr int kPrepThreads = 512;
-// Tiles per CTA of a system that shares the GPU: a CTA takes about 5 us per
-// iteration and 1.2 us more for every tile, so more tiles use fewer SMs per
-// system and fewer tiles finish one sooner.  24 requests of 1k to 20k vertices
-// with 2, 3, 4 and 6 tiles: 106, 80, 71, 66 ms; 6 requests of 1k to 4k: 8.4,
-// 8.5, 8.8, 10.4 ms.
-constexpr int kSharedTiles = 4;
 
 // ---------------------------------------------------------------------------
 // Tables of one matrix (PersistLayout), one CTA per CTA of the solve.
@@ -124,9 +118,13 @@ size_t smem_bytes(int slots, int R, int halo, size_t word) {
 
 }  // namespace
 
+int persist_ctas_for(int n_tiles, int per_cta, int sms) {
+  const int most = n_tiles <= kPersistClusterTiles ? kPersistCluster : sms - 1;
+  return std::min((n_tiles + per_cta - 1) / per_cta, most);
+}
+
 double persist_iteration_us(int n_tiles) {
-  const int most = n_tiles <= kPersistClusterTiles ? kPersistCluster : 151;
-  const int ctas = std::max(1, std::min((n_tiles + kSharedTiles - 1) / kSharedTiles, most));
+  const int ctas = std::max(1, persist_ctas_for(n_tiles, kSharedTiles, 152));
   return 5.0 + 1.2 * (double)((n_tiles + ctas - 1) / ctas - 1);   // (kSharedTiles' figures)
 }
 
@@ -143,11 +141,11 @@ void PersistTables::release(cudaStream_t s) {
   release();
 }
 
-cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared) {
+cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta) {
   int most = 0, *d = nullptr;
   NLGB_CUDA_TRY(cudaMallocAsync((void**)&d, sizeof(int), s));
   cudaError_t e = cudaMemsetAsync(d, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = begin(A, tile_rows, n_tiles, s, shared, d);
+  if (e == cudaSuccess) e = begin(A, tile_rows, n_tiles, s, per_cta, d);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&most, d, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaFreeAsync(d, s);
@@ -156,14 +154,13 @@ cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles,
   return cudaSuccess;
 }
 
-cudaError_t PersistTables::begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, bool shared,
+cudaError_t PersistTables::begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta,
                                  int* most) {
   release();
   int sms = 0, smem_max = 0;
   if (A.n <= 0 || A.nnz <= 0 || A.n != A.m || tile_rows > 512 || !device_limits(&sms, &smem_max)) return cudaSuccess;
   cluster_ = n_tiles <= kPersistClusterTiles;
-  const int most_ctas = cluster_ ? kPersistCluster : sms - 1;
-  const int ctas = std::min(shared ? (n_tiles + kSharedTiles - 1) / kSharedTiles : n_tiles, most_ctas);
+  const int ctas = persist_ctas_for(n_tiles, per_cta, sms);
   if (ctas < 1) return cudaSuccess;
   const int slots = (n_tiles + ctas - 1) / ctas;
   const int cap = slots * tile_rows;

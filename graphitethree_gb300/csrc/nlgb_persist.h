@@ -41,6 +41,14 @@ inline void persist_bind(PersistArgs& a, void* exch) {
   a.zslot = a.ctl + 16;
   a.err = reinterpret_cast<int*>(a.zslot + a.s.n);
 }
+// Tiles per CTA of a system that shares the GPU: a CTA takes about 5 us per
+// iteration and 1.2 us more for every tile, so more tiles use fewer SMs per
+// system and fewer tiles finish one sooner.  24 requests of 1k to 20k vertices
+// with 2, 3, 4 and 6 tiles: 106, 80, 71, 66 ms; 6 requests of 1k to 4k: 8.4,
+// 8.5, 8.8, 10.4 ms.
+constexpr int kSharedTiles = 4;
+// CTAs that own a system's tiles, with per_cta tiles on each or as many as there have to be.
+int persist_ctas_for(int n_tiles, int per_cta, int sms);
 // About the time of an iteration of a system that shares the GPU, us.
 double persist_iteration_us(int n_tiles);
 cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& a, cudaStream_t s);

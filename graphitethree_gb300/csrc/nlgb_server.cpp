@@ -283,7 +283,7 @@ size_t exchange_bytes(const Req& r) {
 // the request's systems fit it and the budget has room for them.
 cudaError_t persist_tables(nlgb_server_s* S, Req* r, cudaStream_t s) {
   const SysView& v = r->slots[0].view;
-  cudaError_t e = r->tables.build(r->A, v.tile_rows, v.n_tiles, s, true);
+  cudaError_t e = r->tables.build(r->A, v.tile_rows, v.n_tiles, s, kSharedTiles);
   if (e != cudaSuccess || !r->tables.usable()) return e;
   const size_t exch = exchange_bytes(*r) * (size_t)r->n_rhs, extra = r->tables.bytes() + exch;
   {

@@ -1,5 +1,5 @@
 """Batches on the persistent single-system kernel (csrc/nlgb_batch.cu): its
-layouts (four tiles per CTA; one CTA, one cluster, cluster to grid at 64 / 65
+layouts (one to four tiles per CTA; one CTA, one cluster, cluster to grid at 64 / 65
 tiles, more than four tiles per CTA), more systems than run at a time, matrices
 used twice, mixed systems that continue in FP64, a layout changed between two
 batches, two threads with the same matrices, and both sides of the rule that
@@ -78,3 +78,28 @@ def test_two_threads_share_matrices(gpu_ok):
         for xs in got[k]:
             for x, y in zip(xs, want):
                 assert np.array_equal(x, y)
+
+
+def test_threads_with_other_layouts_of_a_matrix(gpu_ok):
+    """A matrix alone (a tile per CTA) and among many (four): each batch keeps
+    the tables that it runs on while the other thread's replaces the matrix's."""
+    M, b = _system("lscm", 60, 50)
+    many = [(M, b)] + [_system("fairing", 90, 80 + k, k) for k in range(12)]
+    want = [m.solve(c)[0] for m, c in many]
+    bad = []
+
+    def run(systems, expect):
+        for _ in range(6):
+            xs = solver.batch_solve([m for m, _ in systems], [c for _, c in systems])[0]
+            bad.extend(k for k, (x, y) in enumerate(zip(xs, expect)) if not np.array_equal(x, y))
+    threads = [threading.Thread(target=run, args=a) for a in ((many[:1], want[:1]), (many, want))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 5, 9])
+def test_tiles_per_cta_follow_the_batch(gpu_ok, count):
+    _check([_system("lscm", 60, 50 + k, k) for k in range(count)] + [_system("fairing", 150, 131)])
