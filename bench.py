@@ -505,7 +505,7 @@ def profile_case(which):
         return
     if which == "batch_small":
         # one small LSCM system (4,604 unknowns, 36 tiles) as a batch: the
-        # persistent single-system kernel on a cluster of nine CTAs, 1000 FP64
+        # persistent single-system kernel on a cluster of 16 CTAs, 1000 FP64
         # iterations
         M, rhs, _ = solver.assemble(systems.lscm_system(48, 48, seed=1))
         xs, infos, ks = solver.batch_solve([M], [rhs[0]], max_iter=1000, eps=1e-30)
