@@ -160,6 +160,7 @@ struct SysView {
   const volatile int* abort_flag;   // host-mapped; nonzero -> stop
   long long budget;      // persistent kernel: iterations in this launch (> 0; else the launch's own)
   SellView sell;
+  const short* ci16;     // columns relative to the row, or null (mixed iteration of large systems)
 };
 
 // ---------------------------------------------------------------------------
@@ -264,13 +265,14 @@ __device__ __forceinline__ A subwarp_sum(A v) {
 // read-only path may return stale data there.  L1-cached gathers after the
 // team barrier's acquire measured the same on GB300.)
 // ---------------------------------------------------------------------------
-template <int T, typename VT, typename XT, typename A, bool kCoh = false>
-__device__ __forceinline__ A row_dot(const int* __restrict__ rp, const int* __restrict__ ci,
+template <int T, typename VT, typename XT, typename A, bool kCoh = false, typename CT = int>
+__device__ __forceinline__ A row_dot(const int* __restrict__ rp, const CT* __restrict__ ci,
                                      const VT* __restrict__ va, const XT* __restrict__ x,
                                      int row, bool valid, int lane) {
   A sum = A(0);
   if (valid) {
     const int k0 = __ldg(rp + row), k1 = __ldg(rp + row + 1);
+    const int origin = sizeof(CT) == 2 ? row : 0;   // 16-bit columns are relative to the row
     if constexpr (sizeof(VT) == 4) {
       // three nonzeros in flight: FP32 rows are bound by latency (FP64 ones by
       // the FP64 pipe, where this costs: 176 -> 180 us per iteration at
@@ -281,7 +283,7 @@ __device__ __forceinline__ A row_dot(const int* __restrict__ rp, const int* __re
         XT xc[3];
 #pragma unroll
         for (int u = 0; u < 3; ++u)
-          if (k + u * T < k1) { c[u] = __ldg(ci + k + u * T); av[u] = __ldg(va + k + u * T); }
+          if (k + u * T < k1) { c[u] = origin + (int)__ldg(ci + k + u * T); av[u] = __ldg(va + k + u * T); }
 #pragma unroll
         for (int u = 0; u < 3; ++u)
           if (k + u * T < k1) xc[u] = kCoh ? __ldcg(x + c[u]) : __ldg(x + c[u]);
@@ -292,7 +294,7 @@ __device__ __forceinline__ A row_dot(const int* __restrict__ rp, const int* __re
     } else {
 #pragma unroll 2
       for (int k = k0 + lane; k < k1; k += T) {
-        const int c = __ldg(ci + k);
+        const int c = origin + (int)__ldg(ci + k);
         const XT xc = kCoh ? __ldcg(x + c) : __ldg(x + c);
         sum = fma(A(__ldg(va + k)), A(xc), sum);
       }
@@ -307,8 +309,8 @@ __device__ __forceinline__ A row_dot(const int* __restrict__ rp, const int* __re
 // 7-nonzero Laplacian SpMV) and a "stream" layout staging each tile's
 // nonzeros in shared memory (3.3 vs 5.2 TB/s there, 2.6 vs 4.4 on the
 // 14-nonzero LSCM normal matrix).
-template <int T, typename VT, typename XT, typename A, bool kCoh, typename Epi>
-__device__ __forceinline__ void tile_rows_dot(const int* __restrict__ rp, const int* __restrict__ ci,
+template <int T, typename VT, typename XT, typename A, bool kCoh, typename CT, typename Epi>
+__device__ __forceinline__ void tile_rows_dot(const int* __restrict__ rp, const CT* __restrict__ ci,
                                               const VT* __restrict__ va, const XT* __restrict__ x,
                                               int lo, int hi, Epi&& epi) {
   const int sub = threadIdx.x / T, lane = threadIdx.x % T;
@@ -316,7 +318,7 @@ __device__ __forceinline__ void tile_rows_dot(const int* __restrict__ rp, const 
   for (int base = lo; base < hi; base += RPP) {
     const int row = base + sub;
     const bool valid = row < hi;
-    const A v = row_dot<T, VT, XT, A, kCoh>(rp, ci, va, x, row, valid, lane);
+    const A v = row_dot<T, VT, XT, A, kCoh, CT>(rp, ci, va, x, row, valid, lane);
     if (valid && lane == 0) epi(row, v);
   }
 }
@@ -777,15 +779,16 @@ __device__ void tile_mx_outer(const SysView& s, int tile, double (&out)[4]) {
 }
 
 // q32 = A32 p32 (FP32 row sums); returns sum p.q accumulated in FP64.
-template <int T, bool kCoh = false>
+template <int T, bool kCoh = false, bool C16 = false>
 __device__ double tile_mx_spmv_pq(const SysView& s, int tile) {
   const int lo = tile_lo(s, tile), hi = tile_hi(s, tile);
   double acc[1] = {0.0};
-  tile_rows_dot<T, float, float, float, kCoh>(s.rp, s.ci, s.va32, s.p32, lo, hi,
-    [&](int row, float qv) {
-      s.q32[row] = qv;
-      acc[0] += to_double_int(__ldcg(s.p32 + row) * qv);   // FP32 product, FP64 accumulation
-    });
+  const auto epi = [&](int row, float qv) {
+    s.q32[row] = qv;
+    acc[0] += to_double_int(__ldcg(s.p32 + row) * qv);   // FP32 product, FP64 accumulation
+  };
+  if constexpr (C16) tile_rows_dot<T, float, float, float, kCoh>(s.rp, s.ci16, s.va32, s.p32, lo, hi, epi);
+  else tile_rows_dot<T, float, float, float, kCoh>(s.rp, s.ci, s.va32, s.p32, lo, hi, epi);
   block_sum<1>(acc);
   return acc[0];
 }

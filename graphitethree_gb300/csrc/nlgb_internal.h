@@ -51,6 +51,8 @@ struct DeviceCRS {
   int* ci = nullptr;
   double* va = nullptr;
   float* va32 = nullptr;   // lazily built for the mixed-precision solver
+  short* ci16 = nullptr;   // columns relative to the row, for its large systems (crs_prepare_c16)
+  bool c16_tried = false;
   double* dinv = nullptr;  // Jacobi inverse diagonal (lazily built)
   float* dinv32 = nullptr;
   float2* vadf = nullptr;    // double-float copies (hi, lo) of va and dinv,
@@ -67,6 +69,9 @@ constexpr long long kSellMinNnz = 1LL << 21;
 // Builds the sliced layout; *usable false: the CRS kernels run (other threads
 // per row, small or uneven matrix, no memory for the copy).
 cudaError_t sell_prepare(DeviceCRS& A, bool* usable, cudaStream_t s);
+// 16-bit columns relative to the row, where the matrix is large and its
+// columns lie within 32,767 of the diagonal (A.ci16; null: the 32-bit ones).
+cudaError_t crs_prepare_c16(DeviceCRS& A, cudaStream_t s);
 void sell_free(SellLayout& L, cudaStream_t s, bool async);
 long long sell_bytes(const DeviceCRS& A);
 

@@ -375,6 +375,7 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
   r->t_prepared = S->now();
   bool dfl = false;   // false also when the matrix is outside double-float's range: FP64 runs
   if (e == cudaSuccess && prec == NL_GB300_PRECISION_DOUBLE_FLOAT) e = crs_prepare_df(r->A, &dfl, s);
+  if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && mixed) e = crs_prepare_c16(r->A, s);
   bool sell = false;  // the chunks' SpMV layout (false: CRS)
   if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && !mixed && !dfl) e = sell_prepare(r->A, &sell, s);
   if (e == cudaSuccess) {

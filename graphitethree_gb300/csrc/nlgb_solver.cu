@@ -423,10 +423,11 @@ __global__ void __launch_bounds__(kCTA) k_mx_outer(SysView s) {
 
 // q32 = A32 p32; stores the tiles' p.q partials (alpha is taken by every CTA
 // of k_mx_update_cr, as in the FP64 iteration).
-template <int T>
+// C16: with 16-bit columns (six bytes a nonzero instead of eight).
+template <int T, bool C16>
 __global__ void __launch_bounds__(kCTA) k_mx_spmv_pq(SysView s) {
   if (ld_status(s.st) != ST_RUNNING || ld_mode(s.st) != 1) return;
-  const double v = tile_mx_spmv_pq<T>(s, blockIdx.x);
+  const double v = tile_mx_spmv_pq<T, false, C16>(s, blockIdx.x);
   if (threadIdx.x == 0) __stcg(s.part + (size_t)blockIdx.x * kParts + kSlotPQ, v);
 }
 
@@ -493,6 +494,19 @@ __global__ void k_jacobi(int n, const int* __restrict__ rp, const int* __restric
   const double inv = (d != 0.0) ? 1.0 / d : 1.0;
   dinv[i] = inv;
   if (dinv32) dinv32[i] = float(inv);
+}
+
+// Columns relative to the row; *far: one does not fit.
+__global__ void k_ci16(int n, const int* __restrict__ rp, const int* __restrict__ ci, short* __restrict__ out, int* far) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  bool bad = false;
+  for (int k = rp[i]; k < rp[i + 1]; ++k) {
+    const int d = ci[k] - i;
+    bad |= d != (int)(short)d;
+    out[k] = (short)d;
+  }
+  if (bad) *far = 1;
 }
 
 __global__ void k_to_f32(long long n, const double* __restrict__ a, float* __restrict__ b) {
@@ -693,7 +707,7 @@ void crs_free(DeviceCRS& A) {
   if (!A.owns) { A = DeviceCRS(); return; }
   cudaFree(A.rp); cudaFree(A.ci); cudaFree(A.va); cudaFree(A.va32);
   cudaFree(A.dinv); cudaFree(A.dinv32);
-  cudaFree(A.vadf); cudaFree(A.dinvdf);
+  cudaFree(A.vadf); cudaFree(A.dinvdf); cudaFree(A.ci16);
   sell_free(A.sell, nullptr, false);
   A = DeviceCRS();
 }
@@ -701,7 +715,7 @@ void crs_free(DeviceCRS& A) {
 void crs_free_async(DeviceCRS& A, cudaStream_t s) {
   if (!A.owns) { A = DeviceCRS(); return; }
   for (void* p : {(void*)A.rp, (void*)A.ci, (void*)A.va, (void*)A.va32, (void*)A.dinv, (void*)A.dinv32,
-                  (void*)A.vadf, (void*)A.dinvdf})
+                  (void*)A.vadf, (void*)A.dinvdf, (void*)A.ci16})
     if (p) cudaFreeAsync(p, s);
   sell_free(A.sell, s, true);
   A = DeviceCRS();
@@ -710,6 +724,7 @@ void crs_free_async(DeviceCRS& A, cudaStream_t s) {
 long long device_bytes(const DeviceCRS& A) {
   long long b = (long long)(A.n + 1) * 4 + A.nnz * 12;
   if (A.va32) b += A.nnz * 4;
+  if (A.ci16) b += A.nnz * 2;
   if (A.dinv) b += (long long)A.n * 8;
   if (A.dinv32) b += (long long)A.n * 4;
   if (A.vadf) b += A.nnz * 8;
@@ -746,6 +761,41 @@ cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
     NLGB_CUDA_TRY(cudaGetLastError());
   }
   return cudaSuccess;
+}
+
+// From 2^21 nonzeros on: smaller matrices stay in L2, or run on the persistent
+// kernel with columns of its own.  us per mixed iteration, 32-bit -> 16-bit:
+// fairing 2048x2048 116.3 -> 108.6, LSCM 808x808 79.8 -> 73.9, fairing
+// 1024x1024 51.9 -> 50.7.  (The FP64 SpMV is bound by the FP64 pipe.)
+cudaError_t crs_prepare_c16(DeviceCRS& A, cudaStream_t s) {
+  if (A.c16_tried || !A.owns || A.n != A.m || A.nnz < (1LL << 21)) return cudaSuccess;
+  A.c16_tried = true;
+  int* far = nullptr;
+  int h = 0;
+  cudaError_t e = cudaMallocAsync((void**)&A.ci16, (size_t)A.nnz * sizeof(short), s);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    A.ci16 = nullptr;
+    return cudaSuccess;
+  }
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&far, sizeof(int), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(far, 0, sizeof(int), s);
+  if (e == cudaSuccess) {
+    k_ci16<<<(A.n + 255) / 256, 256, 0, s>>>(A.n, A.rp, A.ci, A.ci16, far);
+    count_launches(1);
+    e = cudaMemcpyAsync(&h, far, sizeof(int), cudaMemcpyDeviceToHost, s);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (far) cudaFreeAsync(far, s);
+  if ((e != cudaSuccess || h) && A.ci16) {
+    cudaFreeAsync(A.ci16, s);
+    A.ci16 = nullptr;
+  }
+  if (e == cudaErrorMemoryAllocation) {   // the 32-bit columns serve
+    cudaGetLastError();
+    e = cudaSuccess;
+  }
+  return e;
 }
 
 // Exponent range [2^-100, 2^100] for the double-float copies: the low
@@ -880,7 +930,7 @@ struct KernelSet {
 template <int T, bool D>
 static KernelSet kernel_set() {
   return {(const void*)k_init<T, D>, (const void*)k_spmv_pq<T, D>, (const void*)k_final<T, D>,
-          (const void*)k_mx_outer<T>, (const void*)k_mx_spmv_pq<T>, (const void*)k_update_xr<D>, (const void*)k_update_p<D>,
+          (const void*)k_mx_outer<T>, (const void*)k_mx_spmv_pq<T, false>, (const void*)k_update_xr<D>, (const void*)k_update_p<D>,
           (const void*)k_resume_p<D>, (const void*)k_init_chunk<T, D>, (const void*)k_final_if<T, D>};
 }
 template <bool D>
@@ -896,6 +946,19 @@ static KernelSet kernels_for_t(int tpr) {
 }
 static KernelSet kernels_for(int tpr, bool df) {
   return df ? kernels_for_t<true>(tpr) : kernels_for_t<false>(tpr);
+}
+
+// The FP32 SpMV for a system's columns.
+static const void* mx_spmv_kernel(const SysView& v) {
+  if (!v.ci16) return kernels_for(v.tpr, false).mx_spmv;
+  switch (v.tpr) {
+    case 1: return (const void*)k_mx_spmv_pq<1, true>;
+    case 2: return (const void*)k_mx_spmv_pq<2, true>;
+    case 4: return (const void*)k_mx_spmv_pq<4, true>;
+    case 8: return (const void*)k_mx_spmv_pq<8, true>;
+    case 16: return (const void*)k_mx_spmv_pq<16, true>;
+    default: return (const void*)k_mx_spmv_pq<32, true>;
+  }
 }
 
 constexpr int kUnrollPlain = 4;   // CG iterations per while-body pass
@@ -989,6 +1052,7 @@ static SysView make_view(DeviceCRS* A, int tile_rows, int n_tiles, double* b, do
   v.n = A->n; v.tile_rows = tile_rows; v.n_tiles = n_tiles; v.tpr = A->tpr;
   v.df = df ? 1 : 0;
   v.rp = A->rp; v.ci = A->ci; v.va = A->va; v.va32 = A->va32; v.vadf = A->vadf;
+  v.ci16 = A->ci16;
   v.dinv = A->dinv; v.dinv32 = A->dinv32; v.dinvdf = A->dinvdf;
   v.b = b; v.x = x; v.r = r; v.p = p; v.q = q;
   v.r32 = r32; v.p32 = p32; v.q32 = q32; v.c32 = c32;
@@ -1086,7 +1150,7 @@ cudaError_t PcgSolver::build_mixed_graph() {
   for (int u = 0; u < kUnrollInner; ++u) {
     cudaGraphNode_t n1, n2, n3;
     NLGB_CUDA_TRY(add_kernel(body, &n1, prev, (const void*)k_mx_update_p, vg, kCTA, a1));
-    NLGB_CUDA_TRY(add_kernel(body, &n2, n1, ks.mx_spmv, n_tiles_, kCTA, a1));
+    NLGB_CUDA_TRY(add_kernel(body, &n2, n1, mx_spmv_kernel(v), n_tiles_, kCTA, a1));
     void* acr[] = {&v, &h_upd, &use_handle};
     NLGB_CUDA_TRY(add_kernel(body, &n3, n2, (const void*)k_mx_update_cr, vg, kCTA, acr));
     prev = n3;
@@ -1185,7 +1249,7 @@ cudaError_t ViewGraph::build(const SysView& v, bool mixed) {
     for (int u = 0; u < kUnrollInner; ++u) {
       cudaGraphNode_t n1, n2, n3;
       NLGB_CUDA_TRY(add_kernel(body, &n1, prev, (const void*)k_mx_update_p, vg, kCTA, a1));
-      NLGB_CUDA_TRY(add_kernel(body, &n2, n1, ks.mx_spmv, v.n_tiles, kCTA, a1));
+      NLGB_CUDA_TRY(add_kernel(body, &n2, n1, mx_spmv_kernel(v), v.n_tiles, kCTA, a1));
       void* acr[] = {&view_, &h_upd, &use_handle};
       NLGB_CUDA_TRY(add_kernel(body, &n3, n2, (const void*)k_mx_update_cr, vg, kCTA, acr));
       prev = n3;
@@ -1230,7 +1294,7 @@ static bool same_view(const SysView& a, const SysView& b) {
          a.x == b.x && a.r == b.r && a.p == b.p && a.q == b.q && a.part == b.part && a.st == b.st &&
          a.va32 == b.va32 && a.dinv32 == b.dinv32 && a.r32 == b.r32 && a.p32 == b.p32 &&
          a.q32 == b.q32 && a.c32 == b.c32 && a.abort_flag == b.abort_flag &&
-         a.sell.shape == b.sell.shape && a.sell.ci == b.sell.ci && a.sell.va == b.sell.va;
+         a.ci16 == b.ci16 && a.sell.shape == b.sell.shape && a.sell.ci == b.sell.ci && a.sell.va == b.sell.va;
 }
 
 cudaError_t ViewGraph::prepare(const SysView& v, bool mixed) { return prepare(v, mixed, nullptr); }
@@ -1431,7 +1495,7 @@ cudaError_t ViewGraph::run_eager(cudaStream_t s, long long iters) {
         NLGB_CUDA_TRY(go(ks.update_p, vg, kCTA, a1));
       } else {
         NLGB_CUDA_TRY(go((const void*)k_mx_update_p, vg, kCTA, a1));
-        NLGB_CUDA_TRY(go(ks.mx_spmv, view_.n_tiles, kCTA, a1));
+        NLGB_CUDA_TRY(go(mx_spmv_kernel(view_), view_.n_tiles, kCTA, a1));
         NLGB_CUDA_TRY(go((const void*)k_mx_update_cr, vg, kCTA, acr));
         NLGB_CUDA_TRY(go((const void*)k_mx_apply, vg, kCTA, a1));   // return unless an update is due
         NLGB_CUDA_TRY(go(ks.mx_outer, view_.n_tiles, kCTA, a1));
@@ -1506,7 +1570,7 @@ cudaError_t PcgSolver::run_eager(bool mixed, bool df, SysState* h, bool cont) {
     for (int u = 0; u < (mixed ? kUnrollInner : kUnrollPlain); ++u) {
       if (mixed) {
         NLGB_CUDA_TRY(go((const void*)k_mx_update_p, vg, kCTA, a1));
-        NLGB_CUDA_TRY(go(ks.mx_spmv, n_tiles_, kCTA, a1));
+        NLGB_CUDA_TRY(go(mx_spmv_kernel(v), n_tiles_, kCTA, a1));
         NLGB_CUDA_TRY(go((const void*)k_mx_update_cr, vg, kCTA, acr));
         NLGB_CUDA_TRY(go((const void*)k_mx_apply, vg, kCTA, a1));   // return unless an update is due
         NLGB_CUDA_TRY(go(ks.mx_outer, n_tiles_, kCTA, a1));
@@ -1624,7 +1688,10 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
     bool sell = false;   // (false: the CRS kernels)
     NLGB_CUDA_TRY(sell_prepare(*A_, &sell, stream_));
   }
-  if (mixed && !persist && !eager_mode() && !mixed_exec_) NLGB_CUDA_TRY(build_mixed_graph());
+  if (mixed && !persist && !eager_mode() && !mixed_exec_) {
+    NLGB_CUDA_TRY(crs_prepare_c16(*A_, stream_));
+    NLGB_CUDA_TRY(build_mixed_graph());
+  }
   if (!mixed && !persist && !eager_mode() && !*plain) NLGB_CUDA_TRY(build_plain_graph(df));
   SysState* h = (SysState*)st_host_;
   std::memset(h, 0, sizeof(SysState));

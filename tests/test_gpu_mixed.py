@@ -84,3 +84,29 @@ def test_chunk_with_many_updates(gpu_ok):
     assert infos[0].status == info.status == "converged"
     assert infos[0].refinement_steps > 20
     _same((xs[0], infos[0]), (x, info))
+
+
+def _wide_band(n, offset):
+    """Rows of 5 and more nonzeros with the farthest at `offset`, 2^21 nonzeros and more."""
+    k = np.arange(n)
+    i, j, w = [k], [k], [np.full(n, 6.5)]
+    for d, v in ((1, -1.0), (700, -1.0), (offset, -1.0)):
+        a = np.arange(n - d)
+        i += [a, a + d]
+        j += [a + d, a]
+        w += [np.full(n - d, v)] * 2
+    return solver.Matrix(*systems.csr_from_coo(n, np.concatenate(i), np.concatenate(j), np.concatenate(w)))
+
+
+@pytest.mark.parametrize("threads", [1, 2, 8])
+@pytest.mark.parametrize("offset", [32767, 32768])   # 16-bit columns; one too far for them
+def test_columns_relative_to_the_row(gpu_ok, offset, threads):
+    n = 700000
+    b = np.sin(np.arange(n))
+    M = _wide_band(n, offset)
+    M.set_layout(threads, 0)
+    want = _eager(M, b)                    # before any graph: 32-bit columns
+    got = M.solve(b, precision="mixed")
+    assert got[1].status == "converged" and got[1].true_rel_residual <= 1e-10
+    _same(got, want)
+    _same(_eager(M, b), want)
