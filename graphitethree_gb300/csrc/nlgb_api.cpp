@@ -7,6 +7,7 @@
 #include "nlgb_sell.h"
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -22,8 +23,7 @@ struct nlgb_matrix_s {
   bool bound = false;
   cudaStream_t stream = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  std::mutex spmv_mu;
-  long long spmvs = 0;       // products asked for so far
+  std::atomic<long long> spmvs{0};   // products asked for so far
   // batches: the tables of the layout (tpr, tile_rows, tiles per CTA), built by the first
   std::mutex batch_mu;
   std::shared_ptr<PersistTables> tables;
@@ -83,13 +83,10 @@ struct Stage {
 // matrix is multiplied in its sliced layout (nlgb_sell.cu): laying it out
 // costs about as much as four products, a user of one or two never pays it.
 cudaError_t spmv_many(nlgb_matrix M, const double* x, double* y, int count) {
-  bool sell = false;
-  {
-    std::lock_guard<std::mutex> lk(M->spmv_mu);
-    M->spmvs += count;
-    if (M->spmvs > 4) NLGB_CUDA_TRY(sell_prepare(M->A, &sell, M->stream));
-  }
-  for (int r = 0; r < count; ++r) NLGB_CUDA_TRY(sell ? sell_spmv64(M->A, x, y, M->stream) : spmv64(M->A, x, y, M->stream));
+  SellView sell{};
+  if ((M->spmvs += count) > 4) NLGB_CUDA_TRY(sell_prepare(M->A, &sell, M->stream));
+  for (int r = 0; r < count; ++r)
+    NLGB_CUDA_TRY(sell.va ? sell_spmv64(M->A, sell, x, y, M->stream) : spmv64(M->A, x, y, M->stream));
   return cudaSuccess;
 }
 

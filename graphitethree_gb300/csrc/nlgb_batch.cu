@@ -26,7 +26,6 @@
 #include "nlgb_core.cuh"
 #include "nlgb_internal.h"
 #include "nlgb_persist.h"
-#include "nlgb_sell.h"
 
 #include <algorithm>
 #include <cmath>
@@ -931,8 +930,6 @@ cudaError_t SystemSlot::alloc(DeviceCRS* Am, bool mx, cudaStream_t s, bool dfl) 
   view.tpr = A->tpr;
   view.rp = A->rp; view.ci = A->ci; view.va = A->va; view.va32 = A->va32;
   view.dinv = A->dinv; view.dinv32 = A->dinv32;
-  view.sell = sell_view(*A);
-  view.ci16 = A->ci16;
   if (df) {
     view.df = 1;
     view.vadf = A->vadf;

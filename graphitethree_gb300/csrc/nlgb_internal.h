@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -10,6 +12,7 @@ namespace nlgb {
 
 struct SysState;
 struct SysView;
+struct SellView;
 
 // Thread-local error text reported by nlGetErrorString()/nlgb_last_error().
 void set_error(const std::string& msg);
@@ -63,15 +66,20 @@ struct DeviceCRS {
   int max_row = 0;         // longest row (nnz)
   bool owns = true;        // false: a view sharing another matrix's arrays
   SellLayout sell;
+  // Held while a part above is built on demand: a product and a solve of one
+  // matrix may ask for the same part from two threads.
+  std::shared_ptr<std::mutex> lazy = std::make_shared<std::mutex>();
 };
 // Matrices below this have SpMVs of a few microseconds, bound by latency.
 constexpr long long kSellMinNnz = 1LL << 21;
-// Builds the sliced layout; *usable false: the CRS kernels run (other threads
-// per row, small or uneven matrix, no memory for the copy).
-cudaError_t sell_prepare(DeviceCRS& A, bool* usable, cudaStream_t s);
-// 16-bit columns relative to the row, where the matrix is large and its
-// columns lie within 32,767 of the diagonal (A.ci16; null: the 32-bit ones).
-cudaError_t crs_prepare_c16(DeviceCRS& A, cudaStream_t s);
+// Builds the sliced layout; on return it is complete, for any stream.  *view
+// without values: the CRS kernels run (other threads per row, small or uneven
+// matrix, no memory for the copy).
+cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s);
+// 16-bit columns relative to the row (complete, for any stream), where the
+// matrix is large and its columns lie within 32,767 of the diagonal; else *out
+// is null and the 32-bit ones serve.
+cudaError_t crs_prepare_c16(DeviceCRS& A, const short** out, cudaStream_t s);
 void sell_free(SellLayout& L, cudaStream_t s, bool async);
 long long sell_bytes(const DeviceCRS& A);
 
@@ -184,7 +192,7 @@ class PersistTables {
 // as a single CUDA-graph launch (while-conditional node).
 class PcgSolver {
  public:
-  PcgSolver() = default;
+  PcgSolver();
   ~PcgSolver();
   PcgSolver(const PcgSolver&) = delete;
   PcgSolver& operator=(const PcgSolver&) = delete;
@@ -218,6 +226,9 @@ class PcgSolver {
   void* st_ = nullptr;          // SysState (device)
   void* st_host_ = nullptr;     // its copy on the host (pageable: pinning costs 300 us a solver)
   void *mem_ = nullptr, *mem32_ = nullptr;   // one allocation for all of these, one for the floats
+  // the matrix's other layouts as this solver's graphs use them
+  std::unique_ptr<SellView> sell_;
+  const short* ci16_ = nullptr;
   const volatile int* abort_flag_ = nullptr;
   cudaGraphExec_t plain_exec_ = nullptr, mixed_exec_ = nullptr, df_exec_ = nullptr;
   cudaGraphExec_t cont_exec_ = nullptr, cont_df_exec_ = nullptr;

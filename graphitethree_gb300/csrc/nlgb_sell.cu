@@ -165,25 +165,21 @@ bool try_alloc(T** p, size_t count, cudaStream_t s) {
 
 const void* sell_pq_kernel(const SysView& v) { return v.sell.va ? (const void*)k_sell_pq : nullptr; }
 
-SellView sell_view(const DeviceCRS& A) {
-  const SellLayout& L = A.sell;
-  if (L.state <= 0 || L.tpr != A.tpr || L.tile_rows != A.tile_rows) return SellView{};
-  return SellView{L.shape, L.len, L.perm, L.ci, L.va, L.passes};
-}
-
 void sell_free(SellLayout& L, cudaStream_t s, bool async) {
   for (void* p : {(void*)L.shape, (void*)L.len, (void*)L.perm, (void*)L.ci, (void*)L.va})
     if (p) { if (async) cudaFreeAsync(p, s); else cudaFree(p); }
   L = SellLayout();
 }
 
-cudaError_t sell_prepare(DeviceCRS& A, bool* usable, cudaStream_t s) {
-  *usable = false;
+cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s) {
+  *view = SellView{};
+  std::lock_guard<std::mutex> lk(*A.lazy);
   if (!A.owns || A.n <= 0 || A.tpr != 2 || A.tile_rows <= 0 || A.nnz < kSellMinNnz) return cudaSuccess;
   SellLayout& L = A.sell;
   if (L.state != 0 && (L.tpr != A.tpr || L.tile_rows != A.tile_rows)) sell_free(L, s, true);
+  auto hand_out = [&]() { *view = SellView{L.shape, L.len, L.perm, L.ci, L.va, L.passes}; };
   if (L.state != 0) {
-    *usable = L.state > 0;
+    if (L.state > 0) hand_out();
     return cudaSuccess;
   }
   L.state = -1;
@@ -218,8 +214,9 @@ cudaError_t sell_prepare(DeviceCRS& A, bool* usable, cudaStream_t s) {
                                               L.va);
   count_launches(1);
   NLGB_CUDA_TRY(cudaGetLastError());
+  NLGB_CUDA_TRY(cudaStreamSynchronize(s));   // (another thread may use it on a stream of its own)
   L.state = 1;
-  *usable = true;
+  hand_out();
   return cudaSuccess;
 }
 
@@ -230,8 +227,8 @@ long long sell_bytes(const DeviceCRS& A) {
   return ctas * (kSellWarps * (long long)sizeof(uint2) + kCTA) + A.n + 12LL * L.units * 32;
 }
 
-cudaError_t sell_spmv64(const DeviceCRS& A, const double* x, double* y, cudaStream_t s) {
-  k_sell_spmv<<<(A.n + A.tile_rows - 1) / A.tile_rows, kCTA, 0, s>>>(sell_view(A), A.n, A.tile_rows, x, y);
+cudaError_t sell_spmv64(const DeviceCRS& A, const SellView& m, const double* x, double* y, cudaStream_t s) {
+  k_sell_spmv<<<(A.n + A.tile_rows - 1) / A.tile_rows, kCTA, 0, s>>>(m, A.n, A.tile_rows, x, y);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -8,10 +8,9 @@
 
 namespace nlgb {
 
-SellView sell_view(const DeviceCRS& A);
 // The kernel that replaces k_spmv_pq for this view, or null.
 const void* sell_pq_kernel(const SysView& v);
-// y = A x (A prepared).
-cudaError_t sell_spmv64(const DeviceCRS& A, const double* x, double* y, cudaStream_t s);
+// y = A x with a layout of A (sell_prepare).
+cudaError_t sell_spmv64(const DeviceCRS& A, const SellView& m, const double* x, double* y, cudaStream_t s);
 
 }  // namespace nlgb

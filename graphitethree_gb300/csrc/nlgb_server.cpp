@@ -375,8 +375,9 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
   r->t_prepared = S->now();
   bool dfl = false;   // false also when the matrix is outside double-float's range: FP64 runs
   if (e == cudaSuccess && prec == NL_GB300_PRECISION_DOUBLE_FLOAT) e = crs_prepare_df(r->A, &dfl, s);
-  if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && mixed) e = crs_prepare_c16(r->A, s);
-  bool sell = false;  // the chunks' SpMV layout (false: CRS)
+  const short* c16 = nullptr;
+  if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && mixed) e = crs_prepare_c16(r->A, &c16, s);
+  SellView sell{};    // the chunks' SpMV layout (no values: CRS)
   if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && !mixed && !dfl) e = sell_prepare(r->A, &sell, s);
   if (e == cudaSuccess) {
     // true footprint now known
@@ -390,6 +391,8 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
       e = r->slots[k].alloc(&r->A, mixed, s, dfl && df_slots);
       if (e != cudaSuccess) break;
       r->slots[k].view.abort_flag = S->abort_dev;
+      r->slots[k].view.sell = sell;
+      r->slots[k].view.ci16 = c16;
       const double* bk = r->kind == 0 ? r->b.data() + (size_t)k * r->n : r->d_rhs + (size_t)k * r->n;
       const double* xk = r->x0.empty() ? nullptr : r->x0.data() + (size_t)k * r->n;
       e = r->slots[k].start(bk, xk, prm, s);

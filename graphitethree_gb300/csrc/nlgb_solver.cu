@@ -733,7 +733,7 @@ long long device_bytes(const DeviceCRS& A) {
   return b;
 }
 
-cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
+static cudaError_t prepare_locked(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
   if (A.tpr == 0) {
     int hist[33];
     int mx = 0;
@@ -763,11 +763,18 @@ cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
   return cudaSuccess;
 }
 
+cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(*A.lazy);
+  return prepare_locked(A, need_fp32, s);
+}
+
 // From 2^21 nonzeros on: smaller matrices stay in L2, or run on the persistent
 // kernel with columns of its own.  us per mixed iteration, 32-bit -> 16-bit:
 // fairing 2048x2048 116.3 -> 108.6, LSCM 808x808 79.8 -> 73.9, fairing
 // 1024x1024 51.9 -> 50.7.  (The FP64 SpMV is bound by the FP64 pipe.)
-cudaError_t crs_prepare_c16(DeviceCRS& A, cudaStream_t s) {
+cudaError_t crs_prepare_c16(DeviceCRS& A, const short** out, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(*A.lazy);
+  *out = A.ci16;
   if (A.c16_tried || !A.owns || A.n != A.m || A.nnz < (1LL << 21)) return cudaSuccess;
   A.c16_tried = true;
   int* far = nullptr;
@@ -795,6 +802,7 @@ cudaError_t crs_prepare_c16(DeviceCRS& A, cudaStream_t s) {
     cudaGetLastError();
     e = cudaSuccess;
   }
+  *out = A.ci16;
   return e;
 }
 
@@ -819,7 +827,8 @@ static cudaError_t exp_range(long long n, const double* a, int* host2, cudaStrea
 }
 
 cudaError_t crs_prepare_df(DeviceCRS& A, bool* usable, cudaStream_t s) {
-  NLGB_CUDA_TRY(crs_prepare(A, false, s));
+  std::lock_guard<std::mutex> lk(*A.lazy);
+  NLGB_CUDA_TRY(prepare_locked(A, false, s));
   if (A.df_state == 0) {
     int rv[2], rd[2];
     NLGB_CUDA_TRY(exp_range(A.nnz, A.va, rv, s));
@@ -965,6 +974,7 @@ constexpr int kUnrollPlain = 4;   // CG iterations per while-body pass
 constexpr int kUnrollInner = 4;
 constexpr long long kMaxItersBetweenUpdates = 1000;   // mixed: forced reliable update
 
+PcgSolver::PcgSolver() : sell_(new SellView{}) {}
 PcgSolver::~PcgSolver() { release(); }
 
 void PcgSolver::release() {
@@ -977,6 +987,8 @@ void PcgSolver::release() {
   cudaFree(mem_);
   cudaFree(mem32_);
   mem_ = mem32_ = exch_ = nullptr;
+  *sell_ = SellView{};
+  ci16_ = nullptr;
   tables_.release();
   ::operator delete(st_host_);
   if (ev0_) cudaEventDestroy(ev0_);
@@ -1052,12 +1064,10 @@ static SysView make_view(DeviceCRS* A, int tile_rows, int n_tiles, double* b, do
   v.n = A->n; v.tile_rows = tile_rows; v.n_tiles = n_tiles; v.tpr = A->tpr;
   v.df = df ? 1 : 0;
   v.rp = A->rp; v.ci = A->ci; v.va = A->va; v.va32 = A->va32; v.vadf = A->vadf;
-  v.ci16 = A->ci16;
   v.dinv = A->dinv; v.dinv32 = A->dinv32; v.dinvdf = A->dinvdf;
   v.b = b; v.x = x; v.r = r; v.p = p; v.q = q;
   v.r32 = r32; v.p32 = p32; v.q32 = q32; v.c32 = c32;
   v.part = part; v.st = (SysState*)st; v.abort_flag = abort_flag;
-  v.sell = sell_view(*A);
   return v;
 }
 
@@ -1096,6 +1106,7 @@ cudaError_t PcgSolver::add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysVie
 cudaError_t PcgSolver::build_plain_graph(bool df, bool cont) {
   SysView v = make_view(A_, tile_rows_, n_tiles_, b_, x_, r_, p_, q_, nullptr, nullptr, nullptr,
                         nullptr, part_, st_, abort_flag_, df);
+  if (!df) v.sell = *sell_;
   const KernelSet ks = kernels_for(tpr_, df);
   cudaGraph_t g;
   NLGB_CUDA_TRY(cudaGraphCreate(&g, 0));
@@ -1124,6 +1135,7 @@ cudaError_t PcgSolver::build_plain_graph(bool df, bool cont) {
 cudaError_t PcgSolver::build_mixed_graph() {
   SysView v = make_view(A_, tile_rows_, n_tiles_, b_, x_, r_, p_, q_, r32_, p32_, q32_, c32_,
                         part_, st_, abort_flag_);
+  v.ci16 = ci16_;
   const KernelSet ks = kernels_for(tpr_, false);
   // [initial FP64 residual] -> while { ( p update ; q = A32 p, p.q ; c/r
   //   update ) x U -> IF(update due) { x += c ; FP64 residual } ; guard }
@@ -1685,11 +1697,10 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
   const int mode = mixed ? kPersistMixed : df ? kPersistDf : kPersistDouble;
   const bool persist = plan_[mode].usable && !eager_mode();
   if (mode == kPersistDouble && !persist && !eager_mode()) {
-    bool sell = false;   // (false: the CRS kernels)
-    NLGB_CUDA_TRY(sell_prepare(*A_, &sell, stream_));
+    NLGB_CUDA_TRY(sell_prepare(*A_, sell_.get(), stream_));
   }
   if (mixed && !persist && !eager_mode() && !mixed_exec_) {
-    NLGB_CUDA_TRY(crs_prepare_c16(*A_, stream_));
+    NLGB_CUDA_TRY(crs_prepare_c16(*A_, &ci16_, stream_));
     NLGB_CUDA_TRY(build_mixed_graph());
   }
   if (!mixed && !persist && !eager_mode() && !*plain) NLGB_CUDA_TRY(build_plain_graph(df));

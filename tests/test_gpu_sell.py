@@ -3,6 +3,7 @@ the products and the phase-kernel iterates are those of the CRS kernels bit for
 bit -- short last tiles and passes, tiles that are not a multiple of a pass,
 rows without entries -- and matrices it does not suit keep the CRS kernels."""
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -58,3 +59,36 @@ def test_rows_of_any_length(gpu_ok, kind):
     x = rng.standard_normal(n)
     y = [M.spmv(x) for _ in range(7)]
     assert all(np.array_equal(y[0], v) for v in y)
+
+
+def test_products_and_solves_of_one_matrix_in_two_threads(gpu_ok):
+    """Whichever thread asks first builds the layout, and both find it whole."""
+    V, F = meshes.height_field(331, 307, 6)
+    first, b, _ = solver.build_lscm(V, F)
+    first.set_layout(2, 1024)
+    x = np.random.default_rng(3).standard_normal(first.n)
+    y = first.spmv(x)
+    want = first.solve(b, max_iter=40)[0]
+    for _ in range(6):
+        M, _, _ = solver.build_lscm(V, F)
+        M.set_layout(2, 1024)
+        start, bad = threading.Barrier(2), []
+
+        def products():
+            start.wait()
+            for _ in range(12):
+                if not np.array_equal(M.spmv(x), y):
+                    bad.append("product")
+
+        def solves():
+            start.wait()
+            for _ in range(3):
+                if not np.array_equal(M.solve(b, max_iter=40)[0], want):
+                    bad.append("solve")
+        threads = [threading.Thread(target=f) for f in (products, solves)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not bad
+        M.close()
