@@ -65,6 +65,7 @@ struct DeviceCRS {
   int tile_rows = 0;
   int max_row = 0;         // longest row (nnz)
   bool owns = true;        // false: a view sharing another matrix's arrays
+  bool lean = false;       // no copies for speed alone (sliced layout, 16-bit columns)
   SellLayout sell;
   // Held while a part above is built on demand: a product and a solve of one
   // matrix may ask for the same part from two threads.
@@ -82,6 +83,9 @@ cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s);
 cudaError_t crs_prepare_c16(DeviceCRS& A, const short** out, cudaStream_t s);
 void sell_free(SellLayout& L, cudaStream_t s, bool async);
 long long sell_bytes(const DeviceCRS& A);
+// What these two may take of memory for A at most (0: never built).
+long long sell_most_bytes(const DeviceCRS& A);
+long long c16_most_bytes(const DeviceCRS& A);
 
 cudaError_t crs_upload(DeviceCRS& A, int n, int m, const int* rp, const int* ci,
                        const double* va, cudaStream_t s);

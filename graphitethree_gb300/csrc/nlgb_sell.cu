@@ -161,6 +161,17 @@ bool try_alloc(T** p, size_t count, cudaStream_t s) {
   return false;
 }
 
+bool suits(const DeviceCRS& A) {
+  return A.owns && !A.lean && A.n > 0 && A.tpr == 2 && A.tile_rows > 0 && A.nnz >= kSellMinNnz;
+}
+long long most_elements(const DeviceCRS& A) { return A.nnz + A.nnz / 8; }
+long long shape_ctas(int n, int tile_rows) {
+  return (long long)((n + tile_rows - 1) / tile_rows) * ((tile_rows + kSellRows - 1) / kSellRows);
+}
+long long layout_bytes(int n, int tile_rows, long long elements) {
+  return shape_ctas(n, tile_rows) * (kSellWarps * (long long)sizeof(uint2) + kCTA) + n + 12LL * elements;
+}
+
 }  // namespace
 
 const void* sell_pq_kernel(const SysView& v) { return v.sell.va ? (const void*)k_sell_pq : nullptr; }
@@ -174,7 +185,7 @@ void sell_free(SellLayout& L, cudaStream_t s, bool async) {
 cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s) {
   *view = SellView{};
   std::lock_guard<std::mutex> lk(*A.lazy);
-  if (!A.owns || A.n <= 0 || A.tpr != 2 || A.tile_rows <= 0 || A.nnz < kSellMinNnz) return cudaSuccess;
+  if (!suits(A)) return cudaSuccess;
   SellLayout& L = A.sell;
   if (L.state != 0 && (L.tpr != A.tpr || L.tile_rows != A.tile_rows)) sell_free(L, s, true);
   auto hand_out = [&]() { *view = SellView{L.shape, L.len, L.perm, L.ci, L.va, L.passes}; };
@@ -186,7 +197,7 @@ cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s) {
   L.tpr = A.tpr;
   L.tile_rows = A.tile_rows;
   L.passes = (A.tile_rows + kSellRows - 1) / kSellRows;
-  const long long ctas = (long long)((A.n + A.tile_rows - 1) / A.tile_rows) * L.passes;
+  const long long ctas = shape_ctas(A.n, A.tile_rows);
   unsigned* ctl = nullptr;
   if (ctas > (1LL << 30) || !try_alloc(&L.shape, (size_t)ctas * kSellWarps, s) ||
       !try_alloc(&L.len, (size_t)ctas * kCTA, s) || !try_alloc(&L.perm, (size_t)A.n, s) || !try_alloc(&ctl, 2, s))
@@ -203,7 +214,7 @@ cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s) {
   // passes that padding adds more than an eighth: not worth it
   L.units = h[0];
   const size_t el = (size_t)L.units * 32;
-  if (h[1] != 0 || (long long)el > A.nnz + A.nnz / 8 || !try_alloc(&L.ci, el, s) || !try_alloc(&L.va, el, s)) {
+  if (h[1] != 0 || (long long)el > most_elements(A) || !try_alloc(&L.ci, el, s) || !try_alloc(&L.va, el, s)) {
     sell_free(L, s, true);
     L.state = -1;
     L.tpr = A.tpr;
@@ -223,8 +234,11 @@ cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s) {
 long long sell_bytes(const DeviceCRS& A) {
   const SellLayout& L = A.sell;
   if (L.state <= 0) return 0;
-  const long long ctas = (long long)((A.n + L.tile_rows - 1) / L.tile_rows) * L.passes;
-  return ctas * (kSellWarps * (long long)sizeof(uint2) + kCTA) + A.n + 12LL * L.units * 32;
+  return layout_bytes(A.n, L.tile_rows, L.units * 32LL);
+}
+
+long long sell_most_bytes(const DeviceCRS& A) {
+  return suits(A) ? layout_bytes(A.n, A.tile_rows, most_elements(A)) : 0;
 }
 
 cudaError_t sell_spmv64(const DeviceCRS& A, const SellView& m, const double* x, double* y, cudaStream_t s) {

@@ -279,6 +279,21 @@ size_t exchange_bytes(const Req& r) {
   return (persist_bytes(r.n, r.slots.empty() ? 1 : r.slots[0].view.n_tiles) + 255) & ~(size_t)255;
 }
 
+// Takes memory of the budget for something that request r can do without.
+bool reserve(nlgb_server_s* S, Req* r, size_t bytes) {
+  std::lock_guard<std::mutex> lk(S->mu);
+  if (S->used + bytes > S->cfg.hbm_budget_bytes) return false;
+  add_used_locked(S, (long long)bytes);
+  r->bytes += bytes;
+  return true;
+}
+
+// The footprint of request r as it is now.
+void account(nlgb_server_s* S, Req* r, size_t bytes) {
+  add_used(S, (long long)bytes - (long long)r->bytes);
+  r->bytes = bytes;
+}
+
 // The tables and exchange areas for chunks on the persistent kernel, where
 // the request's systems fit it and the budget has room for them.
 cudaError_t persist_tables(nlgb_server_s* S, Req* r, cudaStream_t s) {
@@ -286,15 +301,10 @@ cudaError_t persist_tables(nlgb_server_s* S, Req* r, cudaStream_t s) {
   cudaError_t e = r->tables.build(r->A, v.tile_rows, v.n_tiles, s, kSharedTiles);
   if (e != cudaSuccess || !r->tables.usable()) return e;
   const size_t exch = exchange_bytes(*r) * (size_t)r->n_rhs, extra = r->tables.bytes() + exch;
-  {
-    std::lock_guard<std::mutex> lk(S->mu);
-    if (S->used + extra > S->cfg.hbm_budget_bytes) {
-      r->tables.release(s);
-      return cudaSuccess;
-    }
-    add_used_locked(S, (long long)extra);
+  if (!reserve(S, r, extra)) {
+    r->tables.release(s);
+    return cudaSuccess;
   }
-  r->bytes += extra;
   r->plan[0] = r->tables.plan(v.tile_rows, v.tpr, v.df ? kPersistDf : kPersistDouble);   // (a mixed one may end in FP64)
   if (r->slots[0].mixed) r->plan[1] = r->tables.plan(v.tile_rows, v.tpr, kPersistMixed);
   e = cudaMallocAsync(&r->exch, exch, s);
@@ -304,6 +314,31 @@ cudaError_t persist_tables(nlgb_server_s* S, Req* r, cudaStream_t s) {
     return cudaSuccess;
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(r->exch, 0, exch, s);
+  return e;
+}
+
+// The layouts that make graph chunks of large systems faster (FP64: sliced;
+// mixed: 16-bit columns), where the budget has room for them.  The serial
+// worker's solver builds them itself.
+cudaError_t chunk_layouts(nlgb_server_s* S, Req* r, cudaStream_t s) {
+  const SysView& v = r->slots[0].view;
+  const size_t most = (size_t)(r->slots[0].mixed ? c16_most_bytes(r->A) : v.df ? 0 : sell_most_bytes(r->A));
+  if (most == 0) return cudaSuccess;
+  if (!reserve(S, r, most)) {
+    r->A.lean = true;
+    return cudaSuccess;
+  }
+  const size_t before = (size_t)device_bytes(r->A);
+  const short* c16 = nullptr;
+  SellView sell{};
+  cudaError_t e = cudaSuccess;
+  if (S->cfg.mode == NLGB_SERVER_BATCHED)
+    e = r->slots[0].mixed ? crs_prepare_c16(r->A, &c16, s) : sell_prepare(r->A, &sell, s);
+  account(S, r, r->bytes - most + ((size_t)device_bytes(r->A) - before));
+  for (SystemSlot& slot : r->slots) {
+    slot.view.sell = sell;
+    slot.view.ci16 = c16;
+  }
   return e;
 }
 
@@ -375,15 +410,9 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
   r->t_prepared = S->now();
   bool dfl = false;   // false also when the matrix is outside double-float's range: FP64 runs
   if (e == cudaSuccess && prec == NL_GB300_PRECISION_DOUBLE_FLOAT) e = crs_prepare_df(r->A, &dfl, s);
-  const short* c16 = nullptr;
-  if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && mixed) e = crs_prepare_c16(r->A, &c16, s);
-  SellView sell{};    // the chunks' SpMV layout (no values: CRS)
-  if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && !mixed && !dfl) e = sell_prepare(r->A, &sell, s);
   if (e == cudaSuccess) {
     // true footprint now known
-    const size_t actual = (size_t)device_bytes(r->A) + (size_t)r->n_rhs * SystemSlot::bytes_for(r->n, r->A.tile_rows, mixed);
-    add_used(S, (long long)actual - (long long)r->bytes);
-    r->bytes = actual;
+    account(S, r, (size_t)device_bytes(r->A) + (size_t)r->n_rhs * SystemSlot::bytes_for(r->n, r->A.tile_rows, mixed));
     r->iter_cost = iteration_cost(*r, mixed);
     r->slots.resize((size_t)r->n_rhs);
     const SolveParams prm = params_of(S, *r, prec);
@@ -391,8 +420,6 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
       e = r->slots[k].alloc(&r->A, mixed, s, dfl && df_slots);
       if (e != cudaSuccess) break;
       r->slots[k].view.abort_flag = S->abort_dev;
-      r->slots[k].view.sell = sell;
-      r->slots[k].view.ci16 = c16;
       const double* bk = r->kind == 0 ? r->b.data() + (size_t)k * r->n : r->d_rhs + (size_t)k * r->n;
       const double* xk = r->x0.empty() ? nullptr : r->x0.data() + (size_t)k * r->n;
       e = r->slots[k].start(bk, xk, prm, s);
@@ -400,6 +427,7 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
   }
   if (e == cudaSuccess && S->cfg.mode == NLGB_SERVER_BATCHED && S->cfg.schedule == NLGB_SCHEDULE_SRPT)
     e = persist_tables(S, r, s);
+  if (e == cudaSuccess) e = chunk_layouts(S, r, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   // host inputs are no longer needed
   std::vector<int>().swap(r->rp); std::vector<int>().swap(r->ci); std::vector<double>().swap(r->va);
@@ -1393,6 +1421,9 @@ void worker_serial(nlgb_server_s* S) {
         S->st.kernel_s += sr.seconds;
         if (r->status == NL_GB300_STATUS_ABORTED) break;
       }
+      // what the solver built of the matrix (within the budget: chunk_layouts)
+      account(S, r, (size_t)device_bytes(r->A) +
+                        (size_t)r->n_rhs * SystemSlot::bytes_for(r->n, r->A.tile_rows, r->slots[0].mixed));
       if (r->status == NL_GB300_STATUS_NONE) r->status = NL_GB300_STATUS_CONVERGED;
     }
     release(S, r, s);

@@ -768,6 +768,10 @@ cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
   return prepare_locked(A, need_fp32, s);
 }
 
+long long c16_most_bytes(const DeviceCRS& A) {
+  return A.owns && !A.lean && A.n == A.m && A.nnz >= (1LL << 21) ? 2 * A.nnz : 0;
+}
+
 // From 2^21 nonzeros on: smaller matrices stay in L2, or run on the persistent
 // kernel with columns of its own.  us per mixed iteration, 32-bit -> 16-bit:
 // fairing 2048x2048 116.3 -> 108.6, LSCM 808x808 79.8 -> 73.9, fairing
@@ -775,7 +779,7 @@ cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
 cudaError_t crs_prepare_c16(DeviceCRS& A, const short** out, cudaStream_t s) {
   std::lock_guard<std::mutex> lk(*A.lazy);
   *out = A.ci16;
-  if (A.c16_tried || !A.owns || A.n != A.m || A.nnz < (1LL << 21)) return cudaSuccess;
+  if (A.c16_tried || c16_most_bytes(A) == 0) return cudaSuccess;
   A.c16_tried = true;
   int* far = nullptr;
   int h = 0;

@@ -5,7 +5,7 @@ the budget, and failures must be reported, not hung."""
 import numpy as np
 import pytest
 
-from graphitethree_gb300 import solver, systems
+from graphitethree_gb300 import meshes, solver, systems
 
 pytestmark = pytest.mark.gpu
 
@@ -331,3 +331,26 @@ def test_srpt_chunks_follow_their_target_length(gpu_ok, tmp_path, monkeypatch):
     long_ = ms[iters > 16]
     assert len(long_) >= 6
     assert 1.0 <= float(np.median(long_)) <= 15.0, ms
+
+
+@pytest.mark.parametrize("mode", ["batched", "serial"])
+@pytest.mark.parametrize("precision", ["double", "mixed"])
+def test_budget_without_room_for_other_layouts(gpu_ok, precision, mode):
+    """The sliced copy (FP64) and the 16-bit columns (mixed) of a large matrix
+    count against the budget: where it has no room for them the request runs
+    without, with the same iterates."""
+    V, F = meshes.height_field(331, 307, 5)
+    M, b, _ = solver.build_lscm(V, F)
+    assert M.threads_per_row == 2 and M.nnz >= 1 << 21
+    rp, ci, va = M.download()
+    sq = systems.SquareSystem(M.n, rp, ci, va, b[None, :].copy())
+    n, mixed = M.n, precision == "mixed"
+    need = (5 * 8 + (4 * 4 if mixed else 0)) * (n + 64) + (n // 128 + 1) * 64 + 1024   # vectors, tile partials, state
+    need += (12 + (4 if mixed else 0)) * M.nnz + 16 * n                                 # matrix, diagonals
+    for budget in (need + 8192, 4 * need):       # (the second one has room for everything)
+        srv = solver.Server(precision=precision, mode=mode, budget_bytes=budget, eps=1e-2)
+        xs, infos, _ = srv.wait(srv.submit_square(sq))
+        assert srv.stats()["peak_bytes"] <= budget
+        srv.close()
+        x, i = M.solve(b, precision=precision, eps=1e-2)
+        assert np.array_equal(xs[0], x) and infos[0].iterations == i.iterations
