@@ -823,7 +823,6 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
   std::vector<int> waiting(order);     // longest first
   std::vector<char> fp64((size_t)n, 0);
   int left = n, sms_busy = 0;
-  unsigned polls = 0;
   auto seq_of = [&](int i) { return __atomic_load_n(&mirrors[i].seq, __ATOMIC_ACQUIRE); };
   auto start = [&](Lane& l) {
     const int i = l.sys;
@@ -834,15 +833,10 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
   };
   while (left > 0 && ok(e)) {
     bool idle = true;
-    ++polls;
     for (Lane& l : lanes) {
       if (l.sys >= 0) {
         if (seq_of(l.sys) == l.seq0) {
           if (!ok(graphs[(size_t)l.sys]->advance(l.s))) break;
-          if ((polls & 4095u) == 0) {   // a failed kernel writes no mirror
-            const cudaError_t r = cudaStreamQuery(l.s);
-            if (r != cudaErrorNotReady && !ok(r)) break;
-          }
           continue;
         }
         idle = false;

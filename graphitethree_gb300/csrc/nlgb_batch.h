@@ -173,7 +173,7 @@ class ViewGraph {
   bool persist_ = false;
   // the chunk in flight: its launch of the persistent kernel that has not been
   // seen to end (0: none), iterations per launch, reliable updates left
-  unsigned int waiting_ = 0, launches_ = 0;
+  unsigned int waiting_ = 0, launches_ = 0, polls_ = 0;
   long long iters_ = 0;
   int rounds_ = 0;
   cudaError_t build(const SysView& v, bool mixed);

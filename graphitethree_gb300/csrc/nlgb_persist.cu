@@ -3,6 +3,7 @@
 #include "nlgb_persist.h"
 
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 
 namespace nlgb {
@@ -259,12 +260,16 @@ PersistPlan PersistTables::plan(int tile_rows, int tpr, int mode) const {
 
 cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& args, cudaStream_t s) {
   PersistArgs a = args;
+  a.wait_ns = 4000000000ULL;
+  if (const char* t = std::getenv("NLGB_BARRIER_TIMEOUT_MS"))
+    if (const double ms = std::atof(t); ms > 0.0) a.wait_ns = (unsigned long long)(ms * 1e6);
+  const char* shortfall = p.cluster ? nullptr : std::getenv("NLGB_TEST_PERSIST_SHORTFALL");
   void* params[] = {&a};
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
   std::memset(&cfg, 0, sizeof(cfg));
   std::memset(&at, 0, sizeof(at));
-  cfg.gridDim = dim3((unsigned)p.grid);
+  cfg.gridDim = dim3((unsigned)(shortfall && shortfall[0] == '1' ? a.lay.ctas : p.grid));
   cfg.blockDim = dim3((unsigned)p.block);
   cfg.dynamicSmemBytes = (size_t)p.smem;
   cfg.stream = s;

@@ -49,8 +49,6 @@
 namespace nlgb {
 namespace {
 
-constexpr unsigned long long kWaitNs = 4000000000ULL;   // limit of one wait
-
 // Codes a reducer publishes with a scalar.
 enum : int { GO = 0, STOP = 1, STOP_AFTER_P = 2 };
 
@@ -113,12 +111,13 @@ __device__ __forceinline__ void cluster_barrier() {
 struct Wait {
   unsigned long long t0 = 0;
   unsigned int spins = 0;
-  __device__ __forceinline__ bool over(int* err) {
+  __device__ __forceinline__ bool over(const PersistArgs& a) {
+    int* err = a.err;
     if ((++spins & 127u) != 0u) return false;
     const unsigned long long t = clock_ns();
     if (t0 == 0) t0 = t;
     if (*((volatile int*)err) != 0) return true;
-    if (t - t0 > kWaitNs) { atomicExch(err, 1); return true; }
+    if (t - t0 > a.wait_ns) { atomicExch(err, 1); return true; }
     return false;
   }
 };
@@ -329,7 +328,7 @@ __device__ void reducer(const PersistArgs& a, SysState& sst) {
         do {
           va = ld_slot(slots + t);
           vb = ld_slot(slots + (two ? t + 16 : t));
-        } while ((va.y != e || vb.y != e) && !w.over(a.err));
+        } while ((va.y != e || vb.y != e) && !w.over(a));
         if (va.y != e || vb.y != e) { failed = 1; break; }
         double v;
         from_bits(va.x, v);
@@ -546,7 +545,7 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
       Wait w;
       ulonglong2 v = ld_slot(slot);
       while ((v.y >> 8) != e) {
-        if (w.over(a.err)) { s_failed = 1; break; }
+        if (w.over(a)) { s_failed = 1; break; }
         v = ld_slot(slot);
       }
       from_bits(v.x, s_scalar[which]);
@@ -893,7 +892,7 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
             if (i < H) { v[m] = ld_slot(a.zslot + __ldg(halo + i)); ready = ready && v[m].y == e; }
           }
           if (ready) break;
-          if (w.over(a.err)) { s_failed = 1; break; }
+          if (w.over(a)) { s_failed = 1; break; }
         }
 #pragma unroll
         for (int m = 0; m < 4; ++m)

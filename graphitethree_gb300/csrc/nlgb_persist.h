@@ -24,6 +24,7 @@ struct PersistArgs {
   ulonglong2* ctl;             // grid form: [0] alpha, [8] beta as (value, 256 epoch + code)
   ulonglong2* zslot;           // grid form: z of every row as (value, epoch)
   int* err;                    // nonzero: a wait ran out
+  unsigned long long wait_ns;  // limit of one wait (persist_launch)
   PersistLayout lay;
   long long iters;             // iterations of this launch at most
   unsigned int* done;          // host-mapped, or null: done_value + a PersistEnd when the launch ends
@@ -51,6 +52,9 @@ constexpr int kSharedTiles = 4;
 int persist_ctas_for(int n_tiles, int per_cta, int sms);
 // About the time of an iteration of a system that shares the GPU, us.
 double persist_iteration_us(int n_tiles);
+// Launches the kernel.  Environment: NLGB_BARRIER_TIMEOUT_MS limits its waits
+// (4 s); for tests of a wait that runs out, NLGB_TEST_PERSIST_SHORTFALL=1 leaves
+// out the CTA of the grid form that publishes alpha and beta.
 cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& a, cudaStream_t s);
 // The kernel for a layout (nlgb_persist_*.cu): nc rows per lane group in registers.
 const void* persist_kernel_f64(int tpr, bool cluster, int nc);

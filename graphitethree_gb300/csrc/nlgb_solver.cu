@@ -1434,9 +1434,16 @@ cudaError_t ViewGraph::persist_next(cudaStream_t s) {
 }
 
 cudaError_t ViewGraph::advance(cudaStream_t s) {
-  if (waiting_ == 0) return cudaSuccess;
-  const unsigned int done = __atomic_load_n(&mirror_->persist, __ATOMIC_ACQUIRE);
-  if ((done >> 2) != waiting_) return cudaSuccess;
+  unsigned int done = __atomic_load_n(&mirror_->persist, __ATOMIC_ACQUIRE);
+  if (waiting_ == 0 || (done >> 2) != waiting_) {
+    // a kernel that failed, or whose reducing CTA did not come to its end, tells nothing
+    if ((++polls_ & 4095u) != 0) return cudaSuccess;
+    const cudaError_t e = cudaStreamQuery(s);
+    if (e == cudaErrorNotReady) return cudaSuccess;
+    if (e != cudaSuccess || waiting_ == 0) return e;
+    done = __atomic_load_n(&mirror_->persist, __ATOMIC_ACQUIRE);
+    if ((done >> 2) != waiting_) done = kPersistPaused;
+  }
   waiting_ = 0;
   const SysView& v = view_;
   const KernelSet ks = kernels_for(v.tpr, !mixed_ && v.df != 0);
@@ -1635,7 +1642,9 @@ cudaError_t PcgSolver::run_cont(bool df, float* ms) {
 // other streams' kernels now and then), the reliable updates of a mixed
 // system between them, the final residual and the true-residual check.  The
 // kernels return at once when it is not their turn, so several launches are
-// queued before the state is read.  Leaves the state in st_.
+// queued before the state is read.  Leaves the state in st_host_; that is
+// where a wait that ran out shows (the CTA that gave up need not be the one
+// that writes the state on the device).
 constexpr long long kPersistIters = 1024;
 
 cudaError_t PcgSolver::run_persist(int mode, const SolveParams& prm) {
@@ -1741,7 +1750,7 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
     NLGB_CUDA_TRY(cudaGraphLaunch(mixed ? mixed_exec_ : *plain, stream_));
   }
   NLGB_CUDA_TRY(cudaEventRecord(ev1_, stream_));
-  NLGB_CUDA_TRY(cudaMemcpyAsync(h, st_, sizeof(SysState), cudaMemcpyDeviceToHost, stream_));
+  if (!persist) NLGB_CUDA_TRY(cudaMemcpyAsync(h, st_, sizeof(SysState), cudaMemcpyDeviceToHost, stream_));
   NLGB_CUDA_TRY(cudaStreamSynchronize(stream_));
   NLGB_CUDA_TRY(cudaEventElapsedTime(ms, ev0_, ev1_));
   if (persist || eager_mode()) return cudaSuccess;   // counted their launches

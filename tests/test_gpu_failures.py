@@ -97,3 +97,47 @@ def test_abort_stops_batched_epochs(gpu_ok):
     assert 0 < infos[0].iterations < 5 * big.n      # the iterations run before the abort
     assert waited < 2.0
     assert st["completed"] == 1 and st["failed"] == 1
+
+
+PERSIST_SCRIPT = r"""
+import json, os, sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+from graphitethree_gb300 import meshes, solver
+V, F = meshes.height_field(72, 57, 4)            # 65 tiles: a grid, whose CTAs wait for alpha and beta
+M, b, _ = solver.build_lscm(V, F)
+out = {}
+for p in ("double", "mixed", "df"):
+    out[p] = M.solve(b, precision=p)[1].status
+    try:
+        solver.batch_solve([M], [b], precision=p)
+        out["batch " + p] = "ok"
+    except solver.SolverError as e:
+        out["batch " + p] = str(e)
+    srv = solver.Server(precision=p)
+    out["server " + p] = srv.wait_result(srv.submit_mesh("lscm", V, F))[2][0].status
+    srv.close()
+os.environ.pop("NLGB_TEST_PERSIST_SHORTFALL")
+x, i = M.solve(b)                                # the same handle, the same context
+out["after"] = [i.status, bool(np.array_equal(solver.batch_solve([M], [b])[0][0], x))]
+srv = solver.Server(precision="double")
+xs, infos, _ = srv.wait(srv.submit_mesh("lscm", V, F))
+out["after server"] = [infos[0].status, bool(np.array_equal(xs[0], x))]
+srv.close()
+print(json.dumps(out))
+"""
+
+
+def test_wait_of_the_persistent_kernel_runs_out(gpu_ok):
+    """Every wait for alpha is given up after 50 ms.  The CTA that writes the
+    state on the device is the one that is missing, so that the error word alone
+    tells of it: each route reports a device error, and goes on afterwards."""
+    env = dict(os.environ, NLGB_BARRIER_TIMEOUT_MS="50", NLGB_TEST_PERSIST_SHORTFALL="1")
+    p = subprocess.run([sys.executable, "-c", PERSIST_SCRIPT, str(ROOT)], env=env, capture_output=True,
+                       text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+    out = json.loads(p.stdout.strip().splitlines()[-1])
+    for name in ("double", "mixed", "df"):
+        assert out[name] == out["server " + name] == "device_err", out
+        assert "timed out" in out["batch " + name], out
+    assert out["after"] == out["after server"] == ["converged", True]
