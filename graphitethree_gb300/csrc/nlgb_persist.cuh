@@ -343,8 +343,9 @@ __device__ void reducer(const PersistArgs& a, SysState& sst) {
 
   for (;;) {
     const unsigned long long e = base + (unsigned long long)it + 1ULL;
-    // the abort flag (host memory) is read every fourth iteration
-    if (tid == 0 && s.abort_flag != nullptr && (it & 3) == 3) abort_now = *s.abort_flag;
+    // the abort flag (host memory) is read every fourth iteration of the solve (a
+    // launch of a mixed system may end after fewer)
+    if (tid == 0 && s.abort_flag != nullptr && ((base + it) & 3) == 3) abort_now = *s.abort_flag;
     if (hv == 0) {
       const double v = gather(a.slot, e);
       if (i == 0) tot[0][cw] = v;
@@ -590,9 +591,9 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
   for (;;) {
     const unsigned long long e = base + (unsigned long long)it + 1ULL;
     if constexpr (CLUSTER) {
-      // the abort flag (host memory) is read every fourth iteration by CTA 0,
-      // which hands it to the others before the iteration's second barrier
-      if (cta == 0 && threadIdx.x == 0 && s.abort_flag != nullptr && (it & 3) == 3) abort_now = *s.abort_flag;
+      // the abort flag (host memory) is read every fourth iteration of the solve by
+      // CTA 0, which hands it to the others before the iteration's second barrier
+      if (cta == 0 && threadIdx.x == 0 && s.abort_flag != nullptr && ((base + it) & 3) == 3) abort_now = *s.abort_flag;
     }
     // q = A p; where a chain is one row, its p.q product too
     auto finish_row = [&](int row, int pos, V q) {

@@ -141,3 +141,20 @@ def test_wait_of_the_persistent_kernel_runs_out(gpu_ok):
         assert out[name] == out["server " + name] == "device_err", out
         assert "timed out" in out["batch " + name], out
     assert out["after"] == out["after server"] == ["converged", True]
+
+
+@pytest.mark.parametrize("side,n_rhs", [(33, 12000), (110, 4000)])      # a cluster, a grid
+def test_abort_between_reliable_updates_of_a_few_iterations(gpu_ok, side, n_rhs):
+    """Right-hand sides that take three iterations per reliable update and converge in ten."""
+    sq = systems.fairing_system(side, side, lam=30.0, seed=3, n_rhs=1)
+    sq.rhs = np.ascontiguousarray(np.repeat(sq.rhs, n_rhs, axis=0))
+    srv = solver.Server(precision="mixed", mode="serial")
+    t = srv.submit_square(sq)
+    time.sleep(0.6)
+    t_abort = time.perf_counter()
+    srv.abort()
+    ok, x, infos, lat = srv.wait_result(t)
+    waited = time.perf_counter() - t_abort
+    srv.close()
+    assert not ok and "aborted" in [i.status for i in infos]
+    assert "converged" in [i.status for i in infos] and waited < 0.5
