@@ -280,6 +280,12 @@ __device__ __forceinline__ double serial_sum(const double* v, int nw) {
   return s;
 }
 
+// Iterations of this launch at most: a chunk of a mixed system takes a launch
+// per reliable update, and ends where its budget does.
+__device__ __forceinline__ long long launch_iters(const PersistArgs& a, const SysState& st) {
+  return st.iter_stop > 0 ? min(a.iters, st.iter_stop - st.iter) : a.iters;
+}
+
 // Tells the host that this launch is over (one thread; the state itself is for
 // the kernels that the host queues then).
 template <int MODE>
@@ -310,6 +316,7 @@ __device__ void reducer(const PersistArgs& a, SysState& sst) {
   Scalars<MODE> sc;
   sc.load(sst);
   const unsigned long long base = (unsigned long long)sst.coop_epoch;
+  const long long iters = launch_iters(a, sst);
   long long it = 0;
   int abort_now = 0;
   if (tid == 0) { failed = 0; stop = 0; }
@@ -372,7 +379,7 @@ __device__ void reducer(const PersistArgs& a, SysState& sst) {
       const double sum = serial_sum(tot[k], nw);
       const double rr = __shfl_sync(0xffffffffu, sum, 1);
       if (tid == 0) {
-        if (sc.after_xr(sum, rr, it) && it + 1 < a.iters && !abort_now && !failed) {
+        if (sc.after_xr(sum, rr, it) && it + 1 < iters && !abort_now && !failed) {
           sc.advance(sum);
           st_slot(a.ctl + 8, bits_of(sc.beta), (e << 8) | (unsigned)GO);
         } else {
@@ -419,7 +426,8 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
 
   if (threadIdx.x == 0) { sst = *s.st; s_code[0] = s_code[1] = GO; s_failed = 0; s_abort = 0; }
   __syncthreads();
-  if (sst.status != ST_RUNNING || (MODE == kPersistMixed && sst.mode != 1)) {
+  const long long iters = launch_iters(a, sst);
+  if (sst.status != ST_RUNNING || (MODE == kPersistMixed && sst.mode != 1) || iters <= 0) {
     if (cta == 0 && threadIdx.x == 0) tell_done<MODE>(a, sst);
     return;
   }
@@ -860,7 +868,7 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persist(PersistArgs a) {
         bar_sync(2, 64);
         if (threadIdx.x == 0) {
           const double rz = s_tot[0][0], rr = s_tot[1][0];
-          if (sc.after_xr(rz, rr, it - 1) && it < a.iters && !s_abort) {
+          if (sc.after_xr(rz, rr, it - 1) && it < iters && !s_abort) {
             sc.advance(rz);
           } else {
             sc.store(sst, it - 1);

@@ -26,7 +26,7 @@ struct PersistArgs {
   int* err;                    // nonzero: a wait ran out
   unsigned long long wait_ns;  // limit of one wait (persist_launch)
   PersistLayout lay;
-  long long iters;             // iterations of this launch at most
+  long long iters;             // iterations of this launch at most (fewer where the chunk's budget ends)
   unsigned int* done;          // host-mapped, or null: done_value + a PersistEnd when the launch ends
   unsigned int done_value;
 };

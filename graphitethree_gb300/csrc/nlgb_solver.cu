@@ -1388,8 +1388,8 @@ cudaError_t ViewGraph::run(const SysView& v, long long iters, cudaStream_t s, fl
   return cudaSuccess;
 }
 
-// What a chunk graph does, with launches of at most `iters` iterations of the
-// persistent kernel.  The stage after the system's last chunk (its mirror)
+// What a chunk graph does, with launches of the persistent kernel, `iters`
+// iterations of it in all.  The stage after the system's last chunk (its mirror)
 // tells which kernels have nothing to do.
 cudaError_t ViewGraph::persist_head(long long iters, cudaStream_t s) {
   const SysView& v = view_;

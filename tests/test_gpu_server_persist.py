@@ -70,3 +70,18 @@ def test_more_work_than_the_persistent_kernel_gains_on(gpu_ok):
     _check(srv, [systems.fairing_system(360 + 4 * i, 300, seed=i, n_rhs=1) for i in range(12)] +
            [systems.fairing_system(60, 50 + i, seed=i, n_rhs=1) for i in range(8)], "double")
     srv.close()
+
+
+@pytest.mark.parametrize("side", [33, 110])      # a cluster, a grid
+def test_a_mixed_chunk_keeps_to_its_budget(gpu_ok, side, tmp_path, monkeypatch):
+    """A new system's first chunk is a probe of 16 iterations, also where reliable
+    updates end the kernel's launches sooner."""
+    sq = systems.fairing_system(side, side, seed=3, n_rhs=1)
+    want, info = solver.Matrix(sq.rp, sq.ci, sq.va).solve(sq.rhs[0], precision="mixed", inner_eps=0.5)
+    monkeypatch.setenv("NLGB_SERVER_TRACE", str(tmp_path / "trace"))
+    srv = solver.Server(precision="mixed", inner_eps=0.5)
+    xs, infos, _ = srv.wait(srv.submit_square(sq))
+    srv.close()
+    assert np.array_equal(xs[0], want) and infos[0].iterations == info.iterations
+    chunks = [line.split(",") for line in (tmp_path / "trace").read_text().splitlines() if line.startswith("C,")]
+    assert 0 < int(chunks[0][6]) - int(chunks[0][5]) <= 16
