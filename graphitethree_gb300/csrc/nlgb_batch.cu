@@ -750,7 +750,9 @@ int sm_count() {
 
 // Expected time of a system there, up to a factor: iterations of a Jacobi-CG on
 // a surface (sqrt(n)) times the time of one.
-double persist_time(const SysView& v) { return std::sqrt((double)v.n) * persist_iteration_us(v.n_tiles); }
+double persist_time(const SysView& v, int n_sm) {
+  return std::sqrt((double)v.n) * persist_iteration_us(v.n_tiles, persist_ctas_for(v.n_tiles, kSharedTiles, n_sm));
+}
 
 }  // namespace
 
@@ -767,8 +769,9 @@ double persist_time(const SysView& v) { return std::sqrt((double)v.n) * persist_
 //   400 of 16..64      61.3 -> 50.7 (71.4)    0.53
 //   300 of 16..24      21.0 -> 20.6 (24.7)    1.09
 bool persist_batch_pays(const std::vector<SysView>& views) {
+  const int n_sm = sm_count();
   double longest = 0.0;
-  for (const SysView& v : views) longest = std::max(longest, persist_time(v));
+  for (const SysView& v : views) longest = std::max(longest, persist_time(v, n_sm));
   return (double)views.size() <= kPersistBatchRatio * longest;
 }
 
@@ -806,7 +809,7 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
   std::vector<int> order((size_t)n);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    return persist_time(systems[a].view) > persist_time(systems[b].view);
+    return persist_time(systems[a].view, n_sm) > persist_time(systems[b].view, n_sm);
   });
   // with room for all at once the clusters go first: spread CTAs of the grids
   // would leave no GPC with enough free SMs

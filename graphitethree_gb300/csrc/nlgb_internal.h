@@ -169,11 +169,12 @@ class PersistTables {
   PersistTables& operator=(const PersistTables&) = delete;
   // Lays a matrix out for the persistent kernel; usable() tells whether it
   // fits (sizes and halos).  per_cta: tiles on a CTA (more where the GPU has
-  // fewer SMs than that takes).
-  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta = 1);
+  // fewer SMs than that takes); leave: SMs to leave free (persist_ctas_for).
+  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta = 1, int leave = 0);
   // The same in two steps, for many matrices with one synchronisation: begin
   // queues the work and raises *most (device, zero before), end takes its value.
-  cudaError_t begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta, int* most);
+  cudaError_t begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta, int* most,
+                    int leave = 0);
   void end(int most, cudaStream_t s);
   bool usable() const { return lay_.ctas > 0; }
   const PersistLayout& layout() const { return lay_; }

@@ -119,14 +119,16 @@ size_t smem_bytes(int slots, int R, int halo, size_t word) {
 
 }  // namespace
 
-int persist_ctas_for(int n_tiles, int per_cta, int sms) {
+int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave) {
   const int most = n_tiles <= kPersistClusterTiles ? kPersistCluster : sms - 1;
-  return std::min((n_tiles + per_cta - 1) / per_cta, most);
+  const int ctas = std::min((n_tiles + per_cta - 1) / per_cta, most), fewer = sms - 1 - leave;
+  if (leave == 0 || ctas <= kPersistCluster || ctas <= fewer || fewer < 1) return ctas;
+  const int slots = (n_tiles + fewer - 1) / fewer;
+  return slots <= kPersistSlots ? (n_tiles + slots - 1) / slots : ctas;
 }
 
-double persist_iteration_us(int n_tiles) {
-  const int ctas = std::max(1, persist_ctas_for(n_tiles, kSharedTiles, 152));
-  return 5.0 + 1.2 * (double)((n_tiles + ctas - 1) / ctas - 1);   // (kSharedTiles' figures)
+double persist_iteration_us(int n_tiles, int ctas) {
+  return 5.0 + 1.2 * (double)((n_tiles + ctas - 1) / std::max(1, ctas) - 1);   // (kSharedTiles' figures)
 }
 
 void PersistTables::release() {
@@ -142,11 +144,12 @@ void PersistTables::release(cudaStream_t s) {
   release();
 }
 
-cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta) {
+cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta,
+                                 int leave) {
   int most = 0, *d = nullptr;
   NLGB_CUDA_TRY(cudaMallocAsync((void**)&d, sizeof(int), s));
   cudaError_t e = cudaMemsetAsync(d, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = begin(A, tile_rows, n_tiles, s, per_cta, d);
+  if (e == cudaSuccess) e = begin(A, tile_rows, n_tiles, s, per_cta, d, leave);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&most, d, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaFreeAsync(d, s);
@@ -156,12 +159,12 @@ cudaError_t PersistTables::build(const DeviceCRS& A, int tile_rows, int n_tiles,
 }
 
 cudaError_t PersistTables::begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta,
-                                 int* most) {
+                                 int* most, int leave) {
   release();
   int sms = 0, smem_max = 0;
   if (A.n <= 0 || A.nnz <= 0 || A.n != A.m || tile_rows > 512 || !device_limits(&sms, &smem_max)) return cudaSuccess;
   cluster_ = n_tiles <= kPersistClusterTiles;
-  const int ctas = persist_ctas_for(n_tiles, per_cta, sms);
+  const int ctas = persist_ctas_for(n_tiles, per_cta, sms, leave);
   if (ctas < 1) return cudaSuccess;
   const int slots = (n_tiles + ctas - 1) / ctas;
   const int cap = slots * tile_rows;

@@ -48,10 +48,19 @@ inline void persist_bind(PersistArgs& a, void* exch) {
 // with 2, 3, 4 and 6 tiles: 106, 80, 71, 66 ms; 6 requests of 1k to 4k: 8.4,
 // 8.5, 8.8, 10.4 ms.
 constexpr int kSharedTiles = 4;
-// CTAs that own a system's tiles, with per_cta tiles on each or as many as there have to be.
-int persist_ctas_for(int n_tiles, int per_cta, int sms);
+// SMs that the server's persistent chunks leave to the kernels of admissions
+// (an admission waits for a dozen of them one after the other, and a CTA of
+// k_persist has its SM's registers to itself), and that one system leaves: for a
+// cluster beside it as well.  Latency of a request of 1.6k vertices beside an
+// LSCM system of 157k unknowns, with all SMs taken -> so: 19.4 -> 2.0 ms.
+constexpr int kAdmissionSms = 7;
+constexpr int kSharedLeave = kAdmissionSms + kPersistCluster;
+// CTAs that own a system's tiles, with per_cta tiles on each or as many as
+// there have to be.  leave > 0: on all but so many SMs (where nine tiles per CTA
+// allow that), and the fewest CTAs with as many tiles on the busiest.
+int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave = 0);
 // About the time of an iteration of a system that shares the GPU, us.
-double persist_iteration_us(int n_tiles);
+double persist_iteration_us(int n_tiles, int ctas);
 // Launches the kernel.  Environment: NLGB_BARRIER_TIMEOUT_MS limits its waits
 // (4 s); for tests of a wait that runs out, NLGB_TEST_PERSIST_SHORTFALL=1 leaves
 // out the CTA of the grid form that publishes alpha and beta.

@@ -298,7 +298,7 @@ void account(nlgb_server_s* S, Req* r, size_t bytes) {
 // the request's systems fit it and the budget has room for them.
 cudaError_t persist_tables(nlgb_server_s* S, Req* r, cudaStream_t s) {
   const SysView& v = r->slots[0].view;
-  cudaError_t e = r->tables.build(r->A, v.tile_rows, v.n_tiles, s, kSharedTiles);
+  cudaError_t e = r->tables.build(r->A, v.tile_rows, v.n_tiles, s, kSharedTiles, kSharedLeave);
   if (e != cudaSuccess || !r->tables.usable()) return e;
   const size_t exch = exchange_bytes(*r) * (size_t)r->n_rhs, extra = r->tables.bytes() + exch;
   if (!reserve(S, r, extra)) {
@@ -1257,7 +1257,7 @@ void worker_streams(nlgb_server_s* S) {
           if (r->sys_done[k]) continue;
           const int c = r->graphs[k]->persist_ctas(r->mixed_now[k] != 0);
           fit = c > 0;
-          us += (double)c * persist_iteration_us(r->slots[k].view.n_tiles) / (double)std::max(1, n_sm);
+          us += (double)c * persist_iteration_us(r->slots[k].view.n_tiles, c) / (double)std::max(1, n_sm);
           systems += 1.0;
         }
       const double graph_us = kGraphIterationUs * std::max(1.0, systems / (double)std::min(ns, 16));
@@ -1277,7 +1277,7 @@ void worker_streams(nlgb_server_s* S) {
           // least-work one that fits runs meanwhile)
           if (cta_cap > 0 && running_ctas > 0 && running_ctas + ctas_of(r) > cta_cap) continue;
           if (persist && sms_busy > 0 &&
-              sms_busy + r->graphs[k]->persist_ctas(r->mixed_now[k] != 0) > n_sm) continue;
+              sms_busy + r->graphs[k]->persist_ctas(r->mixed_now[k] != 0) > n_sm - kAdmissionSms) continue;
           const double key = r->est_left[k] < 0.0 ? -1.0 : r->est_left[k] * r->iter_cost;
           if (!best || key < bkey || (key == bkey && r->id < best->id)) { best = r; bk = k; bkey = key; }
         }

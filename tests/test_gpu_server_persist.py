@@ -4,6 +4,8 @@ at 64 / 65 tiles, more than four tiles per CTA), every precision, a mixed system
 that continues in FP64, a budget without room for the tables, and a load that
 changes between systems that fit and systems that do not -- the same iterates
 bit for bit as the single-system solver."""
+import time
+
 import numpy as np
 import pytest
 
@@ -85,3 +87,19 @@ def test_a_mixed_chunk_keeps_to_its_budget(gpu_ok, side, tmp_path, monkeypatch):
     assert np.array_equal(xs[0], want) and infos[0].iterations == info.iterations
     chunks = [line.split(",") for line in (tmp_path / "trace").read_text().splitlines() if line.startswith("C,")]
     assert 0 < int(chunks[0][6]) - int(chunks[0][5]) <= 16
+
+
+def test_a_wide_system_leaves_room_for_small_ones(gpu_ok):
+    """Beside a system of 613 tiles, whose chunks last 50 ms, a small request is
+    admitted and solved without waiting for their ends."""
+    V, F = meshes.height_field(280, 280, 1)
+    small = [systems.fairing_system(40, 40, seed=i, n_rhs=1) for i in range(4)]
+    srv = solver.Server(precision="double", epoch_ms=50.0)
+    srv.wait(srv.submit_square(small[3]))
+    wide = srv.submit_mesh("lscm", V, F)
+    time.sleep(0.03)
+    lat = [srv.wait(srv.submit_square(s))[2] for s in small[:3]]
+    _, infos, wide_lat = srv.wait(wide)
+    srv.close()
+    assert infos[0].status == "converged" and wide_lat > sum(lat)     # it ran all the while
+    assert sorted(lat)[1] < 0.025
