@@ -95,6 +95,9 @@ struct Req {
   std::vector<int> mirror_idx;       // per system, its ChunkMirror in the server's pool
   std::vector<int> running, mixed_now, need_fallback;
   std::vector<double> ms_per_iter;
+  // Chunks on the persistent kernel, per system, ms: when it could run next, the
+  // time it ran, and the time it waited for SMs
+  std::vector<double> t_ready, ran_ms, waited_ms;
   std::vector<nlgb_result> res;
   double t_done = 0.0;
   double t_built = 0.0, t_prepared = 0.0;   // admission phases (server clock, tracing)
@@ -450,6 +453,9 @@ bool admit(nlgb_server_s* S, Req* r, cudaStream_t s, bool df_slots) {
   r->running.assign((size_t)r->n_rhs, 0);
   r->need_fallback.assign((size_t)r->n_rhs, 0);
   r->ms_per_iter.assign((size_t)r->n_rhs, -1.0);
+  r->t_ready.assign((size_t)r->n_rhs, S->now() * 1e3);
+  r->ran_ms.assign((size_t)r->n_rhs, 0.0);
+  r->waited_ms.assign((size_t)r->n_rhs, 0.0);
   r->mixed_now.assign((size_t)r->n_rhs, 0);
   for (int k = 0; k < r->n_rhs; ++k) r->mixed_now[k] = r->slots[k].mixed ? 1 : 0;
   r->res.assign((size_t)r->n_rhs, nlgb_result{});
@@ -1080,6 +1086,36 @@ void worker_streams(nlgb_server_s* S) {
   int n_sm = 0, sms_busy = 0, graphs_busy = 0;
   bool persist = true;
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, S->device);
+  const double target_ms = S->cfg.epoch_ms > 0.0 ? S->cfg.epoch_ms : 10.0;
+  auto sms_of = [](Req* r, int k) { return r->graphs[k]->persist_ctas(r->mixed_now[k] != 0); };
+  auto fits = [&](int sms) { return sms_busy == 0 || sms_busy + sms <= n_sm - kAdmissionSms; };
+  auto key_of = [](const Req* r, int k) { return r->est_left[k] < 0.0 ? -1.0 : r->est_left[k] * r->iter_cost; };
+  // A system of many SMs seldom finds them free when a lane is: chunks of smaller
+  // ones are launched on what is there, and would be as long as there are any.
+  // `wide` is such a system that is next: no chunk starts before it, so that its
+  // SMs come free.  It is the one with the least work left once the SMs left idle
+  // meanwhile are worth half a chunk of it, or one that waited nine times as long
+  // as it ran and 50 chunks.
+  // Beside 6 streams of LSCM systems of 60 x 60 (660 a second) one of 200 x 200
+  // (alone 104 ms, 288 with graph chunks) was not run at all; it takes 240 ms.
+  Req* wide = nullptr;
+  int wide_k = -1;
+  double idle = 0.0, t_idle = 0.0;   // SM ms
+  auto choose_wide = [&]() {
+    const double t = S->now() * 1e3;
+    Req* least = nullptr;
+    int lk = -1;
+    for (Req* r : S->active)
+      for (int k = 0; k < r->n_rhs; ++k) {
+        if (r->sys_done[k] || r->running[k] || fits(sms_of(r, k))) continue;
+        if (r->waited_ms[k] + (t - r->t_ready[k]) > 9.0 * r->ran_ms[k] + 50.0 * target_ms) { wide = r; wide_k = k; }
+        if (!least || key_of(r, k) < key_of(least, lk)) { least = r; lk = k; }
+      }
+    idle = least ? idle + (double)std::max(0, n_sm - kAdmissionSms - sms_busy) * (t - t_idle) : 0.0;
+    t_idle = t;
+    if (least && !wide && idle > 0.5 * target_ms * (double)sms_of(least, lk)) { wide = least; wide_k = lk; }
+    if (wide) idle = 0.0;
+  };
   auto ctas_of = [](const Req* r) {
     return ((long long)r->A.n + r->A.tile_rows - 1) / std::max(1, r->A.tile_rows);
   };
@@ -1094,7 +1130,6 @@ void worker_streams(nlgb_server_s* S) {
     S->fatal = std::string("server streams: ") + cudaGetErrorString(cudaGetLastError());
     S->cv_admit.notify_all();
   }
-  const double target_ms = S->cfg.epoch_ms > 0.0 ? S->cfg.epoch_ms : 10.0;
   // host time of the worker's loop by part (tracing): retiring chunks,
   // completing requests, launching chunks (of which the graph launches),
   // waiting; and the time lanes sat finished before their next launch
@@ -1151,6 +1186,8 @@ void worker_streams(nlgb_server_s* S) {
       std::fprintf(S->trace, "C,%.6f,%lld,%d,%d,%lld,%lld,%.3f,%d,%d\n", S->now(), r->id, k, mixed_chunk ? 1 : 0,
                    l.iter_before, h.iter, ms, h.status, h.stage);
     if (di > 0) r->ms_per_iter[k] = double(ms) / double(di);
+    r->ran_ms[k] += double(ms);
+    r->t_ready[k] = S->now() * 1e3;
     r->est_left[k] = estimate_left(r, k, h);
     r->sys_stage[k] = h.stage;
     r->sys_iter[k] = h.iter;
@@ -1237,6 +1274,7 @@ void worker_streams(nlgb_server_s* S) {
     if (S->aborting) {
       // running chunks see the abort flag within one loop pass; when they
       // are all back, the active requests end as aborted
+      wide = nullptr;
       if (n_busy == 0) {
         finish_abort_all();
         S->cv_admit.notify_all();
@@ -1263,6 +1301,8 @@ void worker_streams(nlgb_server_s* S) {
       const double graph_us = kGraphIterationUs * std::max(1.0, systems / (double)std::min(ns, 16));
       persist = fit && us <= (persist ? 1.5 : 1.0) * graph_us;
       S->graph_chunks.store(!persist);
+      if (!persist) wide = nullptr;
+      else if (!wide) choose_wide();
     }
     for (Lane& l : lanes) {
       if (l.r || e != cudaSuccess) continue;
@@ -1276,12 +1316,13 @@ void worker_streams(nlgb_server_s* S) {
           // within the CTA budget (a system that does not fit waits; the
           // least-work one that fits runs meanwhile)
           if (cta_cap > 0 && running_ctas > 0 && running_ctas + ctas_of(r) > cta_cap) continue;
-          if (persist && sms_busy > 0 &&
-              sms_busy + r->graphs[k]->persist_ctas(r->mixed_now[k] != 0) > n_sm - kAdmissionSms) continue;
-          const double key = r->est_left[k] < 0.0 ? -1.0 : r->est_left[k] * r->iter_cost;
+          if (persist && (wide ? r != wide || k != wide_k : !fits(sms_of(r, k)))) continue;
+          const double key = key_of(r, k);
           if (!best || key < bkey || (key == bkey && r->id < best->id)) { best = r; bk = k; bkey = key; }
         }
-      if (!best) break;
+      if (!best || (best == wide && !fits(sms_of(best, bk)))) break;
+      wide = nullptr;
+      best->waited_ms[bk] += S->now() * 1e3 - best->t_ready[bk];
       long long iters = kProbeIters;
       if (best->est_left[bk] >= 0.0) {
         const double mpi = best->ms_per_iter[bk] > 0.0 ? best->ms_per_iter[bk] : best->iter_cost / 2e8;

@@ -4,6 +4,7 @@ at 64 / 65 tiles, more than four tiles per CTA), every precision, a mixed system
 that continues in FP64, a budget without room for the tables, and a load that
 changes between systems that fit and systems that do not -- the same iterates
 bit for bit as the single-system solver."""
+import threading
 import time
 
 import numpy as np
@@ -103,3 +104,32 @@ def test_a_wide_system_leaves_room_for_small_ones(gpu_ok):
     srv.close()
     assert infos[0].status == "converged" and wide_lat > sum(lat)     # it ran all the while
     assert sorted(lat)[1] < 0.025
+
+
+@pytest.mark.parametrize("streams", [6, 12])     # SMs left over, but too few; none left over
+def test_a_wide_system_among_a_stream_of_small_ones(gpu_ok, streams):
+    V, F = meshes.height_field(200, 200, 1)      # 625 tiles, 0.1 s alone
+    small = [meshes.height_field(60, 60, i) for i in range(8)]
+    M, b, _ = solver.build_lscm(V, F)
+    want = M.solve(b)[0]
+    srv = solver.Server(precision="double")
+    stop = threading.Event()
+
+    def feed(i):
+        while not stop.is_set():
+            srv.wait(srv.submit_mesh("lscm", *small[i % 8]))
+            i += 1
+    threads = [threading.Thread(target=feed, args=(i,)) for i in range(streams)]
+    for t in threads:
+        t.start()
+    time.sleep(0.1)
+    got = []
+    waiter = threading.Thread(target=lambda t: got.append(srv.wait(t)), args=(srv.submit_mesh("lscm", V, F),))
+    waiter.start()
+    waiter.join(4.0)
+    in_time = not waiter.is_alive()              # beside the stream, not after it
+    stop.set()
+    for t in threads + [waiter]:
+        t.join()
+    srv.close()
+    assert in_time and np.array_equal(got[0][0][0], want)
