@@ -422,8 +422,9 @@ int nlgb_batch_solve(int n_sys, const nlgb_matrix* A, const double* const* b, do
                    batch_tables(n_sys, A, slots, s, ps, &rc);
     if (persist) {
       float ms = 0.f;
-      const cudaError_t e = persist_batch(ps, s, &ms);
-      persist = e != cudaErrorMemoryAllocation;   // (nothing has run yet: the batched kernel needs less)
+      bool ran = false;
+      const cudaError_t e = persist_batch(ps, s, &ms, &ran);
+      persist = e != cudaErrorMemoryAllocation || ran;   // (no room for the exchange areas: the batched kernel)
       if (!persist) cudaGetLastError();
       else if (e != cudaSuccess) rc = NLGB_E_DEVICE;
       st.ms = ms;

@@ -775,7 +775,8 @@ bool persist_batch_pays(const std::vector<SysView>& views) {
   return (double)views.size() <= kPersistBatchRatio * longest;
 }
 
-cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms) {
+cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms, bool* ran) {
+  *ran = false;
   struct Lane {
     cudaStream_t s = nullptr;
     int sys = -1, sms = 0;
@@ -830,6 +831,7 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
   auto start = [&](Lane& l) {
     const int i = l.sys;
     const bool mixed = systems[i].mixed && !fp64[(size_t)i];
+    *ran = true;
     mirrors[i].budget = kPersistBatchIters;
     l.seq0 = seq_of(i);
     if (ok(graphs[(size_t)i]->prepare(systems[i].view, mixed, &mirrors[i], l.s))) ok(graphs[(size_t)i]->launch(l.s));

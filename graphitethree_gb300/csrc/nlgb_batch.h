@@ -205,9 +205,9 @@ struct PersistSystem {
 };
 // Whether a batch is better off there than in one launch of the batched kernel.
 bool persist_batch_pays(const std::vector<SysView>& views);
-// Runs the systems (ready on stream s); on return they have ended.
-// cudaErrorMemoryAllocation: no room for the exchange areas, nothing was run.
-cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms);
+// Runs the systems (ready on stream s); on return they have ended.  *ran: some
+// system was begun (after an error before that, the batched kernel can run them).
+cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms, bool* ran);
 
 // Launches the persistent kernel over a set of resident systems.  Each
 // system's SysState (device) must be initialised by the caller (status

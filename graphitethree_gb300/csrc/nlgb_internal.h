@@ -214,6 +214,7 @@ class PcgSolver {
                         long long done, int outer, float* ms);
   cudaError_t run_eager(bool mixed, bool df, SysState* h, bool cont = false);
   cudaError_t run_persist(int mode, const SolveParams& prm);
+  cudaError_t solve_once(const double* b, double* x, const SolveParams& prm, SolveResult* res);
   // continuation after a failed true-residual check (state: running, stage 4)
   cudaError_t run_cont(bool df, float* ms);
   cudaError_t add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysView* v, bool df,
@@ -242,6 +243,7 @@ class PcgSolver {
   PersistTables tables_;
   PersistPlan plan_[3];
   void* exch_ = nullptr;
+  bool refused_ = false;        // a launch of it failed
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   bool mixed_alloc_ = false;
   long long graph_launches_ = 0;

@@ -3,6 +3,7 @@
 #include "nlgb_persist.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 
@@ -266,6 +267,13 @@ cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& args, cudaSt
   a.wait_ns = 4000000000ULL;
   if (const char* t = std::getenv("NLGB_BARRIER_TIMEOUT_MS"))
     if (const double ms = std::atof(t); ms > 0.0) a.wait_ns = (unsigned long long)(ms * 1e6);
+  if (const char* t = std::getenv("NLGB_TEST_PERSIST_REFUSE")) {
+    static std::atomic<long long> asked{0};
+    if (++asked >= std::atoll(t)) {
+      set_error("persistent kernel: launch refused (NLGB_TEST_PERSIST_REFUSE)");
+      return cudaErrorCooperativeLaunchTooLarge;
+    }
+  }
   const char* shortfall = p.cluster ? nullptr : std::getenv("NLGB_TEST_PERSIST_SHORTFALL");
   void* params[] = {&a};
   cudaLaunchConfig_t cfg;

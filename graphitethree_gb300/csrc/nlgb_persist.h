@@ -62,8 +62,9 @@ int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave = 0);
 // About the time of an iteration of a system that shares the GPU, us.
 double persist_iteration_us(int n_tiles, int ctas);
 // Launches the kernel.  Environment: NLGB_BARRIER_TIMEOUT_MS limits its waits
-// (4 s); for tests of a wait that runs out, NLGB_TEST_PERSIST_SHORTFALL=1 leaves
-// out the CTA of the grid form that publishes alpha and beta.
+// (4 s).  For tests: NLGB_TEST_PERSIST_SHORTFALL=1 leaves out the CTA of the grid
+// form that publishes alpha and beta, so that waits run out;
+// NLGB_TEST_PERSIST_REFUSE=n refuses the launches from the n-th one on.
 cudaError_t persist_launch(const PersistPlan& p, const PersistArgs& a, cudaStream_t s);
 // The kernel for a layout (nlgb_persist_*.cu): nc rows per lane group in registers.
 const void* persist_kernel_f64(int tpr, bool cluster, int nc);

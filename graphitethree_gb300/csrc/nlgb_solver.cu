@@ -1430,7 +1430,15 @@ cudaError_t ViewGraph::persist_next(cudaStream_t s) {
   waiting_ = launches_;
   pa.done = &mirror_->persist;
   pa.done_value = launches_ << 2;
-  return persist_launch(plan_[mixed_ ? 1 : 0], pa, s);
+  if (persist_launch(plan_[mixed_ ? 1 : 0], pa, s) == cudaSuccess) return cudaSuccess;
+  // it cannot be launched here: the chunk's graph, from where the system is
+  cudaGetLastError();
+  waiting_ = 0;
+  plan_[mixed_ ? 1 : 0].usable = false;
+  const SysView v = view_;
+  NLGB_CUDA_TRY(build(v, mixed_));
+  NLGB_CUDA_TRY(cudaGraphUpload(exec_, s));
+  return cudaGraphLaunch(exec_, s);
 }
 
 cudaError_t ViewGraph::advance(cudaStream_t s) {
@@ -1675,7 +1683,9 @@ cudaError_t PcgSolver::run_persist(int mode, const SolveParams& prm) {
     rounds = (int)std::max(1.0, std::min(16.0, std::ceil(std::log(prm.eps) / std::log(prm.inner_eps))));
   for (;;) {
     for (int k = 0; k < rounds; ++k) {
-      NLGB_CUDA_TRY(persist_launch(plan_[mode], pa, stream_));
+      const cudaError_t e = persist_launch(plan_[mode], pa, stream_);
+      refused_ = e != cudaSuccess;
+      if (refused_) return e;
       if (mixed) {
         NLGB_CUDA_TRY(go((const void*)k_mx_apply, vg, kCTA, a1));
         NLGB_CUDA_TRY(go(ks.mx_outer, n_tiles_, kCTA, a1));
@@ -1767,6 +1777,17 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
 }
 
 cudaError_t PcgSolver::solve(const double* b, double* x, const SolveParams& prm, SolveResult* res) {
+  const cudaError_t e = solve_once(b, x, prm, res);
+  if (!refused_) return e;
+  // the persistent kernel cannot be launched here: the graphs, from the start
+  // (x is written at the end) and from now on
+  cudaGetLastError();
+  refused_ = false;
+  for (PersistPlan& plan : plan_) plan.usable = false;
+  return solve_once(b, x, prm, res);
+}
+
+cudaError_t PcgSolver::solve_once(const double* b, double* x, const SolveParams& prm, SolveResult* res) {
   const bool mixed = prm.precision == 1;
   bool df = false;
   if (mixed) {

@@ -158,3 +158,41 @@ def test_abort_between_reliable_updates_of_a_few_iterations(gpu_ok, side, n_rhs)
     srv.close()
     assert not ok and "aborted" in [i.status for i in infos]
     assert "converged" in [i.status for i in infos] and waited < 0.5
+
+
+REFUSE_SCRIPT = r"""
+import json, os, sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+from graphitethree_gb300 import meshes, solver
+meshes_ = [meshes.height_field(72, 57, 4), meshes.height_field(30, 20, 5)]      # a grid, a cluster
+def run():
+    out = []
+    for p in ("double", "mixed", "df"):
+        systems = [solver.build_lscm(V, F)[:2] for V, F in meshes_]
+        out += [M.solve(b, precision=p) for M, b in systems]
+        xs, infos, _ = solver.batch_solve([M for M, _ in systems], [b for _, b in systems], precision=p)
+        out += list(zip(xs, infos))
+        srv = solver.Server(precision=p, epoch_ms=1.0)
+        for t in [srv.submit_mesh("lscm", V, F) for V, F in meshes_]:
+            xs, infos, _ = srv.wait(t)
+            out.append((xs[0], infos[0]))
+        srv.close()
+    return out
+refused = run()
+del os.environ["NLGB_TEST_PERSIST_REFUSE"]
+want = run()
+print(json.dumps([[i.status, i.iterations == j.iterations, bool(np.array_equal(x, y))]
+                  for (x, i), (y, j) in zip(refused, want)]))
+"""
+
+
+@pytest.mark.parametrize("first", [1, 2, 7, 30])
+def test_a_refused_launch_of_the_persistent_kernel_falls_back_to_the_graphs(gpu_ok, first):
+    """From the first launch on, or in the middle of a solve, a batch or a chunk."""
+    p = subprocess.run([sys.executable, "-c", REFUSE_SCRIPT, str(ROOT)],
+                       env=dict(os.environ, NLGB_TEST_PERSIST_REFUSE=str(first)), capture_output=True, text=True,
+                       timeout=300)
+    assert p.returncode == 0, p.stderr
+    out = json.loads(p.stdout.strip().splitlines()[-1])
+    assert len(out) == 18 and all(o[1:] == [True, True] for o in out), out
