@@ -71,8 +71,14 @@ struct DeviceCRS {
   // matrix may ask for the same part from two threads.
   std::shared_ptr<std::mutex> lazy = std::make_shared<std::mutex>();
 };
-// Matrices below this have SpMVs of a few microseconds, bound by latency.
-constexpr long long kSellMinNnz = 1LL << 21;
+// Matrices below this have SpMVs of a few microseconds, bound by latency; above
+// the upper limit the vectors no longer stay in L2 (129 MB) between the kernels
+// of an iteration, which is then bound by DRAM and pays for the copy's padding.
+// us per FP64 iteration of LSCM systems, CRS -> sliced: 600 x 600 (10.1 M
+// nonzeros) 76.1 -> 68.3, 808 (18.3 M) 111.1 -> 100.4, 1100 (33.8 M) 172.1 ->
+// 163.0, 1350 (51.0 M) 238.5 -> 235.2, 1400 (54.8 M) 249.5 -> 251.3, 1450 (58.8 M)
+// 266.6 -> 264.5, 1500 (63.0 M) 275.9 -> 282.3, 2000 (111.9 M) 471.6 -> 490.5.
+constexpr long long kSellMinNnz = 1LL << 21, kSellMaxNnz = 57LL << 20;
 // Builds the sliced layout; on return it is complete, for any stream.  *view
 // without values: the CRS kernels run (other threads per row, small or uneven
 // matrix, no memory for the copy).

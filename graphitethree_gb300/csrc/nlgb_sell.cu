@@ -13,7 +13,7 @@
 // and a pass over the matrix, once per matrix and layout.
 //
 // Measured on GB300, LSCM 808 x 808 (1.31 M rows, 18.3 M nonzeros): SpMV 62.8
-// -> 53.3 us (4.6 TB/s), PCG iteration 117.8 -> 105.3 us.  Not used with other
+// -> 53.3 us (4.6 TB/s), PCG iteration 111.1 -> 100.4 us.  Not used with other
 // numbers of threads per row, where it loses: with one (the cotangent
 // Laplacian, 4.2 M rows) sorting over 256 rows scatters the gathers of x and
 // the SpMV takes 108 us instead of 91; with four or eight it is even; in FP32
@@ -162,7 +162,8 @@ bool try_alloc(T** p, size_t count, cudaStream_t s) {
 }
 
 bool suits(const DeviceCRS& A) {
-  return A.owns && !A.lean && A.n > 0 && A.tpr == 2 && A.tile_rows > 0 && A.nnz >= kSellMinNnz;
+  return A.owns && !A.lean && A.n > 0 && A.tpr == 2 && A.tile_rows > 0 && A.nnz >= kSellMinNnz &&
+         A.nnz <= kSellMaxNnz;
 }
 long long most_elements(const DeviceCRS& A) { return A.nnz + A.nnz / 8; }
 long long shape_ctas(int n, int tile_rows) {

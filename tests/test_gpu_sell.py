@@ -8,7 +8,7 @@ import threading
 import numpy as np
 import pytest
 
-from graphitethree_gb300 import meshes, solver, systems
+from graphitethree_gb300 import _lib, meshes, solver, systems
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +92,17 @@ def test_products_and_solves_of_one_matrix_in_two_threads(gpu_ok):
             t.join()
         assert not bad
         M.close()
+
+
+@pytest.mark.parametrize("side,built", [(600, True), (1500, False)])     # 10 and 63 million nonzeros
+def test_solves_of_the_largest_matrices_keep_the_crs_kernels(gpu_ok, side, built):
+    """The layout costs two kernels; with other threads per row it is not built."""
+    V, F = meshes.height_field(side, side, 1)
+    M, b, _ = solver.build_lscm(V, F)
+    launches = []
+    for tpr in (4, 2):
+        M.set_layout(tpr, M.tile_rows)
+        before = _lib.load().nlgb_kernel_launches()
+        M.solve(b, max_iter=4)
+        launches.append(_lib.load().nlgb_kernel_launches() - before)
+    assert launches[1] - launches[0] == (2 if built else 0)
