@@ -79,15 +79,15 @@ struct Stage {
   }
 };
 
-// y = A x, `count` products at a time.  From the fifth product on a large
-// matrix is multiplied in its sliced layout (nlgb_sell.cu): laying it out
-// costs about as much as four products, a user of one or two never pays it.
-cudaError_t spmv_many(nlgb_matrix M, const double* x, double* y, int count) {
-  SellView sell{};
-  if ((M->spmvs += count) > 4) NLGB_CUDA_TRY(sell_prepare(M->A, &sell, M->stream));
-  for (int r = 0; r < count; ++r)
-    NLGB_CUDA_TRY(sell.va ? sell_spmv64(M->A, sell, x, y, M->stream) : spmv64(M->A, x, y, M->stream));
-  return cudaSuccess;
+// The layout for the next `count` products of a matrix.  From the fifth product
+// on a large matrix is multiplied in its sliced layout (nlgb_sell.cu): laying it
+// out costs about as much as four products, a user of one or two never pays it.
+cudaError_t product_layout(nlgb_matrix M, int count, SellView* view) {
+  *view = SellView{};
+  return (M->spmvs += count) > 4 ? sell_prepare(M->A, view, M->stream) : cudaSuccess;
+}
+cudaError_t product(nlgb_matrix M, const SellView& view, const double* x, double* y) {
+  return view.va ? sell_spmv64(M->A, view, x, y, M->stream) : spmv64(M->A, x, y, M->stream);
 }
 
 cudaError_t matrix_stream(nlgb_matrix M) {
@@ -212,7 +212,8 @@ int nlgb_spmv(nlgb_matrix A, const double* x, double* y) {
   Stage sx, sy;
   if (sx.in(x, A->A.m, s, true) != cudaSuccess || sy.in(y, A->A.n, s, false) != cudaSuccess)
     return NLGB_E_DEVICE;
-  if (spmv_many(A, sx.d, sy.d, 1) != cudaSuccess) return NLGB_E_DEVICE;
+  SellView view;
+  if (product_layout(A, 1, &view) != cudaSuccess || product(A, view, sx.d, sy.d) != cudaSuccess) return NLGB_E_DEVICE;
   if (sy.out(y, A->A.n, s) != cudaSuccess) return NLGB_E_DEVICE;
   if (cudaStreamSynchronize(s) != cudaSuccess) return fail(NLGB_E_DEVICE, cudaGetErrorString(cudaGetLastError()));
   return NLGB_OK;
@@ -229,9 +230,11 @@ int nlgb_spmv32(nlgb_matrix A, const float* x, float* y) {
 int nlgb_spmv_timed(nlgb_matrix A, const double* x, double* y, int reps, double* ms) {
   if (!A || reps <= 0) return fail(NLGB_E_INVALID, "nlgb_spmv_timed: bad arguments");
   cudaStream_t s = A->stream;
-  if (reps > 4 && spmv_many(A, x, y, 5) != cudaSuccess) return NLGB_E_DEVICE;   // (the layout outside the timing)
+  SellView view;
+  if (product_layout(A, reps, &view) != cudaSuccess) return NLGB_E_DEVICE;
   if (cudaEventRecord(A->e0, s) != cudaSuccess) return NLGB_E_DEVICE;
-  if (spmv_many(A, x, y, reps) != cudaSuccess) return NLGB_E_DEVICE;
+  for (int r = 0; r < reps; ++r)
+    if (product(A, view, x, y) != cudaSuccess) return NLGB_E_DEVICE;
   cudaEventRecord(A->e1, s);
   if (cudaEventSynchronize(A->e1) != cudaSuccess) return fail(NLGB_E_DEVICE, cudaGetErrorString(cudaGetLastError()));
   float t = 0.f;

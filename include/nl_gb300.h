@@ -115,7 +115,8 @@ int nlgb_spmv(nlgb_matrix A, const double* x, double* y);
 /* FP32 values/vectors; x, y device pointers. */
 int nlgb_spmv32(nlgb_matrix A, const float* x, float* y);
 /* Time `reps` back-to-back FP64 SpMVs on the library stream with CUDA
- * events (x, y device pointers); *ms = average per launch. */
+ * events (x, y device pointers); *ms = average per launch (what a matrix is
+ * laid out for once is not in it). */
 int nlgb_spmv_timed(nlgb_matrix A, const double* x, double* y, int reps, double* ms);
 int nlgb_spmv32_timed(nlgb_matrix A, const float* x, float* y, int reps, double* ms);
 

@@ -2,6 +2,7 @@
 the products and the phase-kernel iterates are those of the CRS kernels bit for
 bit -- short last tiles and passes, tiles that are not a multiple of a pass,
 rows without entries -- and matrices it does not suit keep the CRS kernels."""
+import ctypes
 import os
 import threading
 
@@ -9,6 +10,7 @@ import numpy as np
 import pytest
 
 from graphitethree_gb300 import _lib, meshes, solver, systems
+from graphitethree_gb300.nlvector import Vector
 
 pytestmark = pytest.mark.gpu
 
@@ -106,3 +108,19 @@ def test_solves_of_the_largest_matrices_keep_the_crs_kernels(gpu_ok, side, built
         M.solve(b, max_iter=4)
         launches.append(_lib.load().nlgb_kernel_launches() - before)
     assert launches[1] - launches[0] == (2 if built else 0)
+
+
+def test_timed_products_are_the_products_asked_for(gpu_ok):
+    """As many kernels as products, and what a layout costs is not in the time."""
+    L = _lib.load()
+    V, F = meshes.height_field(808, 808, 1)
+    M, _, _ = solver.build_lscm(V, F)
+    x, y, ms = Vector(np.ones(M.n)), Vector(M.n), ctypes.c_double()
+    times = []
+    for reps in (3, 3, 3):
+        assert L.nlgb_spmv_timed(M.handle, x.tensor.data_ptr(), y.tensor.data_ptr(), reps, ctypes.byref(ms)) == 0
+        times.append(ms.value)
+    assert max(times[1:]) < 1.5 * times[0]
+    before = L.nlgb_kernel_launches()
+    assert L.nlgb_spmv_timed(M.handle, x.tensor.data_ptr(), y.tensor.data_ptr(), 10, ctypes.byref(ms)) == 0
+    assert L.nlgb_kernel_launches() - before == 10
