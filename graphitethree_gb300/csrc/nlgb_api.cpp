@@ -79,12 +79,20 @@ struct Stage {
   }
 };
 
-// The layout for the next `count` products of a matrix.  From the fifth product
-// on a large matrix is multiplied in its sliced layout (nlgb_sell.cu): laying it
-// out costs about as much as four products, a user of one or two never pays it.
+// The sliced layout (nlgb_sell.cu) for the next `count` products of a matrix:
+// one that a solve has laid out, or, where a product gains enough, its own from
+// the 257th product on.  Laying out costs as much as it gives back in 40 to 95
+// products, so that whoever makes fewer never pays, and who makes a few more
+// loses about 2 %.  nlgb_spmv, LSCM matrices, CRS -> sliced, us, and what laying
+// out costs: 500 x 500 (7.0 M nonzeros) 36.4 -> 34.8, 215; 550 (8.5 M) 41.7 ->
+// 36.1, 250; 808 (18.3 M) 74.6 -> 64.6, 440; 1280 (45.8 M) 152.5 -> 141.6, 1,030;
+// 1350 (51.0 M) 161.4 -> 158.3, 960; 1600 (71.6 M) 208.6 -> 223.4, 1,310.
+constexpr long long kSellProducts = 256, kSellProductMinNnz = 1LL << 23, kSellProductMaxNnz = 48LL << 20;
 cudaError_t product_layout(nlgb_matrix M, int count, SellView* view) {
+  const long long products = (M->spmvs += count);
   *view = SellView{};
-  return (M->spmvs += count) > 4 ? sell_prepare(M->A, view, M->stream) : cudaSuccess;
+  if (M->A.nnz > kSellProductMaxNnz) return cudaSuccess;
+  return sell_prepare(M->A, view, M->stream, products > kSellProducts && M->A.nnz >= kSellProductMinNnz);
 }
 cudaError_t product(nlgb_matrix M, const SellView& view, const double* x, double* y) {
   return view.va ? sell_spmv64(M->A, view, x, y, M->stream) : spmv64(M->A, x, y, M->stream);

@@ -79,10 +79,10 @@ struct DeviceCRS {
 // 163.0, 1350 (51.0 M) 238.5 -> 235.2, 1400 (54.8 M) 249.5 -> 251.3, 1450 (58.8 M)
 // 266.6 -> 264.5, 1500 (63.0 M) 275.9 -> 282.3, 2000 (111.9 M) 471.6 -> 490.5.
 constexpr long long kSellMinNnz = 1LL << 21, kSellMaxNnz = 57LL << 20;
-// Builds the sliced layout; on return it is complete, for any stream.  *view
-// without values: the CRS kernels run (other threads per row, small or uneven
-// matrix, no memory for the copy).
-cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s);
+// Builds the sliced layout (build false: only looks whether there is one); on
+// return it is complete, for any stream.  *view without values: the CRS kernels
+// run (other threads per row, small or uneven matrix, no memory for the copy).
+cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s, bool build = true);
 // 16-bit columns relative to the row (complete, for any stream), where the
 // matrix is large and its columns lie within 32,767 of the diagonal; else *out
 // is null and the 32-bit ones serve.

@@ -183,7 +183,7 @@ void sell_free(SellLayout& L, cudaStream_t s, bool async) {
   L = SellLayout();
 }
 
-cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s) {
+cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s, bool build) {
   *view = SellView{};
   std::lock_guard<std::mutex> lk(*A.lazy);
   if (!suits(A)) return cudaSuccess;
@@ -194,6 +194,7 @@ cudaError_t sell_prepare(DeviceCRS& A, SellView* view, cudaStream_t s) {
     if (L.state > 0) hand_out();
     return cudaSuccess;
   }
+  if (!build) return cudaSuccess;
   L.state = -1;
   L.tpr = A.tpr;
   L.tile_rows = A.tile_rows;

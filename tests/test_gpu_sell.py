@@ -8,6 +8,7 @@ import threading
 
 import numpy as np
 import pytest
+import torch
 
 from graphitethree_gb300 import _lib, meshes, solver, systems
 from graphitethree_gb300.nlvector import Vector
@@ -124,3 +125,36 @@ def test_timed_products_are_the_products_asked_for(gpu_ok):
     before = L.nlgb_kernel_launches()
     assert L.nlgb_spmv_timed(M.handle, x.tensor.data_ptr(), y.tensor.data_ptr(), 10, ctypes.byref(ms)) == 0
     assert L.nlgb_kernel_launches() - before == 10
+
+
+def _launches_of_products(M, x, y, count):
+    L = _lib.load()
+    before = L.nlgb_kernel_launches()
+    for _ in range(count):
+        assert L.nlgb_spmv(M.handle, x.tensor.data_ptr(), y.tensor.data_ptr()) == 0
+    return L.nlgb_kernel_launches() - before
+
+
+# 2.8 M nonzeros: too few to gain; 9.4 M: laid out (two kernels) once that has paid; 63 M: too many
+@pytest.mark.parametrize("side,extra", [(320, 0), (580, 2), (1500, 0)])
+def test_products_are_laid_out_where_that_pays(gpu_ok, side, extra):
+    V, F = meshes.height_field(side, side, 1)
+    M, _, _ = solver.build_lscm(V, F)
+    x, y = Vector(np.random.default_rng(4).standard_normal(M.n)), Vector(M.n)
+    assert _launches_of_products(M, x, y, 256) == 256
+    first = y.tensor.clone()
+    assert _launches_of_products(M, x, y, 2) == 2 + extra
+    assert torch.equal(y.tensor, first)
+
+
+@pytest.mark.parametrize("tile", [1024, 576])
+def test_products_use_the_layout_of_a_solve(gpu_ok, tile):
+    V, F = meshes.height_field(331, 307, 5)
+    M, b, _ = solver.build_lscm(V, F)
+    M.set_layout(2, tile)
+    x = np.random.default_rng(1).standard_normal(M.n)
+    x[:3] = [np.inf, -np.inf, np.nan]          # reach only their own rows
+    y = M.spmv(x)
+    M.solve(b, max_iter=3)
+    for _ in range(2):
+        assert np.array_equal(M.spmv(x), y, equal_nan=True)
