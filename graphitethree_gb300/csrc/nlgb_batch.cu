@@ -33,7 +33,6 @@
 #include <cstring>
 #include <memory>
 #include <numeric>
-#include <thread>
 
 namespace nlgb {
 
@@ -781,7 +780,12 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
     cudaStream_t s = nullptr;
     int sys = -1, sms = 0;
     unsigned int seq0 = 0;
+    double t_due = 0.0;          // us (now_us)
+    long long iter0 = 0;
   };
+  using Clock = std::chrono::steady_clock;
+  const Clock::time_point t_begin = Clock::now();
+  auto now_us = [&]() { return std::chrono::duration<double, std::micro>(Clock::now() - t_begin).count(); };
   const int n = (int)systems.size(), n_sm = sm_count();
   std::vector<Lane> lanes((size_t)std::min(n, kPersistLanes));
   std::vector<std::unique_ptr<ViewGraph>> graphs;
@@ -826,6 +830,7 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
   }
   std::vector<int> waiting(order);     // longest first
   std::vector<char> fp64((size_t)n, 0);
+  std::vector<double> us_per_iter((size_t)n, 0.0);
   int left = n, sms_busy = 0;
   auto seq_of = [&](int i) { return __atomic_load_n(&mirrors[i].seq, __ATOMIC_ACQUIRE); };
   auto start = [&](Lane& l) {
@@ -833,6 +838,8 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
     const bool mixed = systems[i].mixed && !fp64[(size_t)i];
     *ran = true;
     mirrors[i].budget = kPersistBatchIters;
+    l.iter0 = mirrors[i].st.iter;
+    l.t_due = now_us() + chunk_due_us(mixed, kPersistBatchIters, us_per_iter[(size_t)i]);
     l.seq0 = seq_of(i);
     if (ok(graphs[(size_t)i]->prepare(systems[i].view, mixed, &mirrors[i], l.s))) ok(graphs[(size_t)i]->launch(l.s));
   };
@@ -847,6 +854,8 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
         idle = false;
         const int i = l.sys;
         const SysState& h = mirrors[i].st;
+        if (h.iter > l.iter0)
+          us_per_iter[(size_t)i] = (double)mirrors[i].t_ns * 1e-3 / (double)(h.iter - l.iter0);
         if (h.status == ST_STAGNATION && !h.fell_back && h.precision == 1) {
           // FP32 cannot track this system: it continues in FP64 from its x
           fp64[(size_t)i] = 1;
@@ -879,7 +888,12 @@ cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, f
         break;
       }
     }
-    if (idle) std::this_thread::yield();
+    if (idle) {
+      double due = 1e9;
+      for (const Lane& l : lanes)
+        if (l.sys >= 0) due = std::min(due, l.t_due);
+      poll_pause(due - now_us());
+    }
   }
   for (Lane& l : lanes) {
     if (!l.s) continue;

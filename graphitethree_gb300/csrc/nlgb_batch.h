@@ -2,7 +2,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <chrono>
 #include <memory>
+#include <thread>
 #include <vector>
 
 #include "nlgb_core.cuh"
@@ -192,6 +194,20 @@ class ViewGraph {
 // switched to FP64 PCG from its current x (stage 0, iteration count kept);
 // stream-ordered, before the system's next chunk.
 cudaError_t chunk_fallback_fp64(SysState* st, cudaStream_t s);
+
+// Between two polls of chunks on the persistent kernel: a sleep (of about 70 us)
+// while none of them is due, else the processor is only offered to others (a
+// chunk goes on in steps, and each would wait for the sleep to end).
+inline void poll_pause(double due_in_us) {
+  if (due_in_us > 150.0) std::this_thread::sleep_for(std::chrono::microseconds(20));
+  else std::this_thread::yield();
+}
+// When a chunk of `iters` iterations is due, us from its start; us_per_iter from
+// an earlier one (0: unknown).  A mixed one has a step at every reliable update,
+// so it is due at once; a system that converges ends before it is due.
+inline double chunk_due_us(bool mixed, long long iters, double us_per_iter) {
+  return mixed ? 0.0 : 0.9 * (double)iters * us_per_iter;
+}
 
 // Many systems on the persistent single-system kernel (nlgb_persist.cuh), each
 // by itself on a few SMs, as many at a time as the SMs allow.

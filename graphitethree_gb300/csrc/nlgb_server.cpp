@@ -1062,6 +1062,7 @@ void worker_streams(nlgb_server_s* S) {
     double t_free = -1.0;       // server clock when the lane's last chunk was seen done (tracing)
     long long ctas = 0;         // CTAs per phase kernel of the running system
     int sms = 0;                // SMs of a chunk on the persistent kernel (0: a graph)
+    double t_due = 0.0;         // server clock when that chunk is due
   };
   std::vector<Lane> lanes((size_t)ns);
   // CTA budget of the chunks in flight (config.chunk_cta_budget; 0: none)
@@ -1348,6 +1349,8 @@ void worker_streams(nlgb_server_s* S) {
       sms_busy += l.sms;
       graphs_busy += l.sms == 0 ? 1 : 0;
       best->graphs[bk]->persist(persist);
+      l.t_due = S->now() + 1e-6 * chunk_due_us(best->mixed_now[bk] != 0, iters,
+                                               std::max(0.0, best->ms_per_iter[bk]) * 1e3);
       // the budget is read by the chunk's first kernel
       __atomic_store_n(&m->budget, iters, __ATOMIC_RELEASE);
       const double tr = S->now();
@@ -1379,7 +1382,10 @@ void worker_streams(nlgb_server_s* S) {
       // threads' notifications are seen at the top of the loop); idle: sleep
       // until a request is admitted or the server stops
       if (sms_busy > 0) {
-        std::this_thread::yield();   // (a sleep takes 70 us, and a chunk goes on in steps)
+        double due = 1e9;
+        for (const Lane& l : lanes)
+          if (l.r && l.sms > 0) due = std::min(due, l.t_due);
+        poll_pause((due - S->now()) * 1e6);
       } else if (n_busy > 0) {
         std::this_thread::sleep_for(std::chrono::microseconds(20));
       } else {

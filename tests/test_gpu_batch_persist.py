@@ -5,6 +5,7 @@ used twice, mixed systems that continue in FP64, a layout changed between two
 batches, two threads with the same matrices, and both sides of the rule that
 chooses it -- the iterates of the single-system solver bit for bit."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -103,3 +104,19 @@ def test_threads_with_other_layouts_of_a_matrix(gpu_ok):
 @pytest.mark.parametrize("count", [1, 2, 3, 5, 9])
 def test_tiles_per_cta_follow_the_batch(gpu_ok, count):
     _check([_system("lscm", 60, 50 + k, k) for k in range(count)] + [_system("fairing", 150, 131)])
+
+
+@pytest.mark.parametrize("route", ["batch", "server"])
+def test_the_host_sleeps_while_a_long_chunk_runs(gpu_ok, route):
+    V, F = meshes.height_field(250, 240, 3)
+    M, b, _ = solver.build_lscm(V, F)
+    M.solve(b, max_iter=2)
+    srv = solver.Server(precision="double", epoch_ms=20.0)
+    wall, cpu = time.perf_counter(), time.process_time()
+    if route == "batch":
+        solver.batch_solve([M], [b])
+    else:
+        srv.wait(srv.submit_mesh("lscm", V, F))
+    wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
+    srv.close()
+    assert cpu < 0.5 * wall
