@@ -48,13 +48,14 @@ inline void persist_bind(PersistArgs& a, void* exch) {
 // with 2, 3, 4 and 6 tiles: 106, 80, 71, 66 ms; 6 requests of 1k to 4k: 8.4,
 // 8.5, 8.8, 10.4 ms.
 constexpr int kSharedTiles = 4;
-// SMs that the server's persistent chunks leave to the kernels of admissions
-// (an admission waits for a dozen of them one after the other, and a CTA of
-// k_persist has its SM's registers to itself), and that one system leaves: for a
-// cluster beside it as well.  Latency of a request of 1.6k vertices beside an
-// LSCM system of 157k unknowns, with all SMs taken -> so: 19.4 -> 2.0 ms.
-constexpr int kAdmissionSms = 7;
-constexpr int kSharedLeave = kAdmissionSms + kPersistCluster;
+// SMs that one system leaves free on a server: for a cluster beside it, and for
+// the kernels of admissions (an admission waits for a dozen of them one after
+// the other, and a CTA of k_persist has its SM's registers to itself).  Several
+// systems together may take all SMs: their chunks end at different times, and
+// with seven SMs always free two systems of 20k vertices no longer ran side by
+// side (24 requests of 1k to 20k vertices 65 -> 73 ms).  Latency of a request of 1.6k vertices beside an
+// LSCM system of 157k unknowns, with all SMs taken -> so: 19.4 -> 2.2 ms.
+constexpr int kSharedLeave = kPersistCluster + 7;
 // CTAs that own a system's tiles, with per_cta tiles on each or as many as
 // there have to be.  leave > 0: on all but so many SMs (where nine tiles per CTA
 // allow that), and the fewest CTAs with as many tiles on the busiest.

@@ -1089,7 +1089,7 @@ void worker_streams(nlgb_server_s* S) {
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, S->device);
   const double target_ms = S->cfg.epoch_ms > 0.0 ? S->cfg.epoch_ms : 10.0;
   auto sms_of = [](Req* r, int k) { return r->graphs[k]->persist_ctas(r->mixed_now[k] != 0); };
-  auto fits = [&](int sms) { return sms_busy == 0 || sms_busy + sms <= n_sm - kAdmissionSms; };
+  auto fits = [&](int sms) { return sms_busy == 0 || sms_busy + sms <= n_sm; };
   auto key_of = [](const Req* r, int k) { return r->est_left[k] < 0.0 ? -1.0 : r->est_left[k] * r->iter_cost; };
   // A system of many SMs seldom finds them free when a lane is: chunks of smaller
   // ones are launched on what is there, and would be as long as there are any.
@@ -1098,7 +1098,7 @@ void worker_streams(nlgb_server_s* S) {
   // meanwhile are worth half a chunk of it, or one that waited nine times as long
   // as it ran and 50 chunks.
   // Beside 6 streams of LSCM systems of 60 x 60 (660 a second) one of 200 x 200
-  // (alone 104 ms, 288 with graph chunks) was not run at all; it takes 240 ms.
+  // (alone 104 ms, 288 with graph chunks) was not run at all; it takes 207 ms.
   Req* wide = nullptr;
   int wide_k = -1;
   double idle = 0.0, t_idle = 0.0;   // SM ms
@@ -1112,7 +1112,7 @@ void worker_streams(nlgb_server_s* S) {
         if (r->waited_ms[k] + (t - r->t_ready[k]) > 9.0 * r->ran_ms[k] + 50.0 * target_ms) { wide = r; wide_k = k; }
         if (!least || key_of(r, k) < key_of(least, lk)) { least = r; lk = k; }
       }
-    idle = least ? idle + (double)std::max(0, n_sm - kAdmissionSms - sms_busy) * (t - t_idle) : 0.0;
+    idle = least ? idle + (double)std::max(0, n_sm - sms_busy) * (t - t_idle) : 0.0;
     t_idle = t;
     if (least && !wide && idle > 0.5 * target_ms * (double)sms_of(least, lk)) { wide = least; wide_k = lk; }
     if (wide) idle = 0.0;
