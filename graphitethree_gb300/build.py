@@ -22,7 +22,7 @@ LIB_DIR = PKG / "lib"
 LIB_NAME = "libnl_gb300.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-CU_SOURCES = ["nlgb_solver.cu", "nlgb_assembly.cu", "nlgb_blas.cu", "nlgb_batch.cu",
+CU_SOURCES = ["nlgb_solver.cu", "nlgb_assembly.cu", "nlgb_blas.cu", "nlgb_batch.cu", "nlgb_batch_mx.cu",
               "nlgb_noalloc.cu", "nlgb_persist.cu", "nlgb_persist_f64.cu",
               "nlgb_persist_df.cu", "nlgb_sell.cu", "nlgb_persist_mx.cu", "nlgb_build.cu", "nlgb_krylov.cu", "nlgb_ssor.cu"]
 CPP_SOURCES = ["nl_api.cpp", "nl_matrix_api.cpp", "nlgb_api.cpp", "nlgb_server.cpp"]

@@ -225,6 +225,9 @@ bool persist_batch_pays(const std::vector<SysView>& views);
 // system was begun (after an error before that, the batched kernel can run them).
 cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms, bool* ran);
 
+// The batched kernel for launches with mixed systems (nlgb_batch_mx.cu).
+const void* batch_kernel_mixed();
+
 // Launches the persistent kernel over a set of resident systems.  Each
 // system's SysState (device) must be initialised by the caller (status
 // ST_RUNNING, stage 0, thresholds, max_iter, precision); the state is read

@@ -273,10 +273,11 @@ __device__ __forceinline__ A row_dot(const int* __restrict__ rp, const CT* __res
   if (valid) {
     const int k0 = __ldg(rp + row), k1 = __ldg(rp + row + 1);
     const int origin = sizeof(CT) == 2 ? row : 0;   // 16-bit columns are relative to the row
-    if constexpr (sizeof(VT) == 4) {
+    if constexpr (sizeof(VT) == 4 && (!kCoh || T == 2)) {
       // three nonzeros in flight: FP32 rows are bound by latency (FP64 ones by
       // the FP64 pipe, where this costs: 176 -> 180 us per iteration at
-      // 4.2 M rows; FP32 122.5 -> 119.3)
+      // 4.2 M rows; FP32 122.5 -> 119.3).  In the batched kernel (kCoh) for two
+      // threads per row alone: for all six it spills 192 bytes a thread.
       for (int k = k0 + lane; k < k1; k += 3 * T) {
         int c[3];
         VT av[3];
