@@ -343,11 +343,28 @@ double persist_time(const SysView& v, int n_sm) {
 //   150 of 16..32      25.0 -> 11.1 (15.2)    0.44
 //   400 of 16..64      61.3 -> 50.7 (71.4)    0.53
 //   300 of 16..24      21.0 -> 20.6 (24.7)    1.09
+// And the batched kernel has to take longer than the host does here: at least
+// its longest system by itself, at 10 us per iteration and 4.3 for every tile
+// after the first, against 600 us and 35 for each system (87 for a mixed one,
+// whose reliable updates are steps of the host).  Iterations: 5.5 sqrt(n), of a
+// mixed system with two threads per row and more (normal equations, whose
+// condition is a square) 12 sqrt(n).  Whole call, ms:
+//   1 fairing of 8 x 8 vertices        0.62 -> 0.74, 16 x 16  1.54 -> 0.98
+//   5 fairing of 10 x 9                0.88 -> 1.08, 20 x 20  2.37 -> 1.44
+//   20 fairing of 10 x 10 mixed        1.63 -> 3.26, 20 x 20  3.89 -> 3.40
+//   60 LSCM of 12 x 12                 4.04 -> 5.04, 16 x 16  6.01 -> 5.08
+//   60 LSCM of 12 x 12 mixed           5.84 -> 8.24, 16 x 16  9.95 -> 8.15
 bool persist_batch_pays(const std::vector<SysView>& views) {
   const int n_sm = sm_count();
-  double longest = 0.0;
-  for (const SysView& v : views) longest = std::max(longest, persist_time(v, n_sm));
-  return (double)views.size() <= kPersistBatchRatio * longest;
+  double longest = 0.0, batched = 0.0, host = 600.0;
+  for (const SysView& v : views) {
+    longest = std::max(longest, persist_time(v, n_sm));
+    const double iteration = std::min(70.0, 10.0 + 4.3 * (double)(v.n_tiles - 1));
+    const bool mixed = v.r32 != nullptr;
+    batched = std::max(batched, (mixed && v.tpr >= 2 ? 12.0 : 5.5) * std::sqrt((double)v.n) * (v.df ? 0.78 : 1.0) * iteration);
+    host += mixed ? 87.0 : 35.0;
+  }
+  return (double)views.size() <= kPersistBatchRatio * longest && host <= batched;
 }
 
 cudaError_t persist_batch(std::vector<PersistSystem>& systems, cudaStream_t s, float* ms, bool* ran) {

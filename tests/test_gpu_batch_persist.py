@@ -10,7 +10,7 @@ import time
 import numpy as np
 import pytest
 
-from graphitethree_gb300 import meshes, solver
+from graphitethree_gb300 import _lib, meshes, solver
 
 pytestmark = pytest.mark.gpu
 
@@ -120,3 +120,16 @@ def test_the_host_sleeps_while_a_long_chunk_runs(gpu_ok, route):
     wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
     srv.close()
     assert cpu < 0.5 * wall
+
+
+# quick systems run in one launch of the batched kernel (a few launches in all), longer ones here
+@pytest.mark.parametrize("count,side,precision,here", [
+    (5, 4, "double", False), (5, 20, "double", True), (20, 10, "mixed", False), (20, 30, "mixed", True),
+    (60, 12, "df", False), (60, 30, "df", True)])
+def test_batches_of_quick_systems(gpu_ok, count, side, precision, here):
+    systems = [_system("fairing", side, side, k) for k in range(count)]
+    _check(systems, precision=precision)
+    before = _lib.load().nlgb_kernel_launches()
+    solver.batch_solve([M for M, _ in systems], [b for _, b in systems], precision=precision)
+    launches = _lib.load().nlgb_kernel_launches() - before
+    assert (launches >= 3 * count) == here
