@@ -250,6 +250,10 @@ class PcgSolver {
   PersistPlan plan_[3];
   void* exch_ = nullptr;
   bool refused_ = false;        // a launch of it failed
+  // plain graphs: one cooperative kernel per iteration where the tiles allow it
+  // (coop_now_: the FP64 or double-float graph in use has it)
+  bool use_coop_ = false, coop_now_ = false;
+  unsigned long long* coop_bar_ = nullptr;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   bool mixed_alloc_ = false;
   long long graph_launches_ = 0;

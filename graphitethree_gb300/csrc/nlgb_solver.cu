@@ -226,6 +226,107 @@ __global__ void __launch_bounds__(kCTA, 8) k_update_p(SysView s) {
   for (int t = vec_t0(s), t1 = vec_t1(s); t < t1; ++t) phase_update_p<D>(s, t, beta);
 }
 
+// ---------------------------------------------------------------------------
+// One whole FP64 or double-float PCG iteration in one cooperative kernel, for
+// systems of at most 640 tiles that the persistent kernel does not take (rows
+// of far-apart columns, matrices larger than L2, tiles above 512 rows): SpMV +
+// p.q, grid barrier, x / r update, grid barrier, p update; the kernel boundary orders the next
+// iteration's SpMV after this p update.  Every CTA reduces the tile partials
+// in the canonical order and applies the same scalar steps to its own copy
+// of the state (identical results), so the phases need no extra barrier for
+// the scalars; CTA 0 writes the state back.  The tile procedures, reductions
+// and scalar steps are those of the three-kernel iteration: the iterates are
+// bit-identical.  Replaces three kernel boundaries and three last-CTA
+// reduction tails per iteration by two barriers.  us per FP64 iteration, phase
+// kernels -> this: 81,920 rows of 26 scattered columns 40.4 -> 38.4, of 160
+// (152 MB) 104.7 -> 99.4; 150,000 of 80 88.3 -> 84.6; 8,536 LSCM rows in tiles of
+// 576 rows 26.8 -> 24.0.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long coop_atom_add(unsigned long long* p) {
+  unsigned long long old;
+  asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], 1;" : "=l"(old) : "l"(p) : "memory");
+  return old;
+}
+__device__ __forceinline__ unsigned long long coop_ld_acquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long coop_clock_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Grid barrier on a monotonic counter (one arrival per CTA per barrier):
+// returns false in every thread if the wait exceeded 4 s.
+__device__ bool coop_grid_sync(unsigned long long* bar, unsigned long long target) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ok = 1;
+    coop_atom_add(bar);
+    const unsigned long long t0 = coop_clock_ns();
+    unsigned int spins = 0;
+    while (coop_ld_acquire(bar) < target) {
+      if ((++spins & 63u) == 0u && coop_clock_ns() - t0 > 4000000000ULL) { ok = 0; break; }
+    }
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+template <int T, bool D>
+__global__ void __launch_bounds__(kCTA) k_iter(SysView s, unsigned long long* bar) {
+  __shared__ SysState sst;
+  if (threadIdx.x == 0) sst = *s.st;      // written by the previous kernel
+  __syncthreads();
+  if (sst.status != ST_RUNNING) return;
+  const int G = gridDim.x;
+  const unsigned long long base = (unsigned long long)sst.coop_epoch * 2ULL * (unsigned long long)G;
+  for (int t = blockIdx.x; t < s.n_tiles; t += G) {
+    const double v = phase_spmv_pq<D, T>(s, t);
+    if (threadIdx.x == 0) __stcg(s.part + (size_t)t * kParts + kSlotPQ, v);
+  }
+  bool ok = coop_grid_sync(bar, base + G);
+  if (ok) {
+    const int comp[1] = {kSlotPQ};
+    double o[1];
+    canon_reduce<1>(s.part, s.n_tiles, comp, o);
+    if (threadIdx.x == 0) scalar_after_pq(&sst, o[0]);
+    __syncthreads();
+    if (sst.status == ST_RUNNING) {
+      const double alpha = sst.alpha;
+      for (int t = blockIdx.x; t < s.n_tiles; t += G) {
+        double v[2];
+        phase_update_xr<D>(s, t, alpha, v);
+        if (threadIdx.x == 0) {
+          __stcg(s.part + (size_t)t * kParts + kSlotXR, v[0]);
+          __stcg(s.part + (size_t)t * kParts + kSlotXR + 1, v[1]);
+        }
+      }
+    }
+    // every CTA takes the second barrier (the epoch arithmetic counts both)
+    ok = coop_grid_sync(bar, base + 2ULL * G);
+    if (ok && sst.status == ST_RUNNING) {
+      const int comp2[2] = {kSlotXR, kSlotXR + 1};
+      double o2[2];
+      canon_reduce<2>(s.part, s.n_tiles, comp2, o2);
+      if (threadIdx.x == 0) scalar_after_xr(&sst, o2[0], o2[1]);
+      __syncthreads();
+      if (sst.status == ST_RUNNING) {
+        const double beta = sst.beta;
+        for (int t = blockIdx.x; t < s.n_tiles; t += G) phase_update_p<D>(s, t, beta);
+      }
+    }
+  }
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    if (!ok) sst.status = ST_DEVICE_ERR;
+    sst.coop_epoch += 1;
+    *s.st = sst;
+  }
+}
+
 // Termination guard of a while-node body (single thread).  use_handle == 0:
 // launched outside a graph (eager mode), the host reads the status instead.
 __global__ void k_guard(SysView s, cudaGraphConditionalHandle h, int need_mode, int use_handle) {
@@ -599,6 +700,49 @@ static long long resident_slots() {
   return 8LL * sms;
 }
 long long phase_resident_slots() { return resident_slots(); }
+
+// CTAs of the single-kernel iteration k_iter<T> resident at once (0 if the
+// occupancy cannot be queried).
+// Above ~640 CTAs the single-counter barrier and the per-CTA canonical
+// reductions (CTAs x tiles partial reads) cost more than the two kernel
+// boundaries they replace (measured on GB300: 512 CTAs 30 vs 38 us per
+// iteration, 834-1,024 CTAs 47-64 vs 39-50 us).
+constexpr long long kCoopMaxCtas = 640;
+
+template <bool D>
+static const void* iter_kernel(int tpr) {
+  switch (tpr) {
+    case 1: return (const void*)k_iter<1, D>;
+    case 2: return (const void*)k_iter<2, D>;
+    case 4: return (const void*)k_iter<4, D>;
+    case 8: return (const void*)k_iter<8, D>;
+    case 16: return (const void*)k_iter<16, D>;
+    default: return (const void*)k_iter<32, D>;
+  }
+}
+
+// Resident CTAs per SM of the single-kernel iteration: the smaller of its
+// FP64 and double-float forms (0 if it cannot be queried).
+static int coop_per_sm(int tpr) {
+  int a = 0, b = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, iter_kernel<false>(tpr), kCTA, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, iter_kernel<true>(tpr), kCTA, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return std::min(a, b);
+}
+
+static long long coop_wave(int tpr) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const int per_sm = coop_per_sm(tpr);
+  return std::min<long long>((long long)per_sm * sms, kCoopMaxCtas);
+}
 
 // Tiles of the smallest systems' layouts (128 and 256 rows): at most this
 // many, so that a system above 128 x this takes 256-row tiles.
@@ -1014,6 +1158,7 @@ cudaError_t PcgSolver::bind(DeviceCRS* A, cudaStream_t stream) {
   n_tiles_ = std::max(1, (n_ + tile_rows_ - 1) / tile_rows_);
   NLGB_CUDA_TRY(tables_.build(*A, tile_rows_, n_tiles_, stream));
   for (int m = 0; m < 3; ++m) plan_[m] = tables_.plan(tile_rows_, tpr_, m);
+  use_coop_ = n_tiles_ <= coop_wave(tpr_);
   return alloc(false);
 }
 
@@ -1024,7 +1169,7 @@ cudaError_t PcgSolver::alloc(bool mixed) {
   auto up = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
   if (!x_) {
     const size_t n8 = up((size_t)std::max(2, n_ + 2) * sizeof(double));
-    const size_t parts = up((size_t)n_tiles_ * kParts * sizeof(double)), st = up(sizeof(SysState));
+    const size_t parts = up((size_t)n_tiles_ * kParts * sizeof(double)), st = up(sizeof(SysState)) + 256;
     const size_t exch = tables_.usable() ? persist_bytes(n_, n_tiles_) : 0;
     char* p = nullptr;
     cudaError_t e = cudaMalloc(&p, 5 * n8 + parts + st + exch);
@@ -1041,6 +1186,7 @@ cudaError_t PcgSolver::alloc(bool mixed) {
     }
     part_ = reinterpret_cast<double*>(p);
     st_ = p + parts;
+    coop_bar_ = reinterpret_cast<unsigned long long*>(p + parts + st - 256);
     exch_ = p + parts + st;      // (used where a plan is usable)
     st_host_ = ::operator new(sizeof(SysState) + 16);
     NLGB_CUDA_TRY(cudaEventCreate(&ev0_));
@@ -1076,8 +1222,8 @@ static SysView make_view(DeviceCRS* A, int tile_rows, int n_tiles, double* b, do
 }
 
 // The while loop of the plain (FP64 or double-float) iteration, after
-// `dep`: kUnrollPlain iterations per pass (three phase kernels each), then
-// the guard.
+// `dep`: kUnrollPlain iterations per pass (one cooperative kernel each, or
+// three phase kernels), then the guard.
 cudaError_t PcgSolver::add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysView* v, bool df,
                                       cudaGraphNode_t* loop_out) {
   const KernelSet ks = kernels_for(tpr_, df);
@@ -1089,7 +1235,19 @@ cudaError_t PcgSolver::add_plain_loop(cudaGraph_t g, cudaGraphNode_t dep, SysVie
   cudaGraph_t body;
   NLGB_CUDA_TRY(add_while(g, loop_out, dep, h, &body));
   cudaGraphNode_t prev = nullptr;
+  unsigned long long* bar = coop_bar_;
+  void* a_it[] = {v, &bar};
   for (int u = 0; u < kUnrollPlain; ++u) {
+    if (coop_now_) {
+      cudaGraphNode_t n1;
+      NLGB_CUDA_TRY(add_kernel(body, &n1, prev, df ? iter_kernel<true>(tpr_) : iter_kernel<false>(tpr_), n_tiles_, kCTA, a_it));
+      cudaKernelNodeAttrValue coop;
+      std::memset(&coop, 0, sizeof(coop));
+      coop.cooperative = 1;
+      NLGB_CUDA_TRY(cudaGraphKernelNodeSetAttribute(n1, cudaKernelNodeAttributeCooperative, &coop));
+      prev = n1;
+      continue;
+    }
     cudaGraphNode_t n1, n2, n3;
     NLGB_CUDA_TRY(add_kernel(body, &n1, prev, spmv, n_tiles_, kCTA, a1));
     const int vg = (n_tiles_ + vec_tiles_for(tile_rows_) - 1) / vec_tiles_for(tile_rows_);
@@ -1640,7 +1798,7 @@ cudaError_t PcgSolver::run_cont(bool df, float* ms) {
   if (eager_mode()) return cudaSuccess;   // run_eager counted its launches
   ++graph_launches_;
   // resume p update, mark, final residual, check + every while-body pass
-  count_launches(4 + (h->guard - guard0) * (3 * kUnrollPlain + 1));
+  count_launches(4 + (h->guard - guard0) * ((coop_now_ ? 1 : 3) * kUnrollPlain + 1));
   return cudaSuccess;
 }
 
@@ -1726,7 +1884,21 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
     NLGB_CUDA_TRY(crs_prepare_c16(*A_, &ci16_, stream_));
     NLGB_CUDA_TRY(build_mixed_graph());
   }
-  if (!mixed && !persist && !eager_mode() && !*plain) NLGB_CUDA_TRY(build_plain_graph(df));
+  if (!mixed && !persist && !eager_mode()) {
+    coop_now_ = use_coop_ && (df || !sell_->va);
+    cudaError_t e = *plain ? cudaSuccess : build_plain_graph(df);
+    if (e != cudaSuccess && coop_now_) {   // cooperative kernel nodes refused here: one kernel per phase
+      cudaGetLastError();
+      use_coop_ = coop_now_ = false;
+      for (cudaGraphExec_t* g : {&plain_exec_, &df_exec_, &cont_exec_, &cont_df_exec_}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+      }
+      e = build_plain_graph(df);
+    }
+    NLGB_CUDA_TRY(e);
+    NLGB_CUDA_TRY(cudaMemsetAsync(coop_bar_, 0, sizeof(unsigned long long), stream_));   // coop_epoch = 0 too
+  }
   SysState* h = (SysState*)st_host_;
   std::memset(h, 0, sizeof(SysState));
   h->thresh2 = prm.eps * prm.eps;
@@ -1745,6 +1917,7 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
   // Hard cap on while-body passes: enough for max_iter iterations plus the
   // outer steps; reached only if the scalar logic failed to stop the loop.
   const int unroll = mixed ? kUnrollInner : kUnrollPlain;
+  const long long per_iter = !mixed && coop_now_ ? 1 : 3;
   h->guard_cap = std::max(0LL, max_iter - done) / unroll + 2LL * (h->max_outer + 2) + 4;
   NLGB_CUDA_TRY(cudaMemcpyAsync(st_, h, sizeof(SysState), cudaMemcpyHostToDevice, stream_));
   if (mixed) {
@@ -1766,11 +1939,11 @@ cudaError_t PcgSolver::run_graph(bool mixed, bool df, const SolveParams& prm, lo
   if (persist || eager_mode()) return cudaSuccess;   // counted their launches
   ++graph_launches_;
   // Kernel nodes executed: every while-body pass runs all of its kernels
-  // (3 per unrolled iteration + the guard); the mixed graph adds 2 kernels
+  // (1 or 3 per unrolled iteration + the guard); the mixed graph adds 2 kernels
   // per reliable update after the first; plus the first and final kernels
   // (and the true-residual check of the plain graph).
   const long long passes = h->guard;
-  long long k = (mixed ? 2 : 3) + passes * (3LL * unroll + 1);
+  long long k = (mixed ? 2 : 3) + passes * (per_iter * unroll + 1);
   if (mixed) k += 2LL * std::max(0, h->outer - outer - 1);
   count_launches(k);
   return cudaSuccess;

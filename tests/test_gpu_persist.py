@@ -9,7 +9,7 @@ import os
 import numpy as np
 import pytest
 
-from graphitethree_gb300 import meshes, solver, systems
+from graphitethree_gb300 import _lib, meshes, solver, systems
 
 pytestmark = pytest.mark.gpu
 
@@ -84,3 +84,16 @@ def test_no_iteration(gpu_ok, b):
     v = np.zeros_like(rhs) if b == "zero" else np.full_like(rhs, np.nan)
     x, i = M.solve(v)
     assert i.iterations == 0 and i.status == ("converged" if b == "zero" else "breakdown")
+
+
+@pytest.mark.parametrize("precision", ["double", "df"])
+@pytest.mark.parametrize("case", ["tiles_above_512_rows"])
+def test_one_kernel_per_iteration_where_the_persistent_one_does_not_fit(gpu_ok, case, precision):
+    M, b = _system("lscm", 70, 61)
+    M.set_layout(2, 576)
+    _both(M, b, precision, max_iter=40)
+    before = _lib.load().nlgb_kernel_launches()
+    info = M.solve(b, precision=precision, max_iter=40)[1]
+    assert info.iterations == 40
+    assert _lib.load().nlgb_kernel_launches() - before < 2 * info.iterations      # three phases: 3 and more
+    _both(M, b, precision, eps=1e-13, max_iter=1500)                              # continuations too
