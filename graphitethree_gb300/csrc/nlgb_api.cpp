@@ -327,8 +327,9 @@ bool batch_tables(int n_sys, const nlgb_matrix* A, const std::vector<SystemSlot>
   for (; per_cta < kSharedTiles; ++per_cta) {
     int used = 0;
     for (const SystemSlot& sl : slots) {
-      const int c = persist_ctas_for(sl.view.n_tiles, per_cta, sms);
-      used += sl.view.n_tiles > kPersistClusterTiles ? c + 1 : c > 9 ? sms / 8 : c;
+      const int tiles = sl.view.n_tiles;
+      const int c = persist_ctas(*sl.A, tiles, per_cta, sms);
+      used += c > kPersistCluster || tiles > kPersistClusterTiles ? c + 1 : c > 9 ? sms / 8 : c;
     }
     if (used <= sms) break;
   }

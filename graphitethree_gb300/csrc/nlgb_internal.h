@@ -174,9 +174,9 @@ class PersistTables {
   PersistTables(const PersistTables&) = delete;
   PersistTables& operator=(const PersistTables&) = delete;
   // Lays a matrix out for the persistent kernel; usable() tells whether it
-  // fits (sizes and halos).  per_cta: tiles on a CTA (more where the GPU has
-  // fewer SMs than that takes); leave: SMs to leave free (persist_ctas_for).
-  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta = 1, int leave = 0);
+  // fits (sizes and halos).  per_cta: tiles on a CTA, leave: SMs to leave free
+  // (persist_ctas).
+  cudaError_t build(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta, int leave = 0);
   // The same in two steps, for many matrices with one synchronisation: begin
   // queues the work and raises *most (device, zero before), end takes its value.
   cudaError_t begin(const DeviceCRS& A, int tile_rows, int n_tiles, cudaStream_t s, int per_cta, int* most,
@@ -193,6 +193,7 @@ class PersistTables {
   PersistLayout lay_;
   bool cluster_ = false;
   int ctas_ = 0;
+  long long nnz_ = 0;
   void* mem_ = nullptr;
   size_t bytes_ = 0;
 };

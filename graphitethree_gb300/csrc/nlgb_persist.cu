@@ -120,10 +120,18 @@ size_t smem_bytes(int slots, int R, int halo, size_t word) {
 
 }  // namespace
 
-int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave) {
-  const int most = n_tiles <= kPersistClusterTiles ? kPersistCluster : sms - 1;
-  const int ctas = std::min((n_tiles + per_cta - 1) / per_cta, most), fewer = sms - 1 - leave;
-  if (leave == 0 || ctas <= kPersistCluster || ctas <= fewer || fewer < 1) return ctas;
+int persist_ctas(const DeviceCRS& A, int n_tiles, int per_cta, int sms, int leave) {
+  const bool alone = per_cta == kPersistAlone, rows_long = A.tpr > 2 && A.nnz > kPersistCluster * kPersistCtaNnz;
+  int tiles = std::max(1, per_cta);
+  if (A.tpr > 2) tiles = (int)std::max(1LL, std::min<long long>(tiles, kPersistCtaNnz * n_tiles / std::max(1LL, A.nnz)));
+  return persist_ctas_for(n_tiles, tiles, sms, leave, alone || rows_long);
+}
+
+int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave, bool spread) {
+  const int want = (n_tiles + per_cta - 1) / per_cta;
+  if (n_tiles <= kPersistClusterTiles && (want <= kPersistCluster || !spread)) return std::min(want, kPersistCluster);
+  const int ctas = std::min(want, sms - 1), fewer = sms - 1 - leave;
+  if (leave == 0 || ctas <= fewer || fewer < 1) return ctas;
   const int slots = (n_tiles + fewer - 1) / fewer;
   return slots <= kPersistSlots ? (n_tiles + slots - 1) / slots : ctas;
 }
@@ -164,9 +172,10 @@ cudaError_t PersistTables::begin(const DeviceCRS& A, int tile_rows, int n_tiles,
   release();
   int sms = 0, smem_max = 0;
   if (A.n <= 0 || A.nnz <= 0 || A.n != A.m || tile_rows > 512 || !device_limits(&sms, &smem_max)) return cudaSuccess;
-  cluster_ = n_tiles <= kPersistClusterTiles;
-  const int ctas = persist_ctas_for(n_tiles, per_cta, sms, leave);
+  const int ctas = persist_ctas(A, n_tiles, per_cta, sms, leave);
   if (ctas < 1) return cudaSuccess;
+  cluster_ = ctas <= kPersistCluster && n_tiles <= kPersistClusterTiles;
+  nnz_ = A.nnz;
   const int slots = (n_tiles + ctas - 1) / ctas;
   const int cap = slots * tile_rows;
   if (slots > kPersistSlots || cap > 8192) return cudaSuccess;
@@ -222,8 +231,15 @@ void PersistTables::end(int most, cudaStream_t s) {
 
 PersistPlan PersistTables::plan(int tile_rows, int tpr, int mode) const {
   PersistPlan p;
-  int sms = 0, smem_max = 0;
-  if (!usable() || !device_limits(&sms, &smem_max)) return p;
+  int sms = 0, smem_max = 0, dev = 0, l2 = 0;
+  if (!usable() || !device_limits(&sms, &smem_max) || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+    return p;
+  // values and columns within L2: one CTA per SM cannot stream them from HBM (us
+  // per FP64 iteration, cooperative kernel -> this: 126 MB 92.9 -> 81.2, 142 MB
+  // 84.6 -> 91.5, 152 MB 99.4 -> 107.8, 208 MB 110.4 -> 130.2; mixed, graph ->
+  // this: 114 MB 72.7 -> 53.9, 139 MB 83.9 -> 109.9)
+  if (nnz_ * (mode == kPersistMixed ? 8 : 12) > (long long)l2) return p;
   // 256 threads where they hold every row in registers, else 512
   const int per_lane_rows = (lay_.slots * tile_rows * tpr + 255) / 256;
   p.cluster = cluster_;

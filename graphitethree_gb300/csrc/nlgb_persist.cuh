@@ -25,7 +25,7 @@
 //     has rows of 5 to 9: 7 FP64 instructions per row instead of 9);
 //   * block sums run in as few warp instructions as the tree has levels'
 //     adds, spread over the four schedulers.
-// Two forms.  Up to kPersistClusterTiles tiles: one thread-block cluster, partial
+// Two forms.  Systems that kPersistCluster CTAs hold: one thread-block cluster, partial
 // sums and z through distributed shared memory (a cluster barrier costs 378
 // cycles), every CTA taking the scalar steps itself.  Above: a cooperative
 // grid of one CTA per SM, one of which owns no rows, sums the partials and

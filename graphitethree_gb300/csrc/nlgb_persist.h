@@ -11,8 +11,21 @@ enum { kPersistDouble = 0, kPersistDf = 1, kPersistMixed = 2 };
 
 constexpr int kPersistBlock = 512;        // threads per CTA at most (128 registers each)
 constexpr int kPersistSlots = 9;          // tiles per CTA at most (1,216 tiles on 151 CTAs)
-constexpr int kPersistCluster = 16;       // CTAs of the cluster form at most
-constexpr int kPersistClusterTiles = 64;  // tiles of the cluster form at most
+// The cluster form: up to 16 CTAs.  Tiles that share a CTA cost more than the grid
+// form's exchanges, above all with long rows, which a CTA reads from L2.  So a
+// system that has the GPU to itself, or whose rows are long, takes the grid from 17
+// tiles on; one that shares the GPU from 65 on (4 charts of 60 to 128 vertices a
+// side at once 15.0 ms, with grids from 17 on 16.9).  us per FP64 iteration, 64 tiles on 16 CTAs ->
+// a grid of 63 and one: 8,000 rows of 6 nonzeros 10.5 -> 7.4, of 24 22.6 -> 11.2,
+// of 92 42.2 -> 16.5, of 356 105.9 -> 35.7 (one cooperative kernel per iteration
+// 17.1, 22.4, 32.5, 69.5); 16 tiles: 2,000 rows of 6 7.2 in either.
+constexpr int kPersistCluster = 16;
+constexpr int kPersistClusterTiles = 64;  // with four tiles on each
+// Nonzeros of a CTA's tiles where rows have more than two threads (of which one
+// row per lane group stays in registers): above, fewer tiles per CTA.  6,000 rows
+// of 46 nonzeros, 17,400 per CTA: 22.5 us per iteration (25.0 in the cooperative
+// kernel); 8,000 of 47, 23,500: 27.5 (24.9).
+constexpr long long kPersistCtaNnz = 16384;
 constexpr int kPersistRed = 8 * 36;       // 8-byte words of one staged value of a tile
 
 // How a launch left its system: running, at a reliable update, or stopped.
@@ -47,7 +60,7 @@ inline void persist_bind(PersistArgs& a, void* exch) {
 // system and fewer tiles finish one sooner.  24 requests of 1k to 20k vertices
 // with 2, 3, 4 and 6 tiles: 106, 80, 71, 66 ms; 6 requests of 1k to 4k: 8.4,
 // 8.5, 8.8, 10.4 ms.
-constexpr int kSharedTiles = 4;
+constexpr int kSharedTiles = 4, kPersistAlone = 0;
 // SMs that one system leaves free on a server: for a cluster beside it, and for
 // the kernels of admissions (an admission waits for a dozen of them one after
 // the other, and a CTA of k_persist has its SM's registers to itself).  Several
@@ -56,10 +69,14 @@ constexpr int kSharedTiles = 4;
 // side (24 requests of 1k to 20k vertices 65 -> 73 ms).  Latency of a request of 1.6k vertices beside an
 // LSCM system of 157k unknowns, with all SMs taken -> so: 19.4 -> 2.2 ms.
 constexpr int kSharedLeave = kPersistCluster + 7;
-// CTAs that own a system's tiles, with per_cta tiles on each or as many as
+// CTAs that own a system's tiles, with per_cta tiles on each (kPersistAlone: one,
+// the system has the GPU to itself), fewer where rows are long, or as many as
 // there have to be.  leave > 0: on all but so many SMs (where nine tiles per CTA
 // allow that), and the fewest CTAs with as many tiles on the busiest.
-int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave = 0);
+int persist_ctas(const DeviceCRS& A, int n_tiles, int per_cta, int sms, int leave = 0);
+// The same without a look at the rows; spread: a grid rather than more tiles than
+// per_cta on the CTAs of a cluster.
+int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave = 0, bool spread = false);
 // About the time of an iteration of a system that shares the GPU, us.
 double persist_iteration_us(int n_tiles, int ctas);
 // Launches the kernel.  Environment: NLGB_BARRIER_TIMEOUT_MS limits its waits

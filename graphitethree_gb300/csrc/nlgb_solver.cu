@@ -1156,7 +1156,7 @@ cudaError_t PcgSolver::bind(DeviceCRS* A, cudaStream_t stream) {
   tpr_ = A->tpr;
   tile_rows_ = A->tile_rows;
   n_tiles_ = std::max(1, (n_ + tile_rows_ - 1) / tile_rows_);
-  NLGB_CUDA_TRY(tables_.build(*A, tile_rows_, n_tiles_, stream));
+  NLGB_CUDA_TRY(tables_.build(*A, tile_rows_, n_tiles_, stream, kPersistAlone));
   for (int m = 0; m < 3; ++m) plan_[m] = tables_.plan(tile_rows_, tpr_, m);
   use_coop_ = n_tiles_ <= coop_wave(tpr_);
   return alloc(false);

@@ -86,11 +86,45 @@ def test_no_iteration(gpu_ok, b):
     assert i.iterations == 0 and i.status == ("converged" if b == "zero" else "breakdown")
 
 
+def _band(n, per_row, seed):
+    """Diagonally dominant, random columns within a band, about per_row nonzeros a row."""
+    rng = np.random.default_rng(seed)
+    m = n * (per_row - 1) // 2
+    i = rng.integers(0, n, m)
+    j = i + rng.integers(1, max(2, min(2500, n // 3)), m)
+    i, j = i[j < n], j[j < n]
+    w = rng.uniform(0.1, 1.0, i.shape[0])
+    d = np.full(n, 1e-3)
+    np.add.at(d, i, w)
+    np.add.at(d, j, w)
+    k = np.arange(n)
+    rp, ci, va = systems.csr_from_coo(n, np.concatenate([i, j, k]), np.concatenate([j, i, k]),
+                                      np.concatenate([-w, -w, d]))
+    return solver.Matrix(rp, ci, va), rng.standard_normal(n)
+
+
+@pytest.mark.parametrize("n,per_row", [(300, 60), (2048, 30), (2049, 30), (2177, 110), (8192, 200), (8193, 24),
+                                       (20000, 300)])
+def test_long_rows(gpu_ok, n, per_row):
+    """A cluster up to 16 tiles, a grid from 17 on; many nonzeros outside the registers."""
+    M, b = _band(n, per_row, n)
+    assert M.threads_per_row > 2
+    for precision in ("double", "mixed", "df"):
+        _both(M, b, precision, max_iter=60)
+    xs, infos, _ = solver.batch_solve([M, M], [b, 2.0 * b], max_iter=60)
+    for x, i, s in zip(xs, infos, (1.0, 2.0)):
+        y, j = M.solve(s * b, max_iter=60)
+        assert np.array_equal(x, y) and i.iterations == j.iterations
+
+
 @pytest.mark.parametrize("precision", ["double", "df"])
-@pytest.mark.parametrize("case", ["tiles_above_512_rows"])
+@pytest.mark.parametrize("case", ["tiles_above_512_rows", "larger_than_l2"])
 def test_one_kernel_per_iteration_where_the_persistent_one_does_not_fit(gpu_ok, case, precision):
-    M, b = _system("lscm", 70, 61)
-    M.set_layout(2, 576)
+    if case == "larger_than_l2":
+        M, b = _band(60_000, 230, 1)
+    else:
+        M, b = _system("lscm", 70, 61)
+        M.set_layout(2, 576)
     _both(M, b, precision, max_iter=40)
     before = _lib.load().nlgb_kernel_launches()
     info = M.solve(b, precision=precision, max_iter=40)[1]
