@@ -904,11 +904,15 @@ int nlgb_add_rows(long long n_rows, const long long* row_ptr, const int* var, co
     return NLGB_E_INVALID;
   }
   const int ks = c->nb_systems;
-  c->row_ptr.reserve(c->row_ptr.size() + n_rows);
-  c->col.reserve(c->col.size() + total);
-  c->val.reserve(c->val.size() + total);
-  c->rhs.reserve(c->rhs.size() + n_rows * ks);
-  c->weight.reserve(c->weight.size() + n_rows);
+  // (room for twice as much where there is too little: a caller may add row by row)
+  auto room = [](auto& v, long long more) {
+    if (more > 0 && v.size() + (size_t)more > v.capacity()) v.reserve(std::max(v.size() + (size_t)more, 2 * v.size()));
+  };
+  room(c->row_ptr, n_rows);
+  room(c->col, total);
+  room(c->val, total);
+  room(c->rhs, n_rows * ks);
+  room(c->weight, n_rows);
   // A short row without a variable twice goes to the stream as it is; runs of
   // them are appended at once (71,040 rows, 497,280 coefficients: 3.7 -> 1.95 ms).
   // (with at least a coefficient per variable: by the last row that named each)

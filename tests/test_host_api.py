@@ -170,3 +170,25 @@ def test_matrix_api_host_side(nllib):
     assert nl.nlNewSSORPreconditioner(M, 2.5) is None     # relaxation outside (0, 2)
     assert nl.nlMatrixFactorize(M, nl.NL_SUPERLU_EXT) is None
     nl.nlDeleteMatrix(M)
+
+
+def test_rows_one_by_one_are_taken_in_linear_time(nllib):
+    """nlgb_add_rows with a row per call: four times the rows take about four times as long."""
+    import time
+
+    def intake(n):
+        ctx = nl.nlNewContext()
+        nl.nlSolverParameteri(nl.NL_NB_VARIABLES, n)
+        nl.nlSolverParameteri(nl.NL_LEAST_SQUARES, nl.NL_TRUE)
+        nl.nlBegin(nl.NL_SYSTEM)
+        nl.nlBegin(nl.NL_MATRIX)
+        ptr, val, rhs = np.array([0, 8], np.int64), np.ones(8), np.zeros(1)
+        var = np.arange(8, dtype=np.int32)
+        t = time.perf_counter()
+        for _ in range(n):
+            assert nl.nlgbAddRows(ptr, var, val, rhs) == 0
+        t = time.perf_counter() - t
+        nl.nlDeleteContext(ctx)
+        return t
+    intake(1000)
+    assert min(intake(40_000) for _ in range(2)) < 8.0 * min(intake(10_000) for _ in range(2))
