@@ -175,6 +175,7 @@ _SIGS = {
     "nlgb_server_wait": (C.c_int, [C.c_void_p, C.c_longlong, C.POINTER(NlgbResult), f64p]),
     "nlgb_server_drain": (C.c_int, [C.c_void_p]),
     "nlgb_server_get_stats": (C.c_int, [C.c_void_p, C.POINTER(NlgbServerStats)]),
+    "nlgb_server_get_persist_stats": (C.c_int, [C.c_void_p, C.POINTER(C.c_longlong), f64p, f64p]),
     "nlgb_server_abort": (None, [C.c_void_p]),
     "nlgb_server_destroy": (None, [C.c_void_p]),
     "nlgb_add_rows": (C.c_int, [C.c_longlong, i64p, i32p, f64p, f64p, f64p]),

@@ -172,6 +172,9 @@ struct nlgb_server_s {
   size_t used = 0;
   // statistics (guarded by mu)
   nlgb_server_stats st{};
+  long long persist_chunks = 0;  // chunks on the persistent kernel, the time with
+  double persist_s = 0.0;        //   some in flight, and their algorithmic bytes
+  double persist_bytes = 0.0;
   std::vector<double> latencies;
   double first_arrival = -1.0, last_done = 0.0;
   double t_used = 0.0;           // server time of the last change of `used`
@@ -1138,12 +1141,15 @@ void worker_streams(nlgb_server_s* S) {
   long long w_loops = 0, w_launches = 0;
   int n_busy = 0;
   double t_busy0 = 0.0;
+  bool busy_persist = false;       // (chunks of the two kinds are not in flight together)
   auto busy_change = [&](int delta) {
     const double t = S->now();
     if (n_busy > 0 && delta != 0) {
       std::lock_guard<std::mutex> lk(S->mu);
       S->st.kernel_s += t - t_busy0;
+      if (busy_persist) S->persist_s += t - t_busy0;
     }
+    busy_persist = sms_busy > 0;
     t_busy0 = t;
     n_busy += delta;
     S->lanes_busy.store(n_busy);
@@ -1182,6 +1188,10 @@ void worker_streams(nlgb_server_s* S) {
       S->st.graph_s += ms * 1e-3;
       S->st.epoch_algo_bytes += double(di) * bytes_it;
       if (!mixed_chunk) S->st.graph_algo_bytes += double(di) * bytes_it;
+      if (l.sms > 0) {
+        S->persist_chunks += 1;
+        S->persist_bytes += double(di) * bytes_it;
+      }
     }
     if (S->trace)
       std::fprintf(S->trace, "C,%.6f,%lld,%d,%d,%lld,%lld,%.3f,%d,%d\n", S->now(), r->id, k, mixed_chunk ? 1 : 0,
@@ -1788,6 +1798,15 @@ int nlgb_server_get_stats(nlgb_server S, nlgb_server_stats* out) {
   st.wall_s = S->first_arrival >= 0 ? std::max(0.0, S->last_done - S->first_arrival) : 0.0;
   st.solves_per_s = st.wall_s > 0 ? double(st.completed) / st.wall_s : 0.0;
   *out = st;
+  return NLGB_OK;
+}
+
+int nlgb_server_get_persist_stats(nlgb_server S, long long* chunks, double* seconds, double* algo_bytes) {
+  if (!S) return NLGB_E_INVALID;
+  std::lock_guard<std::mutex> lk(S->mu);
+  if (chunks) *chunks = S->persist_chunks;
+  if (seconds) *seconds = S->persist_s;
+  if (algo_bytes) *algo_bytes = S->persist_bytes;
   return NLGB_OK;
 }
 

@@ -319,7 +319,12 @@ class Server:
     def stats(self) -> dict:
         st = _lib.NlgbServerStats()
         _check(_lib.load().nlgb_server_get_stats(self._h, ctypes.byref(st)), "stats")
-        return {f: getattr(st, f) for f, _ in st._fields_}
+        out = {f: getattr(st, f) for f, _ in st._fields_}
+        chunks, secs, nbytes = ctypes.c_longlong(), ctypes.c_double(), ctypes.c_double()
+        _check(_lib.load().nlgb_server_get_persist_stats(self._h, ctypes.byref(chunks), ctypes.byref(secs),
+                                                         ctypes.byref(nbytes)), "persist stats")
+        out.update(persist_chunks=chunks.value, persist_s=secs.value, persist_algo_bytes=nbytes.value)
+        return out
 
     def abort(self):
         _lib.load().nlgb_server_abort(self._h)

@@ -320,6 +320,11 @@ int         nlgb_server_wait(nlgb_server srv, long long ticket, nlgb_result* res
                              double* latency_s);
 int         nlgb_server_drain(nlgb_server srv);
 int         nlgb_server_get_stats(nlgb_server srv, nlgb_server_stats* st);
+/* The part of epochs, kernel_s and epoch_algo_bytes that ran as chunks on the
+ * persistent single-system kernel, which reads a matrix once per launch and
+ * not once per iteration (each may be NULL). */
+int         nlgb_server_get_persist_stats(nlgb_server srv, long long* chunks, double* seconds,
+                                          double* algo_bytes);
 /* Stop admitting and abort: queued requests fail at once, active systems
  * stop at the next epoch boundary (a solve running on a graph executor, e.g.
  * the SERIAL mode's, within one while-loop pass of 4 iterations) with

@@ -133,3 +133,15 @@ def test_a_wide_system_among_a_stream_of_small_ones(gpu_ok, streams):
         t.join()
     srv.close()
     assert in_time and np.array_equal(got[0][0][0], want)
+
+
+def test_chunks_on_the_persistent_kernel_are_counted_apart(gpu_ok):
+    small, large = systems.fairing_system(90, 80, seed=1, n_rhs=1), systems.fairing_system(1300, 1000, seed=3, n_rhs=1)
+    for sq, here in ((small, True), (large, False)):
+        srv = solver.Server(precision="double")
+        srv.wait(srv.submit_square(sq))
+        st = srv.stats()
+        srv.close()
+        part = (st["persist_chunks"], st["persist_algo_bytes"])
+        assert part == ((st["epochs"], st["epoch_algo_bytes"]) if here else (0, 0.0))
+        assert abs(st["persist_s"] - (st["kernel_s"] if here else 0.0)) < 1e-9
