@@ -170,7 +170,7 @@ class Matrix:
 
 def batch_solve(mats, bs, x0s=None, eps: float = 1e-10, max_iter: int = -1,
                 precision: str = "double", inner_eps: float = 0.1, max_outer: int = 100000):
-    """Solve many systems in one persistent-kernel launch.  mats: list of
+    """Solve many systems in one call (nlgb_batch_solve).  mats: list of
     Matrix (may repeat), bs: list of host vectors.  Returns (xs, infos,
     kernel_seconds)."""
     L = _lib.load()

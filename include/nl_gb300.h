@@ -134,7 +134,8 @@ int nlgb_solve(nlgb_matrix A, const double* b, double* x, const nlgb_params* prm
  * system converges (or stops) on its own; results are bit-identical to
  * nlgb_solve on the same system.  The systems run side by side on the
  * persistent single-system kernel, or in one launch of the batched kernel
- * when one of them is too large for it or there are very many small ones.
+ * when one of them is too large for it, there are very many small ones, or
+ * they end in about a millisecond.
  * *kernel_seconds: device time of the solves (CUDA events). */
 int nlgb_batch_solve(int n_sys, const nlgb_matrix* A, const double* const* b, double* const* x,
                      const nlgb_params* prm, nlgb_result* res, double* kernel_seconds);
