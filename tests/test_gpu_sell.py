@@ -158,3 +158,33 @@ def test_products_use_the_layout_of_a_solve(gpu_ok, tile):
     M.solve(b, max_iter=3)
     for _ in range(2):
         assert np.array_equal(M.spmv(x), y, equal_nan=True)
+
+
+@pytest.mark.parametrize("kind", ["short_and_empty", "one_row_of_500", "one_dense_row"])
+def test_rows_of_any_length_in_the_layout_of_a_solve(gpu_ok, kind):
+    """A solve lays the matrix out (two kernels) unless a lane would get more
+    than 255 nonzeros; the products that follow keep their bits."""
+    n = 170_000 + 77                            # a short last tile and pass
+    rng = np.random.default_rng(11)
+    lens = rng.integers(12, 19, n)
+    if kind == "short_and_empty":
+        lens[rng.random(n) < 0.02] = 0
+        lens[rng.random(n) < 0.02] = 1
+    else:
+        lens[n // 2] = 500 if kind == "one_row_of_500" else 700
+    rp = np.zeros(n + 1, np.int64)
+    rp[1:] = np.cumsum(lens)
+    i = np.repeat(np.arange(n), lens)
+    ci = (i + rng.integers(-300, 300, rp[-1])) % n
+    va = rng.standard_normal(rp[-1])
+    x = rng.standard_normal(n)
+    M = solver.Matrix(rp, ci, va)
+    M.set_layout(2, 1024)
+    y = M.spmv(x)
+    launches = []
+    for _ in range(2):
+        before = _lib.load().nlgb_kernel_launches()
+        M.solve(x, max_iter=1)
+        launches.append(_lib.load().nlgb_kernel_launches() - before)
+    assert np.array_equal(M.spmv(x), y)
+    assert launches[0] - launches[1] == (1 if kind == "one_dense_row" else 2)
