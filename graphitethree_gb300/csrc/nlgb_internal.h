@@ -70,6 +70,7 @@ struct DeviceCRS {
   // Held while a part above is built on demand: a product and a solve of one
   // matrix may ask for the same part from two threads.
   std::shared_ptr<std::mutex> lazy = std::make_shared<std::mutex>();
+  cudaEvent_t converted = nullptr;   // behind the kernels that fill va32, vadf and dinvdf
 };
 // Matrices below this have SpMVs of a few microseconds, bound by latency; above
 // the upper limit the vectors no longer stay in L2 (129 MB) between the kernels
@@ -103,7 +104,9 @@ void crs_free(DeviceCRS& A);
 // them must have completed.  The arrays of a DeviceCRS come from
 // cudaMallocAsync (the device's default pool).
 void crs_free_async(DeviceCRS& A, cudaStream_t s);
-cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s);  // jacobi, fp32, tuning
+// Jacobi, fp32, tuning.  Stream s comes after the kernels of the copies, whichever
+// stream builds them (a batch has one of its own).
+cudaError_t crs_prepare(DeviceCRS& A, bool need_fp32, cudaStream_t s);
 // crs_prepare plus the double-float copies; *usable is false (and no copy is
 // made) when a value or 1/diagonal lies outside [2^-100, 2^100] or is not
 // finite: the double-float iteration would lose its precision there, and

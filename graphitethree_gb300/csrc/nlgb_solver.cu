@@ -853,6 +853,7 @@ void crs_free(DeviceCRS& A) {
   cudaFree(A.dinv); cudaFree(A.dinv32);
   cudaFree(A.vadf); cudaFree(A.dinvdf); cudaFree(A.ci16);
   sell_free(A.sell, nullptr, false);
+  if (A.converted) cudaEventDestroy(A.converted);
   A = DeviceCRS();
 }
 
@@ -862,6 +863,7 @@ void crs_free_async(DeviceCRS& A, cudaStream_t s) {
                   (void*)A.vadf, (void*)A.dinvdf, (void*)A.ci16})
     if (p) cudaFreeAsync(p, s);
   sell_free(A.sell, s, true);
+  if (A.converted) cudaEventDestroy(A.converted);
   A = DeviceCRS();
 }
 
@@ -877,7 +879,13 @@ long long device_bytes(const DeviceCRS& A) {
   return b;
 }
 
+static cudaError_t mark_converted(DeviceCRS& A, cudaStream_t s) {
+  if (!A.converted) NLGB_CUDA_TRY(cudaEventCreateWithFlags(&A.converted, cudaEventDisableTiming));
+  return cudaEventRecord(A.converted, s);
+}
+
 static cudaError_t prepare_locked(DeviceCRS& A, bool need_fp32, cudaStream_t s) {
+  if (A.converted) NLGB_CUDA_TRY(cudaStreamWaitEvent(s, A.converted, 0));
   if (A.tpr == 0) {
     int hist[33];
     int mx = 0;
@@ -903,6 +911,7 @@ static cudaError_t prepare_locked(DeviceCRS& A, bool need_fp32, cudaStream_t s) 
       count_launches(1);
     }
     NLGB_CUDA_TRY(cudaGetLastError());
+    NLGB_CUDA_TRY(mark_converted(A, s));
   }
   return cudaSuccess;
 }
@@ -997,6 +1006,7 @@ cudaError_t crs_prepare_df(DeviceCRS& A, bool* usable, cudaStream_t s) {
       count_launches(1);
     }
     NLGB_CUDA_TRY(cudaGetLastError());
+    NLGB_CUDA_TRY(mark_converted(A, s));
   }
   *usable = A.df_state > 0;
   return cudaSuccess;

@@ -133,3 +133,30 @@ def test_batches_of_quick_systems(gpu_ok, count, side, precision, here):
     solver.batch_solve([M for M, _ in systems], [b for _, b in systems], precision=precision)
     launches = _lib.load().nlgb_kernel_launches() - before
     assert (launches >= 3 * count) == here
+
+
+@pytest.mark.parametrize("precision", ["mixed", "df"])
+def test_a_batch_and_a_solve_convert_one_matrix(gpu_ok, precision):
+    """Whichever comes first converts the values, on a stream of its own; the
+    other waits for them."""
+    V, F = meshes.height_field(331, 307, 6)
+    first, b, _ = solver.build_lscm(V, F)
+    want = first.solve(b, precision=precision, max_iter=8)[0]
+    for _ in range(10):
+        M, _, _ = solver.build_lscm(V, F)
+        start, got = threading.Barrier(2), {}
+
+        def batch():
+            start.wait()
+            got["batch"] = solver.batch_solve([M], [b], precision=precision, max_iter=8)[0][0]
+
+        def solve():
+            start.wait()
+            got["solve"] = M.solve(b, precision=precision, max_iter=8)[0]
+        threads = [threading.Thread(target=f) for f in (batch, solve)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert np.array_equal(got["batch"], want) and np.array_equal(got["solve"], want)
+        M.close()
