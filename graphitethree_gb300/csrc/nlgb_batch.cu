@@ -26,14 +26,6 @@ namespace nlgb {
 
 static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-namespace {
-
-// A batch on the persistent single-system kernel: systems at a time, iterations
-// of one launch, and the rule it is chosen by (persist_batch_pays).
-constexpr int kPersistLanes = 32;
-constexpr long long kPersistBatchIters = 1024;
-constexpr double kPersistBatchRatio = 0.5;
-
 // Small pinned allocations share a chunk of the driver's: to map the first one
 // and to give the last one back takes 0.3 ms.  64 bytes stay, so that a batch does
 // not pay that (a call with one small system 0.55 -> 0.24 ms).
@@ -46,6 +38,14 @@ void keep_pinned_chunk() {
   }();
   (void)kept;
 }
+
+namespace {
+
+// A batch on the persistent single-system kernel: systems at a time, iterations
+// of one launch, and the rule it is chosen by (persist_batch_pays).
+constexpr int kPersistLanes = 32;
+constexpr long long kPersistBatchIters = 1024;
+constexpr double kPersistBatchRatio = 0.5;
 
 __global__ void k_gather_states(const SysView* views, int n, SysState* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

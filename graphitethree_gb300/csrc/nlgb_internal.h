@@ -14,6 +14,8 @@ struct SysState;
 struct SysView;
 struct SellView;
 
+// Called before small pinned allocations that come and go.
+void keep_pinned_chunk();
 // Thread-local error text reported by nlGetErrorString()/nlgb_last_error().
 void set_error(const std::string& msg);
 const char* last_error();
@@ -254,6 +256,7 @@ class PcgSolver {
   PersistPlan plan_[3];
   void* exch_ = nullptr;
   bool refused_ = false;        // a launch of it failed
+  unsigned int* done_ = nullptr;   // pinned: how its last launch of a mixed solve ended
   // plain graphs: one cooperative kernel per iteration where the tiles allow it
   // (coop_now_: the FP64 or double-float graph in use has it)
   bool use_coop_ = false, coop_now_ = false;

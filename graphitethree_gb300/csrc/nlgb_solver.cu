@@ -1144,6 +1144,8 @@ void PcgSolver::release() {
   plain_exec_ = mixed_exec_ = df_exec_ = cont_exec_ = cont_df_exec_ = nullptr;
   cudaFree(mem_);
   cudaFree(mem32_);
+  if (done_) cudaFreeHost(done_);
+  done_ = nullptr;
   mem_ = mem32_ = exch_ = nullptr;
   *sell_ = SellView{};
   ci16_ = nullptr;
@@ -1845,12 +1847,38 @@ cudaError_t PcgSolver::run_persist(int mode, const SolveParams& prm) {
   void* ast[] = {&st};
   NLGB_CUDA_TRY(cudaMemsetAsync(exch_, 0, persist_bytes(n_, n_tiles_), stream_));   // coop_epoch = 0 too
   NLGB_CUDA_TRY(go(mixed ? ks.mx_outer : ks.init, n_tiles_, kCTA, a1));
-  // Mixed: a round per reliable update that is expected (one per inner_eps).
+  // Mixed: a round per reliable update that is expected (one per inner_eps), but
+  // no more than two ahead of the GPU, whose launches tell how they ended: a round
+  // of three kernels with nothing to do takes 12 us, so that a solve of few
+  // iterations took longer than its graph (fairing 33 x 33, no iterations 265 -> 142
+  // us, graph 135; three 288 -> 177, graph 204).
   int rounds = 1;
-  if (mixed && prm.eps > 0.0 && prm.eps < 1.0)
-    rounds = (int)std::max(1.0, std::min(16.0, std::ceil(std::log(prm.eps) / std::log(prm.inner_eps))));
+  unsigned int seq = 0;
+  if (mixed) {
+    keep_pinned_chunk();
+    if (!done_ && cudaMallocHost(&done_, sizeof(*done_)) != cudaSuccess) {
+      cudaGetLastError();
+      done_ = nullptr;
+    }
+    if (done_) __atomic_store_n(done_, 0u, __ATOMIC_RELEASE);
+    pa.done = done_;
+    if (prm.eps > 0.0 && prm.eps < 1.0)
+      rounds = (int)std::max(1.0, std::min(16.0, std::ceil(std::log(prm.eps) / std::log(prm.inner_eps))));
+  }
+  auto over = [&]() {
+    for (unsigned int polls = 1; pa.done; ++polls) {
+      const unsigned int v = __atomic_load_n(done_, __ATOMIC_ACQUIRE);
+      if ((v & 3u) == kPersistStopped) return true;
+      if ((v >> 2) + 2 > seq) break;
+      // (a launch whose reducing CTA did not come to its end tells nothing)
+      if ((polls & 1023u) == 0 && cudaStreamQuery(stream_) != cudaErrorNotReady) break;
+    }
+    return false;
+  };
   for (;;) {
     for (int k = 0; k < rounds; ++k) {
+      if (over()) break;
+      pa.done_value = ++seq << 2;
       const cudaError_t e = persist_launch(plan_[mode], pa, stream_);
       refused_ = e != cudaSuccess;
       if (refused_) return e;

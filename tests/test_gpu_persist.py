@@ -131,3 +131,20 @@ def test_one_kernel_per_iteration_where_the_persistent_one_does_not_fit(gpu_ok, 
     assert info.iterations == 40
     assert _lib.load().nlgb_kernel_launches() - before < 2 * info.iterations      # three phases: 3 and more
     _both(M, b, precision, eps=1e-13, max_iter=1500)                              # continuations too
+
+
+@pytest.mark.parametrize("side", [12, 110])      # a cluster, a grid
+def test_a_mixed_solve_that_ends_at_once_queues_few_kernels(gpu_ok, side):
+    """Ten reliable updates are expected at 1e-10, three kernels each; a solve
+    that is over before does not queue them all (the fewest of some calls: the
+    host sees the end when it comes)."""
+    M, b = _system("fairing", side, side)
+    x, info = M.solve(b, precision="mixed", eps=1e-12)
+    assert info.status == "converged"
+    launches = []
+    for _ in range(8):
+        before = _lib.load().nlgb_kernel_launches()
+        y, again = M.solve(b, x0=x, precision="mixed")
+        launches.append(_lib.load().nlgb_kernel_launches() - before)
+        assert again.status == "converged" and again.iterations == 0 and np.array_equal(x, y)
+    assert min(launches) < 20
