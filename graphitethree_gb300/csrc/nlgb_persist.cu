@@ -124,7 +124,8 @@ int persist_ctas(const DeviceCRS& A, int n_tiles, int per_cta, int sms, int leav
   const bool alone = per_cta == kPersistAlone, rows_long = A.tpr > 2 && A.nnz > kPersistCluster * kPersistCtaNnz;
   int tiles = std::max(1, per_cta);
   if (A.tpr > 2) tiles = (int)std::max(1LL, std::min<long long>(tiles, kPersistCtaNnz * n_tiles / std::max(1LL, A.nnz)));
-  return persist_ctas_for(n_tiles, tiles, sms, leave, alone || rows_long);
+  const bool spread = alone && (A.tpr > 2 || (A.tpr == 2 && n_tiles > 2 * kPersistCluster));
+  return persist_ctas_for(n_tiles, tiles, sms, leave, spread || rows_long);
 }
 
 int persist_ctas_for(int n_tiles, int per_cta, int sms, int leave, bool spread) {

@@ -11,14 +11,19 @@ enum { kPersistDouble = 0, kPersistDf = 1, kPersistMixed = 2 };
 
 constexpr int kPersistBlock = 512;        // threads per CTA at most (128 registers each)
 constexpr int kPersistSlots = 9;          // tiles per CTA at most (1,216 tiles on 151 CTAs)
-// The cluster form: up to 16 CTAs.  Tiles that share a CTA cost more than the grid
-// form's exchanges, above all with long rows, which a CTA reads from L2.  So a
-// system that has the GPU to itself, or whose rows are long, takes the grid from 17
-// tiles on; one that shares the GPU from 65 on (4 charts of 60 to 128 vertices a
-// side at once 15.0 ms, with grids from 17 on 16.9).  us per FP64 iteration, 64 tiles on 16 CTAs ->
-// a grid of 63 and one: 8,000 rows of 6 nonzeros 10.5 -> 7.4, of 24 22.6 -> 11.2,
-// of 92 42.2 -> 16.5, of 356 105.9 -> 35.7 (one cooperative kernel per iteration
-// 17.1, 22.4, 32.5, 69.5); 16 tiles: 2,000 rows of 6 7.2 in either.
+// The cluster form: up to 16 CTAs, whose exchanges cost less than the grid form's.
+// Tiles that share a CTA cost more the more nonzeros they have, above all with long
+// rows, which a CTA reads from L2.  So rows of more than two threads take the grid
+// from 17 tiles on (where the system has the GPU to itself, or they are long), rows
+// of two (LSCM) from 33 on where it has, others from 65 on.  Sharing the GPU: 4
+// charts of 60 to 128 vertices a side at once 15.0 ms, with grids from 17 on 16.9.
+// us per iteration, cluster -> grid (FP64; mixed):
+//   fairing  17 tiles 5.2 -> 6.2; 5.5 -> 6.8    32  5.6 -> 5.7; 5.8 -> 5.9
+//            48       6.3 -> 6.0; 6.0 -> 6.3    64  6.8 -> 6.3; 6.3 -> 6.3
+//   LSCM     17       5.9 -> 6.5; 4.7 -> 5.9    32  6.3 -> 6.1; 5.0 -> 5.7
+//            33       6.8 -> 6.2; 5.2 -> 5.4    64  8.1 -> 6.2; 5.8 -> 5.6
+//   64 tiles of rows of 24 nonzeros 22.6 -> 11.2, of 92 42.2 -> 16.5, of 356 105.9 ->
+//   35.7 (one cooperative kernel per iteration 22.4, 32.5, 69.5)
 constexpr int kPersistCluster = 16;
 constexpr int kPersistClusterTiles = 64;  // with four tiles on each
 // Nonzeros of a CTA's tiles where rows have more than two threads (of which one

@@ -148,3 +148,11 @@ def test_a_mixed_solve_that_ends_at_once_queues_few_kernels(gpu_ok, side):
         launches.append(_lib.load().nlgb_kernel_launches() - before)
         assert again.status == "converged" and again.iterations == 0 and np.array_equal(x, y)
     assert min(launches) < 20
+
+
+@pytest.mark.parametrize("kind,nx,ny", [("fairing", 47, 46), ("fairing", 90, 91), ("lscm", 46, 44), ("lscm", 46, 46)])
+def test_cluster_and_grid_by_threads_per_row(gpu_ok, kind, nx, ny):
+    """17 and 64 tiles of one thread per row: a cluster; 32 and 34 of two: both sides."""
+    M, b = _system(kind, nx, ny)
+    for precision in ("double", "mixed", "df"):
+        _both(M, b, precision, max_iter=60)
